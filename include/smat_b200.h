@@ -87,7 +87,7 @@ int smat_spmm_bcsr_f16_static(const void* bcsrValuesA, const int* bcsrRowPtrA, c
  * No counterpart in the reference (its kernel re-reads bcsrColIdx per tile, mmaCBT.cu:38-43). */
 typedef struct smat_plan smat_plan;
 /* N_hint: the number of columns of B the plan will mostly be used with (0 = unknown).  It only steers
- * how many block-rows form a work item (8 to 24) and which of the two kernels multiplies, so that small matrices or
+ * how many block-rows form a work item (8 to 24) and which of the kernels multiplies, so that small matrices or
  * shards still fill the SMs.
  * A plan also owns scratch for work items that a launch computes in segments (38.8 MB on a 148-SM device, twice
  * that for matrices whose work is very unevenly spread over the block-rows) and may be used by one stream at a
@@ -111,7 +111,8 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
 int smat_plan_destroy(smat_plan* plan);
 /* What a plan turned out to be (informational, no reference counterpart): *rows_per_item = block-rows of a work item
  * (8..16: the kernel that reads both operands from shared memory; 16..24 with *tall = 1: the kernel that reads the
- * B panels from tensor memory), *steps = steps of the walk order.  Any pointer may be NULL. */
+ * B panels from tensor memory; 1: the kernel that walks single block-rows), *steps = steps of the walk order (pieces of
+ * block-rows for the last kernel).  Any pointer may be NULL. */
 int smat_plan_info(const smat_plan* plan, int* tall, int* rows_per_item, size_t* steps);
 
 /* Kernel variant used by every multiplication of this process: 0 = chosen per matrix (default),
@@ -119,7 +120,9 @@ int smat_plan_info(const smat_plan* plan, int* tall, int* rows_per_item, size_t*
  * 2 = B panels copied to tensor memory and read from there (one accumulator buffer),
  * 3 = work items 256 columns of C wide: two MMAs per block, one accumulator buffer (default for N >= 256),
  * 4 = plans created from now on use work items of up to 24 block-rows and the kernel that reads the B panels
- *     from tensor memory (affects smat_plan_create, not plans that exist).
+ *     from tensor memory (affects smat_plan_create, not plans that exist),
+ * 5 = plans created from now on, and products without a plan, use the kernel that walks single block-rows with
+ *     warp-level MMAs (chosen by itself for narrow C, scattered blocks and small products).
  * Meant for benchmarks and tests; no counterpart in the reference. */
 int smat_spmm_set_variant(int variant);
 

@@ -69,13 +69,25 @@ def launch_count():
 
 
 def set_variant(v):
-    """0 = automatic, 1 = shared-memory-operand kernel, 2 = tensor-memory-operand kernel."""
+    """0 = automatic, 1 = shared-memory-operand kernel, 2 = tensor-memory-operand kernel, 3 = 256-column items, 4 = tall plans,
+    5 = stream kernel (see smat_spmm_set_variant)."""
     _check(lib().smat_spmm_set_variant(int(v)))
 
 
 def _stream():
+    """The current CUDA stream of the current device as an integer.  The raw lookup takes 0.1 us, the Stream object that
+    torch.cuda.current_stream() makes 3.2 us: as much as a small product."""
+    global _stream
     import torch
-    return torch.cuda.current_stream().cuda_stream
+    torch.cuda.current_stream()  # initialises CUDA
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is not None and device is not None:
+        def _stream():
+            return raw(device())
+    else:
+        def _stream():
+            return torch.cuda.current_stream().cuda_stream
+    return _stream()
 
 
 # ------------------------------------------------------------------------------------------------
@@ -454,10 +466,12 @@ def spmm(A, B, Cout, check=False):
     B: Matrix / tensor [N, K]; Cout: Matrix / tensor [M, N]."""
     Bt = B.data if isinstance(B, Matrix) else B
     Ct = Cout.data if isinstance(Cout, Matrix) else Cout
-    N = Bt.shape[0]
-    assert Bt.shape[1] == A.K and tuple(Ct.shape) == (A.M, N) and Bt.is_contiguous() and Ct.is_contiguous()
-    _check(lib().smat_spmm_bcsr_f16(A.getBcsrValues(), A.getBcsrRowPtr(), A.getBcsrColIdx(), Bt.data_ptr(),
-                                    Ct.data_ptr(), A.M, N, A.K, A.nnzb, None, None, _stream()))
+    N, K = Bt.shape
+    assert K == A.K and Ct.shape == (A.M, N) and Bt.is_contiguous() and Ct.is_contiguous()
+    rc = lib().smat_spmm_bcsr_f16(A.bcsrVal.data_ptr(), A.bcsrRowPtr.data_ptr(), A.bcsrColIdx.data_ptr(), Bt.data_ptr(),
+                                  Ct.data_ptr(), A.M, N, K, A.nnzb, None, None, _stream())
+    if rc:
+        _check(rc)
     if check:
         _check(lib().smat_device_status(_stream()))
 
@@ -485,6 +499,7 @@ class Plan:
         _check(lib().smat_plan_create(C.byref(h), A.getBcsrValues(), A.getBcsrRowPtr(), A.getBcsrColIdx(), A.M, A.K,
                                       A.nnzb, self.brow_begin, self.brow_end, int(n_hint), _stream()))
         self._h = h
+        self._spmm = lib().smat_plan_spmm
 
     def set_values(self):
         """Re-reads A's value array after it changed (same structure)."""
@@ -495,15 +510,17 @@ class Plan:
         t, r, n = C.c_int(0), C.c_int(0), C.c_size_t(0)
         _check(lib().smat_plan_info(self._h, C.addressof(t), C.addressof(r), C.addressof(n)))
         return {"tall": bool(t.value), "rows_per_item": r.value, "steps": n.value,
-                "kernel": "spmm_bcsr_tall_kernel" if t.value else "spmm_bcsr_tc_kernel"}
+                "kernel": "spmm_bcsr_tall_kernel" if t.value else "spmm_bcsr_stream_kernel" if r.value == 1 else "spmm_bcsr_tc_kernel"}
 
     def spmm(self, B, Cout, check=False):
         Bt = B.data if isinstance(B, Matrix) else B
         Ct = Cout.data if isinstance(Cout, Matrix) else Cout
-        N = Bt.shape[0]
-        assert Bt.shape[1] == self.A.K and tuple(Ct.shape) == ((self.brow_end - self.brow_begin) * 16, N)
+        N, K = Bt.shape
+        assert K == self.A.K and Ct.shape == ((self.brow_end - self.brow_begin) * 16, N)
         assert Bt.is_contiguous() and Ct.is_contiguous()
-        _check(lib().smat_plan_spmm(self._h, Bt.data_ptr(), Ct.data_ptr(), N, _stream()))
+        rc = self._spmm(self._h, Bt.data_ptr(), Ct.data_ptr(), N, _stream())
+        if rc:
+            _check(rc)
         if check:
             _check(lib().smat_device_status(_stream()))
 

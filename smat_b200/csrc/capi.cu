@@ -9,6 +9,7 @@
 
 #include "smat_internal.h"
 #include "spmm_sched.cuh"
+#include "spmm_stream.h"
 
 namespace smat {
 
@@ -150,6 +151,16 @@ static int spmm_transient_plan(const void* vals, const int* rowptr, const int* c
     v.brow_end = brow_end;
     DeviceCtx* ctx = nullptr;
     if (int rc0 = get_device_ctx(&ctx)) return rc0;
+    if (nnzb && stream_for_call(N, brow_end - brow_begin, nnzb, K, ctx->sm_count)) {
+        const StreamShape shape = stream_shape(N, brow_end - brow_begin, nnzb, K, ctx->sm_count, false);
+        const size_t bytes = stream_call_bytes(shape, N, brow_end - brow_begin, nnzb, K);
+        void* scratch = nullptr;
+        if (bytes) SMAT_CUDA_TRY(cudaMallocFromPoolAsync(&scratch, bytes, ctx->pool, stream));
+        int rc = stream_call(shape, vals, rowptr, colidx, B, C, N, K, nnzb, brow_begin, brow_end, scratch, ctx, stream);
+        const cudaError_t e = bytes ? cudaFreeAsync(scratch, stream) : cudaSuccess;
+        if (rc == SMAT_OK && e != cudaSuccess) return fail(SMAT_ERR_CUDA, "cudaFreeAsync failed: %s", cudaGetErrorString(e));
+        return rc;
+    }
     const size_t rg = choose_rows_per_group(brow_end - brow_begin, N, ctx->sm_count, true, nnzb, K);
     const PlanSizes sz = plan_sizes(nnzb, brow_begin, brow_end, rg);
     v.n_groups = sz.n_groups;
@@ -197,7 +208,7 @@ int smat_spmm_bcsr_f16_rows(const void* vals, const int* rowptr, const int* coli
 
 int smat_spmm_set_variant(int variant) {
     clear_error();
-    if (variant < 0 || variant > 4) return fail(SMAT_ERR_BAD_ARG, "unknown SpMM variant %d", variant);
+    if (variant < 0 || variant > 5) return fail(SMAT_ERR_BAD_ARG, "unknown SpMM variant %d", variant);
     g_spmm_variant = variant;
     return SMAT_OK;
 }

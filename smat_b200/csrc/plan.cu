@@ -26,6 +26,7 @@
 #include <algorithm>
 
 #include "smat_internal.h"
+#include "spmm_stream.h"
 
 namespace smat {
 namespace {
@@ -619,6 +620,7 @@ struct smat_plan {
     void* buffer = nullptr;
     void* gsp_buffer = nullptr;
     void* fix_buffer = nullptr;  // partial tiles of cut work items
+    StreamPlan stream;           // buffers of a stream plan
     void* sched_buffer = nullptr;  // listed schedule: offsets per CTA, then the groups
     int device = -1;
     // smat_plan_spmm_host: device staging (B and C whole), the copy streams, per-chunk and per-range events
@@ -756,6 +758,7 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     // already).  Both plans are counted and the estimates compared; smat_spmm_set_variant(4) forces a tall plan,
     // 1..3 exclude it.
     bool tall = false;
+    double est_cycles = 0.0;  // of the tcgen05 kernel that would be taken
     size_t rg_used = rg;
     const size_t rows = brow_end - brow_begin, tiles = ((N_hint ? N_hint : 128) + 127) / 128;
     const bool tall_forced = g_spmm_variant == 4;
@@ -808,6 +811,7 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
             const double est_tall =
                 rounds_for(sz_tall.n_groups * tiles, (size_t)ctx->sm_count, true, (size_t)steps_per_tall, false) * steps_per_tall * 550.0;
             tall = tall_forced || est_tall < 0.97 * est16;
+            est_cycles = tall ? est_tall : est16;
             if (std::getenv("SMAT_PLAN_DEBUG"))
                 fprintf(stderr, "[smat plan] estimates: 16-row %.0f cycles, tall (rg %zu, %d steps) %.0f cycles -> %s\n", est16, rg_tall,
                         tall_total_and_max[0], est_tall, tall ? "tall" : "16-row");
@@ -823,6 +827,46 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
             cap = kTallBlocksPerStep;
         } else {
             cudaFree(gsp_tall);
+        }
+    }
+    // Stream plan (spmm_stream_sm100.cu): taken where its estimate is below that of the kernel chosen so far.
+    if (rc == SMAT_OK && total_steps > 0 && (g_spmm_variant == 5 || (g_spmm_variant == 0 && N_hint > 0))) {
+        const double us = stream_estimate_us(N_hint ? N_hint : 128, rows, range_blocks, K, ctx->sm_count);
+        if (est_cycles == 0.0) {
+            const double per_group = (double)total_steps / (double)sz.n_groups, per_step = (double)range_blocks / (double)total_steps;
+            const double rounds = balanced || p->v.sched_list ? (double)(sz.n_groups * tiles) / (double)ctx->sm_count
+                                                              : rounds_for(sz.n_groups * tiles, (size_t)ctx->sm_count, true, (size_t)per_group, false);
+            est_cycles = rounds * per_group * (per_step * 45.0 > 470.0 ? per_step * 45.0 : 470.0);
+        }
+        const double other = 8.0 + est_cycles / 1850.0;
+        const bool take = g_spmm_variant == 5 || us < other;
+        if (std::getenv("SMAT_PLAN_DEBUG")) fprintf(stderr, "[smat plan] stream %.1f us, %s %.1f us\n", us, tall ? "tall" : "16-row", other);
+        if (take) {
+            std::vector<int> h_rowptr(rows + 1);
+            e = cudaMemcpyAsync(h_rowptr.data(), bcsrRowPtrA + brow_begin, (rows + 1) * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
+            if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
+            if (rc == SMAT_OK && std::is_sorted(h_rowptr.begin(), h_rowptr.end())) {
+                p->v.K = K;
+                p->v.nnzb = range_blocks;
+                p->v.brow_begin = brow_begin;
+                p->v.brow_end = brow_end;
+                rc = stream_plan_build(p->stream, p->v, h_rowptr.data(), bcsrValuesA, bcsrColIdxA, N_hint ? N_hint : 128, ctx->sm_count,
+                                       (cudaStream_t)stream);
+                cudaFree(p->gsp_buffer);
+                cudaFree(p->fix_buffer);
+                cudaFree(p->sched_buffer);
+                p->gsp_buffer = p->fix_buffer = p->sched_buffer = nullptr;
+                p->v.sched_list = p->v.sched_off = nullptr;
+                p->v.total_steps = p->stream.row_piece.empty() ? 0 : (size_t)p->stream.row_piece.back();
+                if (rc) {
+                    cudaFree(p->stream.buffer);
+                    delete p;
+                    return rc;
+                }
+                *out = p;
+                return SMAT_OK;
+            }
         }
     }
     const int steps_final = total_and_max[0];
@@ -898,6 +942,11 @@ int smat_plan_set_values(smat_plan* plan, const void* bcsrValuesA, void* stream)
     if (!plan || (plan->v.nnzb && !bcsrValuesA)) return fail(SMAT_ERR_BAD_ARG, "NULL argument");
     if ((uintptr_t)bcsrValuesA & 15) return fail(SMAT_ERR_BAD_ARG, "bcsrValuesA must be 16-byte aligned");
     if (int rc = check_plan_device(plan)) return rc;
+    if (plan->v.stream) {
+        DeviceCtx* ctx = nullptr;
+        if (int rc = get_device_ctx(&ctx)) return rc;
+        return stream_plan_values(plan->v, bcsrValuesA, nullptr, ctx->sm_count, (cudaStream_t)stream);
+    }
     if (plan->v.tall)
         return pack_values_tall_async(plan->v.rowptr, bcsrValuesA, plan->v.gsp, plan->v.steps, plan->v.blk,
                                       const_cast<void*>(plan->v.packed), plan->v.brow_begin, plan->v.brow_end, plan->v.rg,
@@ -941,6 +990,7 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
     DeviceCtx* ctx = nullptr;
     if (int rc0 = get_device_ctx(&ctx)) return rc0;
     size_t n_ranges = (n_groups * ((W + 127) / 128) + (size_t)ctx->sm_count / 2) / (size_t)ctx->sm_count;
+    if (plan->v.stream) n_ranges = n_groups / 16 * ((W + 127) / 128) / (size_t)ctx->sm_count;
     if (plan->v.sched_list || plan->v.balanced) n_ranges = 1;  // such plans balance a launch over all their groups
     if (const char* e = std::getenv("SMAT_HOST_RANGES")) n_ranges = (size_t)std::atoi(e);  // tuning knob
     if (n_ranges > 4) n_ranges = 4;
@@ -1041,6 +1091,7 @@ int smat_plan_destroy(smat_plan* plan) {
     const cudaError_t e2 = cudaFree(plan->gsp_buffer);
     const cudaError_t e3 = cudaFree(plan->fix_buffer);
     cudaFree(plan->sched_buffer);
+    cudaFree(plan->stream.buffer);
     if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess) e = e3;
     delete plan;

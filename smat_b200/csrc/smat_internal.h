@@ -141,6 +141,9 @@ struct PlanView {
     // Scratch for work items that are computed in segments by several CTAs (null: items are never cut):
     // fix_scratch_bytes(SMs) bytes, used by one launch at a time.
     float* fix_scratch = nullptr;
+    // Stream plan (spmm_stream_sm100.cu): everything its kernel needs; n_groups counts block-rows, rg is 1, the fields of
+    // the other kernels are null.
+    const struct StreamPlan* stream = nullptr;
 };
 
 // Work-list sizes for a block-row range and the asynchronous build on `stream` (plan.cu).
@@ -187,7 +190,7 @@ int launch_sum_cut_items(bool wide, int cut_items, const float* scratch, void* C
                          int n_tiles, int n_full, int parts, size_t ldc, cudaStream_t stream);
 
 // 0 = choose per call, 1 = shared-memory-operand kernel, 2 = tensor-memory-operand kernel, 3 = 256-column items,
-// 4 = plans created from now on are tall plans (tall kernel).
+// 4 = plans created from now on are tall plans (tall kernel), 5 = stream plans and calls (stream kernel).
 extern int g_spmm_variant;
 
 }  // namespace smat

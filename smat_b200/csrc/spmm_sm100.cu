@@ -58,6 +58,7 @@
 #include "ptx_sm100.cuh"
 #include "smat_internal.h"
 #include "spmm_sched.cuh"
+#include "spmm_stream.h"
 
 namespace smat {
 
@@ -652,6 +653,7 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
     if (ldc == 0) ldc = N;
     // the view of the groups asked for: steps, blocks and row pointers are addressed absolutely, so a sub-range is
     // the same plan with its first group, first block-row and group count moved
+    if (whole.stream) return launch_stream(whole, B, C, N, stream, ctx, ldc, group_begin, group_end);
     if (whole.tall) return launch_spmm_tall(whole, B, C, N, stream, ctx, ldc, group_begin, group_end);
     if (group_end > whole.n_groups) group_end = whole.n_groups;
     if (group_begin >= group_end) return SMAT_OK;

@@ -30,6 +30,7 @@
 #include <mutex>
 
 #include "smat_internal.h"
+#include "spmm_stream.h"
 
 namespace smat {
 namespace {
@@ -121,6 +122,11 @@ extern "C" int smat_spmm_bcsr_f16_static(const void* vals, const int* rowptr, co
     if (int rc = static_device(&d)) return rc;
 
     const size_t Mb = M / 16;
+    if (nnzb && stream_for_call(N, Mb, nnzb, K, d->ctx.sm_count)) {
+        const StreamShape shape = stream_shape(N, Mb, nnzb, K, d->ctx.sm_count, false);
+        if (stream_call_bytes(shape, N, Mb, nnzb, K) <= kStaticScratchBytes - kStatusBytes)
+            return stream_call(shape, vals, rowptr, colidx, B, C, N, K, nnzb, 0, Mb, d->base, &d->ctx, stream);
+    }
     PlanView v;
     v.rowptr = rowptr;
     v.K = K;

@@ -1,0 +1,586 @@
+// Block-sparse SpMM for NVIDIA B200 (sm_100a), "stream" variant: no panels, no pipeline of roles -- every warp walks the
+// blocks of (a piece of) ONE block-row and feeds warp-level MMAs straight from global memory through L2 and L1.  Same
+// boundary and layouts as spmm_sm100.cu (replaces mmaCBTKernel, src/cuda_hgemm/src/mma/mmaCBT.cu:13-88).
+//
+// What it is for.  The tcgen05 kernels pay ~470-550 cycles per step (four block-columns of a group of block-rows)
+// whatever the step holds and however narrow C is, and their items are 128 columns wide.  Three kinds of work leave them
+// far from their bounds: a narrow C (decoding: the matrix has to stream from HBM, hardly any arithmetic), scattered
+// blocks (a step holds one or two), and small products, where set-up and hand-overs are most of the time.  Here a block
+// costs its 512 bytes of A, its 16 x N slice of B and N / 8 MMAs, and nothing is needed beforehand, so that a product
+// without a plan reads the boundary's arrays as they are.
+//
+// What bounds it (measured, one B200): A from HBM while C is narrow; then the slices of B that every block fetches through
+// L2, 32 N bytes per block.  From the [N][K] array a slice is N sectors of 32 bytes, each in a line of its own, and an SM takes one such
+// sector per cycle from L2 or L1 (131 cycles per slice of 128 columns); contiguous slices come at 64 bytes per cycle (60
+// cycles; 33 out of L1).  So where the blocks outnumber the block-columns enough, B is first rewritten as slabs [K / 16][N][16],
+// one pass over B.  mma.sync runs at 2.1-2.6 cycles per 16x8x16 MMA and SM (34 cycles per block of 128 columns) and
+// is not what bounds it; a tcgen05.mma on one block would need its slice in shared memory (39 cycles for the operand
+// port alone) and a barrier round trip per hand-over.
+//
+// Measured against the tcgen05 kernels (before -> now): 8192 x 28672 layer, 183 000 blocks, N = 16: 67.7 -> 22.6 us (4.2 TB/s);
+// power-law matrix of 2.05 million blocks, N = 128: 1714 -> 797 us, N = 8 (1.78 million): 2076 -> 208 us; band matrix of
+// 2284 blocks, N = 64: 10 -> 4.5 us.  Where blocks share their slices of B (a layer or a random matrix at N >= 128: the
+// tall kernel takes 8-10 ns per block, 128 columns and SM, this one 55-60) the tcgen05 kernels stay.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <type_traits>
+#include <vector>
+
+#include "smat_internal.h"
+#include "spmm_stream.h"
+
+namespace smat {
+namespace {
+
+
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint4& a, const uint2& b) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a.x), "r"(a.z), "r"(a.y), "r"(a.w), "r"(b.x), "r"(b.y));
+}
+// Values of A are read once per column tile: not kept in L1, which the slices of B need.
+__device__ __forceinline__ uint4 load_a16(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 load_a8(const void* p) {
+    uint2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
+template <int NT, int W, int kWarps, int U, int MINB, bool SLAB, bool PLAN>
+__global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(const StreamArgs p) {
+    constexpr int T = NT / 8;                                       // MMAs (8 columns each) per block
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int tile = (int)(blockIdx.x % (unsigned)p.n_tiles);
+    const int piece = (int)(blockIdx.x / (unsigned)p.n_tiles) * (kWarps / W) + warp / W;
+    const int n0 = tile * p.tile_cols;
+    // launched while the kernel before it still runs (programmatic dependent launch); nothing is read before this
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // ---- the piece: blocks [b0, b1) of block-row `row`; count > 1: one of `count` pieces of a long block-row ----
+    int row = 0, b0 = 0, b1 = 0, count = 1, my_slot = 0, first_slot = 0;
+    bool live = piece < p.n_pieces;
+    if (live) {
+        if (PLAN) {
+            const uint4 d = __ldg(p.pieces + piece);
+            row = (int)d.x; b0 = (int)d.y; b1 = (int)d.z;
+            if (d.w) {
+                const int2 s = __ldg(p.slots + (d.w - 1));
+                my_slot = (int)d.w - 1; first_slot = s.x; count = s.y;
+            }
+        } else {
+            const int n_rows = p.brow_end - p.brow_begin;
+            if (piece < n_rows) {
+                const int lo = __ldg(p.rowptr + p.brow_begin), hi = __ldg(p.rowptr + p.brow_end);
+                // row pointers that would lead past the arrays: an empty product and a status code
+                const bool bad = lo < 0 || hi < lo || hi > p.nnzb || (p.long_rows && __ldg(p.long_rows) > p.n_pieces - n_rows);
+                if (bad && piece == 0 && lane == 0) atomicCAS(p.status, 0, kStatusBadRowptr);
+                row = piece;
+                b0 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + row), lo), hi);
+                b1 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + row + 1), b0), hi);
+                if (b1 - b0 > p.chunk && p.long_rows) {
+                    my_slot = first_slot = __ldg(p.row_slot + row);
+                    count = (b1 - b0 + p.chunk - 1) / p.chunk;
+                    b1 = b0 + p.chunk;
+                }
+            } else {
+                const int listed = __ldg(p.long_rows);
+                live = piece - n_rows < listed && listed <= p.n_pieces - n_rows;
+                if (live) {
+                    const uint4 d = __ldg(p.pieces + (piece - n_rows));
+                    row = (int)d.x; b0 = (int)d.y; b1 = (int)d.z; my_slot = (int)d.w;
+                    const int2 s = __ldg(p.slots + my_slot);
+                    first_slot = s.x; count = s.y;
+                }
+            }
+        }
+    }
+    if (W == 1 && !live) return;
+    // this warp's share of the piece
+    int c0 = b0, c1 = b1;
+    if (W > 1) {
+        const int per = (b1 - b0 + W - 1) / W, w = warp % W;
+        c0 = min(b1, b0 + w * per);
+        c1 = min(b1, c0 + per);
+        if (!live) c0 = c1 = 0;
+    }
+    float acc[T][4];
+#pragma unroll
+    for (int j = 0; j < T; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+
+    // k inside a block is permuted the same way for both operands, so that a thread's four values of a row are adjacent
+    // in memory: thread t of a quad holds k = 4t .. 4t + 3
+    const uint2* __restrict__ b_lane;
+    size_t b_step;   // uint2 between neighbouring column octets
+    if (SLAB) {
+        b_lane = reinterpret_cast<const uint2*>(p.B) + (size_t)(n0 + g) * 4 + t;
+        b_step = 32;
+    } else {
+        b_lane = reinterpret_cast<const uint2*>(p.B) + ((size_t)(n0 + g) * p.K >> 2) + t;
+        b_step = (size_t)p.K * 2;
+    }
+    const size_t slab = SLAB ? (size_t)p.N * 4 : 4;  // uint2 between neighbouring block-columns
+    const int octets = min(p.tile_cols, p.N - n0) >> 3;
+    const uint8_t* a_lane = reinterpret_cast<const uint8_t*>(p.vals) + (PLAN ? lane * 16 : lane * 8);
+    const int Kb = p.K >> 4;
+
+    uint4 a[2][U];
+    uint2 b[2][U][T];
+#pragma unroll
+    for (int s = 0; s < 2; s++)
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int j = 0; j < T; j++) b[s][u][j] = make_uint2(0u, 0u);
+    bool ok[2][U];
+    int cols = 0, cols_at = c0;  // 32 column indices at a time, one per lane
+    auto load_cols = [&](int at) {
+        cols_at = at;
+        int c = (at + lane < c1) ? __ldg(p.colidx + at + lane) >> (PLAN ? 0 : 4) : 0;
+        if (!PLAN && (c < 0 || c >= Kb)) {
+            atomicCAS(p.status, 0, kStatusBadColumns);
+            c = -1;
+        }
+        cols = c;
+        // what the warp will read of A after this batch of 32 blocks is on its way to L2 meanwhile
+        const int ahead = min(c1 - (at + 32), 32);
+        if (lane == 0 && ahead > 0)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const uint8_t*>(p.vals) + (size_t)(at + 32) * 512), "r"(ahead * 512) : "memory");
+    };
+    load_cols(c0);
+    auto fetch = [&](auto S, int at) {
+        constexpr int s = decltype(S)::value;
+        if (at - cols_at >= 32) load_cols(at);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int cb = __shfl_sync(0xffffffffu, cols, (at + u - cols_at) & 31);
+            ok[s][u] = at + u < c1 && cb >= 0;
+            if (ok[s][u]) {
+                const uint8_t* ap = a_lane + (size_t)(at + u) * 512;
+                if (PLAN) {
+                    a[s][u] = load_a16(ap);
+                } else {
+                    const uint2 lo = load_a8(ap), hi = load_a8(ap + 256);
+                    a[s][u] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                }
+                const uint2* bp = b_lane + (size_t)cb * slab;
+#pragma unroll
+                for (int j = 0; j < T; j++)
+                    if (j < octets) b[s][u][j] = __ldg(bp + j * b_step);
+            }
+        }
+    };
+    auto multiply = [&](auto S) {
+        constexpr int s = decltype(S)::value;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (ok[s][u]) {
+#pragma unroll
+                for (int j = 0; j < T; j++) mma_16816(acc[j], a[s][u], b[s][u][j]);
+            }
+    };
+    using I0 = std::integral_constant<int, 0>;
+    using I1 = std::integral_constant<int, 1>;
+    fetch(I0{}, c0);
+    for (int at = c0; at < c1; at += 2 * U) {
+        fetch(I1{}, at + U);
+        multiply(I0{});
+        fetch(I0{}, at + 2 * U);
+        multiply(I1{});
+    }
+
+    // ---- sum over the W warps of the piece (fixed order) ----
+    if constexpr (W > 1) {
+        __shared__ float4 red[kWarps / 2][T][32];
+        const int w = warp % W, base = (warp / W) * (W / 2);
+#pragma unroll
+        for (int half = W / 2; half >= 1; half >>= 1) {
+            if (w >= half && w < 2 * half) {
+#pragma unroll
+                for (int j = 0; j < T; j++) red[base + w - half][j][lane] = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+            }
+            __syncthreads();
+            if (w < half) {
+#pragma unroll
+                for (int j = 0; j < T; j++) {
+                    const float4 v = red[base + w][j][lane];
+                    acc[j][0] += v.x; acc[j][1] += v.y; acc[j][2] += v.z; acc[j][3] += v.w;
+                }
+            }
+            if (half > 1) __syncthreads();
+        }
+        if (w != 0 || !live) return;
+    }
+
+    // ---- a piece of a long block-row: partial sums to scratch; the last piece to arrive adds them up in order ----
+    if (count > 1) {
+        float4* mine = p.partial + ((size_t)my_slot * p.n_tiles + tile) * (T * 32) + lane;
+#pragma unroll
+        for (int j = 0; j < T; j++) __stcg(mine + j * 32, make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]));
+        __threadfence();
+        int old = 0;
+        if (lane == 0) old = atomicAdd(p.counters + (size_t)first_slot * p.n_tiles + tile, 1);
+        old = __shfl_sync(0xffffffffu, old, 0);
+        if (old != count - 1) return;
+        __threadfence();
+        if (lane == 0) p.counters[(size_t)first_slot * p.n_tiles + tile] = 0;  // ready for the next launch
+#pragma unroll
+        for (int j = 0; j < T; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+        for (int i = 0; i < count; i++) {
+            const float4* src = p.partial + ((size_t)(first_slot + i) * p.n_tiles + tile) * (T * 32) + lane;
+#pragma unroll
+            for (int j = 0; j < T; j++) {
+                const float4 v = __ldcg(src + j * 32);
+                acc[j][0] += v.x; acc[j][1] += v.y; acc[j][2] += v.z; acc[j][3] += v.w;
+            }
+        }
+    }
+
+    // ---- fp16 rows of C: neighbouring threads exchange halves of two octets, so that a quad stores 32 contiguous bytes ----
+    __half* crow = p.C + (size_t)(row * 16 + g) * p.ldc + n0;
+    if constexpr (T == 1) {
+        *reinterpret_cast<__half2*>(crow + 2 * t) = __floats2half2_rn(acc[0][0], acc[0][1]);
+        *reinterpret_cast<__half2*>(crow + 8 * p.ldc + 2 * t) = __floats2half2_rn(acc[0][2], acc[0][3]);
+    } else {
+        const bool odd = t & 1;
+#pragma unroll
+        for (int j = 0; j < T; j += 2) {
+            if (j >= octets) break;
+            const __half2 x0 = __floats2half2_rn(acc[j][0], acc[j][1]), y0 = __floats2half2_rn(acc[j][2], acc[j][3]);
+            const __half2 x1 = __floats2half2_rn(acc[j + 1][0], acc[j + 1][1]), y1 = __floats2half2_rn(acc[j + 1][2], acc[j + 1][3]);
+            const __half2 rx = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1), ry = __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 1);
+            const int col = 8 * j + (odd ? 8 + 2 * (t - 1) : 2 * t);
+            if (!odd || j + 1 < octets) {
+                union { __half2 h[2]; uint2 u; } vx, vy;
+                vx.h[0] = odd ? rx : x0; vx.h[1] = odd ? x1 : rx;
+                vy.h[0] = odd ? ry : y0; vy.h[1] = odd ? y1 : ry;
+                *reinterpret_cast<uint2*>(crow + col) = vx.u;
+                *reinterpret_cast<uint2*>(crow + 8 * p.ldc + col) = vy.u;
+            }
+        }
+    }
+}
+
+// B ([N][K], k contiguous) -> slabs [K / 16][N][16]: the 16 x N slice of one block-column becomes contiguous.
+__global__ void __launch_bounds__(256) slab_kernel(const uint4* __restrict__ B, uint4* __restrict__ out, int N, int K8) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // a warp moves 16 rows x 32 bytes; the eight warps of a CTA take neighbouring block-columns
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = blockIdx.x * 8 + warp;  // block-column
+    if (2 * c >= K8) return;
+    for (int n = blockIdx.y * 16 + (lane >> 1); n < N; n += gridDim.y * 16)
+        out[((size_t)c * N + n) * 2 + (lane & 1)] = __ldg(B + (size_t)n * K8 + 2 * c + (lane & 1));
+}
+
+// Product without a plan: the block-rows of more than `chunk` blocks, cut into pieces.  The first piece stays with the
+// row's own warps; the others are listed here, in whatever order the rows arrive (the sums of a row are added up by
+// piece number, so the order does not show in the result).  head[0], head[1]: pieces listed, slots taken (zero before).
+__global__ void __launch_bounds__(256) long_rows_kernel(const int* __restrict__ rowptr, int brow_begin, int brow_end, int nnzb, int chunk,
+                                                       int room, int* head, uint4* __restrict__ pieces, int2* __restrict__ slots,
+                                                       int* __restrict__ row_slot) {
+    const int lo = __ldg(rowptr + brow_begin), hi = __ldg(rowptr + brow_end);
+    const int row = blockIdx.x * 256 + threadIdx.x;
+    if (lo < 0 || hi < lo || hi > nnzb || row >= brow_end - brow_begin) return;
+    const int b0 = min(max(__ldg(rowptr + brow_begin + row), lo), hi), b1 = min(max(__ldg(rowptr + brow_begin + row + 1), b0), hi);
+    if (b1 - b0 <= chunk) return;
+    const int k = (b1 - b0 + chunk - 1) / chunk;
+    const int at = atomicAdd(head, k - 1), slot = atomicAdd(head + 1, k);
+    if (at + k - 1 > room) return;  // row pointers that overlap: the kernel sees more pieces than there can be and refuses
+    row_slot[row] = slot;
+    slots[slot] = make_int2(slot, k);
+    for (int i = 1; i < k; i++) {
+        pieces[at + i - 1] = make_uint4((uint32_t)row, (uint32_t)(b0 + i * chunk), (uint32_t)min(b1, b0 + (i + 1) * chunk), (uint32_t)(slot + i));
+        slots[slot + i] = make_int2(slot, k);
+    }
+}
+
+// The plan's copy of the values in the order a warp's lanes read them (lane (g, t): rows g and g + 8, k = 4t .. 4t + 3), and
+// of the block columns; a column outside the matrix becomes -1.
+__global__ void __launch_bounds__(256) stream_pack_kernel(const uint2* __restrict__ vals, const int* __restrict__ colidx,
+                                                         uint4* __restrict__ packed, int* __restrict__ cols, int first, int n, int Kb) {
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+        const uint2 lo = __ldg(vals + (size_t)(first + i) * 64 + lane), hi = __ldg(vals + (size_t)(first + i) * 64 + 32 + lane);
+        packed[(size_t)i * 32 + lane] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        if (cols && lane == 0) {
+            const int c = __ldg(colidx + first + i) >> 4;
+            cols[i] = (c >= 0 && c < Kb) ? c : -1;
+        }
+    }
+}
+
+// warps of a CTA, blocks per load batch (two batches in flight) and CTAs per SM of the kernel for NT columns, W warps per piece
+template <int NT, int W>
+struct Tune {
+    static constexpr int WARPS = W == 8 ? 8 : 4;
+    static constexpr int U = NT == 8 ? 4 : NT <= 32 ? 2 : 1;
+    static constexpr int MINB = W == 8 ? (NT <= 16 ? 4 : NT <= 64 ? 2 : 1) : (NT <= 16 ? 8 : NT == 32 ? 5 : NT == 64 ? 4 : 3);
+};
+
+template <int NT, int W, bool SLAB, bool PLAN>
+cudaError_t launch_one(const StreamArgs& a, cudaStream_t stream) {
+    using Q = Tune<NT, W>;
+    constexpr long long per = Q::WARPS / W;
+    const long long grid = (((long long)a.n_pieces + per - 1) / per) * a.n_tiles;
+    if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(Q::WARPS * 32);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, spmm_bcsr_stream_kernel<NT, W, Q::WARPS, Q::U, Q::MINB, SLAB, PLAN>, a);
+}
+
+template <bool PLAN, bool SLAB, int W>
+cudaError_t launch_nt(int nt, const StreamArgs& a, cudaStream_t stream) {
+    if constexpr (W < 8) {
+        if (nt == 128) return launch_one<128, W, SLAB, PLAN>(a, stream);
+    }
+    if (nt == 64) return launch_one<64, W, SLAB, PLAN>(a, stream);
+    if (nt == 32) return launch_one<32, W, SLAB, PLAN>(a, stream);
+    if constexpr (!SLAB) {
+        if (nt == 16) return launch_one<16, W, SLAB, PLAN>(a, stream);
+        if (nt == 8) return launch_one<8, W, SLAB, PLAN>(a, stream);
+    }
+    return cudaErrorInvalidValue;
+}
+
+template <bool PLAN, bool SLAB>
+cudaError_t launch_w(const StreamShape& s, const StreamArgs& a, cudaStream_t stream) {
+    if (s.w == 8 && s.nt < 128) return launch_nt<PLAN, SLAB, 8>(s.nt, a, stream);
+    if (s.w >= 4) return launch_nt<PLAN, SLAB, 4>(s.nt, a, stream);
+    if (s.w == 2) return launch_nt<PLAN, SLAB, 2>(s.nt, a, stream);
+    return launch_nt<PLAN, SLAB, 1>(s.nt, a, stream);
+}
+
+template <bool PLAN>
+int launch(const StreamShape& s, const StreamArgs& a, cudaStream_t stream) {
+    const cudaError_t e = s.slab ? launch_w<PLAN, true>(s, a, stream) : launch_w<PLAN, false>(s, a, stream);
+    if (e != cudaSuccess) return fail(SMAT_ERR_CUDA, "launch of the stream kernel failed: %s", cudaGetErrorString(e));
+    count_launch();
+    return SMAT_OK;
+}
+
+int make_slabs(const void* B, void* slabs, size_t N, size_t K, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((K / 16 + 7) / 8), (unsigned)std::min<size_t>((N + 15) / 16, 65535));
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    SMAT_CUDA_TRY(cudaLaunchKernelEx(&cfg, slab_kernel, reinterpret_cast<const uint4*>(B), reinterpret_cast<uint4*>(slabs), (int)N, (int)(K / 8)));
+    count_launch();
+    return SMAT_OK;
+}
+
+// Columns of a tile: N spread evenly over the tiles, in octets.
+int tile_cols(size_t N, int tiles) { return (int)((N / 8 + (size_t)tiles - 1) / (size_t)tiles) * 8; }
+
+size_t round256(size_t x) { return (x + 255) / 256 * 256; }
+
+}  // namespace
+
+// Columns per warp, warps per piece, blocks per piece, and whether B is rewritten as slabs.
+StreamShape stream_shape(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count, bool plan) {
+    StreamShape s;
+    const size_t sms = (size_t)sm_count, avg = rows ? nnzb / rows : 0;
+    // One tile across C as long as it holds in registers: A is then read once.
+    s.nt = N <= 8 ? 8 : N <= 16 ? 16 : N <= 32 ? 32 : N <= 64 ? 64 : 128;
+    // Slabs: a slice then costs 0.27 ns less per column and SM; the pass costs its launch and B twice at 5.5 TB/s.
+    const double gain = (double)nnzb * (double)N * 0.27e-3 / (double)sms, cost = 2.0 + 4e-6 * (double)N * (double)K / 5.5;
+    s.slab = s.nt >= 32 && gain > cost;
+    // Enough warps to keep the SMs' load queues full (12 of 128 columns, 16 of 64, 32 of fewer): first several warps per
+    // block-row, each with at least four blocks, then narrower tiles.
+    auto tiles = [&] { return (N + (size_t)s.nt - 1) / (size_t)s.nt; };
+    auto wanted = [&] { return sms * (s.nt == 128 ? 12 : s.nt == 64 ? 16 : 32); };
+    while (s.w < (s.nt == 128 ? 4 : 8) && rows * tiles() * (size_t)s.w < wanted() && avg >= 8 * (size_t)s.w) s.w *= 2;
+    while (s.nt > (s.slab ? 32 : 16) && rows * tiles() * (size_t)s.w * 2 < wanted()) s.nt /= 2;
+    // A piece: a few rounds of work per resident warp, so that long block-rows neither trail nor pay much for their
+    // partial tiles.  Measured on power-law matrices of 0.2 to 2.2 million blocks: 96 to 192, flat in between.
+    const size_t per_warp = nnzb / (sms * 12) / 2;
+    const size_t warp_chunk = std::min<size_t>(std::max<size_t>(per_warp, 96), 192);
+    // Without a plan long block-rows have to be listed first (two more operations on the stream, ~4 us): small matrices go
+    // without, with enough warps per block-row that even a full one is no longer than their pieces.
+    if (!plan && nnzb < 32 * 1024)
+        while (s.w < (s.nt == 128 ? 4 : 8) && K / 16 > warp_chunk * (size_t)s.w && K / 16 <= warp_chunk * 8) s.w *= 2;
+    s.chunk = (int)(warp_chunk * (size_t)s.w);
+    return s;
+}
+
+// Microseconds a product takes with this kernel (one B200), within some 20 %.
+double stream_estimate_us(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count) {
+    const StreamShape s = stream_shape(N, rows, nnzb, K, sm_count, true);
+    const double n = (double)N, full = (double)(N / 128), rest = (double)(N % 128);
+    const double slice = s.slab ? 0.38 : 0.60;  // ns per column of a block and SM
+    const double per_block = full * (10.0 + 128.0 * slice) + (rest > 0 ? 10.0 + rest * slice : 0.0);
+    return 4.0 + (s.slab ? 2.0 + 4e-6 * n * (double)K / 5.5 : 0.0) + (double)nnzb / sm_count * per_block * 1e-3 + (double)(rows * 16) * n * 2.0 / 6e6;
+}
+
+// A product without a plan takes this kernel unless building a plan inside the call (reading and writing all blocks, a
+// dozen launches) and a tcgen05 kernel are estimated to be faster: many blocks, each used by many columns.
+bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count) {
+    if (g_spmm_variant) return g_spmm_variant == 5;
+    const double plan_us = 50.0 + 1028.0 * (double)nnzb / 5e6 + (double)nnzb * (double)((N + 127) / 128) / sm_count * 20e-3;
+    return stream_estimate_us(N, rows, nnzb, K, sm_count) < plan_us;
+}
+
+int stream_plan_build(StreamPlan& sp, PlanView& v, const int* h_rowptr, const void* vals, const int* colidx, size_t N_hint, int sm_count,
+                      cudaStream_t stream) {
+    const size_t rows = v.brow_end - v.brow_begin, first = (size_t)h_rowptr[0], n = v.nnzb;
+    const StreamShape s = stream_shape(N_hint, rows, n, v.K, sm_count, true);
+    std::vector<uint4> pieces;
+    std::vector<int2> slots;
+    pieces.reserve(rows + n / (size_t)s.chunk + 1);
+    sp.row_piece.resize(rows + 1);
+    for (size_t r = 0; r < rows; r++) {
+        const unsigned b0 = (unsigned)(h_rowptr[r] - (int)first), len = (unsigned)(h_rowptr[r + 1] - h_rowptr[r]);
+        const unsigned k = len ? (len + (unsigned)s.chunk - 1) / (unsigned)s.chunk : 1, per = (len + k - 1) / k;
+        sp.row_piece[r] = (int)pieces.size();
+        const int slot0 = (int)slots.size();
+        for (unsigned i = 0; i < k; i++) {
+            if (k > 1) slots.push_back(make_int2(slot0, (int)k));
+            pieces.push_back(make_uint4((unsigned)r, b0 + std::min(len, i * per), b0 + std::min(len, (i + 1) * per), k > 1 ? (unsigned)slots.size() : 0u));
+        }
+    }
+    sp.row_piece[rows] = (int)pieces.size();
+    sp.n_cap = (N_hint + 127) / 128 * 128;
+    const size_t pieces_bytes = round256(pieces.size() * sizeof(uint4)), slots_bytes = round256(slots.size() * sizeof(int2)),
+                 counter_bytes = round256(slots.size() * (sp.n_cap / 8) * sizeof(int)), partial_bytes = round256(slots.size() * sp.n_cap * 64),
+                 cols_bytes = round256(n * sizeof(int)), packed_bytes = n * 512, slab_bytes = s.slab ? sp.n_cap * v.K * 2 : 0;
+    SMAT_CUDA_TRY(cudaMalloc(&sp.buffer, pieces_bytes + slots_bytes + counter_bytes + partial_bytes + cols_bytes + packed_bytes + slab_bytes));
+    char* b = static_cast<char*>(sp.buffer);
+    StreamArgs& a = sp.args;
+    a = StreamArgs{};
+    a.pieces = reinterpret_cast<uint4*>(b); b += pieces_bytes;
+    a.slots = reinterpret_cast<int2*>(b); b += slots_bytes;
+    a.counters = reinterpret_cast<int*>(b); b += counter_bytes;
+    a.partial = reinterpret_cast<float4*>(b); b += partial_bytes;
+    a.colidx = reinterpret_cast<int*>(b); b += cols_bytes;
+    a.vals = b; b += packed_bytes;
+    sp.slabs = slab_bytes ? b : nullptr;
+    sp.first = first;
+    SMAT_CUDA_TRY(cudaMemcpyAsync(const_cast<uint4*>(a.pieces), pieces.data(), pieces.size() * sizeof(uint4), cudaMemcpyHostToDevice, stream));
+    if (!slots.empty()) {
+        SMAT_CUDA_TRY(cudaMemcpyAsync(const_cast<int2*>(a.slots), slots.data(), slots.size() * sizeof(int2), cudaMemcpyHostToDevice, stream));
+        SMAT_CUDA_TRY(cudaMemsetAsync(a.counters, 0, counter_bytes, stream));
+    }
+    v.stream = &sp;
+    v.n_groups = rows;
+    v.rg = 1;
+    return stream_plan_values(v, vals, colidx, sm_count, stream);  // pageable sources: the copies above have left them
+}
+
+int stream_plan_values(const PlanView& v, const void* vals, const int* colidx, int sm_count, cudaStream_t stream) {
+    if (v.nnzb == 0) return SMAT_OK;
+    const StreamArgs& a = v.stream->args;
+    const unsigned grid = (unsigned)std::min((v.nnzb + 7) / 8, (size_t)sm_count * 8);
+    stream_pack_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const uint2*>(vals), colidx, reinterpret_cast<uint4*>(const_cast<void*>(a.vals)),
+                                                 colidx ? const_cast<int*>(a.colidx) : nullptr, (int)v.stream->first, (int)v.nnzb, (int)(v.K / 16));
+    count_launch();
+    SMAT_CUDA_TRY(cudaGetLastError());
+    return SMAT_OK;
+}
+
+int launch_stream(const PlanView& v, const void* B, void* C, size_t N, cudaStream_t stream, const DeviceCtx* ctx, size_t ldc,
+                  size_t row_begin, size_t row_end) {
+    const StreamPlan& sp = *v.stream;
+    const size_t rows = v.brow_end - v.brow_begin;
+    if (row_end > rows) row_end = rows;
+    if (row_begin >= row_end) return SMAT_OK;
+    // scratch and slabs were sized for n_cap columns: wider products go in several passes
+    for (size_t n0 = 0; n0 < N; n0 += sp.n_cap) {
+        const size_t n = std::min(sp.n_cap, N - n0);
+        StreamShape s = stream_shape(n, rows, v.nnzb, v.K, ctx->sm_count, true);
+        if (!sp.slabs) s.slab = false;
+        StreamArgs a = sp.args;
+        a.B = static_cast<const char*>(B) + n0 * v.K * 2;
+        a.C = static_cast<__half*>(C) + n0 - row_begin * 16 * ldc;  // pieces count block-rows from the plan's first
+        a.status = ctx->d_status;
+        a.ldc = ldc;
+        a.pieces += sp.row_piece[row_begin];
+        a.n_pieces = sp.row_piece[row_end] - sp.row_piece[row_begin];
+        a.N = (int)n;
+        a.K = (int)v.K;
+        a.n_tiles = (int)((n + (size_t)s.nt - 1) / (size_t)s.nt);
+        a.tile_cols = tile_cols(n, a.n_tiles);
+        if (s.slab) {
+            if (int rc = make_slabs(a.B, sp.slabs, n, v.K, stream)) return rc;
+            a.B = sp.slabs;
+        }
+        if (int rc = launch<true>(s, a, stream)) return rc;
+    }
+    return SMAT_OK;
+}
+
+// Scratch of a product without a plan: slabs, and where a block-row can be longer than a piece the list of pieces,
+// their partial tiles and counters.
+size_t stream_call_bytes(const StreamShape& s, size_t N, size_t rows, size_t nnzb, size_t K) {
+    const size_t extra = K / 16 > (size_t)s.chunk ? nnzb / (size_t)s.chunk + 1 : 0, n_pad = (N + (size_t)s.nt - 1) / (size_t)s.nt * (size_t)s.nt;
+    return (s.slab ? round256(N * K * 2) : 0) +
+           (extra ? 256 + round256(2 * extra * (n_pad / (size_t)s.nt) * sizeof(int)) + round256(extra * sizeof(uint4)) + round256(2 * extra * sizeof(int2)) +
+                        round256(rows * sizeof(int)) + 2 * extra * n_pad * 64
+                  : 0);
+}
+
+int stream_call(const StreamShape& s, const void* vals, const int* rowptr, const int* colidx, const void* B, void* C, size_t N, size_t K,
+                size_t nnzb, size_t brow_begin, size_t brow_end, void* scratch, const DeviceCtx* ctx, cudaStream_t stream) {
+    const size_t rows = brow_end - brow_begin;
+    const size_t extra = K / 16 > (size_t)s.chunk ? nnzb / (size_t)s.chunk + 1 : 0, tiles = (N + (size_t)s.nt - 1) / (size_t)s.nt;
+    char* b = static_cast<char*>(scratch);
+    StreamArgs a = {};
+    a.vals = vals;
+    a.rowptr = rowptr;
+    a.colidx = colidx;
+    a.B = B;
+    a.C = static_cast<__half*>(C);
+    a.status = ctx->d_status;
+    a.ldc = N;
+    a.n_pieces = (int)(rows + extra);
+    a.n_tiles = (int)tiles;
+    a.tile_cols = tile_cols(N, a.n_tiles);
+    a.N = (int)N;
+    a.K = (int)K;
+    a.brow_begin = (int)brow_begin;
+    a.brow_end = (int)brow_end;
+    a.nnzb = (int)nnzb;
+    a.chunk = s.chunk;
+    if (extra) {
+        int* head = reinterpret_cast<int*>(b); b += 256;
+        a.long_rows = head;
+        a.counters = reinterpret_cast<int*>(b);
+        const size_t counter_bytes = round256(2 * extra * tiles * sizeof(int)); b += counter_bytes;
+        uint4* pieces = reinterpret_cast<uint4*>(b); b += round256(extra * sizeof(uint4));
+        int2* slots = reinterpret_cast<int2*>(b); b += round256(2 * extra * sizeof(int2));
+        int* row_slot = reinterpret_cast<int*>(b); b += round256(rows * sizeof(int));
+        a.partial = reinterpret_cast<float4*>(b); b += 2 * extra * tiles * (size_t)s.nt * 64;
+        a.pieces = pieces;
+        a.slots = slots;
+        a.row_slot = row_slot;
+        SMAT_CUDA_TRY(cudaMemsetAsync(head, 0, 256 + counter_bytes, stream));
+        long_rows_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, stream>>>(rowptr, (int)brow_begin, (int)brow_end, (int)nnzb, s.chunk, (int)extra, head,
+                                                                             pieces, slots, row_slot);
+        count_launch();
+        SMAT_CUDA_TRY(cudaGetLastError());
+    }
+    if (s.slab) {
+        if (int rc = make_slabs(B, b, N, K, stream)) return rc;
+        a.B = b;
+    }
+    return launch<false>(s, a, stream);
+}
+
+}  // namespace smat
