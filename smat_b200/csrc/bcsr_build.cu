@@ -11,7 +11,10 @@
 // The reference's two dense Mb*Kb int maps (:381, :425-431) are not materialised: one CTA owns one
 // block-row at a time and keeps that block-row's column-block bitmap in shared memory.
 //
-// One CTA of 512 threads per block-row (grid-stride); warp w walks CSR row 16*blockrow + w.
+// One CTA per block-row.  The entries of its 16 CSR rows are contiguous and dealt out to all threads, whatever the rows'
+// lengths: a warp per row made the longest row of the matrix the time of the whole kernel (power-law graph, 65536 rows,
+// longest 8192 entries, 490 000 blocks: count and fill together 370 -> 110 us; what is left is zeroing 250 MB of values).  Which of several equal entries is last matters only where there are equal ones: block-rows whose rows
+// ascend strictly (checked on the way) scatter in any order, the others keep a warp per row and its order.
 #include <cuda_fp16.h>
 
 #include "smat_internal.h"
@@ -19,21 +22,33 @@
 namespace smat {
 namespace {
 
-constexpr int kBuildThreads = 512;
+constexpr int kBuildThreads = 256;
+constexpr int kBuildWarps = kBuildThreads / 32;
 
-// Marks the block-columns touched by the 16 rows of block-row `br` in the shared bitmap.
-__device__ __forceinline__ void mark_block_columns(const int* __restrict__ rowptr, const int* __restrict__ colidx, int br,
-                                                   uint32_t* bitmap, int words) {
-    for (int w = threadIdx.x; w < words; w += blockDim.x) bitmap[w] = 0u;
+// Marks the block-columns touched by the 16 rows of block-row `br` in the shared bitmap and leaves the 17 row pointers in
+// `ptr`.  Returns whether any row holds two columns that do not ascend (CHECK only; same value for all threads).
+template <bool CHECK>
+__device__ __forceinline__ bool mark_block_columns(const int* __restrict__ rowptr, const int* __restrict__ colidx, int br,
+                                                   uint32_t* bitmap, int words, int* ptr) {
+    if (threadIdx.x < 17) ptr[threadIdx.x] = __ldg(rowptr + br * 16 + threadIdx.x);
+    for (int w = threadIdx.x; w < words; w += kBuildThreads) bitmap[w] = 0u;
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = br * 16 + warp;
-    const int beg = __ldg(rowptr + row), end = __ldg(rowptr + row + 1);
-    for (int j = beg + lane; j < end; j += 32) {
-        const int bc = __ldg(colidx + j) >> 4;
+    const int beg = ptr[0], end = ptr[16];
+    bool tangled = false;
+#pragma unroll 4
+    for (int j = beg + (int)threadIdx.x; j < end; j += kBuildThreads) {
+        const int col = __ldg(colidx + j), bc = col >> 4;
+        if (CHECK && j > beg && __ldg(colidx + j - 1) >= col) {  // fine where a row begins at j
+            bool first = false;
+#pragma unroll
+            for (int r = 1; r < 16; r++) first |= ptr[r] == j;
+            tangled |= !first;
+        }
         atomicOr(&bitmap[bc >> 5], 1u << (bc & 31));
     }
+    if (CHECK) return __syncthreads_or(tangled);
     __syncthreads();
+    return false;
 }
 
 __device__ __forceinline__ int block_sum(int v, int* scratch) {
@@ -55,18 +70,16 @@ __device__ __forceinline__ int block_sum(int v, int* scratch) {
 
 // counts[br + 1] = number of nonzero blocks of block-row br (counts[0] is set to 0).
 __global__ void __launch_bounds__(kBuildThreads)
-bcsr_count_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int Mb, int words, int* counts) {
+bcsr_count_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int words, int* counts) {
     extern __shared__ uint32_t sm[];
-    uint32_t* bitmap = sm;
-    __shared__ int red[33];
-    for (int br = blockIdx.x; br < Mb; br += gridDim.x) {
-        mark_block_columns(rowptr, colidx, br, bitmap, words);
-        int c = 0;
-        for (int w = threadIdx.x; w < words; w += blockDim.x) c += __popc(bitmap[w]);
-        c = block_sum(c, red);
-        if (threadIdx.x == 0) counts[br + 1] = c;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) counts[0] = 0;
+    __shared__ int red[33], ptr[17];
+    const int br = (int)blockIdx.x;
+    mark_block_columns<false>(rowptr, colidx, br, sm, words, ptr);
+    int c = 0;
+    for (int w = threadIdx.x; w < words; w += kBuildThreads) c += __popc(sm[w]);
+    c = block_sum(c, red);
+    if (threadIdx.x == 0) counts[br + 1] = c;
+    if (br == 0 && threadIdx.x == 0) counts[0] = 0;
 }
 
 // In-place inclusive scan of data[0..n) by a single CTA (n = Mb + 1 is small next to nnz).
@@ -106,72 +119,83 @@ __global__ void __launch_bounds__(1024) scan_inplace_kernel(int* data, int n) {
 }
 
 __global__ void __launch_bounds__(kBuildThreads)
-bcsr_fill_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, const __half* __restrict__ vals, int Mb,
+bcsr_fill_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, const __half* __restrict__ vals,
                  int words, const int* __restrict__ brp, int* __restrict__ bcol, __half* __restrict__ bvals) {
     extern __shared__ uint32_t sm[];
     uint32_t* bitmap = sm;          // [words]
     uint32_t* prefix = sm + words;  // [words] exclusive prefix of popcounts
-    __shared__ int warp_tot[16];
-    __shared__ int carry_s;
+    __shared__ int warp_tot[kBuildWarps], ptr[17];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int br = blockIdx.x; br < Mb; br += gridDim.x) {
-        mark_block_columns(rowptr, colidx, br, bitmap, words);
-        const int first = __ldg(brp + br);
-        const int nblk = __ldg(brp + br + 1) - first;
-        if (nblk == 0) { __syncthreads(); continue; }
-        // exclusive scan of popcounts over the bitmap words
-        if (threadIdx.x == 0) carry_s = 0;
-        __syncthreads();
-        for (int base = 0; base < words; base += kBuildThreads) {
-            const int w = base + threadIdx.x;
-            const int c = w < words ? __popc(bitmap[w]) : 0;
-            int v = c;
+    const int br = (int)blockIdx.x;
+    const int first = __ldg(brp + br), nblk = __ldg(brp + br + 1) - first;
+    if (nblk == 0) return;
+    // zero this block-row's values (nblk * 512 bytes, 16-byte stores); the scatter below follows a barrier
+    uint4* z = reinterpret_cast<uint4*>(bvals + (size_t)first * 256);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nblk * 32; i += kBuildThreads) z[i] = make_uint4(0, 0, 0, 0);
+    const bool tangled = mark_block_columns<true>(rowptr, colidx, br, bitmap, words, ptr);
+    // exclusive scan of popcounts over the bitmap words
+    int carry = 0;
+    for (int base = 0; base < words; base += kBuildThreads) {
+        const int w = base + threadIdx.x;
+        const int c = w < words ? __popc(bitmap[w]) : 0;
+        int v = c;
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, v, d);
-                if (lane >= d) v += t;
-            }
-            if (lane == 31) warp_tot[warp] = v;
-            __syncthreads();
-            int woff = 0;
-            for (int k = 0; k < warp; k++) woff += warp_tot[k];
-            const int carry = carry_s;
-            if (w < words) prefix[w] = (uint32_t)(carry + woff + v - c);
-            __syncthreads();
-            if (threadIdx.x == kBuildThreads - 1) carry_s = carry + woff + v;
-            __syncthreads();
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, v, d);
+            if (lane >= d) v += t;
         }
-        // column index of every block, ascending
-        for (int w = threadIdx.x; w < words; w += blockDim.x) {
-            uint32_t bits = bitmap[w];
-            int pos = first + (int)prefix[w];
-            while (bits) {
-                const int b = __ffs(bits) - 1;
-                bits &= bits - 1;
-                bcol[pos++] = ((w << 5) + b) << 4;
-            }
-        }
-        // zero this block-row's values (nblk * 512 bytes, 16-byte stores)
-        uint4* z = reinterpret_cast<uint4*>(bvals + (size_t)first * 256);
-        for (int i = threadIdx.x; i < nblk * 32; i += blockDim.x) z[i] = make_uint4(0, 0, 0, 0);
+        if (lane == 31) warp_tot[warp] = v;
         __syncthreads();
-        // scatter: warp w owns CSR row 16*br + w and walks it in order, 32 entries at a time; inside
-        // a 32-entry step the highest lane holding a given column stores, so the last entry wins
-        const int row = br * 16 + warp;
-        const int beg = __ldg(rowptr + row), end = __ldg(rowptr + row + 1);
+        int before = 0, total = 0;
+#pragma unroll
+        for (int k = 0; k < kBuildWarps; k++) {
+            if (k < warp) before += warp_tot[k];
+            total += warp_tot[k];
+        }
+        if (w < words) prefix[w] = (uint32_t)(carry + before + v - c);
+        carry += total;
+        __syncthreads();
+    }
+    // column index of every block, ascending
+    for (int w = threadIdx.x; w < words; w += kBuildThreads) {
+        uint32_t bits = bitmap[w];
+        int pos = first + (int)prefix[w];
+        while (bits) {
+            const int b = __ffs(bits) - 1;
+            bits &= bits - 1;
+            bcol[pos++] = ((w << 5) + b) << 4;
+        }
+    }
+    auto place = [&](int row, int col) {
+        const int bc = col >> 4;
+        const int slot = first + (int)prefix[bc >> 5] + __popc(bitmap[bc >> 5] & ((1u << (bc & 31)) - 1u));
+        return bvals + (size_t)slot * 256 + row * 16 + (col & 15);
+    };
+    if (!tangled) {
+        const int beg = ptr[0], end = ptr[16];
+#pragma unroll 4
+        for (int j = beg + (int)threadIdx.x; j < end; j += kBuildThreads) {
+            int row = 0;  // the last row that begins at or before j
+#pragma unroll
+            for (int step = 8; step; step >>= 1)
+                if (ptr[row + step] <= j) row += step;
+            *place(row, __ldg(colidx + j)) = vals[j];
+        }
+        return;
+    }
+    // a warp walks a CSR row in order, 32 entries at a time; inside a 32-entry step the highest lane holding a given
+    // column stores, so the last entry wins
+    for (int row = warp; row < 16; row += kBuildWarps) {
+        const int beg = ptr[row], end = ptr[row + 1];
         for (int j0 = beg; j0 < end; j0 += 32) {
             const int j = j0 + lane;
             const bool act = j < end;
             const int col = act ? __ldg(colidx + j) : -1 - lane;
             const uint32_t same = __match_any_sync(0xffffffffu, col);
-            if (act && lane == 31 - __clz(same)) {
-                const int bc = col >> 4;
-                const int slot = first + (int)prefix[bc >> 5] + __popc(bitmap[bc >> 5] & ((1u << (bc & 31)) - 1u));
-                bvals[(size_t)slot * 256 + warp * 16 + (col & 15)] = vals[j];
-            }
+            if (act && lane == 31 - __clz(same)) *place(row, col) = vals[j];
             __syncwarp();
         }
-        __syncthreads();
     }
 }
 
@@ -205,8 +229,7 @@ int smat_bcsr_count(const int* csr_rowptr, const int* csr_colidx, size_t M, size
     if (Mb > 0) {
         const size_t smem = (size_t)words * 4;
         SMAT_CUDA_TRY(cudaFuncSetAttribute(bcsr_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        const int grid = Mb < ctx->sm_count * 4 ? Mb : ctx->sm_count * 4;
-        bcsr_count_kernel<<<grid, kBuildThreads, smem, stream>>>(csr_rowptr, csr_colidx, Mb, words, bcsr_rowptr);
+        bcsr_count_kernel<<<Mb, kBuildThreads, smem, stream>>>(csr_rowptr, csr_colidx, words, bcsr_rowptr);
         count_launch();
         SMAT_CUDA_TRY(cudaGetLastError());
     } else {
@@ -239,9 +262,8 @@ int smat_bcsr_fill(const int* csr_rowptr, const int* csr_colidx, const void* csr
     const int Mb = (int)(M / 16);
     const size_t smem = (size_t)words * 8;
     SMAT_CUDA_TRY(cudaFuncSetAttribute(bcsr_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int grid = Mb < ctx->sm_count * 4 ? Mb : ctx->sm_count * 4;
-    bcsr_fill_kernel<<<grid, kBuildThreads, smem, stream>>>(csr_rowptr, csr_colidx, reinterpret_cast<const __half*>(csr_vals),
-                                                            Mb, words, bcsr_rowptr, bcsr_colidx,
+    bcsr_fill_kernel<<<Mb, kBuildThreads, smem, stream>>>(csr_rowptr, csr_colidx, reinterpret_cast<const __half*>(csr_vals),
+                                                            words, bcsr_rowptr, bcsr_colidx,
                                                             reinterpret_cast<__half*>(bcsr_vals));
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
