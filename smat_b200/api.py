@@ -378,26 +378,34 @@ class Matrix:
 
 
 _UPLOAD_CHUNK = 1 << 21  # bytes
+_UPLOAD_RING = 4  # chunks of one upload in pinned memory at a time
 
 
 def _upload(array, dev):
     """Host array (one dimension, pageable memory, as numpy gives it) -> device tensor.
 
     The driver copies pageable memory through its own staging buffers at about 16 GB/s.  Here the CPU threads fill
-    pinned chunks (from torch's caching host allocator, which hands a chunk out again once its copy is done) while the
-    chunks before them are on their way: 5.6 MB of three arrays in 215 instead of 380 us.  Below two chunks, or with too few
-    threads to outrun the link, the plain copy is as fast."""
+    pinned chunks (at most four, from torch's caching host allocator, refilled once their copy is done) while the
+    chunks before them are on their way: 5.6 MB of three arrays in 215 instead of 380 us.  For arrays of an eighth of a
+    chunk, or with too few threads to outrun the link, the plain copy is as fast."""
     import torch
     src = torch.from_numpy(array)
     if array.nbytes < _UPLOAD_CHUNK // 8 or torch.get_num_threads() < 4:
         return src.to(dev)
     dst = torch.empty_like(src, device=dev)
     step = _UPLOAD_CHUNK // array.itemsize
-    for at in range(0, array.size, step):
+    ring = []  # (pinned chunk, event behind its copy)
+    for i, at in enumerate(range(0, array.size, step)):
         part = src[at:at + step]
-        pinned = torch.empty(part.numel(), dtype=src.dtype, pin_memory=True)
+        if i < _UPLOAD_RING:
+            ring.append((torch.empty(part.numel(), dtype=src.dtype, pin_memory=True), torch.cuda.Event()))
+        pinned, copied = ring[i % _UPLOAD_RING]
+        if i >= _UPLOAD_RING:
+            copied.synchronize()
+        pinned = pinned[:part.numel()]
         pinned.copy_(part)
         dst[at:at + step].copy_(pinned, non_blocking=True)
+        copied.record()
     return dst
 
 

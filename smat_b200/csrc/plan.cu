@@ -18,6 +18,7 @@
 
 #include <new>
 
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -100,7 +101,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* total, int* sh) 
 template <bool FILL>
 __global__ void __launch_bounds__(kPlanThreads)
 plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int brow_begin, int brow_end, int rg, int CAP, int Kb,
-            int n_groups, int* __restrict__ gsp, uint4* __restrict__ steps, int* __restrict__ blk, int nnzb, int* status) {
+            int n_groups, int* __restrict__ gsp, uint4* __restrict__ steps, int* __restrict__ blk, int nnzb, int* status, int* units) {
     extern __shared__ uint32_t sm[];
     uint32_t* masks = sm;                                 // [kWindow] row mask per block-column
     int* blk_pre = reinterpret_cast<int*>(sm + kWindow);  // [kWindow] exclusive block number (FILL only)
@@ -140,6 +141,12 @@ plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int 
                               __popc(masks[i0 + 4 * qd + 3]);
                 ns += (c + CAP - 1) / CAP;
                 nb += c;
+            }
+            if (!FILL && units) {  // MMAs of the 16-row kernel: one per block or pair of blocks in rows 2m, 2m + 1
+                int nu = 0;
+                for (int i = 0; i < PER; i++) nu += __popc((masks[i0 + i] | (masks[i0 + i] >> 1)) & 0x55555555u);
+                nu = __reduce_add_sync(0xffffffffu, nu);
+                if (lane == 0 && nu) atomicAdd(units, nu);
             }
             int tot_s, tot_b = 0;
             const int pre_s = block_exclusive_scan(ns, &tot_s, scan_sh);
@@ -227,25 +234,31 @@ __global__ void __launch_bounds__(1024) plan_scan_kernel(int* data, int n) {
     if (threadIdx.x == 0) data[n] = max_s;
 }
 
-// One warp per step: copies the step's value blocks to their place in the packed stream; lane l moves
-// the 16-byte chunk l of a block (row l/2, half l%2) to chunk l ^ ((l >> 3) & 1), i.e. the 32-byte swizzle.
-__global__ void __launch_bounds__(256) pack_kernel(const uint4* __restrict__ vals, const int* __restrict__ blk,
-                                                  const int* __restrict__ gsp, const uint4* __restrict__ steps,
-                                                  uint8_t* __restrict__ packed, const int* __restrict__ rowptr, int brow_begin,
-                                                  int n_groups) {
-    const int rfirst = __ldg(rowptr + brow_begin);
-    const int total = __ldg(gsp + n_groups);
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < total; i += warps) {
-        const uint4 d = __ldg(steps + i);
-        const int cnt = __popc(d.z) + __popc(d.w);
-        const int first = rfirst + (int)(d.y >> 1);  // position of the step's first block in blk
-        uint4* dst = reinterpret_cast<uint4*>(packed + (size_t)d.y * 256);
-        for (int q = 0; q < cnt; q++) {
-            const int src = __ldg(blk + first + q);
-            dst[q * 32 + (lane ^ ((lane >> 3) & 1))] = __ldg(vals + (size_t)src * 32 + lane);
+// Copies the value blocks into walk order: position p of the packed stream holds block blk[first block of the range + p].
+// A warp moves four blocks at a time, all loads before the stores (a warp per step, which went through the step's record and
+// then its blocks one after the other, left most of the memory latency exposed: 8.4 MB of blocks 8.6 -> 3.5 us).  Lane l
+// moves the 16-byte chunk l of a block (row l/2, half l%2) to chunk l ^ ((l >> 3) & 1), i.e. the 32-byte swizzle.
+// Positions behind the blocks of a group whose columns were found inconsistent hold nothing: skipped by the range check.
+__global__ void __launch_bounds__(256) pack_kernel(const uint4* __restrict__ vals, const int* __restrict__ blk, uint4* __restrict__ packed,
+                                                  const int* __restrict__ rowptr, int brow_begin, int brow_end, int nnzb) {
+    constexpr int U = 4;
+    if (range_is_bad(rowptr, brow_begin, brow_end, nnzb)) return;
+    const int first = __ldg(rowptr + brow_begin), n = __ldg(rowptr + brow_end) - first;
+    const int lane = threadIdx.x & 31, to = lane ^ ((lane >> 3) & 1);
+    const int stride = (int)((gridDim.x * blockDim.x) >> 5) * U;
+    for (int p = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * U; p < n; p += stride) {
+        const int src_l = lane < U && p + lane < n ? __ldg(blk + first + p + lane) - first : -1;
+        uint4 v[U];
+        bool ok[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int src = __shfl_sync(0xffffffffu, src_l, u);
+            ok[u] = (unsigned)src < (unsigned)n;
+            if (ok[u]) v[u] = __ldg(vals + (size_t)(first + src) * 32 + lane);
         }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (ok[u]) packed[(size_t)(p + u) * 32 + to] = v[u];
     }
 }
 
@@ -416,32 +429,10 @@ __global__ void __launch_bounds__(256) tall_pair_kernel(const uint32_t* __restri
     }
 }
 
-// One warp per step of a tall plan: copies the step's value blocks to their place in the packed stream (32-byte swizzle).
-__global__ void __launch_bounds__(256) pack_tall_kernel(const uint4* __restrict__ vals, const int* __restrict__ blk,
-                                                       const int* __restrict__ gsp, const uint4* __restrict__ steps,
-                                                       uint8_t* __restrict__ packed, const int* __restrict__ rowptr, int brow_begin,
-                                                       int n_groups) {
-    const int rfirst = __ldg(rowptr + brow_begin);
-    const int total = __ldg(gsp + n_groups);
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < total; i += warps) {
-        const uint4 d = __ldg(steps + i);
-        const int cnt = (int)d.z;
-        const int first = rfirst + (int)(d.y >> 1);
-        uint4* dst = reinterpret_cast<uint4*>(packed + (size_t)d.y * 256);
-        for (int q = 0; q < cnt; q++) {
-            const int src = __ldg(blk + first + q);
-            dst[q * 32 + (lane ^ ((lane >> 3) & 1))] = __ldg(vals + (size_t)src * 32 + lane);
-        }
-    }
-}
-
 }  // namespace
 
-int pack_values_async(const int* rowptr, const void* vals, const int* gsp, const void* steps, const int* blk, void* packed,
-                      size_t brow_begin, size_t brow_end, size_t rg, size_t nnzb, cudaStream_t stream,
-                      const DeviceCtx* ctx_in) {
+int pack_values_async(const int* rowptr, const void* vals, const int* blk, void* packed, size_t brow_begin, size_t brow_end, size_t nnzb,
+                      cudaStream_t stream, const DeviceCtx* ctx_in) {
     if (nnzb == 0 || brow_end == brow_begin) return SMAT_OK;
     const DeviceCtx* ctx = ctx_in;
     if (!ctx) {
@@ -449,10 +440,10 @@ int pack_values_async(const int* rowptr, const void* vals, const int* gsp, const
         if (int rc = get_device_ctx(&c)) return rc;
         ctx = c;
     }
-    const size_t n_groups = (brow_end - brow_begin + rg - 1) / rg;
-    pack_kernel<<<ctx->sm_count * 8, 256, 0, stream>>>(reinterpret_cast<const uint4*>(vals), blk, gsp,
-                                                       reinterpret_cast<const uint4*>(steps), reinterpret_cast<uint8_t*>(packed),
-                                                       rowptr, (int)brow_begin, (int)n_groups);
+    const size_t want = (nnzb + 31) / 32, most = (size_t)ctx->sm_count * 8;  // 32 blocks per CTA and trip
+    pack_kernel<<<(unsigned)(want < most ? want : most), 256, 0, stream>>>(reinterpret_cast<const uint4*>(vals), blk,
+                                                                          reinterpret_cast<uint4*>(packed), rowptr, (int)brow_begin,
+                                                                          (int)brow_end, (int)nnzb);
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
@@ -491,7 +482,7 @@ size_t choose_rows_per_group(size_t block_rows, size_t N, int sm_count, bool can
 PlanSizes plan_sizes(size_t nnzb, size_t brow_begin, size_t brow_end, size_t rg, size_t max_steps) {
     PlanSizes s;
     s.n_groups = (brow_end - brow_begin + rg - 1) / rg;
-    s.gsp_bytes = ((s.n_groups + 2) * sizeof(int) + 255) / 256 * 256;  // + the largest step count of a group
+    s.gsp_bytes = ((s.n_groups + 3) * sizeof(int) + 255) / 256 * 256;  // + the largest step count of a group and the MMA count
     // a step holds at least one block, so nnzb bounds the number of steps
     const size_t steps = max_steps ? max_steps : (nnzb ? nnzb : 1);
     s.steps_bytes = (steps * sizeof(uint4) + 255) / 256 * 256;
@@ -511,7 +502,7 @@ static int plan_launch_setup(const DeviceCtx* ctx_in, const DeviceCtx** ctx) {
 }
 
 int plan_count_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
-                     size_t rg, int* gsp, cudaStream_t stream, const DeviceCtx* ctx_in, size_t cap) {
+                     size_t rg, int* gsp, cudaStream_t stream, const DeviceCtx* ctx_in, size_t cap, int* units) {
     const DeviceCtx* ctx = nullptr;
     if (int rc = plan_launch_setup(ctx_in, &ctx)) return rc;
     const size_t n_groups = (brow_end - brow_begin + rg - 1) / rg;
@@ -525,7 +516,7 @@ int plan_count_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb
     SMAT_CUDA_TRY(cudaFuncSetAttribute(plan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
     plan_kernel<false><<<grid, kPlanThreads, smem_count, stream>>>(rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap,
                                                                   (int)(K / 16), (int)n_groups, gsp, nullptr, nullptr, (int)nnzb,
-                                                                  ctx->d_status);
+                                                                  ctx->d_status, units);
     count_launch();
     plan_scan_kernel<<<1, 1024, 0, stream>>>(gsp, (int)n_groups + 1);
     count_launch();
@@ -544,7 +535,7 @@ int plan_fill_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb,
     SMAT_CUDA_TRY(cudaFuncSetAttribute(plan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fill));
     plan_kernel<true><<<grid, kPlanThreads, smem_fill, stream>>>(rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap,
                                                                  (int)(K / 16), (int)n_groups, const_cast<int*>(gsp),
-                                                                 reinterpret_cast<uint4*>(steps), blk, (int)nnzb, ctx->d_status);
+                                                                 reinterpret_cast<uint4*>(steps), blk, (int)nnzb, ctx->d_status, nullptr);
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
@@ -596,21 +587,6 @@ int plan_fill_tall_async(const int* rowptr, const int* colidx, size_t K, size_t 
     return SMAT_OK;
 }
 
-int pack_values_tall_async(const int* rowptr, const void* vals, const int* gsp, const void* steps, const int* blk, void* packed,
-                           size_t brow_begin, size_t brow_end, size_t rg, size_t nnzb, cudaStream_t stream,
-                           const DeviceCtx* ctx_in) {
-    if (nnzb == 0 || brow_end == brow_begin) return SMAT_OK;
-    const DeviceCtx* ctx = nullptr;
-    if (int rc = plan_launch_setup(ctx_in, &ctx)) return rc;
-    const size_t n_groups = (brow_end - brow_begin + rg - 1) / rg;
-    pack_tall_kernel<<<ctx->sm_count * 8, 256, 0, stream>>>(reinterpret_cast<const uint4*>(vals), blk, gsp,
-                                                            reinterpret_cast<const uint4*>(steps), reinterpret_cast<uint8_t*>(packed),
-                                                            rowptr, (int)brow_begin, (int)n_groups);
-    count_launch();
-    SMAT_CUDA_TRY(cudaGetLastError());
-    return SMAT_OK;
-}
-
 }  // namespace smat
 
 using namespace smat;
@@ -623,6 +599,7 @@ struct smat_plan {
     StreamPlan stream;           // buffers of a stream plan
     void* sched_buffer = nullptr;  // listed schedule: offsets per CTA, then the groups
     int device = -1;
+    size_t nnzb = 0;  // blocks of the whole arrays, as given
     // smat_plan_spmm_host: device staging (B and C whole), the copy streams, per-chunk and per-range events
     void* host_B = nullptr;
     void* host_C = nullptr;
@@ -673,13 +650,21 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         return fail(SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
     }
     int* gsp = static_cast<int*>(p->gsp_buffer);
-    int rc = plan_count_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg, gsp, (cudaStream_t)stream);
-    int total_and_max[2] = {0, 0};
+    int* units = nnzb && sz.n_groups ? gsp + sz.n_groups + 2 : nullptr;  // behind the scanned counts and their maximum
+    int rc = SMAT_OK;
+    if (units) {
+        e = cudaMemsetAsync(units, 0, sizeof(int), (cudaStream_t)stream);
+        if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
+    }
+    if (rc == SMAT_OK)
+        rc = plan_count_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg, gsp, (cudaStream_t)stream, nullptr, kPlanBlocksPerStep, units);
+    int total_and_max[3] = {0, 0, 0};
     if (rc == SMAT_OK && sz.n_groups) {
-        e = cudaMemcpyAsync(total_and_max, gsp + sz.n_groups, 2 * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+        e = cudaMemcpyAsync(total_and_max, gsp + sz.n_groups, (units ? 3 : 2) * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
         if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
     }
+    const int mmas16 = total_and_max[2];
     // blocks of THIS range (nonzeroBlocks counts the whole arrays): what the choices below and at launch go by
     size_t range_blocks = nnzb;
     if (rc == SMAT_OK && nnzb) {
@@ -751,34 +736,44 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         }
     }
     // Tall plan: groups of up to 24 block-rows for the kernel that reads the B panels from tensor memory.  Its steps
-    // cost a little more than those of the 16-row kernels (measured ~550 against ~470 cycles, the latter growing with
-    // the blocks of the step: ~45 cycles each with the hand-overs, the shared-memory operand port), so it pays where taller groups mean
+    // cost a little more than those of the 16-row kernels (tall_step_cycles() against ~480 cycles, the latter growing with
+    // the MMAs of the step: ~58 cycles each with the hand-overs, the shared-memory operand port; vertical neighbours
+    // share one, which is what keeps dense clusters with this kernel), so it pays where taller groups mean
     // fewer steps: matrices whose quads mostly hold a block (a block-sparse layer, a reordered random matrix: three
     // quarters of the steps), not scattered ones (as many steps as before) and not dense clusters (steps of 32 blocks
     // already).  Both plans are counted and the estimates compared; smat_spmm_set_variant(4) forces a tall plan,
     // 1..3 exclude it.
+    const double mma_per_step = total_steps > 0 ? (double)mmas16 / (double)total_steps : 0.0;
+// cycles of a 16-row step: an MMA per block or pair of vertical neighbours, or, where whole columns of blocks are there
+    // (dense clusters), one per column
+    const bool vertical = mmas16 > 0 && (double)range_blocks >= 1.7 * (double)mmas16;
+    const double work16 = vertical ? 20.0 * (double)range_blocks / (double)(total_steps > 0 ? total_steps : 1) : 58.0 * mma_per_step;
+    const double step16 = work16 > 480.0 ? work16 : 480.0;
     bool tall = false;
     double est_cycles = 0.0;  // of the tcgen05 kernel that would be taken
     size_t rg_used = rg;
     const size_t rows = brow_end - brow_begin, tiles = ((N_hint ? N_hint : 128) + 127) / 128;
     const bool tall_forced = g_spmm_variant == 4;
+    const double kTallExtraCycles = 5000.0;  // of a launch: its pipeline takes longer to fill and to drain (measured, smallest plans)
     const bool tall_possible = rc == SMAT_OK && !balanced && !p->v.sched_list && total_steps > 0 && rows > 0 &&
-                               (tall_forced || (g_spmm_variant == 0 && cap == (size_t)kPlanBlocksPerStep && rows >= 16 && N_hint >= 128 &&
-                                                (size_t)total_steps * tiles >= 64 * (size_t)ctx->sm_count));
+                               (tall_forced || (g_spmm_variant == 0 && rows >= 12 && N_hint >= 16 &&
+                                                (size_t)total_steps * tiles >= 16 * (size_t)ctx->sm_count));
     if (tall_possible) {
-        // Height of the groups: what a launch costs is about (rounds of work items) x (steps of an item) x (bytes a
-        // step moves from L2: a 16 KB panel and its blocks).  The steps of an item hardly change with the height as
-        // long as most quads hold a block, so compare rounds x bytes per step.
+        // Height of the groups: what a launch costs is about (rounds of work items) x (steps of an item) x (cycles of
+        // a step, which grow with its blocks).  The quads of an item hardly change with the height as
+        // long as most hold a block, but those with more blocks than a step holds are cut into several steps: with the
+        // blocks of a quad spread like a binomial count, the share of them is taken from the logistic curve closest to it.
         size_t rg_tall = kTallRows;
         double best = 0.0;
-        const double steps_per_group = (double)total_steps / (double)sz.n_groups;
-        for (size_t r = kTallRows; r >= 16; r -= 2) {
+        const double quads = std::max(1.0, std::min((double)total_steps / (double)sz.n_groups, std::ceil((double)K / 64.0)));
+        for (size_t r = kTallRows; r >= 12; r -= 2) {
             const size_t groups = (rows + r - 1) / r;
-            // (blocks per step of a full group: the heaviest item sets the time of a round)
-            const double blocks_per_step =
-                (double)range_blocks / (double)rows * (double)(r < rows ? r : rows) / (steps_per_group > 1.0 ? steps_per_group : 1.0);
-            const double cost = rounds_for(groups * tiles, (size_t)ctx->sm_count, true, (size_t)steps_per_group, false) *
-                                (16384.0 + 512.0 * blocks_per_step);
+            const double per_quad = (double)range_blocks / (double)rows * (double)(r < rows ? r : rows) / quads;
+            double pieces = 1.0;
+            for (int k = 1; k <= 3; k++)
+                pieces += 1.0 / (1.0 + std::exp(((double)(k * kTallBlocksPerStep) + 0.5 - per_quad) / (0.5 * std::sqrt(per_quad) + 1e-9)));
+            const double steps = quads * pieces;
+            const double cost = tall_rounds(groups * tiles, (size_t)ctx->sm_count, steps) * steps * tall_step_cycles(per_quad / pieces);
             if (r == (size_t)kTallRows || cost < best * 0.97) {
                 best = cost;
                 rg_tall = r;
@@ -804,13 +799,14 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
             if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
         }
         if (rc == SMAT_OK) {
-            const double per_step = (double)range_blocks / (double)total_steps;
-            const double est16 = rounds_for(sz.n_groups * tiles, (size_t)ctx->sm_count, true, (size_t)steps_per_group, false) * steps_per_group *
-                                 (per_step * 45.0 > 470.0 ? per_step * 45.0 : 470.0);
+            const double steps_per_group = (double)total_steps / (double)sz.n_groups;
+            const double est16 = rounds_for(sz.n_groups * tiles, (size_t)ctx->sm_count, true, (size_t)steps_per_group, false) * steps_per_group * step16;
             const double steps_per_tall = (double)tall_total_and_max[0] / (double)sz_tall.n_groups;
             const double est_tall =
-                rounds_for(sz_tall.n_groups * tiles, (size_t)ctx->sm_count, true, (size_t)steps_per_tall, false) * steps_per_tall * 550.0;
-            tall = tall_forced || est_tall < 0.97 * est16;
+                tall_rounds(sz_tall.n_groups * tiles, (size_t)ctx->sm_count, steps_per_tall) * steps_per_tall *
+                    tall_step_cycles((double)range_blocks / (double)(tall_total_and_max[0] > 0 ? tall_total_and_max[0] : 1)) +
+                kTallExtraCycles;
+            tall = tall_forced || est_tall < est16;
             est_cycles = tall ? est_tall : est16;
             if (std::getenv("SMAT_PLAN_DEBUG"))
                 fprintf(stderr, "[smat plan] estimates: 16-row %.0f cycles, tall (rg %zu, %d steps) %.0f cycles -> %s\n", est16, rg_tall,
@@ -831,12 +827,12 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     }
     // Stream plan (spmm_stream_sm100.cu): taken where its estimate is below that of the kernel chosen so far.
     if (rc == SMAT_OK && total_steps > 0 && (g_spmm_variant == 5 || (g_spmm_variant == 0 && N_hint > 0))) {
-        const double us = stream_estimate_us(N_hint ? N_hint : 128, rows, range_blocks, K, ctx->sm_count);
+        const double us = stream_estimate_us(N_hint ? N_hint : 128, rows, range_blocks, K, ctx->sm_count, true);
         if (est_cycles == 0.0) {
-            const double per_group = (double)total_steps / (double)sz.n_groups, per_step = (double)range_blocks / (double)total_steps;
+            const double per_group = (double)total_steps / (double)sz.n_groups;
             const double rounds = balanced || p->v.sched_list ? (double)(sz.n_groups * tiles) / (double)ctx->sm_count
                                                               : rounds_for(sz.n_groups * tiles, (size_t)ctx->sm_count, true, (size_t)per_group, false);
-            est_cycles = rounds * per_group * (per_step * 45.0 > 470.0 ? per_step * 45.0 : 470.0);
+            est_cycles = rounds * per_group * step16;
         }
         const double other = 8.0 + est_cycles / 1850.0;
         const bool take = g_spmm_variant == 5 || us < other;
@@ -893,6 +889,7 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         return rc;
     }
     char* b = static_cast<char*>(p->buffer);
+    p->nnzb = nnzb;
     p->v.rowptr = bcsrRowPtrA;
     p->v.gsp = gsp;
     p->v.steps = b;
@@ -908,6 +905,7 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     p->v.total_steps = (size_t)(steps_final > 0 ? steps_final : 0);
     p->v.balanced = balanced;
     p->v.cap = cap;
+    p->v.vertical = vertical;
     p->v.tall = tall;
     if (tall) {
         // behind the step records, in the same region: the per-step words (only read while the plan is built), then the per-pair lists
@@ -915,16 +913,12 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         p->v.winfo = wstep + (size_t)(steps_final > 0 ? steps_final : 1) * 64;
         rc = plan_fill_tall_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg_used, gsp, const_cast<void*>(p->v.steps), wstep,
                                   const_cast<void*>(p->v.winfo), const_cast<int*>(p->v.blk), (cudaStream_t)stream);
-        if (rc == SMAT_OK)
-            rc = pack_values_tall_async(bcsrRowPtrA, bcsrValuesA, gsp, p->v.steps, p->v.blk, const_cast<void*>(p->v.packed),
-                                        brow_begin, brow_end, rg_used, nnzb, (cudaStream_t)stream);
     } else {
         rc = plan_fill_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg, gsp, const_cast<void*>(p->v.steps),
                              const_cast<int*>(p->v.blk), (cudaStream_t)stream, nullptr, cap);
-        if (rc == SMAT_OK)
-            rc = pack_values_async(bcsrRowPtrA, bcsrValuesA, gsp, p->v.steps, p->v.blk, const_cast<void*>(p->v.packed), brow_begin,
-                                   brow_end, rg, nnzb, (cudaStream_t)stream);
     }
+    if (rc == SMAT_OK)
+        rc = pack_values_async(bcsrRowPtrA, bcsrValuesA, p->v.blk, const_cast<void*>(p->v.packed), brow_begin, brow_end, nnzb, (cudaStream_t)stream);
     if (rc) {
         cudaFree(p->buffer);
         cudaFree(p->gsp_buffer);
@@ -947,13 +941,9 @@ int smat_plan_set_values(smat_plan* plan, const void* bcsrValuesA, void* stream)
         if (int rc = get_device_ctx(&ctx)) return rc;
         return stream_plan_values(plan->v, bcsrValuesA, nullptr, ctx->sm_count, (cudaStream_t)stream);
     }
-    if (plan->v.tall)
-        return pack_values_tall_async(plan->v.rowptr, bcsrValuesA, plan->v.gsp, plan->v.steps, plan->v.blk,
-                                      const_cast<void*>(plan->v.packed), plan->v.brow_begin, plan->v.brow_end, plan->v.rg,
-                                      plan->v.nnzb, (cudaStream_t)stream);
-    return pack_values_async(plan->v.rowptr, bcsrValuesA, plan->v.gsp, plan->v.steps, plan->v.blk,
-                             const_cast<void*>(plan->v.packed), plan->v.brow_begin, plan->v.brow_end, plan->v.rg,
-                             plan->v.nnzb, (cudaStream_t)stream);
+    // (the row pointers were checked against the whole arrays' block count, which only bounds what the kernel may read)
+    return pack_values_async(plan->v.rowptr, bcsrValuesA, plan->v.blk, const_cast<void*>(plan->v.packed), plan->v.brow_begin,
+                             plan->v.brow_end, plan->nnzb, (cudaStream_t)stream);
 }
 
 int smat_plan_spmm(const smat_plan* plan, const void* B, void* C, size_t N, void* stream) {

@@ -75,6 +75,15 @@ inline double rounds_for(size_t items, size_t sms, bool can_cut, size_t est_step
     const size_t P = tail_parts_for(items, sms, can_cut, est_steps);
     return (double)(items / sms) + 1.0 / (double)P + (P > 1 ? (wide ? 0.08 : 0.35) : 0.0);
 }
+// The same for the tall kernel, whose items are longer: a cut costs about forty steps (12 us: the partial
+// tiles of 196 KB, their summation, another filling of the pipeline) whatever the item's length.
+inline double tall_rounds(size_t items, size_t sms, double est_steps) {
+    if (items % sms == 0) return (double)(items / sms);
+    const size_t P = tail_parts_for(items, sms, true, (size_t)est_steps);
+    return (double)(items / sms) + 1.0 / (double)P + (P > 1 ? 40.0 / est_steps : 0.0);
+}
+// Cycles of a step of the tall kernel that holds `blocks` blocks (measured with 12 to 20 blocks a step: 544 to 640).
+inline double tall_step_cycles(double blocks) { return 350.0 + 15.0 * blocks > 500.0 ? 350.0 + 15.0 * blocks : 500.0; }
 // Measured cost of a 256-column item relative to a 128-column item of the same group.
 constexpr double kWideItemCost = 1.95;
 // Group height for a range of `block_rows` block-rows when C is N columns wide (0 = unknown): the height in
@@ -123,6 +132,7 @@ struct PlanView {
     size_t K = 0, nnzb = 0, brow_begin = 0, brow_end = 0, n_groups = 0, rg = kPlanRowsPerGroup;
     size_t total_steps = 0;  // number of steps of the range when the host knows it, else 0
     size_t cap = kPlanBlocksPerStep;  // most blocks of a step: kPlanBlocksPerStep or kPlanBlocksPerStepDense
+    bool vertical = false;  // most blocks have a neighbour above or below in their block-column (dense clusters)
     // Tall plan: groups of rg <= kTallRows block-rows with an even number of steps, at most kTallBlocksPerStep blocks
     // per step.  A step record is {element column of the quad, position of the first block in the packed stream in
     // 256-byte units, number of blocks (0: a step that only pads its group), non-empty sub-columns (bit s)}; winfo
@@ -153,25 +163,21 @@ PlanSizes plan_sizes(size_t nnzb, size_t brow_begin, size_t brow_end, size_t rg,
 // `ctx` (here and below): per-device state to use; nullptr = the lazily created one of get_device_ctx.
 // Phase 1 fills gsp (step counts, scanned); phase 2 fills steps and blk.
 int plan_count_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
-                     size_t rg, int* gsp, cudaStream_t stream, const DeviceCtx* ctx = nullptr, size_t cap = kPlanBlocksPerStep);
+                     size_t rg, int* gsp, cudaStream_t stream, const DeviceCtx* ctx = nullptr, size_t cap = kPlanBlocksPerStep,
+                     int* units = nullptr);  // units (zeroed before, or null): += MMAs the 16-row kernel needs per 128 columns
 int plan_fill_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
                     size_t rg, const int* gsp, void* steps, int* blk, cudaStream_t stream, const DeviceCtx* ctx = nullptr,
                     size_t cap = kPlanBlocksPerStep);
 // Copies the value blocks of block-rows [brow_begin, brow_end) into their places in the packed stream.
-int pack_values_async(const int* rowptr, const void* vals, const int* gsp, const void* steps, const int* blk, void* packed,
-                      size_t brow_begin, size_t brow_end, size_t rg, size_t nnzb, cudaStream_t stream,
-                      const DeviceCtx* ctx = nullptr);
+int pack_values_async(const int* rowptr, const void* vals, const int* blk, void* packed, size_t brow_begin, size_t brow_end, size_t nnzb,
+                      cudaStream_t stream, const DeviceCtx* ctx = nullptr);
 
-// The same three phases for a tall plan.
+// The first two phases for a tall plan.
 int plan_count_tall_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
                           size_t rg, int* gsp, cudaStream_t stream, const DeviceCtx* ctx = nullptr);
 int plan_fill_tall_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
                          size_t rg, const int* gsp, void* steps, void* wstep, void* winfo, int* blk, cudaStream_t stream,
                          const DeviceCtx* ctx = nullptr);
-int pack_values_tall_async(const int* rowptr, const void* vals, const int* gsp, const void* steps, const int* blk, void* packed,
-                           size_t brow_begin, size_t brow_end, size_t rg, size_t nnzb, cudaStream_t stream,
-                           const DeviceCtx* ctx = nullptr);
-
 // Launch of the SpMM kernel (spmm_sm100.cu).  `ldc`: elements between rows of C (0 = N, i.e. C is exactly N wide).
 // [group_begin, group_end): the groups of the plan to multiply (default: all); C points at the first row of
 // group_begin.

@@ -38,7 +38,7 @@ namespace {
 constexpr size_t kMaxBlocks = 32768;          // SMAT_STATIC_MAX_BLOCKS
 constexpr size_t kMaxRows = 1048576;          // SMAT_STATIC_MAX_ROWS
 constexpr size_t kMaxGroups = kMaxRows / 16 / 4;  // the smallest group height (SMAT_ROWS_PER_GROUP override) is 4 block-rows
-constexpr size_t kGspBytes = ((kMaxGroups + 2) * sizeof(int) + 255) / 256 * 256;  // prefix of step counts + the largest count
+constexpr size_t kGspBytes = ((kMaxGroups + 3) * sizeof(int) + 255) / 256 * 256;  // prefix of step counts + the largest count
 constexpr size_t kStepsBytes = kMaxBlocks * 16;   // a group never has more steps than blocks
 constexpr size_t kBlkBytes = kMaxBlocks * sizeof(int);
 constexpr size_t kPackedBytes = kMaxBlocks * 512;  // the blocks in walk order
@@ -146,6 +146,6 @@ extern "C" int smat_spmm_bcsr_f16_static(const void* vals, const int* rowptr, co
     v.packed = packed;
     if (int rc = plan_count_async(rowptr, colidx, K, nnzb, 0, Mb, rg, gsp, stream, &d->ctx)) return rc;
     if (int rc = plan_fill_async(rowptr, colidx, K, nnzb, 0, Mb, rg, gsp, steps, blk, stream, &d->ctx)) return rc;
-    if (int rc = pack_values_async(rowptr, vals, gsp, steps, blk, packed, 0, Mb, rg, nnzb, stream, &d->ctx)) return rc;
+    if (int rc = pack_values_async(rowptr, vals, blk, packed, 0, Mb, nnzb, stream, &d->ctx)) return rc;
     return launch_spmm(v, B, C, N, stream, &d->ctx);
 }

@@ -35,7 +35,7 @@ struct StreamShape {
 };
 StreamShape stream_shape(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count, bool plan);
 bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count);
-double stream_estimate_us(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count);
+double stream_estimate_us(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count, bool plan);
 
 // What a plan for this kernel owns (PlanView::stream): the values in fragment order, the block-columns, the pieces.
 struct StreamPlan {
