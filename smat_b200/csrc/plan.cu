@@ -609,6 +609,31 @@ struct smat_plan {
     std::vector<cudaEvent_t> ev_in, ev_done, ev_out;
 };
 
+// One chunk of columns of C, rows x `width16` 16-byte words, from device memory to pinned host memory that the device can
+// address, both `pitch16` words from row to row.  A 2-D copy of the copy engine moves rows of 512 bytes at 8 GB/s
+// (measured; 50 GB/s in one piece), stores from the SMs at the rate of the link.
+static __global__ void __launch_bounds__(256) copy_out_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t rows, size_t pitch16,
+                                                             unsigned width16) {
+    const size_t n = rows * width16, stride = (size_t)gridDim.x * 256;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += stride) {
+        const size_t row = i / width16, at = row * pitch16 + (i - row * width16);
+        dst[at] = __ldg(src + at);
+    }
+}
+
+// The device's address of `bytes` of host memory, or null when it is not pinned (then only the copy engine can reach it).
+static char* device_view_of_host(void* p, size_t bytes) {
+    cudaPointerAttributes first, last;
+    if (((uintptr_t)p & 15) || cudaPointerGetAttributes(&first, p) != cudaSuccess ||
+        cudaPointerGetAttributes(&last, static_cast<char*>(p) + bytes - 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer || !last.devicePointer) return nullptr;
+    if (static_cast<char*>(last.devicePointer) - static_cast<char*>(first.devicePointer) != (ptrdiff_t)(bytes - 1)) return nullptr;
+    return static_cast<char*>(first.devicePointer);
+}
+
 // A plan's memory and tuning belong to the device it was created on.
 static int check_plan_device(const smat_plan* plan) {
     int dev = -1;
@@ -641,11 +666,8 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     PlanSizes sz = plan_sizes(nnzb, brow_begin, brow_end, rg);
     cudaError_t e = cudaGetDevice(&p->device);
     if (e == cudaSuccess) e = cudaMalloc(&p->gsp_buffer, sz.gsp_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&p->fix_buffer, fix_scratch_bytes(ctx->sm_count));
     if (e != cudaSuccess) {
         cudaFree(p->gsp_buffer);
-        cudaFree(p->fix_buffer);
-        cudaFree(p->sched_buffer);
         delete p;
         return fail(SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
     }
@@ -658,23 +680,20 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     }
     if (rc == SMAT_OK)
         rc = plan_count_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg, gsp, (cudaStream_t)stream, nullptr, kPlanBlocksPerStep, units);
-    int total_and_max[3] = {0, 0, 0};
+    // ... and the blocks of THIS range (nonzeroBlocks counts the whole arrays): what the choices below and at launch go by
+    int total_and_max[3] = {0, 0, 0}, ends[2] = {0, 0};
     if (rc == SMAT_OK && sz.n_groups) {
         e = cudaMemcpyAsync(total_and_max, gsp + sz.n_groups, (units ? 3 : 2) * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+        if (e == cudaSuccess && nnzb)
+            e = cudaMemcpyAsync(&ends[0], bcsrRowPtrA + brow_begin, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+        if (e == cudaSuccess && nnzb)
+            e = cudaMemcpyAsync(&ends[1], bcsrRowPtrA + brow_end, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
         if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
     }
     const int mmas16 = total_and_max[2];
-    // blocks of THIS range (nonzeroBlocks counts the whole arrays): what the choices below and at launch go by
     size_t range_blocks = nnzb;
-    if (rc == SMAT_OK && nnzb) {
-        int ends[2] = {0, 0};
-        e = cudaMemcpyAsync(&ends[0], bcsrRowPtrA + brow_begin, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&ends[1], bcsrRowPtrA + brow_end, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
-        if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
-        else if (ends[1] >= ends[0] && (size_t)(ends[1] - ends[0]) <= nnzb) range_blocks = (size_t)(ends[1] - ends[0]);
-    }
+    if (rc == SMAT_OK && nnzb && sz.n_groups && ends[1] >= ends[0] && (size_t)(ends[1] - ends[0]) <= nnzb) range_blocks = (size_t)(ends[1] - ends[0]);
     // Densely filled quads (dense clusters: every quad of a cluster holds all 64 blocks) are cut into pieces of at most 24
     // blocks that each fetch the B panel again; when the steps are that full on average, recount with 32 per step.
     size_t cap = kPlanBlocksPerStep;
@@ -850,9 +869,8 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
                 rc = stream_plan_build(p->stream, p->v, h_rowptr.data(), bcsrValuesA, bcsrColIdxA, N_hint ? N_hint : 128, ctx->sm_count,
                                        (cudaStream_t)stream);
                 cudaFree(p->gsp_buffer);
-                cudaFree(p->fix_buffer);
                 cudaFree(p->sched_buffer);
-                p->gsp_buffer = p->fix_buffer = p->sched_buffer = nullptr;
+                p->gsp_buffer = p->sched_buffer = nullptr;
                 p->v.sched_list = p->v.sched_off = nullptr;
                 p->v.total_steps = p->stream.row_piece.empty() ? 0 : (size_t)p->stream.row_piece.back();
                 if (rc) {
@@ -870,10 +888,8 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         fprintf(stderr, "[smat plan] rows %zu blocks %zu: 16-row plan rg %zu steps %d cap %zu balanced %d listed %d; tall %d rg %zu steps %d max/group %d\n",
                 brow_end - brow_begin, range_blocks, rg, total_steps, cap, (int)balanced, p->v.sched_list != nullptr, (int)tall, rg_used,
                 steps_final, total_and_max[1]);
-    if (rc == SMAT_OK && balanced) {  // two partial tiles per CTA
-        cudaFree(p->fix_buffer);
-        p->fix_buffer = nullptr;
-        e = cudaMalloc(&p->fix_buffer, 2 * fix_scratch_bytes(ctx->sm_count));
+    if (rc == SMAT_OK) {  // a partial tile per CTA, two for the balanced schedule
+        e = cudaMalloc(&p->fix_buffer, (balanced ? 2 : 1) * fix_scratch_bytes(ctx->sm_count));
         if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
     }
     if (rc == SMAT_OK) {
@@ -968,12 +984,21 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
     if (!B_host || !C_host) return fail(SMAT_ERR_BAD_ARG, "B_host or C_host is NULL");
     if (int rc = check_plan_device(plan)) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    // B comes in by column chunks as wide as the kernel's widest work item (rows of the [N][K] array: contiguous);
-    // every chunk but the last is multiplied for all block-rows as soon as it has arrived; the last chunk is
-    // multiplied group range by group range, and the rows of C that it completes go out at once (rows of the
-    // row-major C: contiguous), under the multiplication of the next range.
+    // B comes in by column chunks (rows of the [N][K] array: contiguous), each multiplied for all block-rows as soon as it has
+    // arrived.  Where the device can address C_host, the columns of C that a chunk completes go out at once, under the
+    // arrival of the next chunks; what is left after the last arrival is one chunk's product and its columns, so the
+    // last chunks are half as wide.  Else C has to go out in whole rows: the last chunk is multiplied group range by
+    // group range, and the rows that it completes go out under the multiplication of the next range.
+    char* const out_view = device_view_of_host(C_host, rows * N * 2);
     const size_t W = N >= 512 ? 256 : (N > 128 ? 128 : N);
-    const size_t n_chunks = (N + W - 1) / W;
+    std::vector<size_t> chunk_at;  // first column of every chunk, then N
+    for (size_t n0 = 0; n0 < N; n0 += W) {
+        chunk_at.push_back(n0);
+        const size_t w = N - n0 < W ? N - n0 : W;
+        if (out_view && n0 + W >= N && w >= 64) chunk_at.push_back(n0 + (w / 2 + 7) / 8 * 8);
+    }
+    chunk_at.push_back(N);
+    const size_t n_chunks = chunk_at.size() - 1;
     const size_t n_groups = plan->v.n_groups;
     // ranges of the last chunk: each should still fill the SMs for about one round of work items (shorter launches
     // lose more to partly filled rounds than the overlap of the copy-out wins back); at most 4
@@ -983,6 +1008,7 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
     if (plan->v.stream) n_ranges = n_groups / 16 * ((W + 127) / 128) / (size_t)ctx->sm_count;
     if (plan->v.sched_list || plan->v.balanced) n_ranges = 1;  // such plans balance a launch over all their groups
     if (const char* e = std::getenv("SMAT_HOST_RANGES")) n_ranges = (size_t)std::atoi(e);  // tuning knob
+    if (out_view) n_ranges = 1;
     if (n_ranges > 4) n_ranges = 4;
     if (n_ranges > n_groups) n_ranges = n_groups;
     if (n_ranges < 1) n_ranges = 1;
@@ -1010,7 +1036,7 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
         SMAT_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         plan->ev_in.push_back(e);
     }
-    while (plan->ev_done.size() < n_ranges) {
+    while (plan->ev_done.size() < (out_view ? n_chunks : n_ranges)) {
         cudaEvent_t a = nullptr, b = nullptr;
         SMAT_CUDA_TRY(cudaEventCreateWithFlags(&a, cudaEventDisableTiming));
         plan->ev_done.push_back(a);
@@ -1026,13 +1052,25 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
     char* Bd = static_cast<char*>(plan->host_B);
     char* Cd = static_cast<char*>(plan->host_C);
     for (size_t j = 0; j < n_chunks; j++) {
-        const size_t n0 = j * W, w = (N - n0 < W) ? N - n0 : W;
+        const size_t n0 = chunk_at[j], w = chunk_at[j + 1] - n0;
         SMAT_CUDA_TRY(cudaMemcpyAsync(Bd + n0 * K * 2, Bh + n0 * K * 2, w * K * 2, cudaMemcpyHostToDevice, plan->s_in));
         SMAT_CUDA_TRY(cudaEventRecord(plan->ev_in[j], plan->s_in));
     }
     for (size_t j = 0; j < n_chunks; j++) {
-        const size_t n0 = j * W, w = (N - n0 < W) ? N - n0 : W;
+        const size_t n0 = chunk_at[j], w = chunk_at[j + 1] - n0;
         SMAT_CUDA_TRY(cudaStreamWaitEvent(s, plan->ev_in[j], 0));
+        if (out_view) {
+            if (int rc = launch_spmm(plan->v, Bd + n0 * K * 2, Cd + n0 * 2, w, s, nullptr, N)) return rc;
+            SMAT_CUDA_TRY(cudaEventRecord(plan->ev_done[j], s));
+            SMAT_CUDA_TRY(cudaStreamWaitEvent(plan->s_out, plan->ev_done[j], 0));
+            const size_t words = rows * w / 8, ctas = (words + 1023) / 1024;
+            copy_out_kernel<<<(unsigned)(ctas < 64 ? ctas : 64), 256, 0, plan->s_out>>>(
+                reinterpret_cast<const uint4*>(Cd + n0 * 2), reinterpret_cast<uint4*>(out_view + n0 * 2), rows, N / 8, (unsigned)(w / 8));
+            count_launch();
+            SMAT_CUDA_TRY(cudaGetLastError());
+            if (j + 1 == n_chunks) SMAT_CUDA_TRY(cudaEventRecord(plan->ev_out[0], plan->s_out));
+            continue;
+        }
         if (j + 1 < n_chunks) {
             if (int rc = launch_spmm(plan->v, Bd + n0 * K * 2, Cd + n0 * 2, w, s, nullptr, N)) return rc;
             continue;
@@ -1050,7 +1088,7 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
         }
     }
     // the caller's stream ends after the last copy out, so that ordering on it covers the whole call
-    SMAT_CUDA_TRY(cudaStreamWaitEvent(s, plan->ev_out[n_ranges - 1], 0));
+    SMAT_CUDA_TRY(cudaStreamWaitEvent(s, plan->ev_out[out_view ? 0 : n_ranges - 1], 0));
     return SMAT_OK;
 }
 
