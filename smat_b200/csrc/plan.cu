@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
+#include <type_traits>
 #include <utility>
 #include <queue>
 #include <algorithm>
@@ -34,16 +35,19 @@ namespace {
 
 constexpr int RG = kPlanRowsPerGroup;
 constexpr int kPlanThreads = RG * 32;
-constexpr int kWindow = 16384;  // block-columns per pass: 64 KB of masks + 64 KB of block prefixes
+// Block-columns per pass, a template parameter WIN: 16384 (64 KB of masks + 64 KB of block prefixes), or as few as the matrix
+// has.  Masks are cleared and scanned for the whole window, so a window of 16384 for a matrix of 1024 block-columns left the
+// scan to 32 of the 512 threads, each with eight quads one after the other.
+constexpr int kWindow = 16384;
 
-// Fills masks[0..kWindow) for block-columns [w0, w0 + kWindow) of the group; cursor[] (one per warp,
+// Fills masks[0..WIN) for block-columns [w0, w0 + WIN) of the group; cursor[] (one per warp,
 // kept by lane 0 semantics via registers) walks each row once over all windows.
 // A block column below the window start (columns not ascending, or negative) or beyond the matrix is not marked; the
 // status word then tells the host that the structure is inconsistent.
-template <int THREADS = kPlanThreads>
+template <int THREADS, int WIN>
 __device__ __forceinline__ void mark_window(const int* __restrict__ colidx, int& cur, int end, int w0, int Kb, uint32_t* masks,
                                             int warp, int lane, int* status) {
-    for (int i = threadIdx.x; i < kWindow; i += THREADS) masks[i] = 0u;
+    for (int i = threadIdx.x; i < WIN; i += THREADS) masks[i] = 0u;
     __syncthreads();
     // every lane keeps the same `cur`; lanes stride over the row until the window ends
     for (;;) {
@@ -53,7 +57,7 @@ __device__ __forceinline__ void mark_window(const int* __restrict__ colidx, int&
             if (status) atomicCAS(status, 0, kStatusBadColumns);
             cb = w0 - 1;
         }
-        const bool in = cb < w0 + kWindow;
+        const bool in = cb < w0 + WIN;
         if (in && cb >= w0) atomicOr(&masks[cb - w0], 1u << warp);
         else if (in && status) atomicCAS(status, 0, kStatusBadColumns);
         const uint32_t b = __ballot_sync(0xffffffffu, in);
@@ -98,13 +102,13 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* total, int* sh) 
     return before + inc - v;
 }
 
-template <bool FILL>
+template <bool FILL, int WIN>
 __global__ void __launch_bounds__(kPlanThreads)
 plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int brow_begin, int brow_end, int rg, int CAP, int Kb,
             int n_groups, int* __restrict__ gsp, uint4* __restrict__ steps, int* __restrict__ blk, int nnzb, int* status, int* units) {
     extern __shared__ uint32_t sm[];
-    uint32_t* masks = sm;                                 // [kWindow] row mask per block-column
-    int* blk_pre = reinterpret_cast<int*>(sm + kWindow);  // [kWindow] exclusive block number (FILL only)
+    uint32_t* masks = sm;                                 // [WIN] row mask per block-column
+    int* blk_pre = reinterpret_cast<int*>(sm + WIN);  // [WIN] exclusive block number (FILL only)
     __shared__ int scan_sh[64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // The buffers of the plan are sized from the caller's block count: a range of row pointers that is not monotone or
@@ -127,11 +131,11 @@ plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int 
         int cur = beg;
         int steps_done = 0, blocks_done = 0;
         const int gs = FILL ? __ldg(gsp + g) : 0;
-        for (int w0 = 0; w0 < Kb; w0 += kWindow) {
+        for (int w0 = 0; w0 < Kb; w0 += WIN) {
             const int cur_before = cur;
-            mark_window(colidx, cur, end, w0, Kb, masks, warp, lane, status);
+            mark_window<kPlanThreads, WIN>(colidx, cur, end, w0, Kb, masks, warp, lane, status);
             // per-thread chunk of the window: PER consecutive block-columns = PER / 4 quads
-            constexpr int PER = kWindow / kPlanThreads;
+            constexpr int PER = WIN / kPlanThreads;
             static_assert(PER % 4 == 0, "a thread owns whole quads");
             const int i0 = threadIdx.x * PER;
             int ns = 0, nb = 0;
@@ -181,7 +185,7 @@ plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int 
                 for (int j = cur_before + lane; j < cur; j += 32) {
                     const int cbx = __ldg(colidx + j) >> 4;
                     const int cb = cbx - w0;
-                    if (cb < 0 || cb >= kWindow || cbx >= Kb) continue;  // not marked above (status set there)
+                    if (cb < 0 || cb >= WIN || cbx >= Kb) continue;  // not marked above (status set there)
                     blk[gfirst + blk_pre[cb] + __popc(masks[cb] & ((1u << warp) - 1u))] = j;
                 }
                 blocks_done += tot_b;
@@ -268,14 +272,14 @@ __global__ void __launch_bounds__(256) pack_kernel(const uint4* __restrict__ val
 constexpr int kTallPlanThreads = 1024;  // warp w owns block-row w of the group
 static_assert(kTallRows == 24 && kTallBlocksPerStep <= 32, "the per-warp step words below are laid out for 12 warps of two rows and 5-bit block positions");
 
-template <bool FILL>
+template <bool FILL, int WIN>
 __global__ void __launch_bounds__(kTallPlanThreads)
 plan_tall_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int brow_begin, int brow_end, int rg, int CAP, int Kb,
                  int n_groups, int* __restrict__ gsp, uint4* __restrict__ steps, uint4* __restrict__ winfo, int* __restrict__ blk,
                  int nnzb, int* status) {
     extern __shared__ uint32_t sm[];
-    uint32_t* masks = sm;                                 // [kWindow] row mask per block-column
-    int* blk_pre = reinterpret_cast<int*>(sm + kWindow);  // [kWindow] exclusive block number (FILL only)
+    uint32_t* masks = sm;                                 // [WIN] row mask per block-column
+    int* blk_pre = reinterpret_cast<int*>(sm + WIN);  // [WIN] exclusive block number (FILL only)
     __shared__ int scan_sh[64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // The buffers of the plan are sized from the caller's block count: a range of row pointers that is not monotone or
@@ -298,10 +302,10 @@ plan_tall_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx,
         int cur = beg;
         int steps_done = 0, blocks_done = 0;
         const int gs = FILL ? __ldg(gsp + g) : 0;
-        for (int w0 = 0; w0 < Kb; w0 += kWindow) {
+        for (int w0 = 0; w0 < Kb; w0 += WIN) {
             const int cur_before = cur;
-            mark_window<kTallPlanThreads>(colidx, cur, end, w0, Kb, masks, warp, lane, status);
-            constexpr int PER = kWindow / kTallPlanThreads;
+            mark_window<kTallPlanThreads, WIN>(colidx, cur, end, w0, Kb, masks, warp, lane, status);
+            constexpr int PER = WIN / kTallPlanThreads;
             static_assert(PER % 4 == 0, "a thread owns whole quads");
             const int i0 = threadIdx.x * PER;
             int ns = 0, nb = 0;
@@ -375,7 +379,7 @@ plan_tall_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx,
                 for (int j = cur_before + lane; j < cur; j += 32) {
                     const int cbx = __ldg(colidx + j) >> 4;
                     const int cb = cbx - w0;
-                    if (cb < 0 || cb >= kWindow || cbx >= Kb) continue;  // not marked above (status set there)
+                    if (cb < 0 || cb >= WIN || cbx >= Kb) continue;  // not marked above (status set there)
                     blk[gfirst + blk_pre[cb] + __popc(masks[cb] & ((1u << warp) - 1u))] = j;
                 }
                 blocks_done += tot_b;
@@ -491,6 +495,19 @@ PlanSizes plan_sizes(size_t nnzb, size_t brow_begin, size_t brow_end, size_t rg,
     return s;
 }
 
+// Launches a plan kernel with the smallest window that holds the matrix, with as many CTAs as fit the SMs.
+template <int THREADS, class Launch>
+static int launch_windowed(size_t Kb, size_t n_groups, int words_per_column, int sm_count, Launch&& launch) {
+    auto go = [&](auto win) -> int {
+        const size_t smem = (size_t)decltype(win)::value * 4 * (size_t)words_per_column;
+        const size_t resident = std::max<size_t>(1, std::min<size_t>(2048 / THREADS, (200 * 1024) / (smem + 1024)));
+        return launch(win, (int)std::min(n_groups, (size_t)sm_count * resident), smem);
+    };
+    if (Kb <= THREADS * 4) return go(std::integral_constant<int, THREADS * 4>{});
+    if (THREADS * 8 < kWindow && Kb <= THREADS * 8) return go(std::integral_constant<int, THREADS * 8>{});
+    return go(std::integral_constant<int, kWindow>{});
+}
+
 static int plan_launch_setup(const DeviceCtx* ctx_in, const DeviceCtx** ctx) {
     *ctx = ctx_in;
     if (!*ctx) {
@@ -511,12 +528,15 @@ int plan_count_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb
         SMAT_CUDA_TRY(cudaMemsetAsync(gsp, 0, (n_groups + 1) * sizeof(int), stream));
         return SMAT_OK;
     }
-    const int grid = (int)(n_groups < (size_t)ctx->sm_count ? n_groups : (size_t)ctx->sm_count);
-    const size_t smem_count = (size_t)kWindow * 4;
-    SMAT_CUDA_TRY(cudaFuncSetAttribute(plan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
-    plan_kernel<false><<<grid, kPlanThreads, smem_count, stream>>>(rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap,
-                                                                  (int)(K / 16), (int)n_groups, gsp, nullptr, nullptr, (int)nnzb,
-                                                                  ctx->d_status, units);
+    const int rc = launch_windowed<kPlanThreads>(K / 16, n_groups, 1, ctx->sm_count, [&](auto win, int grid, size_t smem) -> int {
+        auto kernel = plan_kernel<false, decltype(win)::value>;
+        SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<grid, kPlanThreads, smem, stream>>>(
+            rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap, (int)(K / 16),
+            (int)n_groups, gsp, nullptr, nullptr, (int)nnzb, ctx->d_status, units);
+        return SMAT_OK;
+    });
+    if (rc) return rc;
     count_launch();
     plan_scan_kernel<<<1, 1024, 0, stream>>>(gsp, (int)n_groups + 1);
     count_launch();
@@ -530,12 +550,16 @@ int plan_fill_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb,
     if (int rc = plan_launch_setup(ctx_in, &ctx)) return rc;
     const size_t n_groups = (brow_end - brow_begin + rg - 1) / rg;
     if (n_groups == 0 || nnzb == 0) return SMAT_OK;
-    const int grid = (int)(n_groups < (size_t)ctx->sm_count ? n_groups : (size_t)ctx->sm_count);
-    const size_t smem_fill = (size_t)kWindow * 8;
-    SMAT_CUDA_TRY(cudaFuncSetAttribute(plan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fill));
-    plan_kernel<true><<<grid, kPlanThreads, smem_fill, stream>>>(rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap,
-                                                                 (int)(K / 16), (int)n_groups, const_cast<int*>(gsp),
-                                                                 reinterpret_cast<uint4*>(steps), blk, (int)nnzb, ctx->d_status, nullptr);
+    const int rc = launch_windowed<kPlanThreads>(K / 16, n_groups, 2, ctx->sm_count, [&](auto win, int grid, size_t smem) -> int {
+        auto kernel = plan_kernel<true, decltype(win)::value>;
+        SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<grid, kPlanThreads, smem, stream>>>(
+            rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap, (int)(K / 16),
+            (int)n_groups, const_cast<int*>(gsp), reinterpret_cast<uint4*>(steps), blk, (int)nnzb,
+            ctx->d_status, nullptr);
+        return SMAT_OK;
+    });
+    if (rc) return rc;
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
@@ -552,12 +576,16 @@ int plan_count_tall_async(const int* rowptr, const int* colidx, size_t K, size_t
         SMAT_CUDA_TRY(cudaMemsetAsync(gsp, 0, (n_groups + 1) * sizeof(int), stream));
         return SMAT_OK;
     }
-    const int grid = (int)(n_groups < (size_t)ctx->sm_count ? n_groups : (size_t)ctx->sm_count);
-    const size_t smem_count = (size_t)kWindow * 4;
-    SMAT_CUDA_TRY(cudaFuncSetAttribute(plan_tall_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
-    plan_tall_kernel<false><<<grid, kTallPlanThreads, smem_count, stream>>>(rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg,
-                                                                           kTallBlocksPerStep, (int)(K / 16), (int)n_groups, gsp, nullptr,
-                                                                           nullptr, nullptr, (int)nnzb, ctx->d_status);
+    const int rc = launch_windowed<kTallPlanThreads>(K / 16, n_groups, 1, ctx->sm_count, [&](auto win, int grid, size_t smem) -> int {
+        auto kernel = plan_tall_kernel<false, decltype(win)::value>;
+        SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<grid, kTallPlanThreads, smem, stream>>>(
+            rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, kTallBlocksPerStep,
+            (int)(K / 16), (int)n_groups, gsp, nullptr, nullptr, nullptr, (int)nnzb,
+            ctx->d_status);
+        return SMAT_OK;
+    });
+    if (rc) return rc;
     count_launch();
     plan_scan_kernel<<<1, 1024, 0, stream>>>(gsp, (int)n_groups + 1);
     count_launch();
@@ -572,13 +600,16 @@ int plan_fill_tall_async(const int* rowptr, const int* colidx, size_t K, size_t 
     if (int rc = plan_launch_setup(ctx_in, &ctx)) return rc;
     const size_t n_groups = (brow_end - brow_begin + rg - 1) / rg;
     if (n_groups == 0 || nnzb == 0) return SMAT_OK;
-    const int grid = (int)(n_groups < (size_t)ctx->sm_count ? n_groups : (size_t)ctx->sm_count);
-    const size_t smem_fill = (size_t)kWindow * 8;
-    SMAT_CUDA_TRY(cudaFuncSetAttribute(plan_tall_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fill));
-    plan_tall_kernel<true><<<grid, kTallPlanThreads, smem_fill, stream>>>(rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg,
-                                                                         kTallBlocksPerStep, (int)(K / 16), (int)n_groups,
-                                                                         const_cast<int*>(gsp), reinterpret_cast<uint4*>(steps),
-                                                                         reinterpret_cast<uint4*>(wstep), blk, (int)nnzb, ctx->d_status);
+    const int rc = launch_windowed<kTallPlanThreads>(K / 16, n_groups, 2, ctx->sm_count, [&](auto win, int grid, size_t smem) -> int {
+        auto kernel = plan_tall_kernel<true, decltype(win)::value>;
+        SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<grid, kTallPlanThreads, smem, stream>>>(
+            rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, kTallBlocksPerStep,
+            (int)(K / 16), (int)n_groups, const_cast<int*>(gsp), reinterpret_cast<uint4*>(steps),
+            reinterpret_cast<uint4*>(wstep), blk, (int)nnzb, ctx->d_status);
+        return SMAT_OK;
+    });
+    if (rc) return rc;
     count_launch();
     tall_pair_kernel<<<ctx->sm_count * 4, 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(wstep), reinterpret_cast<uint4*>(winfo), gsp,
                                                             (int)n_groups);
@@ -611,13 +642,24 @@ struct smat_plan {
 
 // One chunk of columns of C, rows x `width16` 16-byte words, from device memory to pinned host memory that the device can
 // address, both `pitch16` words from row to row.  A 2-D copy of the copy engine moves rows of 512 bytes at 8 GB/s
-// (measured; 50 GB/s in one piece), stores from the SMs at the rate of the link.
+// (measured; 50 GB/s in one piece), stores from the SMs at the rate of the link; eight CTAs are enough for that and leave
+// the other SMs to the product of the next chunk.
 static __global__ void __launch_bounds__(256) copy_out_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t rows, size_t pitch16,
                                                              unsigned width16) {
     const size_t n = rows * width16, stride = (size_t)gridDim.x * 256;
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += stride) {
-        const size_t row = i / width16, at = row * pitch16 + (i - row * width16);
-        dst[at] = __ldg(src + at);
+    constexpr int U = 4;
+    for (size_t i0 = (size_t)blockIdx.x * 256 + threadIdx.x; i0 < n; i0 += U * stride) {
+        uint4 v[U];
+        size_t at[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const size_t i = i0 + u * stride, row = i / width16;
+            at[u] = row * pitch16 + (i - row * width16);
+            if (i < n) v[u] = __ldg(src + at[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i0 + u * stride < n) dst[at[u]] = v[u];
     }
 }
 
@@ -1064,7 +1106,7 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
             SMAT_CUDA_TRY(cudaEventRecord(plan->ev_done[j], s));
             SMAT_CUDA_TRY(cudaStreamWaitEvent(plan->s_out, plan->ev_done[j], 0));
             const size_t words = rows * w / 8, ctas = (words + 1023) / 1024;
-            copy_out_kernel<<<(unsigned)(ctas < 64 ? ctas : 64), 256, 0, plan->s_out>>>(
+            copy_out_kernel<<<(unsigned)(ctas < 8 ? ctas : 8), 256, 0, plan->s_out>>>(
                 reinterpret_cast<const uint4*>(Cd + n0 * 2), reinterpret_cast<uint4*>(out_view + n0 * 2), rows, N / 8, (unsigned)(w / 8));
             count_launch();
             SMAT_CUDA_TRY(cudaGetLastError());
