@@ -27,6 +27,7 @@
 #include <queue>
 #include <algorithm>
 
+#include "ptx_sm100.cuh"
 #include "smat_internal.h"
 #include "spmm_stream.h"
 
@@ -106,6 +107,7 @@ template <bool FILL, int WIN>
 __global__ void __launch_bounds__(kPlanThreads)
 plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int brow_begin, int brow_end, int rg, int CAP, int Kb,
             int n_groups, int* __restrict__ gsp, uint4* __restrict__ steps, int* __restrict__ blk, int nnzb, int* status, int* units) {
+    ptx::pdl_wait();
     extern __shared__ uint32_t sm[];
     uint32_t* masks = sm;                                 // [WIN] row mask per block-column
     int* blk_pre = reinterpret_cast<int*>(sm + WIN);  // [WIN] exclusive block number (FILL only)
@@ -200,6 +202,7 @@ plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int 
 
 // In-place inclusive scan of data[0..n) by one CTA.
 __global__ void __launch_bounds__(1024) plan_scan_kernel(int* data, int n) {
+    ptx::pdl_wait();
     __shared__ int warp_tot[32];
     __shared__ int carry_s, max_s;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -245,6 +248,7 @@ __global__ void __launch_bounds__(1024) plan_scan_kernel(int* data, int n) {
 // Positions behind the blocks of a group whose columns were found inconsistent hold nothing: skipped by the range check.
 __global__ void __launch_bounds__(256) pack_kernel(const uint4* __restrict__ vals, const int* __restrict__ blk, uint4* __restrict__ packed,
                                                   const int* __restrict__ rowptr, int brow_begin, int brow_end, int nnzb) {
+    ptx::pdl_wait();
     constexpr int U = 4;
     if (range_is_bad(rowptr, brow_begin, brow_end, nnzb)) return;
     const int first = __ldg(rowptr + brow_begin), n = __ldg(rowptr + brow_end) - first;
@@ -277,6 +281,7 @@ __global__ void __launch_bounds__(kTallPlanThreads)
 plan_tall_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int brow_begin, int brow_end, int rg, int CAP, int Kb,
                  int n_groups, int* __restrict__ gsp, uint4* __restrict__ steps, uint4* __restrict__ winfo, int* __restrict__ blk,
                  int nnzb, int* status) {
+    ptx::pdl_wait();
     extern __shared__ uint32_t sm[];
     uint32_t* masks = sm;                                 // [WIN] row mask per block-column
     int* blk_pre = reinterpret_cast<int*>(sm + WIN);  // [WIN] exclusive block number (FILL only)
@@ -409,6 +414,7 @@ plan_tall_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx,
 // and the number of entries in bits [28, 32) of word 0 (the spare bits of its second entry).
 __global__ void __launch_bounds__(256) tall_pair_kernel(const uint32_t* __restrict__ wstep, uint4* __restrict__ winfo,
                                                        const int* __restrict__ gsp, int n_groups) {
+    ptx::pdl_wait();
     const int pairs = __ldg(gsp + n_groups) >> 1;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs * 16; i += gridDim.x * blockDim.x) {
         const int pr = i >> 4, m = i & 15;
@@ -445,9 +451,10 @@ int pack_values_async(const int* rowptr, const void* vals, const int* blk, void*
         ctx = c;
     }
     const size_t want = (nnzb + 31) / 32, most = (size_t)ctx->sm_count * 8;  // 32 blocks per CTA and trip
-    pack_kernel<<<(unsigned)(want < most ? want : most), 256, 0, stream>>>(reinterpret_cast<const uint4*>(vals), blk,
-                                                                          reinterpret_cast<uint4*>(packed), rowptr, (int)brow_begin,
-                                                                          (int)brow_end, (int)nnzb);
+    SMAT_CUDA_TRY(launch_pdl(pack_kernel, dim3((unsigned)(want < most ? want : most)), dim3(256), 0, stream,
+                             reinterpret_cast<const uint4*>(vals), blk,
+                             reinterpret_cast<uint4*>(packed), rowptr, (int)brow_begin,
+                             (int)brow_end, (int)nnzb));
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
@@ -531,14 +538,15 @@ int plan_count_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb
     const int rc = launch_windowed<kPlanThreads>(K / 16, n_groups, 1, ctx->sm_count, [&](auto win, int grid, size_t smem) -> int {
         auto kernel = plan_kernel<false, decltype(win)::value>;
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<grid, kPlanThreads, smem, stream>>>(
-            rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap, (int)(K / 16),
-            (int)n_groups, gsp, nullptr, nullptr, (int)nnzb, ctx->d_status, units);
+        SMAT_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(kPlanThreads), smem, stream,
+                                 rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap, (int)(K / 16),
+                                 (int)n_groups, gsp, nullptr, nullptr, (int)nnzb, ctx->d_status, units));
         return SMAT_OK;
     });
     if (rc) return rc;
     count_launch();
-    plan_scan_kernel<<<1, 1024, 0, stream>>>(gsp, (int)n_groups + 1);
+    SMAT_CUDA_TRY(launch_pdl(plan_scan_kernel, dim3(1), dim3(1024), 0, stream,
+                             gsp, (int)n_groups + 1));
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
@@ -553,10 +561,10 @@ int plan_fill_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb,
     const int rc = launch_windowed<kPlanThreads>(K / 16, n_groups, 2, ctx->sm_count, [&](auto win, int grid, size_t smem) -> int {
         auto kernel = plan_kernel<true, decltype(win)::value>;
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<grid, kPlanThreads, smem, stream>>>(
-            rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap, (int)(K / 16),
-            (int)n_groups, const_cast<int*>(gsp), reinterpret_cast<uint4*>(steps), blk, (int)nnzb,
-            ctx->d_status, nullptr);
+        SMAT_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(kPlanThreads), smem, stream,
+                                 rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap, (int)(K / 16),
+                                 (int)n_groups, const_cast<int*>(gsp), reinterpret_cast<uint4*>(steps), blk, (int)nnzb,
+                                 ctx->d_status, nullptr));
         return SMAT_OK;
     });
     if (rc) return rc;
@@ -579,15 +587,16 @@ int plan_count_tall_async(const int* rowptr, const int* colidx, size_t K, size_t
     const int rc = launch_windowed<kTallPlanThreads>(K / 16, n_groups, 1, ctx->sm_count, [&](auto win, int grid, size_t smem) -> int {
         auto kernel = plan_tall_kernel<false, decltype(win)::value>;
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<grid, kTallPlanThreads, smem, stream>>>(
-            rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, kTallBlocksPerStep,
-            (int)(K / 16), (int)n_groups, gsp, nullptr, nullptr, nullptr, (int)nnzb,
-            ctx->d_status);
+        SMAT_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(kTallPlanThreads), smem, stream,
+                                 rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, kTallBlocksPerStep,
+                                 (int)(K / 16), (int)n_groups, gsp, nullptr, nullptr, nullptr, (int)nnzb,
+                                 ctx->d_status));
         return SMAT_OK;
     });
     if (rc) return rc;
     count_launch();
-    plan_scan_kernel<<<1, 1024, 0, stream>>>(gsp, (int)n_groups + 1);
+    SMAT_CUDA_TRY(launch_pdl(plan_scan_kernel, dim3(1), dim3(1024), 0, stream,
+                             gsp, (int)n_groups + 1));
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
@@ -603,16 +612,17 @@ int plan_fill_tall_async(const int* rowptr, const int* colidx, size_t K, size_t 
     const int rc = launch_windowed<kTallPlanThreads>(K / 16, n_groups, 2, ctx->sm_count, [&](auto win, int grid, size_t smem) -> int {
         auto kernel = plan_tall_kernel<true, decltype(win)::value>;
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<grid, kTallPlanThreads, smem, stream>>>(
-            rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, kTallBlocksPerStep,
-            (int)(K / 16), (int)n_groups, const_cast<int*>(gsp), reinterpret_cast<uint4*>(steps),
-            reinterpret_cast<uint4*>(wstep), blk, (int)nnzb, ctx->d_status);
+        SMAT_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(kTallPlanThreads), smem, stream,
+                                 rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, kTallBlocksPerStep,
+                                 (int)(K / 16), (int)n_groups, const_cast<int*>(gsp), reinterpret_cast<uint4*>(steps),
+                                 reinterpret_cast<uint4*>(wstep), blk, (int)nnzb, ctx->d_status));
         return SMAT_OK;
     });
     if (rc) return rc;
     count_launch();
-    tall_pair_kernel<<<ctx->sm_count * 4, 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(wstep), reinterpret_cast<uint4*>(winfo), gsp,
-                                                            (int)n_groups);
+    SMAT_CUDA_TRY(launch_pdl(tall_pair_kernel, dim3(ctx->sm_count * 4), dim3(256), 0, stream,
+                             reinterpret_cast<const uint32_t*>(wstep), reinterpret_cast<uint4*>(winfo), gsp,
+                             (int)n_groups));
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;

@@ -167,7 +167,7 @@ spmm_bcsr_tc_kernel(const __grid_constant__ CUtensorMap mapB, const __grid_const
     const int n_full = n_items / (int)gridDim.x * (int)gridDim.x;  // items of the complete rounds
     Flat flat;
     flat.gsp = gsp; flat.n_tiles = n_tiles; flat.n_groups = n_groups;
-    flat.total = balanced ? (long long)(__ldg(gsp + n_groups) - __ldg(gsp)) * n_tiles : 0;
+    flat.total = 0;
     auto make_gen = [&]() {
         SegGen<SCHED> sg;
         sg.gsp = gsp; sg.n_tiles = n_tiles; sg.n_items = n_items; sg.n_ctas = (int)gridDim.x; sg.cta = (int)blockIdx.x;
@@ -210,8 +210,10 @@ spmm_bcsr_tc_kernel(const __grid_constant__ CUtensorMap mapB, const __grid_const
         tmem_st_wait();
     }
     tc_fence_before();
+    pdl_wait();  // everything above may run while the kernel before this one still does
     __syncthreads();
     tc_fence_after();
+    if (balanced) flat.total = (long long)(__ldg(gsp + n_groups) - __ldg(gsp)) * n_tiles;
 
     // ------------------------------ epilogue: tensor memory -> fp16 -> C ------------------------------
     auto epilogue = [&](const int grp) {
@@ -539,6 +541,7 @@ __global__ void zero_rows_kernel(uint4* dst, size_t n16) {
 template <int NH>
 __global__ void __launch_bounds__(512) sum_cut_items_kernel(const float* __restrict__ scratch, __half* __restrict__ C, int brow_begin,
                                                            int brow_end, int rg, int N, int n_tiles, int n_full, int parts, size_t ldc) {
+    pdl_wait();
     const int item = n_full + (int)blockIdx.x;
     const int g = item / n_tiles, t = item - g * n_tiles;
     const int r0 = brow_begin + g * rg;
@@ -571,6 +574,7 @@ template <int NH>
 __global__ void __launch_bounds__(512) sum_split_items_kernel(const float* __restrict__ scratch, const int* __restrict__ gsp,
                                                              __half* __restrict__ C, int brow_begin, int brow_end, int rg, int N,
                                                              int n_tiles, int n_groups, int n_ctas, size_t ldc) {
+    pdl_wait();
     Flat flat;
     flat.gsp = gsp; flat.n_tiles = n_tiles; flat.n_groups = n_groups;
     flat.total = (long long)(__ldg(gsp + n_groups) - __ldg(gsp)) * n_tiles;
@@ -632,11 +636,13 @@ PlanView plan_group_range(const PlanView& whole, size_t group_begin, size_t grou
 int launch_sum_cut_items(bool wide, int cut_items, const float* scratch, void* C, int brow_begin, int brow_end, int rg, int N,
                          int n_tiles, int n_full, int parts, size_t ldc, cudaStream_t stream) {
     if (wide)
-        sum_cut_items_kernel<2><<<cut_items, dim3(128, 4), 0, stream>>>(scratch, reinterpret_cast<__half*>(C), brow_begin, brow_end, rg, N,
-                                                                       n_tiles, n_full, parts, ldc);
+        SMAT_CUDA_TRY(launch_pdl(sum_cut_items_kernel<2>, dim3(cut_items), dim3(128, 4), 0, stream,
+                                 scratch, reinterpret_cast<__half*>(C), brow_begin, brow_end, rg, N,
+                                 n_tiles, n_full, parts, ldc));
     else
-        sum_cut_items_kernel<1><<<cut_items, dim3(128, 4), 0, stream>>>(scratch, reinterpret_cast<__half*>(C), brow_begin, brow_end, rg, N,
-                                                                       n_tiles, n_full, parts, ldc);
+        SMAT_CUDA_TRY(launch_pdl(sum_cut_items_kernel<1>, dim3(cut_items), dim3(128, 4), 0, stream,
+                                 scratch, reinterpret_cast<__half*>(C), brow_begin, brow_end, rg, N,
+                                 n_tiles, n_full, parts, ldc));
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
@@ -724,11 +730,11 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
     if (const char* ev = std::getenv("SMAT_L2_PREFETCH")) pf = std::atoi(ev) != 0;  // tuning knob
     auto launch = [&](auto kernel, uint32_t smem_bytes) -> int {
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
-        kernel<<<grid, kThreads, smem_bytes, stream>>>(
-            mapB, mapC, reinterpret_cast<const uint8_t*>(plan.packed), reinterpret_cast<const uint4*>(plan.steps), plan.gsp,
-            plan.rowptr, reinterpret_cast<__half*>(C), (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles,
-            (int)n_items, (int)plan.n_groups, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, ldc,
-            listed ? plan.sched_off : nullptr, listed ? plan.sched_list : nullptr, nm, pf);
+        SMAT_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(kThreads), smem_bytes, stream,
+                                 mapB, mapC, reinterpret_cast<const uint8_t*>(plan.packed), reinterpret_cast<const uint4*>(plan.steps), plan.gsp,
+                                 plan.rowptr, reinterpret_cast<__half*>(C), (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles,
+                                 (int)n_items, (int)plan.n_groups, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, ldc,
+                                 listed ? plan.sched_off : nullptr, listed ? plan.sched_list : nullptr, nm, pf));
         count_launch();
         SMAT_CUDA_TRY(cudaGetLastError());
         return SMAT_OK;
@@ -753,13 +759,15 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
     if (balanced) {
         if (grid < 2) return SMAT_OK;
         if (variant == 3)
-            sum_split_items_kernel<2><<<grid - 1, dim3(128, 4), 0, stream>>>(plan.fix_scratch, plan.gsp, reinterpret_cast<__half*>(C),
-                                                                            (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N,
-                                                                            n_tiles, (int)plan.n_groups, grid, ldc);
+            SMAT_CUDA_TRY(launch_pdl(sum_split_items_kernel<2>, dim3(grid - 1), dim3(128, 4), 0, stream,
+                                     plan.fix_scratch, plan.gsp, reinterpret_cast<__half*>(C),
+                                     (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N,
+                                     n_tiles, (int)plan.n_groups, grid, ldc));
         else
-            sum_split_items_kernel<1><<<grid - 1, dim3(128, 4), 0, stream>>>(plan.fix_scratch, plan.gsp, reinterpret_cast<__half*>(C),
-                                                                            (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N,
-                                                                            n_tiles, (int)plan.n_groups, grid, ldc);
+            SMAT_CUDA_TRY(launch_pdl(sum_split_items_kernel<1>, dim3(grid - 1), dim3(128, 4), 0, stream,
+                                     plan.fix_scratch, plan.gsp, reinterpret_cast<__half*>(C),
+                                     (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N,
+                                     n_tiles, (int)plan.n_groups, grid, ldc));
         count_launch();
         SMAT_CUDA_TRY(cudaGetLastError());
         return SMAT_OK;

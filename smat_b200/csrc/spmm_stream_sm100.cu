@@ -28,6 +28,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "ptx_sm100.cuh"
 #include "smat_internal.h"
 #include "spmm_stream.h"
 
@@ -60,9 +61,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
     const int tile = (int)(blockIdx.x % (unsigned)p.n_tiles);
     const int piece = (int)(blockIdx.x / (unsigned)p.n_tiles) * (kWarps / W) + warp / W;
     const int n0 = tile * p.tile_cols;
-    // launched while the kernel before it still runs (programmatic dependent launch); nothing is read before this
-    asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    ptx::pdl_wait();
     // ---- the piece: blocks [b0, b1) of block-row `row`; count > 1: one of `count` pieces of a long block-row ----
     int row = 0, b0 = 0, b1 = 0, count = 1, my_slot = 0, first_slot = 0;
     bool live = piece < p.n_pieces;
@@ -269,8 +268,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
 
 // B ([N][K], k contiguous) -> slabs [K / 16][N][16]: the 16 x N slice of one block-column becomes contiguous.
 __global__ void __launch_bounds__(256) slab_kernel(const uint4* __restrict__ B, uint4* __restrict__ out, int N, int K8) {
-    asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    ptx::pdl_wait();
     // a warp moves 16 rows x 32 bytes; the eight warps of a CTA take neighbouring block-columns
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x * 8 + warp;  // block-column
@@ -285,6 +283,7 @@ __global__ void __launch_bounds__(256) slab_kernel(const uint4* __restrict__ B, 
 __global__ void __launch_bounds__(256) long_rows_kernel(const int* __restrict__ rowptr, int brow_begin, int brow_end, int nnzb, int chunk,
                                                        int room, int* head, uint4* __restrict__ pieces, int2* __restrict__ slots,
                                                        int* __restrict__ row_slot) {
+    ptx::pdl_wait();
     const int lo = __ldg(rowptr + brow_begin), hi = __ldg(rowptr + brow_end);
     const int row = blockIdx.x * 256 + threadIdx.x;
     if (lo < 0 || hi < lo || hi > nnzb || row >= brow_end - brow_begin) return;
@@ -305,6 +304,7 @@ __global__ void __launch_bounds__(256) long_rows_kernel(const int* __restrict__ 
 // of the block columns; a column outside the matrix becomes -1.
 __global__ void __launch_bounds__(256) stream_pack_kernel(const uint2* __restrict__ vals, const int* __restrict__ colidx,
                                                          uint4* __restrict__ packed, int* __restrict__ cols, int first, int n, int Kb) {
+    ptx::pdl_wait();
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
@@ -331,16 +331,7 @@ cudaError_t launch_one(const StreamArgs& a, cudaStream_t stream) {
     constexpr long long per = Q::WARPS / W;
     const long long grid = (((long long)a.n_pieces + per - 1) / per) * a.n_tiles;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(Q::WARPS * 32);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, spmm_bcsr_stream_kernel<NT, W, Q::WARPS, Q::U, Q::MINB, SLAB, PLAN>, a);
+    return launch_pdl(spmm_bcsr_stream_kernel<NT, W, Q::WARPS, Q::U, Q::MINB, SLAB, PLAN>, dim3((unsigned)grid), dim3(Q::WARPS * 32), 0, stream, a);
 }
 
 template <bool PLAN, bool SLAB, int W>
@@ -374,16 +365,8 @@ int launch(const StreamShape& s, const StreamArgs& a, cudaStream_t stream) {
 }
 
 int make_slabs(const void* B, void* slabs, size_t N, size_t K, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((K / 16 + 7) / 8), (unsigned)std::min<size_t>((N + 15) / 16, 65535));
-    cfg.blockDim = dim3(256);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    SMAT_CUDA_TRY(cudaLaunchKernelEx(&cfg, slab_kernel, reinterpret_cast<const uint4*>(B), reinterpret_cast<uint4*>(slabs), (int)N, (int)(K / 8)));
+    SMAT_CUDA_TRY(launch_pdl(slab_kernel, dim3((unsigned)((K / 16 + 7) / 8), (unsigned)std::min<size_t>((N + 15) / 16, 65535)), dim3(256), 0, stream,
+                             reinterpret_cast<const uint4*>(B), reinterpret_cast<uint4*>(slabs), (int)N, (int)(K / 8)));
     count_launch();
     return SMAT_OK;
 }
@@ -493,8 +476,9 @@ int stream_plan_values(const PlanView& v, const void* vals, const int* colidx, i
     if (v.nnzb == 0) return SMAT_OK;
     const StreamArgs& a = v.stream->args;
     const unsigned grid = (unsigned)std::min((v.nnzb + 7) / 8, (size_t)sm_count * 8);
-    stream_pack_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const uint2*>(vals), colidx, reinterpret_cast<uint4*>(const_cast<void*>(a.vals)),
-                                                 colidx ? const_cast<int*>(a.colidx) : nullptr, (int)v.stream->first, (int)v.nnzb, (int)(v.K / 16));
+    SMAT_CUDA_TRY(launch_pdl(stream_pack_kernel, dim3(grid), dim3(256), 0, stream,
+                             reinterpret_cast<const uint2*>(vals), colidx, reinterpret_cast<uint4*>(const_cast<void*>(a.vals)),
+                             colidx ? const_cast<int*>(a.colidx) : nullptr, (int)v.stream->first, (int)v.nnzb, (int)(v.K / 16)));
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
@@ -576,8 +560,9 @@ int stream_call(const StreamShape& s, const void* vals, const int* rowptr, const
         a.slots = slots;
         a.row_slot = row_slot;
         SMAT_CUDA_TRY(cudaMemsetAsync(head, 0, 256 + counter_bytes, stream));
-        long_rows_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, stream>>>(rowptr, (int)brow_begin, (int)brow_end, (int)nnzb, s.chunk, (int)extra, head,
-                                                                             pieces, slots, row_slot);
+        SMAT_CUDA_TRY(launch_pdl(long_rows_kernel, dim3((unsigned)((rows + 255) / 256)), dim3(256), 0, stream,
+                                 rowptr, (int)brow_begin, (int)brow_end, (int)nnzb, s.chunk, (int)extra, head,
+                                 pieces, slots, row_slot));
         count_launch();
         SMAT_CUDA_TRY(cudaGetLastError());
     }

@@ -187,6 +187,7 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
         tmem_st_wait();
     }
     tc_fence_before();
+    pdl_wait();  // everything above may run while the kernel before this one still does
     __syncthreads();
     tc_fence_after();
 
@@ -522,10 +523,10 @@ int launch_spmm_tall(const PlanView& whole, const void* B, void* C, size_t N, cu
     if (const char* ev = std::getenv("SMAT_L2_PREFETCH")) pf = std::atoi(ev) != 0;  // tuning knob
     auto launch = [&](auto kernel, int threads) -> int {
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
-        kernel<<<grid, threads, SMEM_BYTES, stream>>>(
-            mapB, reinterpret_cast<const uint8_t*>(plan.packed), reinterpret_cast<const uint4*>(plan.steps),
-            reinterpret_cast<const uint4*>(plan.winfo), plan.gsp, plan.rowptr, reinterpret_cast<__half*>(C), ldc, (int)plan.brow_begin,
-            (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles, (int)n_items, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, pf);
+        SMAT_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(threads), SMEM_BYTES, stream,
+                                 mapB, reinterpret_cast<const uint8_t*>(plan.packed), reinterpret_cast<const uint4*>(plan.steps),
+                                 reinterpret_cast<const uint4*>(plan.winfo), plan.gsp, plan.rowptr, reinterpret_cast<__half*>(C), ldc, (int)plan.brow_begin,
+                                 (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles, (int)n_items, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, pf));
         return SMAT_OK;
     };
     // the smallest shape that holds the plan's groups: fewer accumulators leave tensor memory for more panel slots
