@@ -29,7 +29,7 @@ void clear_error();
 // touches global memory.  What this hides is the launch itself and the kernel's set-up (barriers, tensor memory):
 // 1 to 3 us per launch.
 template <class... Params, class... Args>
-cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+cudaError_t launch_pdl_if(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -39,9 +39,17 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
+template <class... Params, class... Args>
+cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_pdl_if(true, kernel, grid, block, smem, stream, args...);
+}
+// Whether a persistent SpMM kernel begins early: CTAs that start as SMs come free end up on other SMs than those of a launch
+// into an idle device, which costs long launches more than it hides (dense clusters, 55 rounds of items: 277 -> 282 us; 85 us
+// layer, 1.2 rounds: 88 -> 86; one round: 33.6 -> 30.1).
+inline bool spmm_begins_early(size_t items, size_t sms) { return items <= 8 * sms; }
 
 // Per-device state created lazily on first use (with that device current): SM count and a small
 // device status word that kernels set when one of their bounded waits runs out.

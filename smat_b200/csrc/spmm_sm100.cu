@@ -633,16 +633,18 @@ PlanView plan_group_range(const PlanView& whole, size_t group_begin, size_t grou
     return plan;
 }
 
+// (Not launched with launch_pdl: its CTAs, resident early beside the last work items, made those take 14 us longer -- 4096 x
+// 8192 layer, N = 2048: 88 -> 102 us.  It lets the kernel after it begin its set-up, though.)
 int launch_sum_cut_items(bool wide, int cut_items, const float* scratch, void* C, int brow_begin, int brow_end, int rg, int N,
                          int n_tiles, int n_full, int parts, size_t ldc, cudaStream_t stream) {
     if (wide)
-        SMAT_CUDA_TRY(launch_pdl(sum_cut_items_kernel<2>, dim3(cut_items), dim3(128, 4), 0, stream,
-                                 scratch, reinterpret_cast<__half*>(C), brow_begin, brow_end, rg, N,
-                                 n_tiles, n_full, parts, ldc));
+        sum_cut_items_kernel<2><<<cut_items, dim3(128, 4), 0, stream>>>(
+                       scratch, reinterpret_cast<__half*>(C), brow_begin, brow_end, rg, N,
+                       n_tiles, n_full, parts, ldc);
     else
-        SMAT_CUDA_TRY(launch_pdl(sum_cut_items_kernel<1>, dim3(cut_items), dim3(128, 4), 0, stream,
-                                 scratch, reinterpret_cast<__half*>(C), brow_begin, brow_end, rg, N,
-                                 n_tiles, n_full, parts, ldc));
+        sum_cut_items_kernel<1><<<cut_items, dim3(128, 4), 0, stream>>>(
+                       scratch, reinterpret_cast<__half*>(C), brow_begin, brow_end, rg, N,
+                       n_tiles, n_full, parts, ldc);
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
@@ -730,7 +732,7 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
     if (const char* ev = std::getenv("SMAT_L2_PREFETCH")) pf = std::atoi(ev) != 0;  // tuning knob
     auto launch = [&](auto kernel, uint32_t smem_bytes) -> int {
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
-        SMAT_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(kThreads), smem_bytes, stream,
+        SMAT_CUDA_TRY(launch_pdl_if(spmm_begins_early(n_items, sms), kernel, dim3(grid), dim3(kThreads), smem_bytes, stream,
                                  mapB, mapC, reinterpret_cast<const uint8_t*>(plan.packed), reinterpret_cast<const uint4*>(plan.steps), plan.gsp,
                                  plan.rowptr, reinterpret_cast<__half*>(C), (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles,
                                  (int)n_items, (int)plan.n_groups, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, ldc,
@@ -759,15 +761,15 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
     if (balanced) {
         if (grid < 2) return SMAT_OK;
         if (variant == 3)
-            SMAT_CUDA_TRY(launch_pdl(sum_split_items_kernel<2>, dim3(grid - 1), dim3(128, 4), 0, stream,
-                                     plan.fix_scratch, plan.gsp, reinterpret_cast<__half*>(C),
-                                     (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N,
-                                     n_tiles, (int)plan.n_groups, grid, ldc));
+            sum_split_items_kernel<2><<<grid - 1, dim3(128, 4), 0, stream>>>(
+                       plan.fix_scratch, plan.gsp, reinterpret_cast<__half*>(C),
+                       (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N,
+                       n_tiles, (int)plan.n_groups, grid, ldc);
         else
-            SMAT_CUDA_TRY(launch_pdl(sum_split_items_kernel<1>, dim3(grid - 1), dim3(128, 4), 0, stream,
-                                     plan.fix_scratch, plan.gsp, reinterpret_cast<__half*>(C),
-                                     (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N,
-                                     n_tiles, (int)plan.n_groups, grid, ldc));
+            sum_split_items_kernel<1><<<grid - 1, dim3(128, 4), 0, stream>>>(
+                       plan.fix_scratch, plan.gsp, reinterpret_cast<__half*>(C),
+                       (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N,
+                       n_tiles, (int)plan.n_groups, grid, ldc);
         count_launch();
         SMAT_CUDA_TRY(cudaGetLastError());
         return SMAT_OK;
