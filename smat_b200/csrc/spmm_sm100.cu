@@ -699,7 +699,9 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
     if (variant == 0 && (balanced || listed)) variant = (N >= 256 && plan.nnzb / plan.n_groups >= 256 && est_steps >= 64) ? 3 : 1;
     if (variant == 0) {
         variant = 1;
-        if (N >= 256 && plan.nnzb / plan.n_groups >= 256 && est_steps >= 64 &&
+        // (a plan built inside a call does not know its steps: items of dense clusters would be taken for long ones,
+        // 65536 rows, N = 512: 108 us against 70)
+        if (plan.total_steps && N >= 256 && plan.nnzb / plan.n_groups >= 256 && est_steps >= 64 &&
             kWideItemCost * rounds(plan.n_groups * ((N + 255) / 256), true) < rounds(plan.n_groups * ((N + 127) / 128), false))
             variant = 3;
     }

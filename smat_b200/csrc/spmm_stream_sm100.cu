@@ -418,12 +418,22 @@ double stream_estimate_us(size_t N, size_t rows, size_t nnzb, size_t K, int sm_c
     return 4.0 + (s.slab ? 2.0 + 4e-6 * n * (double)K / 5.5 : 0.0) + (double)nnzb / sm_count * per_block * 1e-3 + (double)(rows * 16) * n * 2.0 / 6e6;
 }
 
-// A product without a plan takes this kernel unless building a plan inside the call (reading and writing all blocks, a
-// dozen launches) and a tcgen05 kernel are estimated to be faster: many blocks, each used by many columns.
+// A product without a plan takes this kernel unless building a plan inside the call and a tcgen05 kernel are estimated to be
+// faster: 24 us for the launches and small plan kernels, 0.2 ns per block for reading and writing it, and the product --
+// rounds of items at 0.26 us a step, or 20 ns per block, tile and SM, whichever is more.
 bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count) {
     if (g_spmm_variant) return g_spmm_variant == 5;
-    const double plan_us = 50.0 + 1028.0 * (double)nnzb / 5e6 + (double)nnzb * (double)((N + 127) / 128) / sm_count * 20e-3;
-    return stream_estimate_us(N, rows, nnzb, K, sm_count, false) < plan_us;
+    const size_t rg = choose_rows_per_group(rows, N, sm_count, true, nnzb, K), groups = (rows + rg - 1) / rg, tiles = (N + 127) / 128;
+    const double throughput = (double)nnzb * (double)tiles / sm_count * 20e-3, build = 24.0 + 0.2e-3 * (double)nnzb;
+    const double stream = stream_estimate_us(N, rows, nnzb, K, sm_count, false);
+    if ((double)nnzb < 0.08 * (double)rows * (double)(K / 16)) {
+        // Few of the possible blocks: how they lie is not known here.  Short block-rows are taken to be clustered, which suits
+        // the other kernel; long ones may be skewed, which makes some items many times longer than the rest (power-law graph
+        // of 65536 rows, N = 128: 951 us against 229), while this kernel cuts long block-rows.
+        return stream < (nnzb > 24 * rows ? 2.0 : 1.0) * (build + throughput);
+    }
+    const double quads = std::ceil((double)K / 64.0), steps = quads * (1.0 - std::exp(-(double)nnzb / (double)groups / quads));
+    return stream < build + std::max(throughput, rounds_for(groups * tiles, (size_t)sm_count, true, (size_t)steps, false) * steps * 0.26);
 }
 
 int stream_plan_build(StreamPlan& sp, PlanView& v, const int* h_rowptr, const void* vals, const int* colidx, size_t N_hint, int sm_count,
