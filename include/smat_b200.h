@@ -100,8 +100,9 @@ int smat_plan_spmm(const smat_plan* plan, const void* B, void* C, size_t N, void
 
 /* The same product with B and C in HOST memory (pinned memory for copies that overlap), pipelined on two
  * internal streams: B comes in by column chunks of one work-item width, each multiplied as soon as it has
- * arrived; the last chunk is multiplied range of block-rows by range, and the rows of C it completes are copied
- * out under the multiplication of the next range.  B_host is [N][K] (k contiguous), C_host row-major
+ * arrived.  Where C_host is pinned (and 16-byte aligned) the columns a chunk completes are stored to it at once; else the
+ * last chunk is multiplied range of block-rows by range, and the rows of C it completes are copied out under the
+ * multiplication of the next range.  B_host is [N][K] (k contiguous), C_host row-major
  * [(brow_end - brow_begin) * 16][N].  Everything is ordered after earlier work on `stream`, and `stream` ends
  * after the last copy.  The staging buffers (all of B and C) and the streams belong to the plan and are created
  * by the first call, which therefore must not happen inside a stream capture.
@@ -110,7 +111,7 @@ int smat_plan_spmm(const smat_plan* plan, const void* B, void* C, size_t N, void
 int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_t N, void* stream);
 int smat_plan_destroy(smat_plan* plan);
 /* What a plan turned out to be (informational, no reference counterpart): *rows_per_item = block-rows of a work item
- * (8..16: the kernel that reads both operands from shared memory; 16..24 with *tall = 1: the kernel that reads the
+ * (8..16: the kernel that reads both operands from shared memory; 12..24 with *tall = 1: the kernel that reads the
  * B panels from tensor memory; 1: the kernel that walks single block-rows), *steps = steps of the walk order (pieces of
  * block-rows for the last kernel).  Any pointer may be NULL. */
 int smat_plan_info(const smat_plan* plan, int* tall, int* rows_per_item, size_t* steps);
