@@ -222,12 +222,16 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
         float4* mine = p.partial + ((size_t)my_slot * p.n_tiles + tile) * (T * 32) + lane;
 #pragma unroll
         for (int j = 0; j < T; j++) __stcg(mine + j * 32, make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]));
+        // lane 0's arrival stands for all 32 lanes: their stores and fences come before it only through a warp barrier (a
+        // shuffle does not order memory), and what it has seen reaches their loads only through another
         __threadfence();
+        __syncwarp();
         int old = 0;
         if (lane == 0) old = atomicAdd(p.counters + (size_t)first_slot * p.n_tiles + tile, 1);
         old = __shfl_sync(0xffffffffu, old, 0);
         if (old != count - 1) return;
         __threadfence();
+        __syncwarp();
         if (lane == 0) p.counters[(size_t)first_slot * p.n_tiles + tile] = 0;  // ready for the next launch
 #pragma unroll
         for (int j = 0; j < T; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;

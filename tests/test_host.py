@@ -27,6 +27,19 @@ def test_library_exports_every_declared_symbol():
         assert hasattr(L, n), f"{n} is declared in include/smat_b200.h but not exported"
 
 
+def test_partial_tiles_are_published_by_the_whole_warp():
+    """Stream kernel: 32 lanes store a partial tile, lane 0 alone counts its arrival.  No run can show that the others' stores
+    come first, so the source is read: a fence and then a warp barrier between the stores and the arrival, and again
+    between the arrival and the loads of the other pieces' tiles."""
+    src = open(os.path.join(ROOT, "smat_b200", "csrc", "spmm_stream_sm100.cu")).read()
+    src = re.sub(r"//[^\n]*", "", src)
+    tail = src[src.index("__stcg(mine"):]
+    before, after = tail.split("atomicAdd(p.counters", 1)
+    ordered = r"__threadfence\(\);\s*__syncwarp\(\);"
+    assert re.search(ordered, before)
+    assert re.search(ordered, after[:after.index("__ldcg(src")])
+
+
 def test_no_gpu_means_loud_failure_not_fallback():
     import torch
     if torch.cuda.is_available():
