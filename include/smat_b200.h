@@ -129,10 +129,13 @@ int smat_spmm_set_variant(int variant);
 
 /* Synchronises `stream` and reports whether any kernel launched by this library on the current
  * device recorded a device-side error: a bounded wait that ran out (SMAT_ERR_DEVICE_WAIT), or BCSR
- * arrays found inconsistent while a plan was built -- row pointers that are not monotone or exceed
- * nonzeroBlocks, a block column outside the matrix or out of order (SMAT_ERR_RANGE; such input gets
- * an empty or partial plan instead of an out-of-bounds write).  Clears the device status words (the
- * allocating entry points' and the static entry point's).
+ * arrays found inconsistent while a plan was built or by a product without one -- row pointers of the
+ * range that end before they begin, are negative or exceed nonzeroBlocks, a block column outside the
+ * matrix, or block columns out of order (SMAT_ERR_RANGE; such input gets an empty or partial plan or
+ * product instead of an out-of-bounds access).  Order is looked at window by window of 16384
+ * block-columns: a block must not lie in an earlier window than the one before it in its block-row;
+ * inside a window the order does not show in the product and is not reported.  Clears the device status
+ * words (the allocating entry points' and the static entry point's).
  * The reference never checks its launches (src/cuda_hgemm/src/mma/mmaCBT.cu:87). */
 int smat_device_status(void* stream);
 

@@ -39,12 +39,13 @@ constexpr int kPlanThreads = RG * 32;
 // Block-columns per pass, a template parameter WIN: 16384 (64 KB of masks + 64 KB of block prefixes), or as few as the matrix
 // has.  Masks are cleared and scanned for the whole window, so a window of 16384 for a matrix of 1024 block-columns left the
 // scan to 32 of the 512 threads, each with eight quads one after the other.
-constexpr int kWindow = 16384;
+constexpr int kWindow = kOrderWindow;
 
 // Fills masks[0..WIN) for block-columns [w0, w0 + WIN) of the group; cursor[] (one per warp,
 // kept by lane 0 semantics via registers) walks each row once over all windows.
-// A block column below the window start (columns not ascending, or negative) or beyond the matrix is not marked; the
-// status word then tells the host that the structure is inconsistent.
+// A block column below the window start (columns not ascending, or negative) or beyond the matrix is not marked, and a
+// batch of 32 in which one of this window follows one of a later window is not consumed whole; the status word then
+// tells the host that the structure is inconsistent.
 template <int THREADS, int WIN>
 __device__ __forceinline__ void mark_window(const int* __restrict__ colidx, int& cur, int end, int w0, int Kb, uint32_t* masks,
                                             int warp, int lane, int* status) {
@@ -62,6 +63,7 @@ __device__ __forceinline__ void mark_window(const int* __restrict__ colidx, int&
         if (in && cb >= w0) atomicOr(&masks[cb - w0], 1u << warp);
         else if (in && status) atomicCAS(status, 0, kStatusBadColumns);
         const uint32_t b = __ballot_sync(0xffffffffu, in);
+        if (lane == 0 && status && (b & (b + 1u))) atomicCAS(status, 0, kStatusBadColumns);
         cur += __popc(b);
         if (b != 0xffffffffu) break;
     }

@@ -68,9 +68,12 @@ int static_status_take(int* out);
 
 // Device status codes (the word kernels set): 1..99 a bounded wait ran out at that wait site; 100.. the input
 // structure is inconsistent (101: row pointers disagree with the number of blocks, 102: a block column is out of range
-// or the columns of a block-row are not ascending).
+// or the columns of a block-row are not ascending, see kOrderWindow).
 constexpr int kStatusBadRowptr = 101;
 constexpr int kStatusBadColumns = 102;
+// Most block-columns that the plan kernels look at together.  Inside such a window they sort for themselves, so the order of
+// a block-row's columns shows nowhere; a block in an earlier window than the block before it is refused, by every kernel.
+constexpr int kOrderWindow = 16384;
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point lookup (no link against libcuda).
 int encode_tensor_map_2d_f16(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint64_t row_pitch_bytes,

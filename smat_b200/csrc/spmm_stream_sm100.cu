@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
     ptx::pdl_wait();
     // ---- the piece: blocks [b0, b1) of block-row `row`; count > 1: one of `count` pieces of a long block-row ----
     int row = 0, b0 = 0, b1 = 0, count = 1, my_slot = 0, first_slot = 0;
+    int after = 0;  // no plan: the blocks behind this one follow another block of their block-row
     bool live = piece < p.n_pieces;
     if (live) {
         if (PLAN) {
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
                 row = piece;
                 b0 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + row), lo), hi);
                 b1 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + row + 1), b0), hi);
+                after = b0;
                 if (b1 - b0 > p.chunk && p.long_rows) {
                     my_slot = first_slot = __ldg(p.row_slot + row);
                     count = (b1 - b0 + p.chunk - 1) / p.chunk;
@@ -94,6 +96,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
                 if (live) {
                     const uint4 d = __ldg(p.pieces + (piece - n_rows));
                     row = (int)d.x; b0 = (int)d.y; b1 = (int)d.z; my_slot = (int)d.w;
+                    after = b0 - 1;
                     const int2 s = __ldg(p.slots + my_slot);
                     first_slot = s.x; count = s.y;
                 }
@@ -142,9 +145,13 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
     auto load_cols = [&](int at) {
         cols_at = at;
         int c = (at + lane < c1) ? __ldg(p.colidx + at + lane) >> (PLAN ? 0 : 4) : 0;
-        if (!PLAN && (c < 0 || c >= Kb)) {
-            atomicCAS(p.status, 0, kStatusBadColumns);
-            c = -1;
+        if (!PLAN) {
+            // (what plan creation refuses is refused here as well)
+            bool bad = c < 0 || c >= Kb;
+            if (Kb > kOrderWindow && at + lane < c1 && at + lane > after)
+                bad |= c / kOrderWindow < (__ldg(p.colidx + at + lane - 1) >> 4) / kOrderWindow;
+            if (bad) atomicCAS(p.status, 0, kStatusBadColumns);
+            if (c < 0 || c >= Kb) c = -1;
         }
         cols = c;
         // what the warp will read of A after this batch of 32 blocks is on its way to L2 meanwhile

@@ -1,5 +1,5 @@
 """Edges of the plan builder's and the launchers' choices: windows of block-columns, low tall groups, column chunks of the
-host-buffer product, value updates of a range -- each against the CPU oracle."""
+host-buffer product, value updates of a range -- each against the CPU oracle; what every route refuses."""
 import numpy as np
 import pytest
 
@@ -86,3 +86,54 @@ def test_host_buffers_by_column_chunks(N, pinned):
         torch.cuda.synchronize()
         assert _error(C_host.numpy().view(np.float16), brp, bci, bv, B_nk, (0, 50)) <= TOL
     plan.close()
+
+
+# (variant, entry): the kernels that see the boundary's arrays first -- plan kernels of both walk orders, stream kernel
+ROUTES = [(0, "call"), (1, "call"), (5, "call"), (1, "static"), (5, "static"), (0, "plan"), (1, "plan"), (4, "plan"), (5, "plan")]
+
+
+def _status_of(route, A, B, C):
+    import torch
+    variant, entry = route
+    L, stream, (N, K) = S.lib(), torch.cuda.current_stream().cuda_stream, B.data.shape
+    S.set_variant(variant)
+    try:
+        if entry == "plan":
+            plan = S.Plan(A, n_hint=N)
+            plan.spmm(B, C)
+            rc = L.smat_device_status(stream)
+            plan.close()
+        else:
+            S.spmm(A, B, C) if entry == "call" else S.api._check(L.smat_spmm_bcsr_f16_static(
+                A.getBcsrValues(), A.getBcsrRowPtr(), A.getBcsrColIdx(), B.data.data_ptr(), C.data.data_ptr(), A.M, N, K, A.nnzb, stream))
+            rc = L.smat_device_status(stream)
+    finally:
+        S.set_variant(0)
+    assert L.smat_device_status(stream) == 0
+    return rc
+
+
+@pytest.mark.parametrize("route", ROUTES)
+@pytest.mark.parametrize("late,early", [(1, 1), (40, 1), (300, 3)])
+def test_block_columns_out_of_order_are_reported_by_every_kernel(route, late, early):
+    """A block-row whose first `late` blocks lie in the second window of 16384 block-columns and whose next `early` ones in
+    the first: within 32 columns read together, across two such batches, across the warps and pieces of a long row."""
+    Kb, N = 20000, 16
+    good = np.sort(np.random.default_rng(late).choice(Kb, 9, replace=False))
+    cols = [good, np.concatenate([16384 + 7 * np.arange(late), 5 + np.arange(early)]), good]
+    brp = np.cumsum([0] + [len(c) for c in cols]).astype(np.int32)
+    bci = (np.concatenate(cols) * 16).astype(np.int32)
+    A = S.SparseMatrix.from_bcsr(48, Kb * 16, brp, bci, np.ones(brp[-1] * 256, np.float16))
+    B, C = S.Matrix(N, Kb * 16, fill=1.0), S.Matrix(48, N, fill=0.0)
+    assert _status_of(route, A, B, C) == -6 and b"ascending" in S.lib().smat_last_error_string()
+
+
+@pytest.mark.parametrize("route", ROUTES)
+def test_order_inside_a_window_does_not_matter(route):
+    rng = np.random.default_rng(8)
+    brp, bci, bv, B_nk = _problem(3, 40, 700, 16, 60)
+    order = np.concatenate([rng.permutation(np.arange(brp[r], brp[r + 1])) for r in range(40)])
+    A = S.SparseMatrix.from_bcsr(640, 11200, brp, bci[order], bv.reshape(-1, 256)[order].reshape(-1))
+    C = S.Matrix(640, 16, fill=float("nan"))
+    assert _status_of(route, A, S.Matrix.from_host(B_nk), C) == 0
+    assert _error(C.data.cpu().numpy(), brp, bci, bv, B_nk, (0, 40)) <= TOL
