@@ -27,6 +27,7 @@
 #include <queue>
 #include <algorithm>
 
+#include "host_range.h"
 #include "ptx_sm100.cuh"
 #include "smat_internal.h"
 #include "spmm_stream.h"
@@ -675,17 +676,35 @@ static __global__ void __launch_bounds__(256) copy_out_kernel(const uint4* __res
     }
 }
 
-// The device's address of `bytes` of host memory, or null when it is not pinned (then only the copy engine can reach it).
+// The device's address of `bytes` of host memory, or null when not all of it is pinned (then only the copy engine can reach it).
 static char* device_view_of_host(void* p, size_t bytes) {
-    cudaPointerAttributes first, last;
-    if (((uintptr_t)p & 15) || cudaPointerGetAttributes(&first, p) != cudaSuccess ||
-        cudaPointerGetAttributes(&last, static_cast<char*>(p) + bytes - 1) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer || !last.devicePointer) return nullptr;
-    if (static_cast<char*>(last.devicePointer) - static_cast<char*>(first.devicePointer) != (ptrdiff_t)(bytes - 1)) return nullptr;
-    return static_cast<char*>(first.devicePointer);
+    if ((uintptr_t)p & 15) return nullptr;
+    typedef CUresult (*AttributeFn)(void*, CUpointer_attribute, CUdeviceptr);
+    static const AttributeFn attribute = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return (AttributeFn)fn;
+    }();
+    if (!attribute) return nullptr;
+    return device_view_of_range(p, bytes, [](uintptr_t at, HostMapping* m) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, reinterpret_cast<void*>(at)) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        CUdeviceptr base = 0;
+        if (a.type != cudaMemoryTypeHost || attribute(&base, CU_POINTER_ATTRIBUTE_MAPPING_BASE_ADDR, at) != CUDA_SUCCESS ||
+            attribute(&m->size, CU_POINTER_ATTRIBUTE_MAPPING_SIZE, at) != CUDA_SUCCESS)
+            return false;
+        m->base = base;
+        m->device = static_cast<char*>(a.devicePointer);
+        return true;
+    });
 }
 
 // A plan's memory and tuning belong to the device it was created on.

@@ -88,6 +88,28 @@ def test_host_buffers_by_column_chunks(N, pinned):
     plan.close()
 
 
+def test_part_of_a_pinned_buffer_is_stored_to_by_the_kernels():
+    """C inside a larger pinned allocation goes out by columns (a store kernel per chunk), as a whole allocation does; the
+    same buffer in pageable memory takes no such kernel."""
+    import torch
+    brp, bci, bv, B_nk = _problem(11, 50, 90, 200, 30)
+    plan = S.Plan(S.SparseMatrix.from_bcsr(800, 1440, brp, bci, bv), n_hint=200)
+    B_host = torch.from_numpy(B_nk.view(np.int16)).pin_memory()
+    launches = {}
+    for name, flat in (("pinned", torch.empty(800 * 200 + 4096, dtype=torch.int16).pin_memory()),
+                       ("pageable", torch.empty(800 * 200 + 4096, dtype=torch.int16))):
+        C_host = flat[2048:2048 + 800 * 200].view(800, 200)
+        flat.fill_(-1)
+        before = S.launch_count()
+        plan.spmm_host(B_host, C_host)
+        torch.cuda.synchronize()
+        launches[name] = S.launch_count() - before
+        assert _error(C_host.numpy().view(np.float16), brp, bci, bv, B_nk, (0, 50)) <= TOL
+        assert bool((flat[:2048] == -1).all()) and bool((flat[2048 + 800 * 200:] == -1).all())
+    plan.close()
+    assert launches["pinned"] >= 4 and launches["pinned"] > launches["pageable"]
+
+
 # (variant, entry): the kernels that see the boundary's arrays first -- plan kernels of both walk orders, stream kernel
 ROUTES = [(0, "call"), (1, "call"), (5, "call"), (1, "static"), (5, "static"), (0, "plan"), (1, "plan"), (4, "plan"), (5, "plan")]
 

@@ -40,6 +40,52 @@ def test_partial_tiles_are_published_by_the_whole_warp():
     assert re.search(ordered, after[:after.index("__ldcg(src")])
 
 
+def test_host_range_is_pinned_from_end_to_end(tmp_path):
+    """host_range.h decides whether a kernel may store to the caller's C: compiled with a fake of the driver's answers.  A hole
+    between two pinned ends, a last page that is not pinned and a view the device sees in two places are refused."""
+    import subprocess
+    (tmp_path / "t.cpp").write_text(r"""
+#include "host_range.h"
+#include <cstdio>
+#include <vector>
+struct Pinned { uintptr_t base; size_t size; ptrdiff_t shift; };
+static bool view(std::vector<Pinned> all, uintptr_t p, size_t bytes, ptrdiff_t shift) {
+    int asked = 0;
+    char* v = smat::device_view_of_range((void*)p, bytes, [&](uintptr_t at, smat::HostMapping* m) {
+        asked++;
+        for (auto& x : all)
+            if (at >= x.base && at < x.base + x.size) { *m = {x.base, x.size, (char*)(at + x.shift)}; return true; }
+        return false;
+    });
+    return v && v == (char*)(p + shift) && asked <= 16;
+}
+int main() {
+    const uintptr_t P = 0x10000;
+    std::vector<Pinned> many;
+    for (int i = 0; i < 17; i++) many.push_back({P + i * 0x1000, 0x1000, 0});
+    bool ok[] = {
+        view({{P, 0x3000, 0}}, P, 0x3000, 0),                                     // exactly the mapping
+        view({{P, 0x3000, 64}}, P + 0x110, 0x1000, 64),                           // inside it, another device address
+        view({{P, 0x1000, 0}, {P + 0x1000, 0x2000, 0}}, P, 0x3000, 0),            // two side by side
+        view({{P, 1, 0}}, P, 1, 0),
+        view(many, P, 16 * 0x1000, 0),
+        !view({{P, 0x1000, 0}, {P + 0x2000, 0x1000, 0}}, P, 0x3000, 0),           // a hole between pinned ends
+        !view({{P, 0x2000, 0}}, P, 0x2001, 0),                                    // one byte beyond
+        !view({{P, 0x1000, 0}, {P + 0x1000, 0x2000, 64}}, P, 0x3000, 0),          // two places on the device
+        !view({}, P, 16, 0),
+        !view(many, P, 17 * 0x1000, 0),                                           // more mappings than are looked at
+    };
+    for (bool b : ok) putchar(b ? '1' : '0');
+}
+""")
+    exe = str(tmp_path / "t")
+    subprocess.check_call(["g++", "-std=c++17", "-I", os.path.join(ROOT, "smat_b200", "csrc"), "-o", exe, str(tmp_path / "t.cpp")])
+    assert subprocess.check_output([exe]) == b"1" * 10
+    plan = open(os.path.join(ROOT, "smat_b200", "csrc", "plan.cu")).read()
+    body = plan[plan.index("static char* device_view_of_host("):plan.index("static int check_plan_device")]
+    assert "device_view_of_range(p, bytes," in body
+
+
 def test_no_gpu_means_loud_failure_not_fallback():
     import torch
     if torch.cuda.is_available():
