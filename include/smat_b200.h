@@ -88,7 +88,9 @@ int smat_spmm_bcsr_f16_static(const void* bcsrValuesA, const int* bcsrRowPtrA, c
 typedef struct smat_plan smat_plan;
 /* N_hint: the number of columns of B the plan will mostly be used with (0 = unknown).  It only steers
  * how many block-rows form a work item (8 to 24) and which of the kernels multiplies, so that small matrices or
- * shards still fill the SMs.
+ * shards still fill the SMs.  Any N may be multiplied: where the kernel for N_hint columns is not the one for wide
+ * products of the matrix, the plan holds the walk orders and blocks of both (twice the memory, if the device has it;
+ * smat_plan_set_values refreshes both) and each product takes the kernel estimated to be faster at its width.
  * A plan also owns scratch for work items that a launch computes in segments (38.8 MB on a 148-SM device, twice
  * that for matrices whose work is very unevenly spread over the block-rows) and may be used by one stream at a
  * time. */
@@ -110,7 +112,7 @@ int smat_plan_spmm(const smat_plan* plan, const void* B, void* C, size_t N, void
  * (src/cuda_hgemm/src/common/matrix.h:88-101). */
 int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_t N, void* stream);
 int smat_plan_destroy(smat_plan* plan);
-/* What a plan turned out to be (informational, no reference counterpart): *rows_per_item = block-rows of a work item
+/* What a plan turned out to be for N_hint columns (informational, no reference counterpart): *rows_per_item = block-rows of a work item
  * (8..16: the kernel that reads both operands from shared memory; 12..24 with *tall = 1: the kernel that reads the
  * B panels from tensor memory; 1: the kernel that walks single block-rows), *steps = steps of the walk order (pieces of
  * block-rows for the last kernel).  Any pointer may be NULL. */

@@ -505,6 +505,16 @@ PlanSizes plan_sizes(size_t nnzb, size_t brow_begin, size_t brow_end, size_t rg,
     return s;
 }
 
+double tc_estimate_us(const PlanView& v, size_t N, size_t sms) {
+    const size_t items = v.n_groups * ((N + 127) / 128);
+    const double per_group = (double)v.total_steps / (double)v.n_groups;
+    double cycles;
+    if (v.tall) cycles = tall_rounds(items, sms, per_group) * per_group * v.step_cycles + kTallExtraCycles;
+    else if (v.balanced || v.sched_list) cycles = (double)items / (double)sms * per_group * v.step_cycles;
+    else cycles = rounds_for(items, sms, true, (size_t)per_group, false) * per_group * v.step_cycles;
+    return 8.0 + cycles / 1850.0;
+}
+
 // Launches a plan kernel with the smallest window that holds the matrix, with as many CTAs as fit the SMs.
 template <int THREADS, class Launch>
 static int launch_windowed(size_t Kb, size_t n_groups, int words_per_column, int sm_count, Launch&& launch) {
@@ -636,7 +646,13 @@ int plan_fill_tall_async(const int* rowptr, const int* colidx, size_t K, size_t 
 using namespace smat;
 
 struct smat_plan {
-    PlanView v;
+    PlanView v;          // for products about as wide as the hint
+    // A stream plan of a matrix on which a tcgen05 kernel is faster for wide products: the plan of that kernel, for the products
+    // that are (the kernel is picked by the width of each product; smat_plan_set_values keeps both up to date).
+    PlanView wide;
+    bool has_wide = false;
+    size_t n_hint = 0;
+    int sms = 0;
     void* buffer = nullptr;
     void* gsp_buffer = nullptr;
     void* fix_buffer = nullptr;  // partial tiles of cut work items
@@ -705,6 +721,39 @@ static char* device_view_of_host(void* p, size_t bytes) {
         m->device = static_cast<char*>(a.devicePointer);
         return true;
     });
+}
+
+// What multiplies N columns: the hint steers which plans there are, the two estimates which of them is used.  They are off by
+// some 20 %, so the kernel for the hint stays until the other's is lower by that: dense clusters of 131072 rows planned for 8
+// columns and used with 16 take 16.6 us with it, 25.7 with the other kernel, whose estimate is the lower one.  Where it is
+// wider than that, the other kernel it is: 8192 x 28672 layer planned for 16 columns, 2048 columns in 2560 us by passes of
+// 128, in 484 by it; 256 columns 318 and 73.
+static const PlanView& view_for(const smat_plan* p, size_t N) {
+    if (!p->has_wide) return p->v;
+    const PlanView& v = p->v;
+    return stream_passes_us(N, p->n_hint, v.brow_end - v.brow_begin, v.nnzb, v.K, p->sms) < 1.25 * tc_estimate_us(p->wide, N, (size_t)p->sms) ? v : p->wide;
+}
+
+static cudaError_t free_plan(smat_plan* p) {
+    cudaError_t e = cudaSuccess;
+    for (void* b : {p->buffer, p->gsp_buffer, p->fix_buffer, p->sched_buffer, p->stream.buffer}) {
+        const cudaError_t eb = cudaFree(b);
+        if (e == cudaSuccess) e = eb;
+    }
+    delete p;
+    return e;
+}
+
+// The stream plan of the range that `of` describes, in place of it or beside it, in `p`'s buffers; `out` becomes its view.
+static int build_stream_view(smat_plan* p, const PlanView& of, bool beside, PlanView& out, const int* h_rowptr, const void* vals, const int* colidx,
+                             cudaStream_t stream) {
+    out.K = of.K;
+    out.nnzb = of.nnzb;
+    out.brow_begin = of.brow_begin;
+    out.brow_end = of.brow_end;
+    if (int rc = stream_plan_build(p->stream, out, h_rowptr, vals, colidx, p->n_hint, p->sms, beside ? &of : nullptr, stream)) return rc;
+    out.total_steps = (size_t)p->stream.row_piece.back();
+    return SMAT_OK;
 }
 
 // A plan's memory and tuning belong to the device it was created on.
@@ -836,17 +885,15 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     // already).  Both plans are counted and the estimates compared; smat_spmm_set_variant(4) forces a tall plan,
     // 1..3 exclude it.
     const double mma_per_step = total_steps > 0 ? (double)mmas16 / (double)total_steps : 0.0;
-// cycles of a 16-row step: an MMA per block or pair of vertical neighbours, or, where whole columns of blocks are there
+    // cycles of a 16-row step: an MMA per block or pair of vertical neighbours, or, where whole columns of blocks are there
     // (dense clusters), one per column
     const bool vertical = mmas16 > 0 && (double)range_blocks >= 1.7 * (double)mmas16;
     const double work16 = vertical ? 20.0 * (double)range_blocks / (double)(total_steps > 0 ? total_steps : 1) : 58.0 * mma_per_step;
     const double step16 = work16 > 480.0 ? work16 : 480.0;
     bool tall = false;
-    double est_cycles = 0.0;  // of the tcgen05 kernel that would be taken
     size_t rg_used = rg;
     const size_t rows = brow_end - brow_begin, tiles = ((N_hint ? N_hint : 128) + 127) / 128;
     const bool tall_forced = g_spmm_variant == 4;
-    const double kTallExtraCycles = 5000.0;  // of a launch: its pipeline takes longer to fill and to drain (measured, smallest plans)
     const bool tall_possible = rc == SMAT_OK && !balanced && !p->v.sched_list && total_steps > 0 && rows > 0 &&
                                (tall_forced || (g_spmm_variant == 0 && rows >= 12 && N_hint >= 16 &&
                                                 (size_t)total_steps * tiles >= 16 * (size_t)ctx->sm_count));
@@ -899,7 +946,6 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
                     tall_step_cycles((double)range_blocks / (double)(tall_total_and_max[0] > 0 ? tall_total_and_max[0] : 1)) +
                 kTallExtraCycles;
             tall = tall_forced || est_tall < est16;
-            est_cycles = tall ? est_tall : est16;
             if (std::getenv("SMAT_PLAN_DEBUG"))
                 fprintf(stderr, "[smat plan] estimates: 16-row %.0f cycles, tall (rg %zu, %d steps) %.0f cycles -> %s\n", est16, rg_tall,
                         tall_total_and_max[0], est_tall, tall ? "tall" : "16-row");
@@ -917,46 +963,57 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
             cudaFree(gsp_tall);
         }
     }
-    // Stream plan (spmm_stream_sm100.cu): taken where its estimate is below that of the kernel chosen so far.
+    const int steps_final = total_and_max[0];
+    PlanView& v = p->v;
+    p->n_hint = N_hint ? N_hint : 128;
+    p->sms = ctx->sm_count;
+    v.rowptr = bcsrRowPtrA;
+    v.gsp = gsp;
+    v.K = K;
+    v.nnzb = range_blocks;  // blocks of the plan's range
+    v.brow_begin = brow_begin;
+    v.brow_end = brow_end;
+    v.n_groups = sz.n_groups;
+    v.rg = rg_used;
+    v.total_steps = (size_t)(steps_final > 0 ? steps_final : 0);
+    v.balanced = balanced;
+    v.cap = cap;
+    v.vertical = vertical;
+    v.tall = tall;
+    v.step_cycles = tall ? tall_step_cycles((double)range_blocks / (double)(steps_final > 0 ? steps_final : 1)) : step16;
+    // Stream plan (spmm_stream_sm100.cu): taken where its estimate is below that of the kernel chosen so far.  That one is kept
+    // beside it unless its estimate loses for wide products too: each pass over the matrix with the stream kernel multiplies
+    // 128 columns or as many as the hint names, so a plan made for 16 columns would take 32 passes for 4096.
+    std::vector<int> h_rowptr;
+    bool stream_too = false;
     if (rc == SMAT_OK && total_steps > 0 && (g_spmm_variant == 5 || (g_spmm_variant == 0 && N_hint > 0))) {
-        const double us = stream_estimate_us(N_hint ? N_hint : 128, rows, range_blocks, K, ctx->sm_count, true);
-        if (est_cycles == 0.0) {
-            const double per_group = (double)total_steps / (double)sz.n_groups;
-            const double rounds = balanced || p->v.sched_list ? (double)(sz.n_groups * tiles) / (double)ctx->sm_count
-                                                              : rounds_for(sz.n_groups * tiles, (size_t)ctx->sm_count, true, (size_t)per_group, false);
-            est_cycles = rounds * per_group * step16;
-        }
-        const double other = 8.0 + est_cycles / 1850.0;
-        const bool take = g_spmm_variant == 5 || us < other;
-        if (std::getenv("SMAT_PLAN_DEBUG")) fprintf(stderr, "[smat plan] stream %.1f us, %s %.1f us\n", us, tall ? "tall" : "16-row", other);
-        if (take) {
-            std::vector<int> h_rowptr(rows + 1);
+        const size_t wide = std::max<size_t>(p->n_hint, 4096);
+        const double us = stream_estimate_us(p->n_hint, rows, range_blocks, K, ctx->sm_count, true), other = tc_estimate_us(v, p->n_hint, (size_t)ctx->sm_count);
+        const double us_wide = stream_passes_us(wide, p->n_hint, rows, range_blocks, K, ctx->sm_count), other_wide = tc_estimate_us(v, wide, (size_t)ctx->sm_count);
+        if (std::getenv("SMAT_PLAN_DEBUG"))
+            fprintf(stderr, "[smat plan] stream %.1f us, %s %.1f us; %zu columns: %.1f, %.1f us\n", us, tall ? "tall" : "16-row", other, wide, us_wide, other_wide);
+        if (g_spmm_variant == 5 || us < other) {
+            h_rowptr.resize(rows + 1);
             e = cudaMemcpyAsync(h_rowptr.data(), bcsrRowPtrA + brow_begin, (rows + 1) * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
             if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
-            if (rc == SMAT_OK && std::is_sorted(h_rowptr.begin(), h_rowptr.end())) {
-                p->v.K = K;
-                p->v.nnzb = range_blocks;
-                p->v.brow_begin = brow_begin;
-                p->v.brow_end = brow_end;
-                rc = stream_plan_build(p->stream, p->v, h_rowptr.data(), bcsrValuesA, bcsrColIdxA, N_hint ? N_hint : 128, ctx->sm_count,
-                                       (cudaStream_t)stream);
+            stream_too = rc == SMAT_OK && std::is_sorted(h_rowptr.begin(), h_rowptr.end());
+            if (stream_too && (g_spmm_variant == 5 || us_wide < other_wide)) {
                 cudaFree(p->gsp_buffer);
                 cudaFree(p->sched_buffer);
                 p->gsp_buffer = p->sched_buffer = nullptr;
-                p->v.sched_list = p->v.sched_off = nullptr;
-                p->v.total_steps = p->stream.row_piece.empty() ? 0 : (size_t)p->stream.row_piece.back();
+                PlanView only;
+                rc = build_stream_view(p, v, false, only, h_rowptr.data(), bcsrValuesA, bcsrColIdxA, (cudaStream_t)stream);
                 if (rc) {
-                    cudaFree(p->stream.buffer);
-                    delete p;
-                    return rc;
+                    free_plan(p);
+                    return rc == SMAT_ERR_NOMEM ? SMAT_ERR_CUDA : rc;
                 }
+                v = only;
                 *out = p;
                 return SMAT_OK;
             }
         }
     }
-    const int steps_final = total_and_max[0];
     if (std::getenv("SMAT_PLAN_DEBUG"))
         fprintf(stderr, "[smat plan] rows %zu blocks %zu: 16-row plan rg %zu steps %d cap %zu balanced %d listed %d; tall %d rg %zu steps %d max/group %d\n",
                 brow_end - brow_begin, range_blocks, rg, total_steps, cap, (int)balanced, p->v.sched_list != nullptr, (int)tall, rg_used,
@@ -971,49 +1028,49 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
     }
     if (rc) {
-        cudaFree(p->gsp_buffer);
-        cudaFree(p->fix_buffer);
-        cudaFree(p->sched_buffer);
-        delete p;
+        free_plan(p);
         return rc;
     }
     char* b = static_cast<char*>(p->buffer);
     p->nnzb = nnzb;
-    p->v.rowptr = bcsrRowPtrA;
-    p->v.gsp = gsp;
-    p->v.steps = b;
-    p->v.blk = reinterpret_cast<int*>(b + sz.steps_bytes);
-    p->v.packed = b + sz.steps_bytes + sz.blk_bytes;
-    p->v.K = K;
-    p->v.nnzb = range_blocks;  // blocks of the plan's range
-    p->v.brow_begin = brow_begin;
-    p->v.brow_end = brow_end;
-    p->v.n_groups = sz.n_groups;
-    p->v.rg = rg_used;
-    p->v.fix_scratch = static_cast<float*>(p->fix_buffer);
-    p->v.total_steps = (size_t)(steps_final > 0 ? steps_final : 0);
-    p->v.balanced = balanced;
-    p->v.cap = cap;
-    p->v.vertical = vertical;
-    p->v.tall = tall;
+    v.steps = b;
+    v.blk = reinterpret_cast<int*>(b + sz.steps_bytes);
+    v.packed = b + sz.steps_bytes + sz.blk_bytes;
+    v.fix_scratch = static_cast<float*>(p->fix_buffer);
+    if (stream_too) {  // places without a block stay marked as such (stream_plan_build)
+        e = cudaMemsetAsync(const_cast<int*>(v.blk), 0xff, sz.blk_bytes, (cudaStream_t)stream);
+        if (e != cudaSuccess) {
+            free_plan(p);
+            return fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
+        }
+    }
     if (tall) {
         // behind the step records, in the same region: the per-step words (only read while the plan is built), then the per-pair lists
         char* wstep = b + (size_t)(steps_final > 0 ? steps_final : 1) * 16;
-        p->v.winfo = wstep + (size_t)(steps_final > 0 ? steps_final : 1) * 64;
-        rc = plan_fill_tall_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg_used, gsp, const_cast<void*>(p->v.steps), wstep,
-                                  const_cast<void*>(p->v.winfo), const_cast<int*>(p->v.blk), (cudaStream_t)stream);
+        v.winfo = wstep + (size_t)(steps_final > 0 ? steps_final : 1) * 64;
+        rc = plan_fill_tall_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg_used, gsp, const_cast<void*>(v.steps), wstep,
+                                  const_cast<void*>(v.winfo), const_cast<int*>(v.blk), (cudaStream_t)stream);
     } else {
-        rc = plan_fill_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg, gsp, const_cast<void*>(p->v.steps),
-                             const_cast<int*>(p->v.blk), (cudaStream_t)stream, nullptr, cap);
+        rc = plan_fill_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg, gsp, const_cast<void*>(v.steps),
+                             const_cast<int*>(v.blk), (cudaStream_t)stream, nullptr, cap);
     }
-    if (rc == SMAT_OK)
-        rc = pack_values_async(bcsrRowPtrA, bcsrValuesA, p->v.blk, const_cast<void*>(p->v.packed), brow_begin, brow_end, nnzb, (cudaStream_t)stream);
+    bool packed = false;
+    if (rc == SMAT_OK && stream_too) {
+        PlanView narrow;
+        rc = build_stream_view(p, v, true, narrow, h_rowptr.data(), bcsrValuesA, bcsrColIdxA, (cudaStream_t)stream);
+        if (rc == SMAT_OK) {
+            p->wide = v;
+            p->has_wide = packed = true;
+            v = narrow;
+        } else if (rc == SMAT_ERR_NOMEM) {  // no room for the second copy of the blocks: all products with the first
+            clear_error();
+            rc = SMAT_OK;
+        }
+    }
+    if (rc == SMAT_OK && !packed)
+        rc = pack_values_async(bcsrRowPtrA, bcsrValuesA, v.blk, const_cast<void*>(v.packed), brow_begin, brow_end, nnzb, (cudaStream_t)stream);
     if (rc) {
-        cudaFree(p->buffer);
-        cudaFree(p->gsp_buffer);
-        cudaFree(p->fix_buffer);
-        cudaFree(p->sched_buffer);
-        delete p;
+        free_plan(p);
         return rc;
     }
     *out = p;
@@ -1025,11 +1082,7 @@ int smat_plan_set_values(smat_plan* plan, const void* bcsrValuesA, void* stream)
     if (!plan || (plan->v.nnzb && !bcsrValuesA)) return fail(SMAT_ERR_BAD_ARG, "NULL argument");
     if ((uintptr_t)bcsrValuesA & 15) return fail(SMAT_ERR_BAD_ARG, "bcsrValuesA must be 16-byte aligned");
     if (int rc = check_plan_device(plan)) return rc;
-    if (plan->v.stream) {
-        DeviceCtx* ctx = nullptr;
-        if (int rc = get_device_ctx(&ctx)) return rc;
-        return stream_plan_values(plan->v, bcsrValuesA, nullptr, ctx->sm_count, (cudaStream_t)stream);
-    }
+    if (plan->v.stream) return stream_plan_values(plan->v, bcsrValuesA, nullptr, plan->sms, (cudaStream_t)stream);
     // (the row pointers were checked against the whole arrays' block count, which only bounds what the kernel may read)
     return pack_values_async(plan->v.rowptr, bcsrValuesA, plan->v.blk, const_cast<void*>(plan->v.packed), plan->v.brow_begin,
                              plan->v.brow_end, plan->nnzb, (cudaStream_t)stream);
@@ -1044,7 +1097,7 @@ int smat_plan_spmm(const smat_plan* plan, const void* B, void* C, size_t N, void
     if (((uintptr_t)B | (uintptr_t)C) & 15) return fail(SMAT_ERR_BAD_ARG, "B and C must be 16-byte aligned");
     if (N >= ((size_t)1 << 31)) return fail(SMAT_ERR_RANGE, "N beyond 2^31");
     if (int rc = check_plan_device(plan)) return rc;
-    return launch_spmm(plan->v, B, C, N, (cudaStream_t)stream);
+    return launch_spmm(view_for(plan, N), B, C, N, (cudaStream_t)stream);
 }
 
 int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_t N, void* stream) {
@@ -1072,14 +1125,15 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
     }
     chunk_at.push_back(N);
     const size_t n_chunks = chunk_at.size() - 1;
-    const size_t n_groups = plan->v.n_groups;
+    const PlanView& v = view_for(plan, W);
+    const size_t n_groups = v.n_groups;
     // ranges of the last chunk: each should still fill the SMs for about one round of work items (shorter launches
     // lose more to partly filled rounds than the overlap of the copy-out wins back); at most 4
     DeviceCtx* ctx = nullptr;
     if (int rc0 = get_device_ctx(&ctx)) return rc0;
     size_t n_ranges = (n_groups * ((W + 127) / 128) + (size_t)ctx->sm_count / 2) / (size_t)ctx->sm_count;
-    if (plan->v.stream) n_ranges = n_groups / 16 * ((W + 127) / 128) / (size_t)ctx->sm_count;
-    if (plan->v.sched_list || plan->v.balanced) n_ranges = 1;  // such plans balance a launch over all their groups
+    if (v.stream) n_ranges = n_groups / 16 * ((W + 127) / 128) / (size_t)ctx->sm_count;
+    if (v.sched_list || v.balanced) n_ranges = 1;  // such plans balance a launch over all their groups
     if (const char* e = std::getenv("SMAT_HOST_RANGES")) n_ranges = (size_t)std::atoi(e);  // tuning knob
     if (out_view) n_ranges = 1;
     if (n_ranges > 4) n_ranges = 4;
@@ -1133,7 +1187,7 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
         const size_t n0 = chunk_at[j], w = chunk_at[j + 1] - n0;
         SMAT_CUDA_TRY(cudaStreamWaitEvent(s, plan->ev_in[j], 0));
         if (out_view) {
-            if (int rc = launch_spmm(plan->v, Bd + n0 * K * 2, Cd + n0 * 2, w, s, nullptr, N)) return rc;
+            if (int rc = launch_spmm(v, Bd + n0 * K * 2, Cd + n0 * 2, w, s, nullptr, N)) return rc;
             SMAT_CUDA_TRY(cudaEventRecord(plan->ev_done[j], s));
             SMAT_CUDA_TRY(cudaStreamWaitEvent(plan->s_out, plan->ev_done[j], 0));
             const size_t words = rows * w / 8, ctas = (words + 1023) / 1024;
@@ -1145,14 +1199,14 @@ int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_
             continue;
         }
         if (j + 1 < n_chunks) {
-            if (int rc = launch_spmm(plan->v, Bd + n0 * K * 2, Cd + n0 * 2, w, s, nullptr, N)) return rc;
+            if (int rc = launch_spmm(v, Bd + n0 * K * 2, Cd + n0 * 2, w, s, nullptr, N)) return rc;
             continue;
         }
         for (size_t r = 0; r < n_ranges; r++) {
             const size_t g0 = n_groups * r / n_ranges, g1 = n_groups * (r + 1) / n_ranges;
-            const size_t row0 = g0 * plan->v.rg * 16;
-            const size_t row1 = (g1 * plan->v.rg * 16 < rows) ? g1 * plan->v.rg * 16 : rows;
-            if (int rc = launch_spmm(plan->v, Bd + n0 * K * 2, Cd + (row0 * N + n0) * 2, w, s, nullptr, N, g0, g1)) return rc;
+            const size_t row0 = g0 * v.rg * 16;
+            const size_t row1 = (g1 * v.rg * 16 < rows) ? g1 * v.rg * 16 : rows;
+            if (int rc = launch_spmm(v, Bd + n0 * K * 2, Cd + (row0 * N + n0) * 2, w, s, nullptr, N, g0, g1)) return rc;
             SMAT_CUDA_TRY(cudaEventRecord(plan->ev_done[r], s));
             SMAT_CUDA_TRY(cudaStreamWaitEvent(plan->s_out, plan->ev_done[r], 0));
             SMAT_CUDA_TRY(cudaMemcpyAsync(Ch + row0 * N * 2, Cd + row0 * N * 2, (row1 - row0) * N * 2, cudaMemcpyDeviceToHost,
@@ -1188,14 +1242,7 @@ int smat_plan_destroy(smat_plan* plan) {
         cudaFree(plan->host_B);
         cudaFree(plan->host_C);
     }
-    cudaError_t e = cudaFree(plan->buffer);
-    const cudaError_t e2 = cudaFree(plan->gsp_buffer);
-    const cudaError_t e3 = cudaFree(plan->fix_buffer);
-    cudaFree(plan->sched_buffer);
-    cudaFree(plan->stream.buffer);
-    if (e == cudaSuccess) e = e2;
-    if (e == cudaSuccess) e = e3;
-    delete plan;
+    const cudaError_t e = free_plan(plan);
     if (e != cudaSuccess) return fail(SMAT_ERR_CUDA, "cudaFree failed: %s", cudaGetErrorString(e));
     return SMAT_OK;
 }

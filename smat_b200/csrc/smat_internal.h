@@ -114,6 +114,8 @@ inline double tall_rounds(size_t items, size_t sms, double est_steps) {
 }
 // Cycles of a step of the tall kernel that holds `blocks` blocks (measured with 12 to 20 blocks a step: 544 to 640).
 inline double tall_step_cycles(double blocks) { return 350.0 + 15.0 * blocks > 500.0 ? 350.0 + 15.0 * blocks : 500.0; }
+// ... and what a launch of it costs beyond its steps: its pipeline takes longer to fill and to drain (measured, smallest plans).
+constexpr double kTallExtraCycles = 5000.0;
 // Measured cost of a 256-column item relative to a 128-column item of the same group.
 constexpr double kWideItemCost = 1.95;
 // Group height for a range of `block_rows` block-rows when C is N columns wide (0 = unknown): the height in
@@ -162,6 +164,7 @@ struct PlanView {
     size_t K = 0, nnzb = 0, brow_begin = 0, brow_end = 0, n_groups = 0, rg = kPlanRowsPerGroup;
     size_t total_steps = 0;  // number of steps of the range when the host knows it, else 0
     size_t cap = kPlanBlocksPerStep;  // most blocks of a step: kPlanBlocksPerStep or kPlanBlocksPerStepDense
+    double step_cycles = 0.0;  // what a step is estimated to take (tc_estimate_us)
     bool vertical = false;  // most blocks have a neighbour above or below in their block-column (dense clusters)
     // Tall plan: groups of rg <= kTallRows block-rows with an even number of steps, at most kTallBlocksPerStep blocks
     // per step.  A step record is {element column of the quad, position of the first block in the packed stream in
@@ -213,6 +216,9 @@ int plan_fill_tall_async(const int* rowptr, const int* colidx, size_t K, size_t 
 // group_begin.
 int launch_spmm(const PlanView& plan, const void* B, void* C, size_t N, cudaStream_t stream,
                 const DeviceCtx* ctx = nullptr, size_t ldc = 0, size_t group_begin = 0, size_t group_end = (size_t)-1);
+
+// Microseconds a product of N columns is estimated to take with a 16-row or tall plan whose steps are counted.
+double tc_estimate_us(const PlanView& plan, size_t N, size_t sms);
 
 // The view of groups [group_begin, group_end) of a plan (steps, blocks and row pointers are addressed absolutely, so
 // a sub-range is the same plan with its first group, first block-row and group count moved).

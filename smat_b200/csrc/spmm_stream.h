@@ -36,6 +36,9 @@ struct StreamShape {
 StreamShape stream_shape(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count, bool plan);
 bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count);
 double stream_estimate_us(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count, bool plan);
+// Columns a plan made for N_hint columns multiplies in one pass, and its estimate for N columns.
+inline size_t stream_pass_columns(size_t N_hint) { return (N_hint + 127) / 128 * 128; }
+double stream_passes_us(size_t N, size_t N_hint, size_t rows, size_t nnzb, size_t K, int sm_count);
 
 // What a plan for this kernel owns (PlanView::stream): the values in fragment order, the block-columns, the pieces.
 struct StreamPlan {
@@ -44,11 +47,16 @@ struct StreamPlan {
     void* slabs = nullptr;
     size_t n_cap = 0, first = 0;  // columns that scratch and slabs hold; position of the plan's first block in the boundary's arrays
     std::vector<int> row_piece;   // first piece of every block-row
+    // beside the plan of a tcgen05 kernel (null: none): its copy of the blocks, and every block's place there
+    void* walk = nullptr;
+    int* pos = nullptr;
 };
 // h_rowptr: the plan's row pointers on the host (block-rows brow_begin .. brow_end), checked to be monotone.
+// `walk`: the plan of a tcgen05 kernel that is kept beside this one (or null), its walk order filled (blk -1 where it holds no
+// block), its copy of the blocks filled here.  SMAT_ERR_NOMEM, and nothing launched, where the device has no room.
 int stream_plan_build(StreamPlan& sp, PlanView& v, const int* h_rowptr, const void* vals, const int* colidx, size_t N_hint, int sm_count,
-                      cudaStream_t stream);
-// New values into an existing plan (colidx null) or values and columns into a new one.
+                      const PlanView* walk, cudaStream_t stream);
+// New values into an existing plan (colidx null) or values and columns into a new one; into the plan beside it as well.
 int stream_plan_values(const PlanView& v, const void* vals, const int* colidx, int sm_count, cudaStream_t stream);
 int launch_stream(const PlanView& v, const void* B, void* C, size_t N, cudaStream_t stream, const DeviceCtx* ctx, size_t ldc,
                   size_t row_begin, size_t row_end);

@@ -312,19 +312,40 @@ __global__ void __launch_bounds__(256) long_rows_kernel(const int* __restrict__ 
 }
 
 // The plan's copy of the values in the order a warp's lanes read them (lane (g, t): rows g and g + 8, k = 4t .. 4t + 3), and
-// of the block columns; a column outside the matrix becomes -1.
+// of the block columns; a column outside the matrix becomes -1.  Where the plan holds the blocks in the walk order of a
+// tcgen05 kernel as well, block i also goes to place pos[i] of that copy, in its swizzled form (16-byte chunk index XOR bit 2
+// of the row): read once for both (183 000 blocks: 52 us, 64 with a kernel
+// for each, 33 for one copy alone).
 __global__ void __launch_bounds__(256) stream_pack_kernel(const uint2* __restrict__ vals, const int* __restrict__ colidx,
-                                                         uint4* __restrict__ packed, int* __restrict__ cols, int first, int n, int Kb) {
+                                                         uint4* __restrict__ packed, int* __restrict__ cols, int first, int n, int Kb,
+                                                         const int* __restrict__ pos, uint2* __restrict__ walk) {
     ptx::pdl_wait();
     const int lane = threadIdx.x & 31;
+    const int row = lane >> 2, chunk = 2 * row + ((lane >> 1) & 1), to = 2 * (chunk ^ ((row >> 2) & 1)) + (lane & 1);
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
         const uint2 lo = __ldg(vals + (size_t)(first + i) * 64 + lane), hi = __ldg(vals + (size_t)(first + i) * 64 + 32 + lane);
         packed[(size_t)i * 32 + lane] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        if (pos) {
+            const int p = __ldg(pos + i);
+            if (p >= 0) {
+                walk[(size_t)p * 64 + to] = lo;
+                walk[(size_t)p * 64 + 32 + to] = hi;
+            }
+        }
         if (cols && lane == 0) {
             const int c = __ldg(colidx + first + i) >> 4;
             cols[i] = (c >= 0 && c < Kb) ? c : -1;
         }
+    }
+}
+
+// pos[j] = place of block j in the walk order `blk` (both counted from the range's first block; -1 where it has none).
+__global__ void __launch_bounds__(256) walk_place_kernel(const int* __restrict__ blk, int* __restrict__ pos, int first, int n) {
+    ptx::pdl_wait();
+    for (int p = blockIdx.x * 256 + threadIdx.x; p < n; p += gridDim.x * 256) {
+        const int j = __ldg(blk + first + p) - first;
+        if (j >= 0 && j < n) pos[j] = p;
     }
 }
 
@@ -429,6 +450,12 @@ double stream_estimate_us(size_t N, size_t rows, size_t nnzb, size_t K, int sm_c
     return 4.0 + (s.slab ? 2.0 + 4e-6 * n * (double)K / 5.5 : 0.0) + (double)nnzb / sm_count * per_block * 1e-3 + (double)(rows * 16) * n * 2.0 / 6e6;
 }
 
+double stream_passes_us(size_t N, size_t N_hint, size_t rows, size_t nnzb, size_t K, int sm_count) {
+    const size_t cap = stream_pass_columns(N_hint), rest = N % cap;
+    return (double)(N / cap) * stream_estimate_us(cap, rows, nnzb, K, sm_count, true) +
+           (rest ? stream_estimate_us(rest, rows, nnzb, K, sm_count, true) : 0.0);
+}
+
 // A product without a plan takes this kernel unless building a plan inside the call and a tcgen05 kernel are estimated to be
 // faster: 24 us for the launches and small plan kernels, 0.2 ns per block for reading and writing it, and the product --
 // rounds of items at 0.26 us a step, or 20 ns per block, tile and SM, whichever is more.
@@ -448,7 +475,7 @@ bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count)
 }
 
 int stream_plan_build(StreamPlan& sp, PlanView& v, const int* h_rowptr, const void* vals, const int* colidx, size_t N_hint, int sm_count,
-                      cudaStream_t stream) {
+                      const PlanView* walk, cudaStream_t stream) {
     const size_t rows = v.brow_end - v.brow_begin, first = (size_t)h_rowptr[0], n = v.nnzb;
     const StreamShape s = stream_shape(N_hint, rows, n, v.K, sm_count, true);
     std::vector<uint4> pieces;
@@ -466,11 +493,16 @@ int stream_plan_build(StreamPlan& sp, PlanView& v, const int* h_rowptr, const vo
         }
     }
     sp.row_piece[rows] = (int)pieces.size();
-    sp.n_cap = (N_hint + 127) / 128 * 128;
+    sp.n_cap = stream_pass_columns(N_hint);
     const size_t pieces_bytes = round256(pieces.size() * sizeof(uint4)), slots_bytes = round256(slots.size() * sizeof(int2)),
                  counter_bytes = round256(slots.size() * (sp.n_cap / 8) * sizeof(int)), partial_bytes = round256(slots.size() * sp.n_cap * 64),
-                 cols_bytes = round256(n * sizeof(int)), packed_bytes = n * 512, slab_bytes = s.slab ? sp.n_cap * v.K * 2 : 0;
-    SMAT_CUDA_TRY(cudaMalloc(&sp.buffer, pieces_bytes + slots_bytes + counter_bytes + partial_bytes + cols_bytes + packed_bytes + slab_bytes));
+                 cols_bytes = round256(n * sizeof(int)), packed_bytes = n * 512, pos_bytes = walk ? cols_bytes : 0;
+    // slabs for the widest pass, whatever the hint: where a narrower one wants them the widest does too
+    const size_t slab_bytes = stream_shape(sp.n_cap, rows, n, v.K, sm_count, true).slab ? sp.n_cap * v.K * 2 : 0;
+    const cudaError_t e = cudaMalloc(&sp.buffer, pieces_bytes + slots_bytes + counter_bytes + partial_bytes + cols_bytes + pos_bytes + packed_bytes + slab_bytes);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    if (e != cudaSuccess)
+        return fail(e == cudaErrorMemoryAllocation ? SMAT_ERR_NOMEM : SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
     char* b = static_cast<char*>(sp.buffer);
     StreamArgs& a = sp.args;
     a = StreamArgs{};
@@ -479,6 +511,14 @@ int stream_plan_build(StreamPlan& sp, PlanView& v, const int* h_rowptr, const vo
     a.counters = reinterpret_cast<int*>(b); b += counter_bytes;
     a.partial = reinterpret_cast<float4*>(b); b += partial_bytes;
     a.colidx = reinterpret_cast<int*>(b); b += cols_bytes;
+    if (walk) {
+        sp.pos = reinterpret_cast<int*>(b); b += pos_bytes;
+        sp.walk = const_cast<void*>(walk->packed);
+        SMAT_CUDA_TRY(cudaMemsetAsync(sp.pos, 0xff, pos_bytes, stream));
+        SMAT_CUDA_TRY(launch_pdl(walk_place_kernel, dim3((unsigned)std::min((n + 255) / 256, (size_t)sm_count * 8)), dim3(256), 0, stream,
+                                 walk->blk, sp.pos, (int)first, (int)n));
+        count_launch();
+    }
     a.vals = b; b += packed_bytes;
     sp.slabs = slab_bytes ? b : nullptr;
     sp.first = first;
@@ -499,7 +539,8 @@ int stream_plan_values(const PlanView& v, const void* vals, const int* colidx, i
     const unsigned grid = (unsigned)std::min((v.nnzb + 7) / 8, (size_t)sm_count * 8);
     SMAT_CUDA_TRY(launch_pdl(stream_pack_kernel, dim3(grid), dim3(256), 0, stream,
                              reinterpret_cast<const uint2*>(vals), colidx, reinterpret_cast<uint4*>(const_cast<void*>(a.vals)),
-                             colidx ? const_cast<int*>(a.colidx) : nullptr, (int)v.stream->first, (int)v.nnzb, (int)(v.K / 16)));
+                             colidx ? const_cast<int*>(a.colidx) : nullptr, (int)v.stream->first, (int)v.nnzb, (int)(v.K / 16), v.stream->pos,
+                             static_cast<uint2*>(v.stream->walk)));
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;

@@ -17,13 +17,13 @@ def _blocks(rng, counts, Kb):
     return brp, bci, (rng.standard_normal(brp[-1] * 256) * 0.25).astype(np.float16)
 
 
-def _multiply(brp, bci, bv, B_nk, M, K, plan):
+def _multiply(brp, bci, bv, B_nk, M, K, plan, hint=136):
     N = B_nk.shape[0]
     A, B, C = S.SparseMatrix.from_bcsr(M, K, brp, bci, bv), S.Matrix.from_host(B_nk), S.Matrix(M, N, fill=float("nan"))
     S.set_variant(5)
     try:
         if plan:
-            p = S.Plan(A, n_hint=min(N, 136))  # wider products than the hint go in several passes
+            p = S.Plan(A, n_hint=min(N, hint))  # wider products than the hint rounded up to 128 go in several passes
             assert p.info()["kernel"] == "spmm_bcsr_stream_kernel"
             p.set_values()
             p.spmm(B, C, check=True)
@@ -92,3 +92,71 @@ def test_stream_plan_of_a_range_and_host_buffers():
     mag = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B_nk), Mb * 16, N, Kb * 16, b0, b1)
     for got in (C.data.cpu().numpy(), C_host.numpy().view(np.float16)):
         assert float(np.max(np.abs(got.astype(np.float32) - ref) / (np.maximum(np.abs(ref), 1e-2 * mag) + 1e-30))) <= TOL
+
+
+@pytest.mark.parametrize("Mb,Kb,most,hint,N", [
+    (64, 512, 400, 16, 328),   # three passes, the slabs of one reused by the next, long block-rows in pieces
+    (40, 100, 9, 16, 264),     # no slabs; a last pass of eight columns
+    (3, 3000, 2900, 136, 600),  # passes of 256 columns, every block-row in pieces
+])
+def test_products_in_several_passes(Mb, Kb, most, hint, N):
+    rng = np.random.default_rng(N)
+    counts = rng.integers(0, most + 1, Mb)
+    counts[-1] = most
+    brp, bci, bv = _blocks(rng, counts, Kb)
+    B_nk = rng.standard_normal((N, Kb * 16)).astype(np.float16)
+    assert _close(_multiply(brp, bci, bv, B_nk, Mb * 16, Kb * 16, True, hint), brp, bci, bv, B_nk, Mb * 16, Kb * 16)
+
+
+def test_plan_used_at_other_widths_than_its_hint():
+    """A plan made for 16 columns of a block-sparse layer multiplies wide products with the kernel a plan made for them takes
+    (one or two launches, not one or two per 128 columns) and narrow ones with its own, also after a change of values,
+    from host buffers, and in a captured sequence that is replayed after the values changed again."""
+    import torch
+    rng = np.random.default_rng(12)
+    Mb, Kb = 192, 256
+    brp, bci, bv = _blocks(rng, rng.binomial(Kb, 0.2, Mb), Kb)
+    M, K = Mb * 16, Kb * 16
+    A = S.SparseMatrix.from_bcsr(M, K, brp, bci, bv)
+    plan, wide = S.Plan(A, n_hint=16), S.Plan(A, n_hint=1024)
+    assert plan.info()["kernel"] == "spmm_bcsr_stream_kernel" and wide.info()["kernel"] != "spmm_bcsr_stream_kernel"
+    wide.close()
+    B_nk = rng.standard_normal((1024, K)).astype(np.float16)
+    widths = (8, 16, 64, 136, 520, 1024)
+    B = {N: S.Matrix.from_host(B_nk[:N]) for N in widths}
+    C = {N: S.Matrix(M, N, fill=float("nan")) for N in widths}
+
+    def check(N, got, values):
+        assert _close(got[:, :64], brp, bci, values, B_nk[:min(N, 64)], M, K)  # every column by the same arithmetic: a sample
+        if N > 64:
+            assert _close(got[:, N - 64:], brp, bci, values, B_nk[N - 64:N], M, K)
+
+    values = bv
+    for scale in (1.0, -2.0):
+        if scale != 1.0:
+            A.bcsrVal.mul_(scale)
+            plan.set_values()
+            values = (values * np.float16(scale)).astype(np.float16)
+        for N in widths:
+            before = S.launch_count()
+            plan.spmm(B[N], C[N], check=True)
+            assert S.launch_count() - before <= 2
+            check(N, C[N].data.cpu().numpy(), values)
+    for N in (16, 1024):
+        B_host, C_host = torch.from_numpy(B_nk[:N].view(np.int16)).pin_memory(), torch.full((M, N), -1, dtype=torch.int16).pin_memory()
+        plan.spmm_host(B_host, C_host)
+        torch.cuda.synchronize()
+        check(N, C_host.numpy().view(np.float16), values)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.set_values()
+        for N in (16, 1024):
+            plan.spmm(B[N], C[N])
+    A.bcsrVal.mul_(-2.0)
+    values = (values * np.float16(-2)).astype(np.float16)
+    graph.replay()
+    torch.cuda.synchronize()
+    for N in (16, 1024):
+        check(N, C[N].data.cpu().numpy(), values)
+    del graph
+    plan.close()
