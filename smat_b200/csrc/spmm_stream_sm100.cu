@@ -465,9 +465,16 @@ bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count)
     const double throughput = (double)nnzb * (double)tiles / sm_count * 20e-3, build = 24.0 + 0.2e-3 * (double)nnzb;
     const double stream = stream_estimate_us(N, rows, nnzb, K, sm_count, false);
     if ((double)nnzb < 0.08 * (double)rows * (double)(K / 16)) {
-        // Few of the possible blocks: how they lie is not known here.  Short block-rows are taken to be clustered, which suits
-        // the other kernel; long ones may be skewed, which makes some items many times longer than the rest (power-law graph
-        // of 65536 rows, N = 128: 951 us against 229), while this kernel cuts long block-rows.
+        // Few of the possible blocks: how they lie is not known here, and no rule on these four sizes suits all.  Clustered
+        // blocks suit the other kernel: dense clusters of 65536 rows, N = 512, 71 us against 165 with this one.  Scattered
+        // ones suit this one: random matrix of 65536 rows, 123 blocks a block-row, N = 128, 251 against 474; skewed ones
+        // more (power-law graph of 65536 rows: 235 against 970), since it cuts long block-rows.  So short block-rows are
+        // taken to be clustered, and for long ones this kernel may cost twice the estimate of the other's throughput.
+        // Of 489 products (random, power-law, block-sparse layer, clusters, bands; 8 to 768 columns) the rule takes the slower
+        // kernel for random matrices where both are close (105 us against 84 at worst) and leaves them the other kernel where
+        // N > 200 (2.4 times the time at worst); what pays for it are bands of more than 24 blocks a block-row at 72 to 264
+        // columns (half bandwidth 200: 65 us against 42; 600: 190 against 101).  Counting the other kernel's rounds of
+        // steps, as below, is right for scattered blocks and takes those bands beyond 264 columns as well (120 -> 240 us).
         return stream < (nnzb > 24 * rows ? 2.0 : 1.0) * (build + throughput);
     }
     const double quads = std::ceil((double)K / 64.0), steps = quads * (1.0 - std::exp(-(double)nnzb / (double)groups / quads));
