@@ -294,12 +294,10 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
 #endif
                 tc_fence_after();
                 if (leader) {
-#ifndef SMAT_TALL_NOCP
                     if (subs & 1u) tc_cp_128x256b(tdst, pdesc);
                     if (subs & 2u) tc_cp_128x256b(tdst + 8, pdesc + 2);
                     if (subs & 4u) tc_cp_128x256b(tdst + 16, pdesc + 4);
                     if (subs & 8u) tc_cp_128x256b(tdst + 24, pdesc + 6);
-#endif
                     tc_commit(cp_done(pi % NPAIR));
                     // A plain arrive beside the commit's: it is ordered after this thread's wait for the blocks and
                     // lists of the step, so whoever passes cp_done may read them (the MMA warps wait for nothing else).

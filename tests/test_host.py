@@ -40,6 +40,13 @@ def test_partial_tiles_are_published_by_the_whole_warp():
     assert re.search(ordered, after[:after.index("__ldcg(src")])
 
 
+def test_committed_kernels_have_no_switch_that_skips_work():
+    """Conditional sections of the CUDA sources: the cycle counters, which only add work, and settings with a default."""
+    allowed = {"SMAT_PROFILE", "SMAT_TMA_EPILOGUE", "SMAT_OWNERS"}
+    for path in glob.glob(os.path.join(ROOT, "smat_b200", "csrc", "*.cu*")) + glob.glob(os.path.join(ROOT, "smat_b200", "csrc", "*.h")):
+        assert set(re.findall(r"#\s*(?:if|ifdef|ifndef|elif)\s+(\w+)", open(path).read())) <= allowed, path
+
+
 def test_host_range_is_pinned_from_end_to_end(tmp_path):
     """host_range.h decides whether a kernel may store to the caller's C: compiled with a fake of the driver's answers.  A hole
     between two pinned ends, a last page that is not pinned and a view the device sees in two places are refused."""
