@@ -550,11 +550,16 @@ def main():
 
 
 def run_reference_arm(args, rank, world, log):
-    """The reference's CPU blocked multiply (oracle/_ref when built, else the oracle port) on the same
-    workload, all host cores, each step a bounded sample."""
+    """The reference's CPU blocked multiply (oracle/_ref, compiled from its sources) on the same workload, all host cores,
+    each step a bounded sample.  Without that library there is nothing of the reference to time: the oracle's restatement
+    does not stand in for it."""
     if rank != 0:
         return
     import oracle
+    if not oracle.have_ref():
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libsmat_ref.so is not built: the reference's sources are not "
+                                                              "on this machine"}), flush=True)
+        return
     import smat_b200 as S
     p = build_problem(args.config, args.scale, log)
     rp, ci, v, reorder_s, _ = reorder_if_needed(p, log, None, args.config, args.scale)

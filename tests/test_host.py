@@ -40,6 +40,18 @@ def test_partial_tiles_are_published_by_the_whole_warp():
     assert re.search(ordered, after[:after.index("__ldcg(src")])
 
 
+def test_reference_arm_never_times_the_port():
+    """bench.py --impl reference without the reference's own library says so and ends; it prints no figure."""
+    import json
+    import subprocess
+    import sys
+    if oracle.have_ref():
+        pytest.skip("the reference's library is built")
+    out = subprocess.check_output([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1"], text=True)
+    line = json.loads(out.strip().splitlines()[-1])
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
+
+
 def test_committed_kernels_have_no_switch_that_skips_work():
     """Conditional sections of the CUDA sources: the cycle counters, which only add work, and settings with a default."""
     allowed = {"SMAT_PROFILE", "SMAT_TMA_EPILOGUE", "SMAT_OWNERS"}
