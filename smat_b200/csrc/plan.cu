@@ -653,10 +653,10 @@ struct smat_plan {
     bool has_wide = false;
     size_t n_hint = 0;
     int sms = 0;
+    // everything the plan holds on the device but step counts and schedule: one allocation (each costs 0.3 ms, whatever its size)
     void* buffer = nullptr;
     void* gsp_buffer = nullptr;
-    void* fix_buffer = nullptr;  // partial tiles of cut work items
-    StreamPlan stream;           // buffers of a stream plan
+    StreamPlan stream;
     void* sched_buffer = nullptr;  // listed schedule: offsets per CTA, then the groups
     int device = -1;
     size_t nnzb = 0;  // blocks of the whole arrays, as given
@@ -736,24 +736,12 @@ static const PlanView& view_for(const smat_plan* p, size_t N) {
 
 static cudaError_t free_plan(smat_plan* p) {
     cudaError_t e = cudaSuccess;
-    for (void* b : {p->buffer, p->gsp_buffer, p->fix_buffer, p->sched_buffer, p->stream.buffer}) {
+    for (void* b : {p->buffer, p->gsp_buffer, p->sched_buffer}) {
         const cudaError_t eb = cudaFree(b);
         if (e == cudaSuccess) e = eb;
     }
     delete p;
     return e;
-}
-
-// The stream plan of the range that `of` describes, in place of it or beside it, in `p`'s buffers; `out` becomes its view.
-static int build_stream_view(smat_plan* p, const PlanView& of, bool beside, PlanView& out, const int* h_rowptr, const void* vals, const int* colidx,
-                             cudaStream_t stream) {
-    out.K = of.K;
-    out.nnzb = of.nnzb;
-    out.brow_begin = of.brow_begin;
-    out.brow_end = of.brow_end;
-    if (int rc = stream_plan_build(p->stream, out, h_rowptr, vals, colidx, p->n_hint, p->sms, beside ? &of : nullptr, stream)) return rc;
-    out.total_steps = (size_t)p->stream.row_piece.back();
-    return SMAT_OK;
 }
 
 // A plan's memory and tuning belong to the device it was created on.
@@ -984,8 +972,13 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     // Stream plan (spmm_stream_sm100.cu): taken where its estimate is below that of the kernel chosen so far.  That one is kept
     // beside it unless its estimate loses for wide products too: each pass over the matrix with the stream kernel multiplies
     // 128 columns or as many as the hint names, so a plan made for 16 columns would take 32 passes for 4096.
-    std::vector<int> h_rowptr;
     bool stream_too = false;
+    StreamLayout layout;
+    PlanView narrow;  // the stream plan's
+    narrow.K = K;
+    narrow.nnzb = range_blocks;
+    narrow.brow_begin = brow_begin;
+    narrow.brow_end = brow_end;
     if (rc == SMAT_OK && total_steps > 0 && (g_spmm_variant == 5 || (g_spmm_variant == 0 && N_hint > 0))) {
         const size_t wide = std::max<size_t>(p->n_hint, 4096);
         const double us = stream_estimate_us(p->n_hint, rows, range_blocks, K, ctx->sm_count, true), other = tc_estimate_us(v, p->n_hint, (size_t)ctx->sm_count);
@@ -993,22 +986,26 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         if (std::getenv("SMAT_PLAN_DEBUG"))
             fprintf(stderr, "[smat plan] stream %.1f us, %s %.1f us; %zu columns: %.1f, %.1f us\n", us, tall ? "tall" : "16-row", other, wide, us_wide, other_wide);
         if (g_spmm_variant == 5 || us < other) {
-            h_rowptr.resize(rows + 1);
+            std::vector<int> h_rowptr(rows + 1);
             e = cudaMemcpyAsync(h_rowptr.data(), bcsrRowPtrA + brow_begin, (rows + 1) * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
             if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
             stream_too = rc == SMAT_OK && std::is_sorted(h_rowptr.begin(), h_rowptr.end());
-            if (stream_too && (g_spmm_variant == 5 || us_wide < other_wide)) {
+            const bool alone = g_spmm_variant == 5 || us_wide < other_wide;
+            if (stream_too) layout = stream_plan_layout(h_rowptr.data(), rows, K, p->n_hint, ctx->sm_count, !alone);
+            if (stream_too && alone) {
                 cudaFree(p->gsp_buffer);
                 cudaFree(p->sched_buffer);
                 p->gsp_buffer = p->sched_buffer = nullptr;
-                PlanView only;
-                rc = build_stream_view(p, v, false, only, h_rowptr.data(), bcsrValuesA, bcsrColIdxA, (cudaStream_t)stream);
+                e = cudaMalloc(&p->buffer, layout.bytes());
+                if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
+                if (rc == SMAT_OK)
+                    rc = stream_plan_fill(p->stream, narrow, layout, p->buffer, bcsrValuesA, bcsrColIdxA, ctx->sm_count, nullptr, (cudaStream_t)stream);
                 if (rc) {
                     free_plan(p);
-                    return rc == SMAT_ERR_NOMEM ? SMAT_ERR_CUDA : rc;
+                    return rc;
                 }
-                v = only;
+                v = narrow;
                 *out = p;
                 return SMAT_OK;
             }
@@ -1018,13 +1015,18 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         fprintf(stderr, "[smat plan] rows %zu blocks %zu: 16-row plan rg %zu steps %d cap %zu balanced %d listed %d; tall %d rg %zu steps %d max/group %d\n",
                 brow_end - brow_begin, range_blocks, rg, total_steps, cap, (int)balanced, p->v.sched_list != nullptr, (int)tall, rg_used,
                 steps_final, total_and_max[1]);
-    if (rc == SMAT_OK) {  // a partial tile per CTA, two for the balanced schedule
-        e = cudaMalloc(&p->fix_buffer, (balanced ? 2 : 1) * fix_scratch_bytes(ctx->sm_count));
-        if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
-    }
+    // a partial tile per CTA, two for the balanced schedule; then steps, order and blocks; then the stream plan beside them
+    const size_t fix_bytes = (balanced ? 2 : 1) * fix_scratch_bytes(ctx->sm_count);
+    size_t plan_bytes = 0;
     if (rc == SMAT_OK) {
         sz = plan_sizes(nnzb, brow_begin, brow_end, rg_used, (size_t)(steps_final > 0 ? steps_final : 1) * (tall ? 13 : 1));  // tall: + 64 bytes of per-step words + 128 bytes of the per-pair lists
-        e = cudaMalloc(&p->buffer, sz.steps_bytes + sz.blk_bytes + sz.packed_bytes);
+        plan_bytes = fix_bytes + sz.steps_bytes + sz.blk_bytes + sz.packed_bytes;
+        e = cudaMalloc(&p->buffer, plan_bytes + (stream_too ? layout.bytes() : 0));
+        if (e == cudaErrorMemoryAllocation && stream_too) {  // no room for two copies of the blocks: all products with the first
+            cudaGetLastError();
+            stream_too = false;
+            e = cudaMalloc(&p->buffer, plan_bytes);
+        }
         if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
     }
     if (rc) {
@@ -1033,10 +1035,11 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     }
     char* b = static_cast<char*>(p->buffer);
     p->nnzb = nnzb;
+    v.fix_scratch = reinterpret_cast<float*>(b);
+    b += fix_bytes;
     v.steps = b;
     v.blk = reinterpret_cast<int*>(b + sz.steps_bytes);
     v.packed = b + sz.steps_bytes + sz.blk_bytes;
-    v.fix_scratch = static_cast<float*>(p->fix_buffer);
     if (stream_too) {  // places without a block stay marked as such (stream_plan_build)
         e = cudaMemsetAsync(const_cast<int*>(v.blk), 0xff, sz.blk_bytes, (cudaStream_t)stream);
         if (e != cudaSuccess) {
@@ -1054,21 +1057,15 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         rc = plan_fill_async(bcsrRowPtrA, bcsrColIdxA, K, nnzb, brow_begin, brow_end, rg, gsp, const_cast<void*>(v.steps),
                              const_cast<int*>(v.blk), (cudaStream_t)stream, nullptr, cap);
     }
-    bool packed = false;
     if (rc == SMAT_OK && stream_too) {
-        PlanView narrow;
-        rc = build_stream_view(p, v, true, narrow, h_rowptr.data(), bcsrValuesA, bcsrColIdxA, (cudaStream_t)stream);
-        if (rc == SMAT_OK) {
-            p->wide = v;
-            p->has_wide = packed = true;
-            v = narrow;
-        } else if (rc == SMAT_ERR_NOMEM) {  // no room for the second copy of the blocks: all products with the first
-            clear_error();
-            rc = SMAT_OK;
-        }
-    }
-    if (rc == SMAT_OK && !packed)
+        rc = stream_plan_fill(p->stream, narrow, layout, static_cast<char*>(p->buffer) + plan_bytes, bcsrValuesA, bcsrColIdxA, ctx->sm_count, &v,
+                              (cudaStream_t)stream);
+        p->wide = v;
+        p->has_wide = true;
+        v = narrow;
+    } else if (rc == SMAT_OK) {
         rc = pack_values_async(bcsrRowPtrA, bcsrValuesA, v.blk, const_cast<void*>(v.packed), brow_begin, brow_end, nnzb, (cudaStream_t)stream);
+    }
     if (rc) {
         free_plan(p);
         return rc;

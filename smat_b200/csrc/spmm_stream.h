@@ -40,9 +40,8 @@ double stream_estimate_us(size_t N, size_t rows, size_t nnzb, size_t K, int sm_c
 inline size_t stream_pass_columns(size_t N_hint) { return (N_hint + 127) / 128 * 128; }
 double stream_passes_us(size_t N, size_t N_hint, size_t rows, size_t nnzb, size_t K, int sm_count);
 
-// What a plan for this kernel owns (PlanView::stream): the values in fragment order, the block-columns, the pieces.
+// What a plan for this kernel holds (PlanView::stream): the values in fragment order, the block-columns, the pieces.
 struct StreamPlan {
-    void* buffer = nullptr;
     StreamArgs args = {};         // pieces, slots, counters, partial, colidx, vals
     void* slabs = nullptr;
     size_t n_cap = 0, first = 0;  // columns that scratch and slabs hold; position of the plan's first block in the boundary's arrays
@@ -51,11 +50,20 @@ struct StreamPlan {
     void* walk = nullptr;
     int* pos = nullptr;
 };
-// h_rowptr: the plan's row pointers on the host (block-rows brow_begin .. brow_end), checked to be monotone.
-// `walk`: the plan of a tcgen05 kernel that is kept beside this one (or null), its walk order filled (blk -1 where it holds no
-// block), its copy of the blocks filled here.  SMAT_ERR_NOMEM, and nothing launched, where the device has no room.
-int stream_plan_build(StreamPlan& sp, PlanView& v, const int* h_rowptr, const void* vals, const int* colidx, size_t N_hint, int sm_count,
-                      const PlanView* walk, cudaStream_t stream);
+// Its pieces, and the device memory that it takes (bytes() of it, 256-byte aligned).  h_rowptr: the plan's row pointers on the
+// host (block-rows brow_begin .. brow_end), checked to be monotone.  beside: kept beside the plan of a tcgen05 kernel.
+struct StreamLayout {
+    std::vector<uint4> pieces;
+    std::vector<int2> slots;
+    std::vector<int> row_piece;
+    size_t n_cap = 0, first = 0, pieces_bytes = 0, slots_bytes = 0, counter_bytes = 0, partial_bytes = 0, cols_bytes = 0, pos_bytes = 0, packed_bytes = 0, slab_bytes = 0;
+    size_t bytes() const { return pieces_bytes + slots_bytes + counter_bytes + partial_bytes + cols_bytes + pos_bytes + packed_bytes + slab_bytes; }
+};
+StreamLayout stream_plan_layout(const int* h_rowptr, size_t rows, size_t K, size_t N_hint, int sm_count, bool beside);
+// v: the range, K and blocks of the plan; becomes the stream plan's view.  walk: the plan beside it (or null), its walk order
+// filled (blk -1 where it holds no block); its copy of the blocks is filled here.
+int stream_plan_fill(StreamPlan& sp, PlanView& v, StreamLayout& l, void* memory, const void* vals, const int* colidx, int sm_count,
+                     const PlanView* walk, cudaStream_t stream);
 // New values into an existing plan (colidx null) or values and columns into a new one; into the plan beside it as well.
 int stream_plan_values(const PlanView& v, const void* vals, const int* colidx, int sm_count, cudaStream_t stream);
 int launch_stream(const PlanView& v, const void* B, void* C, size_t N, cudaStream_t stream, const DeviceCtx* ctx, size_t ldc,

@@ -314,29 +314,39 @@ __global__ void __launch_bounds__(256) long_rows_kernel(const int* __restrict__ 
 // The plan's copy of the values in the order a warp's lanes read them (lane (g, t): rows g and g + 8, k = 4t .. 4t + 3), and
 // of the block columns; a column outside the matrix becomes -1.  Where the plan holds the blocks in the walk order of a
 // tcgen05 kernel as well, block i also goes to place pos[i] of that copy, in its swizzled form (16-byte chunk index XOR bit 2
-// of the row): read once for both (183 000 blocks: 52 us, 64 with a kernel
-// for each, 33 for one copy alone).
+// of the row): read once for both (183 000 blocks: 47 us, 64 with a kernel
+// for each, 33 for one copy alone; 52 with a block at a time instead of four).
 __global__ void __launch_bounds__(256) stream_pack_kernel(const uint2* __restrict__ vals, const int* __restrict__ colidx,
                                                          uint4* __restrict__ packed, int* __restrict__ cols, int first, int n, int Kb,
                                                          const int* __restrict__ pos, uint2* __restrict__ walk) {
     ptx::pdl_wait();
     const int lane = threadIdx.x & 31;
     const int row = lane >> 2, chunk = 2 * row + ((lane >> 1) & 1), to = 2 * (chunk ^ ((row >> 2) & 1)) + (lane & 1);
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-        const uint2 lo = __ldg(vals + (size_t)(first + i) * 64 + lane), hi = __ldg(vals + (size_t)(first + i) * 64 + 32 + lane);
-        packed[(size_t)i * 32 + lane] = make_uint4(lo.x, lo.y, hi.x, hi.y);
-        if (pos) {
-            const int p = __ldg(pos + i);
-            if (p >= 0) {
-                walk[(size_t)p * 64 + to] = lo;
-                walk[(size_t)p * 64 + 32 + to] = hi;
+    constexpr int U = 4;  // blocks of a warp at a time, all loads before the stores
+    const int stride = (int)((gridDim.x * blockDim.x) >> 5) * U;
+    for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * U; i < n; i += stride) {
+        uint2 lo[U], hi[U];
+        int p[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i + u < n) {
+                lo[u] = __ldg(vals + (size_t)(first + i + u) * 64 + lane);
+                hi[u] = __ldg(vals + (size_t)(first + i + u) * 64 + 32 + lane);
+                p[u] = pos ? __ldg(pos + i + u) : -1;
             }
-        }
-        if (cols && lane == 0) {
-            const int c = __ldg(colidx + first + i) >> 4;
-            cols[i] = (c >= 0 && c < Kb) ? c : -1;
-        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i + u < n) {
+                packed[(size_t)(i + u) * 32 + lane] = make_uint4(lo[u].x, lo[u].y, hi[u].x, hi[u].y);
+                if (p[u] >= 0) {
+                    walk[(size_t)p[u] * 64 + to] = lo[u];
+                    walk[(size_t)p[u] * 64 + 32 + to] = hi[u];
+                }
+                if (cols && lane == 0) {
+                    const int c = __ldg(colidx + first + i + u) >> 4;
+                    cols[i + u] = (c >= 0 && c < Kb) ? c : -1;
+                }
+            }
     }
 }
 
@@ -481,62 +491,71 @@ bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count)
     return stream < build + std::max(throughput, rounds_for(groups * tiles, (size_t)sm_count, true, (size_t)steps, false) * steps * 0.26);
 }
 
-int stream_plan_build(StreamPlan& sp, PlanView& v, const int* h_rowptr, const void* vals, const int* colidx, size_t N_hint, int sm_count,
-                      const PlanView* walk, cudaStream_t stream) {
-    const size_t rows = v.brow_end - v.brow_begin, first = (size_t)h_rowptr[0], n = v.nnzb;
-    const StreamShape s = stream_shape(N_hint, rows, n, v.K, sm_count, true);
-    std::vector<uint4> pieces;
-    std::vector<int2> slots;
-    pieces.reserve(rows + n / (size_t)s.chunk + 1);
-    sp.row_piece.resize(rows + 1);
+StreamLayout stream_plan_layout(const int* h_rowptr, size_t rows, size_t K, size_t N_hint, int sm_count, bool beside) {
+    StreamLayout l;
+    const int first = h_rowptr[0];
+    const size_t n = (size_t)(h_rowptr[rows] - first);
+    const StreamShape s = stream_shape(N_hint, rows, n, K, sm_count, true);
+    l.pieces.reserve(rows + n / (size_t)s.chunk + 1);
+    l.row_piece.resize(rows + 1);
     for (size_t r = 0; r < rows; r++) {
-        const unsigned b0 = (unsigned)(h_rowptr[r] - (int)first), len = (unsigned)(h_rowptr[r + 1] - h_rowptr[r]);
+        const unsigned b0 = (unsigned)(h_rowptr[r] - first), len = (unsigned)(h_rowptr[r + 1] - h_rowptr[r]);
         const unsigned k = len ? (len + (unsigned)s.chunk - 1) / (unsigned)s.chunk : 1, per = (len + k - 1) / k;
-        sp.row_piece[r] = (int)pieces.size();
-        const int slot0 = (int)slots.size();
+        l.row_piece[r] = (int)l.pieces.size();
+        const int slot0 = (int)l.slots.size();
         for (unsigned i = 0; i < k; i++) {
-            if (k > 1) slots.push_back(make_int2(slot0, (int)k));
-            pieces.push_back(make_uint4((unsigned)r, b0 + std::min(len, i * per), b0 + std::min(len, (i + 1) * per), k > 1 ? (unsigned)slots.size() : 0u));
+            if (k > 1) l.slots.push_back(make_int2(slot0, (int)k));
+            l.pieces.push_back(make_uint4((unsigned)r, b0 + std::min(len, i * per), b0 + std::min(len, (i + 1) * per), k > 1 ? (unsigned)l.slots.size() : 0u));
         }
     }
-    sp.row_piece[rows] = (int)pieces.size();
-    sp.n_cap = stream_pass_columns(N_hint);
-    const size_t pieces_bytes = round256(pieces.size() * sizeof(uint4)), slots_bytes = round256(slots.size() * sizeof(int2)),
-                 counter_bytes = round256(slots.size() * (sp.n_cap / 8) * sizeof(int)), partial_bytes = round256(slots.size() * sp.n_cap * 64),
-                 cols_bytes = round256(n * sizeof(int)), packed_bytes = n * 512, pos_bytes = walk ? cols_bytes : 0;
+    l.row_piece[rows] = (int)l.pieces.size();
+    l.first = (size_t)first;
+    l.n_cap = stream_pass_columns(N_hint);
+    l.pieces_bytes = round256(l.pieces.size() * sizeof(uint4));
+    l.slots_bytes = round256(l.slots.size() * sizeof(int2));
+    l.counter_bytes = round256(l.slots.size() * (l.n_cap / 8) * sizeof(int));
+    l.partial_bytes = round256(l.slots.size() * l.n_cap * 64);
+    l.cols_bytes = round256(n * sizeof(int));
+    l.pos_bytes = beside ? l.cols_bytes : 0;
+    l.packed_bytes = n * 512;
     // slabs for the widest pass, whatever the hint: where a narrower one wants them the widest does too
-    const size_t slab_bytes = stream_shape(sp.n_cap, rows, n, v.K, sm_count, true).slab ? sp.n_cap * v.K * 2 : 0;
-    const cudaError_t e = cudaMalloc(&sp.buffer, pieces_bytes + slots_bytes + counter_bytes + partial_bytes + cols_bytes + pos_bytes + packed_bytes + slab_bytes);
-    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
-    if (e != cudaSuccess)
-        return fail(e == cudaErrorMemoryAllocation ? SMAT_ERR_NOMEM : SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
-    char* b = static_cast<char*>(sp.buffer);
+    l.slab_bytes = stream_shape(l.n_cap, rows, n, K, sm_count, true).slab ? round256(l.n_cap * K * 2) : 0;
+    return l;
+}
+
+int stream_plan_fill(StreamPlan& sp, PlanView& v, StreamLayout& l, void* memory, const void* vals, const int* colidx, int sm_count,
+                     const PlanView* walk, cudaStream_t stream) {
+    char* b = static_cast<char*>(memory);
     StreamArgs& a = sp.args;
     a = StreamArgs{};
-    a.pieces = reinterpret_cast<uint4*>(b); b += pieces_bytes;
-    a.slots = reinterpret_cast<int2*>(b); b += slots_bytes;
-    a.counters = reinterpret_cast<int*>(b); b += counter_bytes;
-    a.partial = reinterpret_cast<float4*>(b); b += partial_bytes;
-    a.colidx = reinterpret_cast<int*>(b); b += cols_bytes;
+    a.pieces = reinterpret_cast<uint4*>(b); b += l.pieces_bytes;
+    a.slots = reinterpret_cast<int2*>(b); b += l.slots_bytes;
+    a.counters = reinterpret_cast<int*>(b); b += l.counter_bytes;
+    a.partial = reinterpret_cast<float4*>(b); b += l.partial_bytes;
+    a.colidx = reinterpret_cast<int*>(b); b += l.cols_bytes;
+    if (walk) sp.pos = reinterpret_cast<int*>(b);
+    b += l.pos_bytes;
+    a.vals = b; b += l.packed_bytes;
+    sp.slabs = l.slab_bytes ? b : nullptr;
+    sp.first = l.first;
+    sp.n_cap = l.n_cap;
+    sp.row_piece = std::move(l.row_piece);
+    SMAT_CUDA_TRY(cudaMemcpyAsync(const_cast<uint4*>(a.pieces), l.pieces.data(), l.pieces.size() * sizeof(uint4), cudaMemcpyHostToDevice, stream));
+    if (!l.slots.empty()) {
+        SMAT_CUDA_TRY(cudaMemcpyAsync(const_cast<int2*>(a.slots), l.slots.data(), l.slots.size() * sizeof(int2), cudaMemcpyHostToDevice, stream));
+        SMAT_CUDA_TRY(cudaMemsetAsync(a.counters, 0, l.counter_bytes, stream));
+    }
     if (walk) {
-        sp.pos = reinterpret_cast<int*>(b); b += pos_bytes;
         sp.walk = const_cast<void*>(walk->packed);
-        SMAT_CUDA_TRY(cudaMemsetAsync(sp.pos, 0xff, pos_bytes, stream));
-        SMAT_CUDA_TRY(launch_pdl(walk_place_kernel, dim3((unsigned)std::min((n + 255) / 256, (size_t)sm_count * 8)), dim3(256), 0, stream,
-                                 walk->blk, sp.pos, (int)first, (int)n));
+        SMAT_CUDA_TRY(cudaMemsetAsync(sp.pos, 0xff, l.pos_bytes, stream));
+        SMAT_CUDA_TRY(launch_pdl(walk_place_kernel, dim3((unsigned)std::min((v.nnzb + 255) / 256, (size_t)sm_count * 8)), dim3(256), 0, stream,
+                                 walk->blk, sp.pos, (int)sp.first, (int)v.nnzb));
         count_launch();
     }
-    a.vals = b; b += packed_bytes;
-    sp.slabs = slab_bytes ? b : nullptr;
-    sp.first = first;
-    SMAT_CUDA_TRY(cudaMemcpyAsync(const_cast<uint4*>(a.pieces), pieces.data(), pieces.size() * sizeof(uint4), cudaMemcpyHostToDevice, stream));
-    if (!slots.empty()) {
-        SMAT_CUDA_TRY(cudaMemcpyAsync(const_cast<int2*>(a.slots), slots.data(), slots.size() * sizeof(int2), cudaMemcpyHostToDevice, stream));
-        SMAT_CUDA_TRY(cudaMemsetAsync(a.counters, 0, counter_bytes, stream));
-    }
     v.stream = &sp;
-    v.n_groups = rows;
+    v.n_groups = v.brow_end - v.brow_begin;
     v.rg = 1;
+    v.total_steps = l.pieces.size();
     return stream_plan_values(v, vals, colidx, sm_count, stream);  // pageable sources: the copies above have left them
 }
 
