@@ -13,8 +13,9 @@
 //
 // One CTA per block-row.  The entries of its 16 CSR rows are contiguous and dealt out to all threads, whatever the rows'
 // lengths: a warp per row made the longest row of the matrix the time of the whole kernel (power-law graph, 65536 rows,
-// longest 8192 entries, 490 000 blocks: count and fill together 370 -> 110 us; what is left is zeroing 250 MB of values).  Which of several equal entries is last matters only where there are equal ones: block-rows whose rows
-// ascend strictly (checked on the way) scatter in any order, the others keep a warp per row and its order.
+// longest 8192 entries, 490 000 blocks: count and fill together 370 -> 110 us; what is left is zeroing 250 MB of values).
+// Which of several equal entries is last matters only where there are equal ones: block-rows whose rows ascend strictly
+// (checked on the way) scatter in any order, the others keep a warp per row and its order.
 #include <cuda_fp16.h>
 
 #include "smat_internal.h"

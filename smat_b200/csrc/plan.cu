@@ -64,7 +64,7 @@ __device__ __forceinline__ void mark_window(const int* __restrict__ colidx, int&
         if (in && cb >= w0) atomicOr(&masks[cb - w0], 1u << warp);
         else if (in && status) atomicCAS(status, 0, kStatusBadColumns);
         const uint32_t b = __ballot_sync(0xffffffffu, in);
-        if (lane == 0 && status && (b & (b + 1u))) atomicCAS(status, 0, kStatusBadColumns);
+        if (WIN == kOrderWindow && lane == 0 && status && (b & (b + 1u))) atomicCAS(status, 0, kStatusBadColumns);  // smaller ones hold all
         cur += __popc(b);
         if (b != 0xffffffffu) break;
     }
@@ -980,11 +980,12 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     narrow.brow_begin = brow_begin;
     narrow.brow_end = brow_end;
     if (rc == SMAT_OK && total_steps > 0 && (g_spmm_variant == 5 || (g_spmm_variant == 0 && N_hint > 0))) {
-        const size_t wide = std::max<size_t>(p->n_hint, 4096);
-        const double us = stream_estimate_us(p->n_hint, rows, range_blocks, K, ctx->sm_count, true), other = tc_estimate_us(v, p->n_hint, (size_t)ctx->sm_count);
-        const double us_wide = stream_passes_us(wide, p->n_hint, rows, range_blocks, K, ctx->sm_count), other_wide = tc_estimate_us(v, wide, (size_t)ctx->sm_count);
+        const size_t hint = p->n_hint, wide = std::max<size_t>(hint, 4096), sms = (size_t)ctx->sm_count;
+        const double us = stream_estimate_us(hint, rows, range_blocks, K, ctx->sm_count, true), other = tc_estimate_us(v, hint, sms);
+        const double us_wide = stream_passes_us(wide, hint, rows, range_blocks, K, ctx->sm_count), other_wide = tc_estimate_us(v, wide, sms);
         if (std::getenv("SMAT_PLAN_DEBUG"))
-            fprintf(stderr, "[smat plan] stream %.1f us, %s %.1f us; %zu columns: %.1f, %.1f us\n", us, tall ? "tall" : "16-row", other, wide, us_wide, other_wide);
+            fprintf(stderr, "[smat plan] stream %.1f us, %s %.1f us; %zu columns: %.1f, %.1f us\n", us, tall ? "tall" : "16-row", other,
+                    wide, us_wide, other_wide);
         if (g_spmm_variant == 5 || us < other) {
             std::vector<int> h_rowptr(rows + 1);
             e = cudaMemcpyAsync(h_rowptr.data(), bcsrRowPtrA + brow_begin, (rows + 1) * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
@@ -1019,7 +1020,8 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     const size_t fix_bytes = (balanced ? 2 : 1) * fix_scratch_bytes(ctx->sm_count);
     size_t plan_bytes = 0;
     if (rc == SMAT_OK) {
-        sz = plan_sizes(nnzb, brow_begin, brow_end, rg_used, (size_t)(steps_final > 0 ? steps_final : 1) * (tall ? 13 : 1));  // tall: + 64 bytes of per-step words + 128 bytes of the per-pair lists
+        // tall: + 64 bytes of per-step words + 128 bytes of the per-pair lists
+        sz = plan_sizes(nnzb, brow_begin, brow_end, rg_used, (size_t)(steps_final > 0 ? steps_final : 1) * (tall ? 13 : 1));
         plan_bytes = fix_bytes + sz.steps_bytes + sz.blk_bytes + sz.packed_bytes;
         e = cudaMalloc(&p->buffer, plan_bytes + (stream_too ? layout.bytes() : 0));
         if (e == cudaErrorMemoryAllocation && stream_too) {  // no room for two copies of the blocks: all products with the first

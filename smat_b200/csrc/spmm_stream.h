@@ -56,7 +56,8 @@ struct StreamLayout {
     std::vector<uint4> pieces;
     std::vector<int2> slots;
     std::vector<int> row_piece;
-    size_t n_cap = 0, first = 0, pieces_bytes = 0, slots_bytes = 0, counter_bytes = 0, partial_bytes = 0, cols_bytes = 0, pos_bytes = 0, packed_bytes = 0, slab_bytes = 0;
+    size_t n_cap = 0, first = 0;
+    size_t pieces_bytes = 0, slots_bytes = 0, counter_bytes = 0, partial_bytes = 0, cols_bytes = 0, pos_bytes = 0, packed_bytes = 0, slab_bytes = 0;
     size_t bytes() const { return pieces_bytes + slots_bytes + counter_bytes + partial_bytes + cols_bytes + pos_bytes + packed_bytes + slab_bytes; }
 };
 StreamLayout stream_plan_layout(const int* h_rowptr, size_t rows, size_t K, size_t N_hint, int sm_count, bool beside);

@@ -10,17 +10,20 @@
 // without a plan reads the boundary's arrays as they are.
 //
 // What bounds it (measured, one B200): A from HBM while C is narrow; then the slices of B that every block fetches through
-// L2, 32 N bytes per block.  From the [N][K] array a slice is N sectors of 32 bytes, each in a line of its own, and an SM takes one such
-// sector per cycle from L2 or L1 (131 cycles per slice of 128 columns); contiguous slices come at 64 bytes per cycle (60
-// cycles; 33 out of L1).  So where the blocks outnumber the block-columns enough, B is first rewritten as slabs [K / 16][N][16],
-// one pass over B.  mma.sync runs at 2.1-2.6 cycles per 16x8x16 MMA and SM (34 cycles per block of 128 columns) and
-// is not what bounds it; a tcgen05.mma on one block would need its slice in shared memory (39 cycles for the operand
-// port alone) and a barrier round trip per hand-over.
+// L2, 32 N bytes per block.  From the [N][K] array a slice is N sectors of 32 bytes, each in a line of its own, and an SM
+// takes one such sector per cycle from L2 or L1 (131 cycles per slice of 128 columns); contiguous slices come at 64 bytes per
+// cycle (60 cycles; 33 out of L1).  So where the blocks outnumber the block-columns enough, B is first rewritten as slabs
+// [K / 16][N][16], one pass over B.  mma.sync runs at 2.1-2.6 cycles per 16x8x16 MMA and SM (34 cycles per block of 128
+// columns) and is not what bounds it; a tcgen05.mma on one block would need its slice in shared memory (39 cycles for the
+// operand port alone) and a barrier round trip per hand-over.  At 128 columns no unit is full (ncu, power-law matrix of
+// 464 000 blocks: L2 at 45 % of its peak, tensor pipe 34 %, HBM 17 %): 166 registers leave 12 warps per SM, each with the
+// loads of one block in flight, 49 bytes per cycle and SM at an L2 latency of about a thousand cycles.
 //
-// Measured against the tcgen05 kernels (before -> now): 8192 x 28672 layer, 183 000 blocks, N = 16: 67.7 -> 22.6 us (4.2 TB/s);
-// power-law matrix of 2.05 million blocks, N = 128: 1714 -> 797 us, N = 8 (1.78 million): 2076 -> 208 us; band matrix of
-// 2284 blocks, N = 64: 10 -> 4.5 us.  Where blocks share their slices of B (a layer or a random matrix at N >= 128: the
-// tall kernel takes 8-10 ns per block, 128 columns and SM, this one 55-60) the tcgen05 kernels stay.
+// Measured against the tcgen05 kernels (before -> now, inputs that change from pass to pass): 8192 x 28672 layer, 183 000
+// blocks, N = 16: 67.7 -> 24.7 us (3.9 TB/s); power-law matrix of 2.05 million blocks, N = 128: 1706 -> 795 us, N = 8 (1.78
+// million): 2076 -> 208 us; band matrix of 2284 blocks, N = 64: 10 -> 4.1 us.  Where blocks share their slices of B (a layer
+// or a random matrix at N >= 128: the tall kernel takes 8-10 ns per block, 128 columns and SM, this one 55-60) the tcgen05
+// kernels stay.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -34,7 +37,6 @@
 
 namespace smat {
 namespace {
-
 
 __device__ __forceinline__ void mma_16816(float (&d)[4], const uint4& a, const uint2& b) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -64,7 +66,6 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
     ptx::pdl_wait();
     // ---- the piece: blocks [b0, b1) of block-row `row`; count > 1: one of `count` pieces of a long block-row ----
     int row = 0, b0 = 0, b1 = 0, count = 1, my_slot = 0, first_slot = 0;
-    int after = 0;  // no plan: the blocks behind this one follow another block of their block-row
     bool live = piece < p.n_pieces;
     if (live) {
         if (PLAN) {
@@ -84,7 +85,6 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
                 row = piece;
                 b0 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + row), lo), hi);
                 b1 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + row + 1), b0), hi);
-                after = b0;
                 if (b1 - b0 > p.chunk && p.long_rows) {
                     my_slot = first_slot = __ldg(p.row_slot + row);
                     count = (b1 - b0 + p.chunk - 1) / p.chunk;
@@ -96,7 +96,6 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
                 if (live) {
                     const uint4 d = __ldg(p.pieces + (piece - n_rows));
                     row = (int)d.x; b0 = (int)d.y; b1 = (int)d.z; my_slot = (int)d.w;
-                    after = b0 - 1;
                     const int2 s = __ldg(p.slots + my_slot);
                     first_slot = s.x; count = s.y;
                 }
@@ -146,9 +145,9 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
         cols_at = at;
         int c = (at + lane < c1) ? __ldg(p.colidx + at + lane) >> (PLAN ? 0 : 4) : 0;
         if (!PLAN) {
-            // (what plan creation refuses is refused here as well)
+            // what plan creation refuses is refused here as well
             bool bad = c < 0 || c >= Kb;
-            if (Kb > kOrderWindow && at + lane < c1 && at + lane > after)
+            if (Kb > kOrderWindow && at + lane < c1 && at + lane > max(__ldg(p.rowptr + p.brow_begin + row), 0))
                 bad |= c / kOrderWindow < (__ldg(p.colidx + at + lane - 1) >> 4) / kOrderWindow;
             if (bad) atomicCAS(p.status, 0, kStatusBadColumns);
             if (c < 0 || c >= Kb) c = -1;
