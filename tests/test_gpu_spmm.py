@@ -396,9 +396,11 @@ def test_bounded_wait_timeout_is_reported():
     assert _rel_err(C, Cref, Cabs) <= TOL
 
 
-def test_inconsistent_row_pointers_are_reported_not_written_past():
+@pytest.mark.parametrize("variant", [0, 1, 5])
+def test_inconsistent_row_pointers_are_reported_not_written_past(variant):
     """nonzeroBlocks smaller than what the row pointers claim: the plan buffers are sized from nonzeroBlocks, so the
-    plan kernels refuse the range (empty plan, status word) and smat_device_status returns SMAT_ERR_RANGE."""
+    plan kernels (variant 1) refuse the range (empty plan, status word), the stream kernel (variant 5, and by itself on this
+    small matrix) multiplies nothing, and smat_device_status returns SMAT_ERR_RANGE."""
     torch = _torch()
     p, brp, bci, bv = _problem("band", 0.1, 8)
     A = S.SparseMatrix.from_bcsr(p.M, p.K, brp, bci, bv)
@@ -406,18 +408,22 @@ def test_inconsistent_row_pointers_are_reported_not_written_past():
     C = S.Matrix(p.M, 8, fill=0.0)
     L = S.lib()
     stream = torch.cuda.current_stream().cuda_stream
-    for entry in ("plain", "static"):
-        lie = A.nnzb - 5  # fewer blocks than bcsrRowPtr[M / 16]
-        if entry == "plain":
-            rc = L.smat_spmm_bcsr_f16(A.getBcsrValues(), A.getBcsrRowPtr(), A.getBcsrColIdx(), B.data.data_ptr(), C.data.data_ptr(),
-                                      p.M, 8, p.K, lie, None, None, stream)
-        else:
-            rc = L.smat_spmm_bcsr_f16_static(A.getBcsrValues(), A.getBcsrRowPtr(), A.getBcsrColIdx(), B.data.data_ptr(),
-                                             C.data.data_ptr(), p.M, 8, p.K, lie, stream)
-        assert rc == 0
-        rc = L.smat_device_status(stream)
-        assert rc == -6 and b"bcsrRowPtr" in L.smat_last_error_string(), entry
-        assert L.smat_device_status(stream) == 0
+    S.set_variant(variant)
+    try:
+        for entry in ("plain", "static"):
+            lie = A.nnzb - 5  # fewer blocks than bcsrRowPtr[M / 16]
+            if entry == "plain":
+                rc = L.smat_spmm_bcsr_f16(A.getBcsrValues(), A.getBcsrRowPtr(), A.getBcsrColIdx(), B.data.data_ptr(), C.data.data_ptr(),
+                                          p.M, 8, p.K, lie, None, None, stream)
+            else:
+                rc = L.smat_spmm_bcsr_f16_static(A.getBcsrValues(), A.getBcsrRowPtr(), A.getBcsrColIdx(), B.data.data_ptr(),
+                                                 C.data.data_ptr(), p.M, 8, p.K, lie, stream)
+            assert rc == 0
+            rc = L.smat_device_status(stream)
+            assert rc == -6 and b"bcsrRowPtr" in L.smat_last_error_string(), entry
+            assert L.smat_device_status(stream) == 0
+    finally:
+        S.set_variant(0)
 
 
 @pytest.mark.parametrize("name,scale", [("uniform", 0.03), ("powerlaw", 0.01)])
