@@ -144,13 +144,9 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
     auto load_cols = [&](int at) {
         cols_at = at;
         int c = (at + lane < c1) ? __ldg(p.colidx + at + lane) >> (PLAN ? 0 : 4) : 0;
-        if (!PLAN) {
-            // what plan creation refuses is refused here as well
-            bool bad = c < 0 || c >= Kb;
-            if (Kb > kOrderWindow && at + lane < c1 && at + lane > max(__ldg(p.rowptr + p.brow_begin + row), 0))
-                bad |= c / kOrderWindow < (__ldg(p.colidx + at + lane - 1) >> 4) / kOrderWindow;
-            if (bad) atomicCAS(p.status, 0, kStatusBadColumns);
-            if (c < 0 || c >= Kb) c = -1;
+        if (!PLAN && (c < 0 || c >= Kb)) {
+            atomicCAS(p.status, 0, kStatusBadColumns);
+            c = -1;
         }
         cols = c;
         // what the warp will read of A after this batch of 32 blocks is on its way to L2 meanwhile
@@ -310,11 +306,28 @@ __global__ void __launch_bounds__(256) long_rows_kernel(const int* __restrict__ 
     }
 }
 
+// Product without a plan of a matrix of several windows of block-columns: what the plan kernels refuse there is refused here as
+// well.  (In the kernel that multiplies, the look costs the eight-column shapes registers they do not have: 43 -> 62 us.)
+__global__ void __launch_bounds__(256) column_order_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int brow_begin,
+                                                          int brow_end, int nnzb, int* status) {
+    ptx::pdl_wait();
+    constexpr int W = kOrderWindow * 16;  // columns of a window
+    const int lo = __ldg(rowptr + brow_begin), hi = __ldg(rowptr + brow_end), lane = threadIdx.x & 31;
+    if (lo < 0 || hi < lo || hi > nnzb) return;
+    const int warps = (int)((gridDim.x * blockDim.x) >> 5);
+    for (int row = brow_begin + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); row < brow_end; row += warps) {
+        const int b0 = min(max(__ldg(rowptr + row), lo), hi), b1 = min(max(__ldg(rowptr + row + 1), b0), hi);
+        bool bad = false;
+        for (int j = b0 + 1 + lane; j < b1; j += 32) bad |= __ldg(colidx + j) / W < __ldg(colidx + j - 1) / W;
+        if (bad) atomicCAS(status, 0, kStatusBadColumns);
+    }
+}
+
 // The plan's copy of the values in the order a warp's lanes read them (lane (g, t): rows g and g + 8, k = 4t .. 4t + 3), and
 // of the block columns; a column outside the matrix becomes -1.  Where the plan holds the blocks in the walk order of a
 // tcgen05 kernel as well, block i also goes to place pos[i] of that copy, in its swizzled form (16-byte chunk index XOR bit 2
-// of the row): read once for both (183 000 blocks: 47 us, 64 with a kernel
-// for each, 33 for one copy alone; 52 with a block at a time instead of four).
+// of the row): read once for both (183 000 blocks: 47 us, 64 with a kernel for each, 33 for one copy alone; 52 with a block at a
+// time instead of four).
 __global__ void __launch_bounds__(256) stream_pack_kernel(const uint2* __restrict__ vals, const int* __restrict__ colidx,
                                                          uint4* __restrict__ packed, int* __restrict__ cols, int first, int n, int Kb,
                                                          const int* __restrict__ pos, uint2* __restrict__ walk) {
@@ -652,6 +665,11 @@ int stream_call(const StreamShape& s, const void* vals, const int* rowptr, const
                                  pieces, slots, row_slot));
         count_launch();
         SMAT_CUDA_TRY(cudaGetLastError());
+    }
+    if (K / 16 > (size_t)kOrderWindow) {
+        SMAT_CUDA_TRY(launch_pdl(column_order_kernel, dim3((unsigned)std::min((rows + 7) / 8, (size_t)ctx->sm_count * 8)), dim3(256), 0, stream,
+                                 rowptr, colidx, (int)brow_begin, (int)brow_end, (int)nnzb, ctx->d_status));
+        count_launch();
     }
     if (s.slab) {
         if (int rc = make_slabs(B, b, N, K, stream)) return rc;
