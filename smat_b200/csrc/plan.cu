@@ -647,11 +647,10 @@ using namespace smat;
 
 struct smat_plan {
     PlanView v;          // for products about as wide as the hint
-    // A stream plan of a matrix on which a tcgen05 kernel is faster for wide products: the plan of that kernel, for the products
-    // that are (the kernel is picked by the width of each product; smat_plan_set_values keeps both up to date).
+    // A stream plan of a matrix on which a tcgen05 kernel is faster for wide products: the plan of that kernel, for products
+    // of `wide_from` columns or more (0: no such plan).  smat_plan_set_values keeps both up to date.
     PlanView wide;
-    bool has_wide = false;
-    size_t n_hint = 0;
+    size_t wide_from = 0;
     int sms = 0;
     // everything the plan holds on the device but step counts and schedule: one allocation (each costs 0.3 ms, whatever its size)
     void* buffer = nullptr;
@@ -723,15 +722,18 @@ static char* device_view_of_host(void* p, size_t bytes) {
     });
 }
 
-// What multiplies N columns: the hint steers which plans there are, the two estimates which of them is used.  They are off by
-// some 20 %, so the kernel for the hint stays until the other's is lower by that: dense clusters of 131072 rows planned for 8
-// columns and used with 16 take 16.6 us with it, 25.7 with the other kernel, whose estimate is the lower one.  Where it is
-// wider than that, the other kernel it is: 8192 x 28672 layer planned for 16 columns, 2048 columns in 2560 us by passes of
-// 128, in 484 by it; 256 columns 318 and 73.
-static const PlanView& view_for(const smat_plan* p, size_t N) {
-    if (!p->has_wide) return p->v;
-    const PlanView& v = p->v;
-    return stream_passes_us(N, p->n_hint, v.brow_end - v.brow_begin, v.nnzb, v.K, p->sms) < 1.25 * tc_estimate_us(p->wide, N, (size_t)p->sms) ? v : p->wide;
+static const PlanView& view_for(const smat_plan* p, size_t N) { return p->wide_from && N >= p->wide_from ? p->wide : p->v; }
+
+// The width from which a matrix planned with the stream kernel for `hint` columns is multiplied by the tcgen05 kernel of `tc`; 0:
+// at no width looked at.  The two estimates are off by some 20 %, so the kernel for the hint stays until the other's is lower
+// by that: dense clusters of 131072 rows planned for 8 columns and used with 16 take 16.6 us with it, 25.7 with the other
+// kernel, whose estimate is the lower one.  From there on it is the other: 8192 x 28672 layer planned for 16 columns,
+// 2048 columns in 2560 us by passes of 128, in 484 by it; 256 columns 318 and 73.
+static size_t wide_from_width(const PlanView& tc, size_t hint, int sms) {
+    const size_t rows = tc.brow_end - tc.brow_begin, cap = stream_pass_columns(hint), last = std::max<size_t>(4096, 2 * cap);
+    for (size_t N = (hint + 7) / 8 * 8; N <= last; N += N < 2 * cap ? 8 : 128)
+        if (N > hint && stream_passes_us(N, hint, rows, tc.nnzb, tc.K, sms) >= 1.25 * tc_estimate_us(tc, N, (size_t)sms)) return N;
+    return 0;
 }
 
 static cudaError_t free_plan(smat_plan* p) {
@@ -953,7 +955,6 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     }
     const int steps_final = total_and_max[0];
     PlanView& v = p->v;
-    p->n_hint = N_hint ? N_hint : 128;
     p->sms = ctx->sm_count;
     v.rowptr = bcsrRowPtrA;
     v.gsp = gsp;
@@ -970,8 +971,8 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     v.tall = tall;
     v.step_cycles = tall ? tall_step_cycles((double)range_blocks / (double)(steps_final > 0 ? steps_final : 1)) : step16;
     // Stream plan (spmm_stream_sm100.cu): taken where its estimate is below that of the kernel chosen so far.  That one is kept
-    // beside it unless its estimate loses for wide products too: each pass over the matrix with the stream kernel multiplies
-    // 128 columns or as many as the hint names, so a plan made for 16 columns would take 32 passes for 4096.
+    // beside it where it is faster for wide products: each pass over the matrix with the stream kernel multiplies 128 columns
+    // or as many as the hint names, so a plan made for 16 columns would take 32 passes for 4096.
     bool stream_too = false;
     StreamLayout layout;
     PlanView narrow;  // the stream plan's
@@ -980,21 +981,22 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     narrow.brow_begin = brow_begin;
     narrow.brow_end = brow_end;
     if (rc == SMAT_OK && total_steps > 0 && (g_spmm_variant == 5 || (g_spmm_variant == 0 && N_hint > 0))) {
-        const size_t hint = p->n_hint, wide = std::max<size_t>(hint, 4096), sms = (size_t)ctx->sm_count;
-        const double us = stream_estimate_us(hint, rows, range_blocks, K, ctx->sm_count, true), other = tc_estimate_us(v, hint, sms);
-        const double us_wide = stream_passes_us(wide, hint, rows, range_blocks, K, ctx->sm_count), other_wide = tc_estimate_us(v, wide, sms);
+        const size_t hint = N_hint ? N_hint : 128;
+        const double us = stream_estimate_us(hint, rows, range_blocks, K, ctx->sm_count, true), other = tc_estimate_us(v, hint, (size_t)ctx->sm_count);
         if (std::getenv("SMAT_PLAN_DEBUG"))
-            fprintf(stderr, "[smat plan] stream %.1f us, %s %.1f us; %zu columns: %.1f, %.1f us\n", us, tall ? "tall" : "16-row", other,
-                    wide, us_wide, other_wide);
+            fprintf(stderr, "[smat plan] stream %.1f us, %s %.1f us; the latter from %zu columns\n", us, tall ? "tall" : "16-row", other,
+                    wide_from_width(v, hint, ctx->sm_count));
         if (g_spmm_variant == 5 || us < other) {
             std::vector<int> h_rowptr(rows + 1);
             e = cudaMemcpyAsync(h_rowptr.data(), bcsrRowPtrA + brow_begin, (rows + 1) * sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
             if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan build failed: %s", cudaGetErrorString(e));
             stream_too = rc == SMAT_OK && std::is_sorted(h_rowptr.begin(), h_rowptr.end());
-            const bool alone = g_spmm_variant == 5 || us_wide < other_wide;
-            if (stream_too) layout = stream_plan_layout(h_rowptr.data(), rows, K, p->n_hint, ctx->sm_count, !alone);
-            if (stream_too && alone) {
+            if (stream_too) {
+                if (g_spmm_variant != 5) p->wide_from = wide_from_width(v, hint, ctx->sm_count);
+                layout = stream_plan_layout(h_rowptr.data(), rows, K, hint, ctx->sm_count, p->wide_from != 0);
+            }
+            if (stream_too && p->wide_from == 0) {
                 cudaFree(p->gsp_buffer);
                 cudaFree(p->sched_buffer);
                 p->gsp_buffer = p->sched_buffer = nullptr;
@@ -1027,6 +1029,7 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         if (e == cudaErrorMemoryAllocation && stream_too) {  // no room for two copies of the blocks: all products with the first
             cudaGetLastError();
             stream_too = false;
+            p->wide_from = 0;
             e = cudaMalloc(&p->buffer, plan_bytes);
         }
         if (e != cudaSuccess) rc = fail(SMAT_ERR_CUDA, "plan allocation failed: %s", cudaGetErrorString(e));
@@ -1063,7 +1066,6 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         rc = stream_plan_fill(p->stream, narrow, layout, static_cast<char*>(p->buffer) + plan_bytes, bcsrValuesA, bcsrColIdxA, ctx->sm_count, &v,
                               (cudaStream_t)stream);
         p->wide = v;
-        p->has_wide = true;
         v = narrow;
     } else if (rc == SMAT_OK) {
         rc = pack_values_async(bcsrRowPtrA, bcsrValuesA, v.blk, const_cast<void*>(v.packed), brow_begin, brow_end, nnzb, (cudaStream_t)stream);
