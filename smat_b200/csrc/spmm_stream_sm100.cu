@@ -492,7 +492,7 @@ bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count)
         // ones suit this one: random matrix of 65536 rows, 123 blocks a block-row, N = 128, 251 against 474; skewed ones
         // more (power-law graph of 65536 rows: 235 against 970), since it cuts long block-rows.  So short block-rows are
         // taken to be clustered, and for long ones this kernel may cost twice the estimate of the other's throughput.
-        // Of 489 products (random, power-law, block-sparse layer, clusters, bands; 8 to 768 columns) the rule takes the slower
+        // Of 489 products (random, power-law, block-sparse layer, clusters, bands; 16 to 768 columns) the rule takes the slower
         // kernel for random matrices where both are close (105 us against 84 at worst) and leaves them the other kernel where
         // N > 200 (2.4 times the time at worst); what pays for it are bands of more than 24 blocks a block-row at 72 to 264
         // columns (half bandwidth 200: 65 us against 42; 600: 190 against 101).  Counting the other kernel's rounds of

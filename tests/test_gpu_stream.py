@@ -160,3 +160,37 @@ def test_plan_used_at_other_widths_than_its_hint():
         check(N, C[N].data.cpu().numpy(), values)
     del graph
     plan.close()
+
+
+@pytest.mark.parametrize("hint,Mb,Kb", [(8, 240, 300), (64, 240, 300), (16, 520, 700)])  # beside it a 16-row plan; a tall one
+def test_both_walk_orders_of_a_range(hint, Mb, Kb):
+    """A plan with two walk orders for block-rows [37, Mb - 10) of a matrix with empty block-rows and block columns in any order:
+    the places of the blocks are counted from the range's first block; new values reach both copies."""
+    rng = np.random.default_rng(hint)
+    b0, b1 = 37, Mb - 10
+    counts = rng.binomial(Kb, 0.3, Mb)
+    counts[[0, 40, 41, 100, b1 - 1]] = 0
+    brp, bci, bv = _blocks(rng, counts, Kb)
+    order = np.concatenate([rng.permutation(np.arange(brp[r], brp[r + 1])) for r in range(Mb)])
+    M, K, rows = Mb * 16, Kb * 16, (b1 - b0) * 16
+    A = S.SparseMatrix.from_bcsr(M, K, brp, bci[order], bv.reshape(-1, 256)[order].reshape(-1))
+    plan = S.Plan(A, b0, b1, n_hint=hint)
+    assert plan.info()["kernel"] == "spmm_bcsr_stream_kernel"
+    B_nk = rng.standard_normal((1032, K)).astype(np.float16)
+    values = bv
+    for scale in (1.0, -2.0):
+        if scale != 1.0:
+            A.bcsrVal.mul_(scale)
+            plan.set_values()
+            values = (values * np.float16(scale)).astype(np.float16)
+        for N in (8, hint, 72, 1032):
+            C = S.Matrix(rows, N, fill=float("nan"))
+            before = S.launch_count()
+            plan.spmm(S.Matrix.from_host(B_nk[:N]), C, check=True)
+            assert S.launch_count() - before <= 2
+            got, n0 = C.data.cpu().numpy(), max(0, N - 40)
+            ref = oracle.bcsr_spmm(values, brp, bci, B_nk[n0:N], M, N - n0, K, b0, b1, threads=8).astype(np.float16).astype(np.float32)
+            mag = oracle.bcsr_spmm(np.abs(values), brp, bci, np.abs(B_nk[n0:N]), M, N - n0, K, b0, b1, threads=8)
+            assert float(np.max(np.abs(got[:, n0:].astype(np.float32) - ref) / (np.maximum(np.abs(ref), 1e-2 * mag) + 1e-30))) <= TOL
+            assert np.all(got.reshape(b1 - b0, -1)[counts[b0:b1] == 0] == 0)
+    plan.close()
