@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const uint4* __restrict__ val
 // ---- tall plans: groups of up to kTallRows block-rows (one warp of this kernel per block-row), 16-byte step records,
 // ---- 64 bytes of per-warp words per step (the input of tall_pair_kernel below), groups padded to an even step count ----
 constexpr int kTallPlanThreads = 1024;  // warp w owns block-row w of the group
-static_assert(kTallRows == 24 && kTallBlocksPerStep <= 32, "the per-warp step words below are laid out for 12 warps of two rows and 5-bit block positions");
+static_assert(kTallRows == 24 && kTallBlocksPerStep <= 64, "the per-warp step words below are laid out for 12 warps of two rows and 6-bit block positions");
 
 template <bool FILL, int WIN>
 __global__ void __launch_bounds__(kTallPlanThreads)
@@ -371,13 +371,13 @@ plan_tall_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx,
                                     const uint32_t own = (part[sub] >> (2 * m)) & 3u;
                                     const uint32_t q = pre[sub] + (uint32_t)__popc(part[sub] & ((1u << (2 * m)) - 1u));
                                     word |= own << (2 * sub);
-                                    word |= (q & 31u) << (8 + 5 * sub);
+                                    word |= (q & 63u) << (8 + 6 * sub);
                                 }
                                 wi[mm] = word;
                             }
                             wdst[v] = make_uint4(wi[0], wi[1], wi[2], wi[3]);
                         }
-                        wdst[3] = make_uint4((part[0] ? 1u : 0u) | (part[1] ? 2u : 0u) | (part[2] ? 4u : 0u) | (part[3] ? 8u : 0u), 0u, 0u, 0u);
+                        wdst[3] = make_uint4((uint32_t)taken, 0u, 0u, 0u);
                         s++;
                         b += taken;
                         c -= taken;
@@ -409,36 +409,43 @@ plan_tall_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx,
 
 // Tall plans, last pass: the kernel hands its MMA warps the steps two at a time, so what each warp has to issue for a
 // pair is listed here once, ready to use.  One thread per (pair, warp m): from the two steps' words (bits 2s, 2s + 1
-// = rows 2m, 2m + 1 have a block in sub-column s; bits [8 + 5s, 13 + 5s) = position of the first of them among the
-// step's blocks) to four words holding up to eight 16-bit entries, one per MMA, in (step, sub-column) order:
-//   bits [0, 6)  block position in the pair's two block slots (24 * step + position in the step)
-//   bits [6, 9)  panel sub-column, 4 * step + s            bit 9  accumulator of row 2m + 1 (else 2m)
-//   bit 10       both rows (one MMA of 32 accumulator columns)
-// and the number of entries in bits [28, 32) of word 0 (the spare bits of its second entry).
+// = rows 2m, 2m + 1 have a block in sub-column s; bits [8 + 6s, 14 + 6s) = position of the first of them among the
+// step's blocks) to the list described at kTallListBytes, its entries in (step, sub-column, row) order.
 __global__ void __launch_bounds__(256) tall_pair_kernel(const uint32_t* __restrict__ wstep, uint4* __restrict__ winfo,
                                                        const int* __restrict__ gsp, int n_groups) {
     ptx::pdl_wait();
-    const int pairs = __ldg(gsp + n_groups) >> 1;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs * 16; i += gridDim.x * blockDim.x) {
-        const int pr = i >> 4, m = i & 15;
-        uint32_t out[4] = {0u, 0u, 0u, 0u};
-        if (m < kTallRows / 2) {
-            uint32_t n = 0;
-            for (uint32_t st = 0; st < 2; st++) {
-                const uint32_t x = __ldg(wstep + ((size_t)(2 * pr) + st) * 16 + m);
-                for (uint32_t sub = 0; sub < 4; sub++) {
-                    const uint32_t own = (x >> (2 * sub)) & 3u;
-                    if (!own) continue;
-                    const uint32_t q = (x >> (8 + 5 * sub)) & 31u;
-                    const uint32_t e = (st * (uint32_t)kTallBlocksPerStep + q) | ((4 * st + sub) << 6) | ((own == 2u ? 1u : 0u) << 9) |
-                                       ((own == 3u ? 1u : 0u) << 10);
-                    out[n >> 1] |= e << (16 * (n & 1));
-                    n++;
-                }
-            }
-            out[0] |= n << 28;
+    constexpr uint32_t NM = kTallRows / 2;
+    const unsigned n_lists = (unsigned)(__ldg(gsp + n_groups) >> 1) * NM;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n_lists; i += gridDim.x * blockDim.x) {
+        const unsigned pr = i / NM, m = i - pr * NM;
+        const uint32_t word[2] = {__ldg(wstep + ((size_t)(2 * pr)) * 16 + m), __ldg(wstep + ((size_t)(2 * pr) + 1) * 16 + m)};
+        const uint32_t first_blocks = __ldg(wstep + ((size_t)(2 * pr)) * 16 + NM);  // of the first step: the second's follow them
+        const uint32_t n = (uint32_t)__popc(word[0] & 0xffu) + (uint32_t)__popc(word[1] & 0xffu);
+        uint32_t left[2] = {word[0], word[1]};  // bits [0, 8): blocks not listed yet
+        auto next = [&]() {                     // entry of the next block
+            const uint32_t st = (left[0] & 0xffu) ? 0u : 1u;
+            const uint32_t x = word[st], bit = (uint32_t)__ffs((int)(left[st] & 0xffu)) - 1u, sub = bit >> 1, row = bit & 1u;
+            left[st] &= left[st] - 1u;
+            // position: that of the first block of the warp in this sub-column, one more for the second row behind the first
+            const uint32_t q = ((x >> (8 + 6 * sub)) & 63u) + (row & (x >> (2 * sub)) & 1u);
+            return ((st * first_blocks + q) * 32u) << 16 | ((4 * st + sub) * 8u) << 8 | row * 16u;
+        };
+        uint4* out = winfo + (size_t)i * (kTallListBytes / 16);
+        uint4 v = make_uint4(0u, 0u, 0u, 0u), z = v, e = v, f = v;
+        const uint32_t last = n == 16 ? 1u : 0u, c = n - last;
+        v.x = (c & 1u ? kTallList1 : 0u) | (c & 2u ? kTallList2 : 0u) | (c & 4u ? kTallList4 : 0u) | (c & 8u ? kTallList8 : 0u);
+        if (c & 1u) v.y = next();
+        if (c & 2u) { v.z = next(); v.w = next(); }
+        if (c & 4u) { z.x = next(); z.y = next(); z.z = next(); z.w = next(); }
+        if (c & 8u) {
+            e.x = next(); e.y = next(); e.z = next(); e.w = next();
+            f.x = next(); f.y = next(); f.z = next(); f.w = next();
         }
-        winfo[(size_t)pr * 16 + m] = make_uint4(out[0], out[1], out[2], out[3]);
+        if (last) v.x |= kTallListLast | next();
+        out[0] = v;
+        out[1] = z;
+        out[2] = e;
+        out[3] = f;
     }
 }
 
@@ -1022,8 +1029,8 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     const size_t fix_bytes = (balanced ? 2 : 1) * fix_scratch_bytes(ctx->sm_count);
     size_t plan_bytes = 0;
     if (rc == SMAT_OK) {
-        // tall: + 64 bytes of per-step words + 128 bytes of the per-pair lists
-        sz = plan_sizes(nnzb, brow_begin, brow_end, rg_used, (size_t)(steps_final > 0 ? steps_final : 1) * (tall ? 13 : 1));
+        // tall: + 64 bytes of per-step words + half a pair's lists
+        sz = plan_sizes(nnzb, brow_begin, brow_end, rg_used, (size_t)(steps_final > 0 ? steps_final : 1) * (tall ? 5 + kTallRows / 2 * kTallListBytes / 32 : 1));
         plan_bytes = fix_bytes + sz.steps_bytes + sz.blk_bytes + sz.packed_bytes;
         e = cudaMalloc(&p->buffer, plan_bytes + (stream_too ? layout.bytes() : 0));
         if (e == cudaErrorMemoryAllocation && stream_too) {  // no room for two copies of the blocks: all products with the first

@@ -112,8 +112,9 @@ inline double tall_rounds(size_t items, size_t sms, double est_steps) {
     const size_t P = tail_parts_for(items, sms, true, (size_t)est_steps);
     return (double)(items / sms) + 1.0 / (double)P + (P > 1 ? 12.0 / est_steps : 0.0);
 }
-// Cycles of a step of the tall kernel that holds `blocks` blocks (measured with 12 to 20 blocks a step: 544 to 640).
-inline double tall_step_cycles(double blocks) { return 350.0 + 15.0 * blocks > 500.0 ? 350.0 + 15.0 * blocks : 500.0; }
+// Cycles of a step of the tall kernel that holds `blocks` blocks (measured on layers: 374 with 9 blocks a step, 482 with 12.5, 513
+// with 15.5, 569 with 18.6, about 800 with 31).
+inline double tall_step_cycles(double blocks) { return 300.0 + 15.0 * blocks > 400.0 ? 300.0 + 15.0 * blocks : 400.0; }
 // ... and what a launch of it costs beyond its steps: its pipeline takes longer to fill and to drain (measured, smallest plans).
 constexpr double kTallExtraCycles = 5000.0;
 // Measured cost of a 256-column item relative to a 128-column item of the same group.
@@ -133,7 +134,16 @@ constexpr int kPlanBlocksPerStepDense = 32;
 // steps of at most kTallBlocksPerStep blocks, an even number of steps per group, and per pair of steps the list of
 // MMAs of each issuing warp (PlanView::winfo).
 constexpr int kTallRows = 24;
-constexpr int kTallBlocksPerStep = 24;
+constexpr int kTallBlocksPerStep = 48;
+// The list of an issuing warp: 16 words.  One MMA per block; an entry holds what is added to the addresses of the pair's slots:
+//   bits [0, 5)   accumulator, in tensor-memory columns (0 or 16)
+//   bits [8, 16)  panel sub-column, in tensor-memory columns (8 each; 32 more for the second step)
+//   bits [16, 28) block of the pair, in 16-byte units (32 each)
+// Word 0 tells which groups there are (so that the warp decides once per group, not per MMA) and holds the entry of the last;
+// word 1: the group of one; words 2, 3: of two; 4 to 7: of four; 8 to 15: of eight.
+constexpr int kTallListBytes = 64;
+constexpr uint32_t kTallList1 = 1u << 31, kTallList2 = 1u << 30, kTallList4 = 1u << 29, kTallList8 = 1u << 28, kTallListLast = 1u << 7;
+static_assert(2 * kTallBlocksPerStep * 32 <= 1 << 12, "an entry's block");
 // MMA-issuing warps of the kernel; each owns kPlanRowsPerGroup / kPlanOwners consecutive accumulators.
 #ifndef SMAT_OWNERS
 #define SMAT_OWNERS 8
@@ -169,8 +179,7 @@ struct PlanView {
     // Tall plan: groups of rg <= kTallRows block-rows with an even number of steps, at most kTallBlocksPerStep blocks
     // per step.  A step record is {element column of the quad, position of the first block in the packed stream in
     // 256-byte units, number of blocks (0: a step that only pads its group), non-empty sub-columns (bit s)}; winfo
-    // holds 16 x 16 bytes per PAIR of steps: entry m < 12 lists the MMAs of the warp that owns block-rows 2m, 2m + 1
-    // (layout: tall_pair_kernel in plan.cu).
+    // holds kTallRows / 2 lists per PAIR of steps: list m has the MMAs of the warp that owns block-rows 2m, 2m + 1.
     bool tall = false;
     const void* winfo = nullptr;
     // The heaviest group has many times the average number of steps: deal out equal step ranges instead of items

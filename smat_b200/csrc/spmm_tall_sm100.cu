@@ -17,25 +17,32 @@
 //     a barrier wait cost the issuing thread ~100-200 cycles each, the tensor pipe nothing.  So 12 warps issue, each
 //     owning two accumulator rows (all MMAs into one accumulator come from one thread, in order: results do not
 //     depend on warp timing), the steps are handed over two at a time, and the plan lists each warp's MMAs of a pair
-//     of steps so that the warp works the list off in straight-line code.
+//     of steps, in groups of 1, 2, 4 and 8, so that the warp decides once per group instead of once per MMA.
+//   * tcgen05.cp and tcgen05.mma of an SM run one after the other, in the order in which they were issued, or nearly so: the
+//     eight copies of a pair take 64 cycles each, 36 MMAs beside them add 107 cycles and 72 MMAs 383.
 //
 // Pipeline per step (four block-columns of a group), all hand-overs by mbarriers, every wait bounded:
-//   loader warps (4, one thread each, every 4th step): TMA box {64 k, 128 n} -> panel slot (6 slots), bulk copy of the
-//     step's packed A blocks -> block slot (10 slots) and, with the first step of a pair, of the pair's MMA lists;
+//   panel loaders (4 warps, one thread each, every 4th step): TMA box {64 k, 128 n} -> panel slot (6 slots);
+//   block loader (1 warp, one thread): per pair, one bulk copy of the packed A blocks of its steps, which follow one another in
+//     the plan, to the next free place of a ring of RING_BLOCKS blocks, and one of the pair's MMA lists.  Slots of a fixed
+//     size would have to be as large as the largest step, so steps would have to be cut short: with a ring a step holds up to
+//     kTallBlocksPerStep blocks, twice as many as with slots, and its panel is fetched and copied once (random matrix of
+//     65536 rows, 22 blocks a step: 217 000 -> 175 000 steps, 831 -> 744 us; layer 8192 x 28672, N = 4096: 737 -> 704);
 //   copier warps (4, one thread each, every 4th step): wait panel + blocks, tcgen05.cp the non-empty sub-columns
 //     shared -> tensor memory ring, commit -> cp_done of the step's pair.  That frees the shared panel slot for the
 //     loader and tells the MMA warps that panels AND blocks of the pair are in place;
 //   MMA warps (one per two accumulator rows): per PAIR of steps wait cp_done once, read their list, issue, commit ->
-//     step_done (a plain arrive when the warp had no block in the pair); step_done frees the block slots (loader)
+//     step_done (a plain arrive when the warp had no block in the pair); step_done frees the blocks (block loader)
 //     and the tensor-memory panel slots (copier) of the pair;
 //   epilogue warps (8 = two per tensor-memory lane quarter, alternating block-rows): tcgen05.ld -> zero the
 //     accumulator -> fp16 -> 4-byte stores to C; cut items write fp32 partial tiles.
 // Groups of at most 16 or 20 block-rows use fewer accumulators and a longer tensor-memory panel ring (8 or 6 slots
 // instead of 4).  Scheduling is the round-robin-with-cut-last-round scheme of spmm_sm100.cu (SegGen<0>); the plan
 // pads every group to an even number of steps and items are cut at even positions, so a pair never spans two items.
-// What bounds the kernel on the block-sparse layer it was written for: every step moves 16 KB of panel and ~10 KB of
-// blocks from L2 to the SM, and 148 SMs doing that every ~600 cycles is ~12 TB/s, two thirds of what L2 delivered
-// to a pure streaming kernel (19-20 TB/s); the rest is latency of the chain copy -> MMAs -> slot release.
+// What bounds the kernel on the block-sparse layer it was written for (1190 cycles per pair of steps at 24 rows): the loop copy ->
+// MMAs -> slot release, with two pairs of panels in tensor memory.  Of it 512 cycles are the copies themselves, 300 the MMAs, the
+// rest hand-overs; without panels, copies and MMAs the loop alone takes 650.  The loads (52 KB a pair) would take 740 at the rate
+// at which L2 serves a pure streaming kernel (70 bytes per cycle and SM).
 #include <cuda_fp16.h>
 #include <limits.h>
 #include <stdlib.h>
@@ -52,35 +59,38 @@ using namespace ptx;
 
 namespace {
 
-constexpr int NLW = 4;           // panel-loader warps, and as many block-loader warps
-constexpr int LW = 2 * NLW;      // loader warps in all
+constexpr int NLW = 4;           // panel-loader warps
+constexpr int LW = NLW + 1;      // loader warps in all: one more loads the blocks
 constexpr int NCW = 4;           // copier warps
 constexpr int NEW = 8;           // epilogue warps
 constexpr uint32_t PS = 6;                                   // panel slots in shared memory (a slot is free once copied to tensor memory)
-constexpr uint32_t BS = 10;                                  // block slots (held until the step's MMAs have completed)
 constexpr uint32_t PANEL_BYTES = 128 * 64 * 2;               // 128 n x 64 k fp16
-constexpr uint32_t BLK_SLOT_BYTES = kTallBlocksPerStep * 512;
+// The blocks of a pair of steps lie one after the other in a ring (never around its end) until the pair's MMAs have completed.
+constexpr uint32_t RING_BLOCKS = 246;
+constexpr uint32_t NLIST = 7;                                 // pairs with blocks in the ring, at most: list slots
+constexpr uint32_t META_BYTES = kTallRows / 2 * kTallListBytes;  // per pair of steps: the MMA lists of the 12 issuing warps
 constexpr uint32_t OFF_PANEL = 0;
 constexpr uint32_t OFF_BLK = OFF_PANEL + PS * PANEL_BYTES;
-constexpr uint32_t META_BYTES = 256;                          // per pair of steps: the MMA lists of the 12 issuing warps
-constexpr uint32_t OFF_META = OFF_BLK + BS * BLK_SLOT_BYTES;
-constexpr uint32_t OFF_SUBS = OFF_META + (BS / 2) * META_BYTES;  // per step: its non-empty sub-columns (written by the loader)
-constexpr uint32_t OFF_BAR = OFF_SUBS + BS * 8;
-// A thread that waits on an mbarrier by parity must see every phase of it.  Loader j and copier j handle the steps
-// st = j (mod 4), so a "full" barrier ring is as long as lcm(slots, 4): barrier st % ring then always belongs to
-// the same loader and the same copier.  The per-pair rings (8 barriers) are visited by a loader or copier at every
-// other pair, i.e. each barrier of its parity class once per 8 pairs: once per phase.
+constexpr uint32_t OFF_META = OFF_BLK + RING_BLOCKS * 512;
+// A thread that waits on an mbarrier by parity must see every phase of it.  Panel loader j and copier j handle the steps
+// st = j (mod 4), so the full_p ring is as long as lcm(PS, 4): barrier st % ring then always belongs to the same loader and the
+// same copier.  The per-pair rings (8 barriers) are visited by a loader or copier at every other pair, i.e. each barrier of
+// its parity class once per 8 pairs: once per phase; the block loader visits them all, in order.
 constexpr uint32_t FP = 12;                                   // full_p ring: lcm(PS, 4)
-constexpr uint32_t FB = 20;                                   // full_b ring: lcm(BS, 4)
-constexpr uint32_t NPAIR = 8;                                 // cp_done / step_done rings (pairs of steps)
-constexpr uint32_t N_BARS = FP + FB + NPAIR + NPAIR + 2;
+constexpr uint32_t NPAIR = 8;                                 // full_b / cp_done / step_done rings (pairs of steps)
+constexpr uint32_t OFF_SUBS = OFF_META + NLIST * META_BYTES;  // per step (full_p ring): its non-empty sub-columns, by the panel loader
+constexpr uint32_t OFF_AT = OFF_SUBS + FP * 4;                // per pair (NPAIR ring): place of its blocks, in blocks, by the block loader
+constexpr uint32_t OFF_END = OFF_AT + NPAIR * 4;              // ... and the count of blocks up to its end, for the block loader itself
+constexpr uint32_t OFF_BAR = OFF_END + NPAIR * 4;
+constexpr uint32_t N_BARS = FP + 3 * NPAIR + 2;
 constexpr uint32_t OFF_MISC = OFF_BAR + N_BARS * 8;
 constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;        // slack for the manual 1024-byte alignment
 constexpr uint32_t TMEM_ACC = 0;                             // accumulators: one per block-row, 16 columns each
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
-static_assert(NLW == 4 && NCW == 4 && FP % PS == 0 && FP % 4 == 0 && FB % BS == 0 && FB % 4 == 0 && PS % 2 == 0 && BS % 2 == 0 &&
-                  NPAIR % 2 == 0 && NPAIR > BS / 2,
+static_assert(NLW == 4 && NCW == 4 && FP % PS == 0 && FP % 4 == 0 && PS % 2 == 0 && NPAIR % 2 == 0 && NLIST < NPAIR && OFF_BAR % 8 == 0,
               "the barrier phase arithmetic below assumes these");
+// a pair that does not fit behind the last one leaves less than its own size unused at the end of the ring
+static_assert(RING_BLOCKS >= 2 * 2 * kTallBlocksPerStep, "any pair must fit an empty ring, wherever the last one ended");
 static_assert(kTallRows * 16 * 128 <= kFixSlotFloats, "a partial tile must fit a scratch slot");
 
 // Shape of a work item: TRG block-rows (accumulators), two of them per MMA-issuing warp.  What tensor memory the
@@ -98,7 +108,6 @@ struct Shape {
 struct TallStep {
     int live;
     int tile;
-    int idx;      // index of the step in the plan
     uint32_t st;  // its position in this CTA's sequence
     uint4 a;      // {element column, packed position (256-byte units), blocks, non-empty sub-columns}
 };
@@ -116,13 +125,13 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bar0 = base + OFF_BAR;
     auto full_p = [&](uint32_t s) { return bar0 + 8 * s; };
-    auto full_b = [&](uint32_t s) { return bar0 + 8 * (FP + s); };
+    auto full_b = [&](uint32_t p) { return bar0 + 8 * (FP + p); };  // blocks and lists of pair p (mod NPAIR) have arrived
     // The MMA warps are handed the steps two at a time (pair p = steps 2p, 2p + 1 of the CTA's sequence, whatever
     // work items they belong to): measured, a barrier wait or a commit costs the issuing thread about as much as an
     // MMA (~100 cycles), so one of each per step and warp would hold the whole pipeline back.
-    auto cp_done = [&](uint32_t p) { return bar0 + 8 * (FP + FB + p); };            // both panels of pair p (mod NPAIR) copied
-    auto step_done = [&](uint32_t p) { return bar0 + 8 * (FP + FB + NPAIR + p); };  // all MMAs of pair p (mod NPAIR) completed
-    const uint32_t acc_full = bar0 + 8 * (FP + FB + 2 * NPAIR), acc_empty = acc_full + 8;
+    auto cp_done = [&](uint32_t p) { return bar0 + 8 * (FP + NPAIR + p); };            // both panels of pair p (mod NPAIR) copied
+    auto step_done = [&](uint32_t p) { return bar0 + 8 * (FP + 2 * NPAIR + p); };  // all MMAs of pair p (mod NPAIR) completed
+    const uint32_t acc_full = bar0 + 8 * (FP + 3 * NPAIR), acc_empty = acc_full + 8;
     const uint32_t tmem_slot = base + OFF_MISC;
     const uint32_t abort_addr = base + OFF_MISC + 4;
 
@@ -164,8 +173,8 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < FP; s++) mbar_init(full_p(s), 1);
-        for (uint32_t s = 0; s < FB; s++) mbar_init(full_b(s), 1);
-        for (uint32_t s = 0; s < NPAIR; s++) { mbar_init(cp_done(s), 4); mbar_init(step_done(s), NMW); }  // cp_done: per step a commit and an arrive
+        // cp_done: a commit for each step of the pair, and an arrive for its blocks and lists
+        for (uint32_t s = 0; s < NPAIR; s++) { mbar_init(full_b(s), 1); mbar_init(cp_done(s), 3); mbar_init(step_done(s), NMW); }
         mbar_init(acc_full, NMW);
         mbar_init(acc_empty, NEW);
         st_shared_u32(abort_addr, 0);
@@ -192,17 +201,15 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
     tc_fence_after();
 
     if (warp < LW) {
-        // ---------------- loader warps: panel loader j and block loader j take the steps j, j + NLW, ... ----------------
-        // (two threads per step, so that neither waits for the other's slot and each has half the work per step)
-        if (lane == 0) {
-            const bool panels = warp < NLW;
-            const int j = warp % NLW;
+        // ---------------- loader warps: panel loader j takes the steps j, j + NLW, ...; the block loader all pairs ----------------
+        if (lane == 0 && warp < NLW) {
+            const int j = warp;
             SegGen<0> sg = make_gen();
             Seg cs;
             bool have = sg.next(cs);
             uint32_t h_st0 = 0, h_next = (uint32_t)j;
             constexpr int U = 4;  // step records in flight per loader (their descriptors are requested U positions ahead)
-            constexpr int PF = 2;  // records ahead (of this loader) whose data is prefetched into L2 when the launch asks for it
+            constexpr int PF = 2;  // records ahead (of this loader) whose panel is prefetched into L2 when the launch asks for it
             TallStep rec[U];
             auto gen = [&](TallStep& r) {
                 while (have && h_next >= h_st0 + (uint32_t)(cs.k1 - cs.k0)) {
@@ -213,16 +220,12 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                 if (have) {
                     r.tile = cs.item % n_tiles;
                     r.st = h_next;
-                    r.idx = cs.gs + cs.k0 + (int)(h_next - h_st0);
-                    r.a = __ldg(steps + r.idx);
+                    r.a = __ldg(steps + (cs.gs + cs.k0 + (int)(h_next - h_st0)));
                     h_next += NLW;
                 }
             };
             auto prefetch = [&](const TallStep& r) {  // HBM latency is hidden in L2: fetched PF records ahead of the copies
-                if (pf && r.live && r.a.z) {
-                    if (panels) tma_prefetch_l2_2d(&mapB, (int)r.a.x, r.tile * 128);
-                    else bulk_prefetch_l2(packed + (size_t)r.a.y * 256, r.a.z * 512u);
-                }
+                if (pf && r.live && r.a.z) tma_prefetch_l2_2d(&mapB, (int)r.a.x, r.tile * 128);
             };
 #pragma unroll
             for (int a = 0; a < U; a++) gen(rec[a]);
@@ -234,30 +237,63 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                 for (int a = 0; a < U; a++) {
                     TallStep& r = rec[a];
                     if (!r.live) { more = false; break; }
-                    const uint32_t ps = r.st % PS, bs = r.st % BS, pi = r.st >> 1;
-                    const uint32_t a_bytes = r.a.z * 512u;  // 0: a step that only pads its group to an even count
-                    if (panels) {
-                        // the panel's slot is free once the copy of the step PS positions back (pair pi - PS / 2) has left it
-                        if (r.st >= PS) TWAIT(cp_done((pi - PS / 2) % NPAIR), ((pi - PS / 2) / NPAIR) & 1, 1);
-                        if (a_bytes) {
-                            mbar_arrive_expect_tx(full_p(r.st % FP), panel_bytes);
-                            tma_load_2d(base + OFF_PANEL + ps * PANEL_BYTES, &mapB, (int)r.a.x, r.tile * 128, full_p(r.st % FP));
-                        } else {
-                            mbar_arrive(full_p(r.st % FP));  // no panel: the phase completes at once
-                        }
+                    const uint32_t ps = r.st % PS, fp = r.st % FP, pi = r.st >> 1;
+                    // the panel's slot is free once the copy of the step PS positions back (pair pi - PS / 2) has left it
+                    if (r.st >= PS) TWAIT(cp_done((pi - PS / 2) % NPAIR), ((pi - PS / 2) / NPAIR) & 1, 1);
+                    st_shared_u32(base + OFF_SUBS + fp * 4, r.a.w);  // for the copier; ordered before its wait by the arrive below
+                    if (r.a.z) {
+                        mbar_arrive_expect_tx(full_p(fp), panel_bytes);
+                        tma_load_2d(base + OFF_PANEL + ps * PANEL_BYTES, &mapB, (int)r.a.x, r.tile * 128, full_p(fp));
                     } else {
-                        // the slot of the blocks is free once the MMAs of the step BS positions back (pair pi - BS / 2) have completed
-                        if (r.st >= BS) TWAIT(step_done((pi - BS / 2) % NPAIR), ((pi - BS / 2) / NPAIR) & 1, 2);
-                        st_shared_u32(base + OFF_SUBS + bs * 8, r.a.w);  // for the copier; ordered before its wait by the arrive below
-                        const uint32_t m_bytes = (r.st & 1u) ? 0u : META_BYTES;  // the pair's lists travel with its first step
-                        if (a_bytes + m_bytes) mbar_arrive_expect_tx(full_b(r.st % FB), a_bytes + m_bytes);
-                        else mbar_arrive(full_b(r.st % FB));
-                        if (m_bytes)
-                            bulk_load(base + OFF_META + (bs >> 1) * META_BYTES, winfo + 16 * (size_t)(r.idx >> 1), META_BYTES, full_b(r.st % FB));
-                        if (a_bytes) bulk_load(base + OFF_BLK + bs * BLK_SLOT_BYTES, packed + (size_t)r.a.y * 256, a_bytes, full_b(r.st % FB));
+                        mbar_arrive(full_p(fp));  // a step that only pads its group: no panel, the phase completes at once
                     }
                     prefetch(rec[(a + PF) % U]);
                     gen(r);
+                }
+            }
+        } else if (lane == 0) {
+            SegGen<0> sg = make_gen();
+            Seg cs;
+            uint32_t pi = 0;                 // the pair to load
+            uint32_t done = 0;               // pairs known to have completed
+            uint32_t head = 0;               // where its blocks go if they fit before the end of the ring
+            uint32_t used = 0, freed = 0;    // blocks of the ring taken (with what was left out at its end) and given back, ever
+            constexpr int U = 4;             // pairs whose step records are requested ahead
+            struct { uint32_t at, n; } rec[U];
+            while (sg.next(cs)) {
+                const int first = (cs.gs + cs.k0) >> 1, n_pairs = (cs.k1 - cs.k0) >> 1;
+                auto gen = [&](int i, int a) {
+                    if (i >= n_pairs) return;
+                    const uint4 s0 = __ldg(steps + 2 * (first + i)), s1 = __ldg(steps + 2 * (first + i) + 1);
+                    rec[a].at = s0.y;
+                    rec[a].n = s0.z + s1.z;  // the blocks of a group's steps follow one another
+                };
+#pragma unroll
+                for (int a = 0; a < U; a++) gen(a, a);
+                for (int i0 = 0; i0 < n_pairs; i0 += U) {
+#pragma unroll
+                    for (int a = 0; a < U; a++) {
+                        if (i0 + a >= n_pairs) break;
+                        const uint32_t n = rec[a].n, pl = pi % NPAIR;
+                        if (head + n > RING_BLOCKS) {
+                            used += RING_BLOCKS - head;
+                            head = 0;
+                        }
+                        used += n;
+                        while (done < pi && (pi - done >= NLIST || used - freed > RING_BLOCKS)) {
+                            TWAIT(step_done(done % NPAIR), (done / NPAIR) & 1, 2);
+                            freed = ld_shared_u32(base + OFF_END + (done % NPAIR) * 4);
+                            done++;
+                        }
+                        st_shared_u32(base + OFF_AT + pl * 4, head);
+                        st_shared_u32(base + OFF_END + pl * 4, used);
+                        mbar_arrive_expect_tx(full_b(pl), n * 512u + META_BYTES);
+                        bulk_load(base + OFF_META + (pi % NLIST) * META_BYTES, winfo + (META_BYTES / 16) * (size_t)(first + i0 + a), META_BYTES, full_b(pl));
+                        if (n) bulk_load(base + OFF_BLK + head * 512u, packed + (size_t)rec[a].at * 256, n * 512u, full_b(pl));
+                        head += n;
+                        pi++;
+                        gen(i0 + a + U, a);
+                    }
                 }
             }
         }
@@ -277,16 +313,15 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
             }
             total = (uint32_t)__shfl_sync(0xffffffffu, total, 0);
             for (uint32_t st = j; st < total; st += NCW) {
-                const uint32_t ps = st % PS, bs = st % BS, pi = st >> 1;
+                const uint32_t ps = st % PS, fp = st % FP, pi = st >> 1;
                 // what is usually there already first: blocks and panel wait in shared memory for a tensor-memory slot,
                 // which is free once the MMAs of the step TS_ positions back (pair pi - TS_ / 2) have completed; only
                 // the copies follow that
-                TWAIT(full_b(st % FB), (st / FB) & 1, 4);
-                const uint32_t subs_l = ld_shared_u32(base + OFF_SUBS + bs * 8);  // non-empty sub-columns
-                const uint32_t subs = __ballot_sync(0xffffffffu, (subs_l >> lane) & 1u);
+                if (!(j & 1u)) TWAIT(full_b(pi % NPAIR), (pi / NPAIR) & 1, 4);  // the copier of a pair's first step looks after its blocks
                 const uint64_t pdesc = smem_desc_k_sw128(base + OFF_PANEL + ps * PANEL_BYTES);
                 const uint32_t tdst = tmem_base + TMEM_PANELS + (st % TS_) * 32;
-                TWAIT(full_p(st % FP), (st / FP) & 1, 3);
+                TWAIT(full_p(fp), (st / FP) & 1, 3);
+                const uint32_t subs = uniform(ld_shared_u32(base + OFF_SUBS + fp * 4));  // non-empty sub-columns
                 if (pi >= TS_ / 2) TWAIT(step_done((pi - TS_ / 2) % NPAIR), ((pi - TS_ / 2) / NPAIR) & 1, 5);
 #ifdef SMAT_PROFILE
                 if (pi >= TS_ / 2) prof_c[13] += (unsigned int)clock() - *(volatile unsigned int*)&stamp_mma[(pi - TS_ / 2) % 8];
@@ -301,7 +336,7 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                     tc_commit(cp_done(pi % NPAIR));
                     // A plain arrive beside the commit's: it is ordered after this thread's wait for the blocks and
                     // lists of the step, so whoever passes cp_done may read them (the MMA warps wait for nothing else).
-                    mbar_arrive(cp_done(pi % NPAIR));
+                    if (!(j & 1u)) mbar_arrive(cp_done(pi % NPAIR));
                 }
 #ifdef SMAT_PROFILE
                 if (leader) atomicMax(&stamp_cp[pi % 8], (unsigned int)clock());
@@ -312,16 +347,18 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
         __syncwarp();
     } else if (warp < LW + NCW + NMW) {
         // ------------------------------ MMA warp m: accumulator rows 2m, 2m + 1 ------------------------------
-        // The whole warp runs the loop converged and one elected lane issues.  Every operand of a tcgen05.mma must
-        // be a value the compiler knows to be warp-uniform (the instruction reads uniform registers): measured, the
+        // The whole warp runs the loop converged and its MMAs are issued under a predicate of one elected lane.  Every operand of a
+        // tcgen05.mma must be a value the compiler knows to be warp-uniform (the instruction reads uniform registers): measured, the
         // same loop run by a single lane on values loaded from shared memory is 10 % slower over the whole kernel.
-        // So the list words, read from shared memory, are turned into ballots before anything is derived from them.
+        // So the list words, read from shared memory, go through a warp reduction before anything is derived from them.
+        // In isolation (12 warps, 3 MMAs each a pair) the loop takes 500 cycles a pair; with one switch on the number of MMAs inside
+        // a region of the elected lane it took 660: 120 of them the jump, 45 to 90 the region's end.
         {
             const uint32_t m = (uint32_t)__shfl_sync(0xffffffffu, warp - LW - NCW, 0);
-            const bool leader = elect_one();
+            const uint32_t leader = elect_one();
             const uint32_t B_HI = (uint32_t)(smem_desc_k_sw32(0) >> 32);
             const uint32_t b_lo0 = (uint32_t)smem_desc_k_sw32(base + OFF_BLK);
-            constexpr uint32_t IDESC16 = idesc_f16_f32(128, 16), IDESC32 = idesc_f16_f32(128, 32);
+            constexpr uint32_t IDESC16 = idesc_f16_f32(128, 16);
             const uint32_t acc_m = tmem_base + TMEM_ACC + 2u * m * 16u;  // this warp's two accumulators
             uint32_t st = 0, it = 0;
             SegGen<0> sg = make_gen();
@@ -331,70 +368,56 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                 tc_fence_after();
                 // segments hold an even number of steps and start at an even position: a pair never spans two of them
                 for (int k = cs.k0; k < cs.k1; k += 2, st += 2) {
-                    const uint32_t pi = st >> 1, bs = st % BS;
+                    const uint32_t pi = st >> 1;
                     PROF_MARK(0);
                     TWAIT(cp_done(pi % NPAIR), (pi / NPAIR) & 1, 7);
 #ifdef SMAT_PROFILE
                     prof_c[12] += (unsigned int)clock() - *(volatile unsigned int*)&stamp_cp[pi % 8];
 #endif
                     tc_fence_after();
-                    // This warp's list for the pair: up to eight 16-bit entries, one per MMA (layout: tall_pair_kernel
-                    // in plan.cu), their number in the top bits of the first word.  Measured: the branches and the
-                    // register arithmetic around a tcgen05.mma cost the issuing thread far more than the instruction
-                    // (~15 cycles), and writing an operand register of an MMA just issued stalls it ~90 cycles.  So
-                    // the plan lists the MMAs, and the list is worked off in straight-line code entered at its length.
-                    const uint4 l = ld_shared_v4(base + OFF_META + (bs >> 1) * META_BYTES + m * 16u);
-                    uint32_t w[4];
-                    w[0] = __ballot_sync(0xffffffffu, (l.x >> lane) & 1u);
-                    w[1] = __ballot_sync(0xffffffffu, (l.y >> lane) & 1u);
-                    w[2] = __ballot_sync(0xffffffffu, (l.z >> lane) & 1u);
-                    w[3] = __ballot_sync(0xffffffffu, (l.w >> lane) & 1u);
+                    // This warp's list for the pair (layout: kTallListBytes in smat_internal.h): which of the groups of 1, 2, 4, 8
+                    // and 1 MMAs it has, and their entries.
+                    const uint32_t list = base + OFF_META + (pi % NLIST) * META_BYTES + m * kTallListBytes;
+                    const uint4 l = ld_shared_v4(list);
+                    const uint32_t b_lo = b_lo0 + uniform(ld_shared_u32(base + OFF_AT + (pi % NPAIR) * 4)) * 32u;
+                    const uint32_t w0 = uniform(l.x), w1 = uniform(l.y), w2 = uniform(l.z), w3 = uniform(l.w);
                     const uint32_t tpanel = tmem_base + TMEM_PANELS + (st % TS_) * 32;
-                    const uint32_t b_lo = b_lo0 + bs * (BLK_SLOT_BYTES >> 4);
-                    const uint32_t count = w[0] >> 28;
                     PROF_MARK(9);
-                    // operands of the first four entries (most lists are no longer) worked out here, where the warp is
-                    // converged and the values stay in uniform registers; the elected lane's region below only issues
-                    uint32_t od[4], oa[4], ob[4], oi[4];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const uint32_t e = (i & 1) ? (w[i >> 1] >> 16) : w[i >> 1];
-                        od[i] = acc_m + ((e >> 5) & 16u);
-                        oa[i] = tpanel + ((e >> 3) & 56u);
-                        ob[i] = b_lo + (e & 63u) * 32u;
-                        oi[i] = IDESC16 + ((e << 8) & (1u << 18));
+                    auto mma = [&](uint32_t e) {
+                        mma_f16_ts_if(leader, acc_m + (e & 0x1fu), tpanel + ((e >> 8) & 0xffu), b_lo + ((e >> 16) & 0xfffu), B_HI, IDESC16);
+                    };
+                    if (w0 & kTallList1) mma(w1);
+                    if (w0 & kTallList2) {
+                        mma(w2);
+                        mma(w3);
                     }
-#define SMAT_TALL_MMA(i)                                                                                               \
-    {                                                                                                                  \
-        if ((i) < 4) {                                                                                                 \
-            mma_f16_ts_lohi(od[(i) & 3], oa[(i) & 3], ob[(i) & 3], B_HI, oi[(i) & 3], 1u);                             \
-        } else {                                                                                                       \
-            const uint32_t e = ((i) & 1) ? (w[(i) >> 1] >> 16) : w[(i) >> 1];                                          \
-            mma_f16_ts_lohi(acc_m + ((e >> 5) & 16u), tpanel + ((e >> 3) & 56u), b_lo + (e & 63u) * 32u, B_HI,         \
-                            IDESC16 + ((e << 8) & (1u << 18)), 1u);                                                    \
-        }                                                                                                              \
-    }
-                    static_assert(IDESC32 == IDESC16 + (1u << 18), "the 32-column descriptor is the 16-column one plus bit 18");
-                    // one region of the elected lane per pair (every separate `if (leader)` costs the warp a divergence
-                    // and a reconvergence: one region instead of one per MMA was worth 7 % of the kernel's time)
-                    if (leader) {
-                        switch (count) {
-                            case 8: SMAT_TALL_MMA(7) [[fallthrough]];
-                            case 7: SMAT_TALL_MMA(6) [[fallthrough]];
-                            case 6: SMAT_TALL_MMA(5) [[fallthrough]];
-                            case 5: SMAT_TALL_MMA(4) [[fallthrough]];
-                            case 4: SMAT_TALL_MMA(3) [[fallthrough]];
-                            case 3: SMAT_TALL_MMA(2) [[fallthrough]];
-                            case 2: SMAT_TALL_MMA(1) [[fallthrough]];
-                            case 1: SMAT_TALL_MMA(0) tc_commit(step_done(pi % NPAIR)); break;
-                            default: mbar_arrive(step_done(pi % NPAIR)); break;
+                    if (w0 & (kTallList4 | kTallList8 | kTallListLast)) {
+                        if (w0 & kTallList4) {
+                            const uint4 q = ld_shared_v4(list + 16);
+                            const uint32_t e0 = uniform(q.x), e1 = uniform(q.y), e2 = uniform(q.z), e3 = uniform(q.w);
+                            mma(e0);
+                            mma(e1);
+                            mma(e2);
+                            mma(e3);
                         }
-#ifdef SMAT_PROFILE
-                        atomicMax(&stamp_mma[pi % 8], (unsigned int)clock());
-#endif
+                        if (w0 & kTallList8) {
+                            const uint4 q = ld_shared_v4(list + 32), r = ld_shared_v4(list + 48);
+                            const uint32_t e0 = uniform(q.x), e1 = uniform(q.y), e2 = uniform(q.z), e3 = uniform(q.w);
+                            const uint32_t e4 = uniform(r.x), e5 = uniform(r.y), e6 = uniform(r.z), e7 = uniform(r.w);
+                            mma(e0);
+                            mma(e1);
+                            mma(e2);
+                            mma(e3);
+                            mma(e4);
+                            mma(e5);
+                            mma(e6);
+                            mma(e7);
+                        }
+                        if (w0 & kTallListLast) mma(w0);
                     }
-#undef SMAT_TALL_MMA
                     PROF_MARK(10);
+                    if (w0) tc_commit_if(leader, step_done(pi % NPAIR));
+                    else if (leader) mbar_arrive(step_done(pi % NPAIR));
                     PROF_MARK(11);
                 }
                 if (leader) tc_commit(acc_full);
