@@ -15,7 +15,7 @@
 // cycle (60 cycles; 33 out of L1).  So where the blocks outnumber the block-columns enough, B is first rewritten as slabs
 // [K / 16][N][16], one pass over B.  mma.sync runs at 2.1-2.6 cycles per 16x8x16 MMA and SM (34 cycles per block of 128
 // columns) and is not what bounds it; a tcgen05.mma on one block would need its slice in shared memory (39 cycles for the
-// operand port alone) and a barrier round trip per hand-over.  At 128 columns no unit is full (ncu, power-law matrix of
+// operand port alone) and a barrier round trip per hand-over.  At 128 columns from slabs no unit is full (ncu, power-law matrix of
 // 464 000 blocks: L2 at 45 % of its peak, tensor pipe 34 %, HBM 17 %): 166 registers leave 12 warps per SM, each with the
 // loads of one block in flight, 49 bytes per cycle and SM at an L2 latency of about a thousand cycles.
 //
@@ -55,6 +55,128 @@ __device__ __forceinline__ uint2 load_a8(const void* p) {
     return v;
 }
 
+__device__ __forceinline__ uint4 lds16(uint32_t at) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 lds8(uint32_t at) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(at) : "memory");
+    return v;
+}
+constexpr int kRingWaitCode = 40;  // status word: a bounded wait of the ring kernel ran out
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
+    if (ptx::mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (!ptx::mbar_try_wait_suspend(bar, parity, 2000u))
+        if (clock64() - t0 > 4000000000LL) return false;  // about two seconds
+    return true;
+}
+
+// The blocks [b0, b1) of block-row `row` that a warp (or several) multiplies; count > 1: one of `count` pieces of a long block-row.
+struct Piece {
+    int row = 0, b0 = 0, b1 = 0, count = 1, my_slot = 0, first_slot = 0;
+    bool live = false;
+};
+template <bool PLAN>
+__device__ __forceinline__ Piece piece_of(const StreamArgs& p, int piece, int lane) {
+    Piece q;
+    q.live = piece < p.n_pieces;
+    if (!q.live) return q;
+    if (PLAN) {
+        const uint4 d = __ldg(p.pieces + piece);
+        q.row = (int)d.x; q.b0 = (int)d.y; q.b1 = (int)d.z;
+        if (d.w) {
+            const int2 s = __ldg(p.slots + (d.w - 1));
+            q.my_slot = (int)d.w - 1; q.first_slot = s.x; q.count = s.y;
+        }
+        return q;
+    }
+    const int n_rows = p.brow_end - p.brow_begin;
+    if (piece < n_rows) {
+        const int lo = __ldg(p.rowptr + p.brow_begin), hi = __ldg(p.rowptr + p.brow_end);
+        // row pointers that would lead past the arrays: an empty product and a status code
+        const bool bad = lo < 0 || hi < lo || hi > p.nnzb || (p.long_rows && __ldg(p.long_rows) > p.n_pieces - n_rows);
+        if (bad && piece == 0 && lane == 0) atomicCAS(p.status, 0, kStatusBadRowptr);
+        q.row = piece;
+        q.b0 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + q.row), lo), hi);
+        q.b1 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + q.row + 1), q.b0), hi);
+        if (q.b1 - q.b0 > p.chunk && p.long_rows) {
+            q.my_slot = q.first_slot = __ldg(p.row_slot + q.row);
+            q.count = (q.b1 - q.b0 + p.chunk - 1) / p.chunk;
+            q.b1 = q.b0 + p.chunk;
+        }
+        return q;
+    }
+    const int listed = __ldg(p.long_rows);
+    q.live = piece - n_rows < listed && listed <= p.n_pieces - n_rows;
+    if (q.live) {
+        const uint4 d = __ldg(p.pieces + (piece - n_rows));
+        q.row = (int)d.x; q.b0 = (int)d.y; q.b1 = (int)d.z; q.my_slot = (int)d.w;
+        const int2 s = __ldg(p.slots + q.my_slot);
+        q.first_slot = s.x; q.count = s.y;
+    }
+    return q;
+}
+
+// What a warp does with its sums (of all warps of the piece): to C, or to scratch and on to C by the last piece of the row.
+template <int T>
+__device__ __forceinline__ void finish_piece(const StreamArgs& p, const Piece& q, float (&acc)[T][4], int tile, int n0, int octets, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    // ---- a piece of a long block-row: partial sums to scratch; the last piece to arrive adds them up in order ----
+    if (q.count > 1) {
+        float4* mine = p.partial + ((size_t)q.my_slot * p.n_tiles + tile) * (T * 32) + lane;
+#pragma unroll
+        for (int j = 0; j < T; j++) __stcg(mine + j * 32, make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]));
+        // lane 0's arrival stands for all 32 lanes: their stores and fences come before it only through a warp barrier (a
+        // shuffle does not order memory), and what it has seen reaches their loads only through another
+        __threadfence();
+        __syncwarp();
+        int old = 0;
+        if (lane == 0) old = atomicAdd(p.counters + (size_t)q.first_slot * p.n_tiles + tile, 1);
+        old = __shfl_sync(0xffffffffu, old, 0);
+        if (old != q.count - 1) return;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) p.counters[(size_t)q.first_slot * p.n_tiles + tile] = 0;  // ready for the next launch
+#pragma unroll
+        for (int j = 0; j < T; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+        for (int i = 0; i < q.count; i++) {
+            const float4* src = p.partial + ((size_t)(q.first_slot + i) * p.n_tiles + tile) * (T * 32) + lane;
+#pragma unroll
+            for (int j = 0; j < T; j++) {
+                const float4 v = __ldcg(src + j * 32);
+                acc[j][0] += v.x; acc[j][1] += v.y; acc[j][2] += v.z; acc[j][3] += v.w;
+            }
+        }
+    }
+
+    // ---- fp16 rows of C: neighbouring threads exchange halves of two octets, so that a quad stores 32 contiguous bytes ----
+    __half* crow = p.C + (size_t)(q.row * 16 + g) * p.ldc + n0;
+    if constexpr (T == 1) {
+        *reinterpret_cast<__half2*>(crow + 2 * t) = __floats2half2_rn(acc[0][0], acc[0][1]);
+        *reinterpret_cast<__half2*>(crow + 8 * p.ldc + 2 * t) = __floats2half2_rn(acc[0][2], acc[0][3]);
+    } else {
+        const bool odd = t & 1;
+#pragma unroll
+        for (int j = 0; j < T; j += 2) {
+            if (j >= octets) break;
+            const __half2 x0 = __floats2half2_rn(acc[j][0], acc[j][1]), y0 = __floats2half2_rn(acc[j][2], acc[j][3]);
+            const __half2 x1 = __floats2half2_rn(acc[j + 1][0], acc[j + 1][1]), y1 = __floats2half2_rn(acc[j + 1][2], acc[j + 1][3]);
+            const __half2 rx = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1), ry = __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 1);
+            const int col = 8 * j + (odd ? 8 + 2 * (t - 1) : 2 * t);
+            if (!odd || j + 1 < octets) {
+                union { __half2 h[2]; uint2 u; } vx, vy;
+                vx.h[0] = odd ? rx : x0; vx.h[1] = odd ? x1 : rx;
+                vy.h[0] = odd ? ry : y0; vy.h[1] = odd ? y1 : ry;
+                *reinterpret_cast<uint2*>(crow + col) = vx.u;
+                *reinterpret_cast<uint2*>(crow + 8 * p.ldc + col) = vy.u;
+            }
+        }
+    }
+}
+
 template <int NT, int W, int kWarps, int U, int MINB, bool SLAB, bool PLAN>
 __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(const StreamArgs p) {
     constexpr int T = NT / 8;                                       // MMAs (8 columns each) per block
@@ -64,44 +186,9 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
     const int piece = (int)(blockIdx.x / (unsigned)p.n_tiles) * (kWarps / W) + warp / W;
     const int n0 = tile * p.tile_cols;
     ptx::pdl_wait();
-    // ---- the piece: blocks [b0, b1) of block-row `row`; count > 1: one of `count` pieces of a long block-row ----
-    int row = 0, b0 = 0, b1 = 0, count = 1, my_slot = 0, first_slot = 0;
-    bool live = piece < p.n_pieces;
-    if (live) {
-        if (PLAN) {
-            const uint4 d = __ldg(p.pieces + piece);
-            row = (int)d.x; b0 = (int)d.y; b1 = (int)d.z;
-            if (d.w) {
-                const int2 s = __ldg(p.slots + (d.w - 1));
-                my_slot = (int)d.w - 1; first_slot = s.x; count = s.y;
-            }
-        } else {
-            const int n_rows = p.brow_end - p.brow_begin;
-            if (piece < n_rows) {
-                const int lo = __ldg(p.rowptr + p.brow_begin), hi = __ldg(p.rowptr + p.brow_end);
-                // row pointers that would lead past the arrays: an empty product and a status code
-                const bool bad = lo < 0 || hi < lo || hi > p.nnzb || (p.long_rows && __ldg(p.long_rows) > p.n_pieces - n_rows);
-                if (bad && piece == 0 && lane == 0) atomicCAS(p.status, 0, kStatusBadRowptr);
-                row = piece;
-                b0 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + row), lo), hi);
-                b1 = bad ? 0 : min(max(__ldg(p.rowptr + p.brow_begin + row + 1), b0), hi);
-                if (b1 - b0 > p.chunk && p.long_rows) {
-                    my_slot = first_slot = __ldg(p.row_slot + row);
-                    count = (b1 - b0 + p.chunk - 1) / p.chunk;
-                    b1 = b0 + p.chunk;
-                }
-            } else {
-                const int listed = __ldg(p.long_rows);
-                live = piece - n_rows < listed && listed <= p.n_pieces - n_rows;
-                if (live) {
-                    const uint4 d = __ldg(p.pieces + (piece - n_rows));
-                    row = (int)d.x; b0 = (int)d.y; b1 = (int)d.z; my_slot = (int)d.w;
-                    const int2 s = __ldg(p.slots + my_slot);
-                    first_slot = s.x; count = s.y;
-                }
-            }
-        }
-    }
+    Piece q = piece_of<PLAN>(p, piece, lane);
+    const bool live = q.live;
+    const int b0 = q.b0, b1 = q.b1;
     if (W == 1 && !live) return;
     // this warp's share of the piece
     int c0 = b0, c1 = b1;
@@ -219,57 +306,134 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
         if (w != 0 || !live) return;
     }
 
-    // ---- a piece of a long block-row: partial sums to scratch; the last piece to arrive adds them up in order ----
-    if (count > 1) {
-        float4* mine = p.partial + ((size_t)my_slot * p.n_tiles + tile) * (T * 32) + lane;
-#pragma unroll
-        for (int j = 0; j < T; j++) __stcg(mine + j * 32, make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]));
-        // lane 0's arrival stands for all 32 lanes: their stores and fences come before it only through a warp barrier (a
-        // shuffle does not order memory), and what it has seen reaches their loads only through another
-        __threadfence();
-        __syncwarp();
-        int old = 0;
-        if (lane == 0) old = atomicAdd(p.counters + (size_t)first_slot * p.n_tiles + tile, 1);
-        old = __shfl_sync(0xffffffffu, old, 0);
-        if (old != count - 1) return;
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) p.counters[(size_t)first_slot * p.n_tiles + tile] = 0;  // ready for the next launch
-#pragma unroll
-        for (int j = 0; j < T; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
-        for (int i = 0; i < count; i++) {
-            const float4* src = p.partial + ((size_t)(first_slot + i) * p.n_tiles + tile) * (T * 32) + lane;
-#pragma unroll
-            for (int j = 0; j < T; j++) {
-                const float4 v = __ldcg(src + j * 32);
-                acc[j][0] += v.x; acc[j][1] += v.y; acc[j][2] += v.z; acc[j][3] += v.w;
-            }
-        }
-    }
+    finish_piece<T>(p, q, acc, tile, n0, octets, lane);
+}
 
-    // ---- fp16 rows of C: neighbouring threads exchange halves of two octets, so that a quad stores 32 contiguous bytes ----
-    __half* crow = p.C + (size_t)(row * 16 + g) * p.ldc + n0;
-    if constexpr (T == 1) {
-        *reinterpret_cast<__half2*>(crow + 2 * t) = __floats2half2_rn(acc[0][0], acc[0][1]);
-        *reinterpret_cast<__half2*>(crow + 8 * p.ldc + 2 * t) = __floats2half2_rn(acc[0][2], acc[0][3]);
-    } else {
-        const bool odd = t & 1;
+// The same product for wide tiles whose B is slabs: a warp's next S slices and blocks are on their way to a ring in shared memory
+// (a bulk copy each) while it multiplies, so that the loads in flight are not bounded by registers: 12 warps of the kernel above
+// (166 registers) have one block of 4.6 KB each on its way.  Power-law matrix of 262144 rows, 128 columns: 826 -> 630 us (58 of
+// the 67-72 bytes per cycle and SM that L2 serves to a pure streaming kernel), 96 columns 731 -> 480, 64 columns 515 -> 403;
+// 65536 rows without a plan, 128 columns: 266 -> 212.  32 columns stay with the kernel above (179 us against 234): a
+// block then costs its two copies, 28 cycles each, more than its bytes.  The blocks of A come as copies too, although a lane
+// could load its 16 bytes itself: a wait for one such load waits for all later ones of the warp as well (1100 cycles a block).
+template <int NT, int S, int W, int kWarps, int MINB, bool PLAN>
+__global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_ring_kernel(const StreamArgs p) {
+    constexpr int T = NT / 8;
+    constexpr uint32_t STAGE = NT * 32 + 512;  // bytes: a slice of NT columns, then the block
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = (int)(blockIdx.x % (unsigned)p.n_tiles);
+    const int piece = (int)(blockIdx.x / (unsigned)p.n_tiles) * (kWarps / W) + warp / W;
+    const int n0 = tile * p.tile_cols;
+    const uint32_t ring = ptx::smem_u32(smem) + warp * (S * STAGE), bars = ptx::smem_u32(smem) + kWarps * (S * STAGE) + warp * (S * 8);
+    if (lane == 0) {
 #pragma unroll
-        for (int j = 0; j < T; j += 2) {
-            if (j >= octets) break;
-            const __half2 x0 = __floats2half2_rn(acc[j][0], acc[j][1]), y0 = __floats2half2_rn(acc[j][2], acc[j][3]);
-            const __half2 x1 = __floats2half2_rn(acc[j + 1][0], acc[j + 1][1]), y1 = __floats2half2_rn(acc[j + 1][2], acc[j + 1][3]);
-            const __half2 rx = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1), ry = __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 1);
-            const int col = 8 * j + (odd ? 8 + 2 * (t - 1) : 2 * t);
-            if (!odd || j + 1 < octets) {
-                union { __half2 h[2]; uint2 u; } vx, vy;
-                vx.h[0] = odd ? rx : x0; vx.h[1] = odd ? x1 : rx;
-                vy.h[0] = odd ? ry : y0; vy.h[1] = odd ? y1 : ry;
-                *reinterpret_cast<uint2*>(crow + col) = vx.u;
-                *reinterpret_cast<uint2*>(crow + 8 * p.ldc + col) = vy.u;
+        for (int s = 0; s < S; s++) ptx::mbar_init(bars + 8 * s, 1);
+        ptx::fence_barrier_init();
+    }
+    __syncwarp();
+    ptx::pdl_wait();
+    const Piece q = piece_of<PLAN>(p, piece, lane);
+    if (W == 1 && !q.live) return;
+    int c0 = q.b0, c1 = q.b1;  // this warp's share of the piece
+    if (W > 1) {
+        const int per = (q.b1 - q.b0 + W - 1) / W, w = warp % W;
+        c0 = min(q.b1, q.b0 + w * per);
+        c1 = min(q.b1, c0 + per);
+        if (!q.live) c0 = c1 = 0;
+    }
+    float acc[T][4];
+#pragma unroll
+    for (int j = 0; j < T; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+    const int octets = min(p.tile_cols, p.N - n0) >> 3, Kb = p.K >> 4;
+    const uint32_t bytes = (uint32_t)octets * 256u;
+    const uint8_t* vals = static_cast<const uint8_t*>(p.vals);
+    const uint8_t* slabs = static_cast<const uint8_t*>(p.B) + (size_t)n0 * 32;
+    const size_t slab = (size_t)p.N * 32;
+    const uint32_t a_lane = ring + NT * 32 + (PLAN ? lane * 16 : lane * 8), b_lane = ring + lane * 8;
+    const uint64_t once = ptx::policy_evict_first();  // a block is read once per column tile: it is not to push slabs out of L2
+    // 32 block-columns at a time, one per lane, and the 32 that follow
+    auto load_cols = [&](int at) {
+        int c = (at + lane < c1) ? __ldg(p.colidx + at + lane) >> (PLAN ? 0 : 4) : 0;
+        if (!PLAN && (c < 0 || c >= Kb)) {
+            atomicCAS(p.status, 0, kStatusBadColumns);
+            c = -1;
+        }
+        return c;
+    };
+    int cols_at = c0, cols = load_cols(c0), cols_next = load_cols(c0 + 32);
+    uint32_t ok = 0, phase = 0;  // bit s: stage s holds a block; parity of its next wait
+    auto fetch = [&](int s, int at) {
+        if (at - cols_at >= 32) {
+            cols_at += 32;
+            cols = cols_next;
+            cols_next = load_cols(cols_at + 32);
+        }
+        const int cb = __shfl_sync(0xffffffffu, cols, at - cols_at);
+        ok &= ~(1u << s);
+        if (at < c1 && cb >= 0) {
+            ok |= 1u << s;
+            if (lane == 0) {
+                ptx::mbar_arrive_expect_tx(bars + 8 * s, bytes + 512u);
+                ptx::bulk_load(ring + s * STAGE, slabs + (size_t)cb * slab, bytes, bars + 8 * s);
+                ptx::bulk_load_hint(ring + s * STAGE + NT * 32, vals + (size_t)at * 512, 512u, bars + 8 * s, once);
             }
         }
+    };
+#pragma unroll
+    for (int s = 0; s < S; s++) fetch(s, c0 + s);
+    bool there = true;
+    for (int at = c0; at < c1 && there; at += S) {
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            if (there && (ok & (1u << s))) {
+                there = ring_wait(bars + 8 * s, (phase >> s) & 1u);
+                phase ^= 1u << s;
+                // all of the stage: what a narrower tile leaves of it goes to columns that are not stored
+                uint4 a;
+                uint2 b[T];
+                if (PLAN) {
+                    a = lds16(a_lane + s * STAGE);
+                } else {
+                    const uint2 lo = lds8(a_lane + s * STAGE), hi = lds8(a_lane + s * STAGE + 256);
+                    a = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                }
+#pragma unroll
+                for (int j = 0; j < T; j++) b[j] = lds8(b_lane + s * STAGE + j * 256);
+#pragma unroll
+                for (int j = 0; j < T; j++) mma_16816(acc[j], a, b[j]);
+            }
+            __syncwarp();  // all lanes have read the stage before it is filled again
+            if (there) fetch(s, at + S + s);
+        }
     }
+    if (!there) {  // a copy did not arrive in time: the host sees a status, copies in flight get time to land
+        if (lane == 0) atomicCAS(p.status, 0, kRingWaitCode);
+        for (int i = 0; i < 64; i++) __nanosleep(1000);
+    }
+    if constexpr (W > 1) {  // sum over the W warps of the piece (fixed order), in the rings
+        const int w = warp % W;
+#pragma unroll
+        for (int half = W / 2; half >= 1; half >>= 1) {
+            float4* red = reinterpret_cast<float4*>(smem + (warp - w + (w < half ? w : w - half)) * (S * STAGE)) + lane;
+            static_assert(T * 32 * 16 <= S * STAGE, "a warp's sums fit its ring");
+            __syncthreads();
+            if (w >= half && w < 2 * half) {
+#pragma unroll
+                for (int j = 0; j < T; j++) red[j * 32] = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+            }
+            __syncthreads();
+            if (w < half) {
+#pragma unroll
+                for (int j = 0; j < T; j++) {
+                    const float4 v = red[j * 32];
+                    acc[j][0] += v.x; acc[j][1] += v.y; acc[j][2] += v.z; acc[j][3] += v.w;
+                }
+            }
+        }
+        if (w != 0 || !q.live) return;
+    }
+    if (there) finish_piece<T>(p, q, acc, tile, n0, octets, lane);
 }
 
 // B ([N][K], k contiguous) -> slabs [K / 16][N][16]: the 16 x N slice of one block-column becomes contiguous.
@@ -388,12 +552,42 @@ cudaError_t launch_one(const StreamArgs& a, cudaStream_t stream) {
     return launch_pdl(spmm_bcsr_stream_kernel<NT, W, Q::WARPS, Q::U, Q::MINB, SLAB, PLAN>, dim3((unsigned)grid), dim3(Q::WARPS * 32), 0, stream, a);
 }
 
+// slabs of more bytes than this are taken not to stay in L2 beside A (126 MB, each half of the SMs by its own half)
+constexpr size_t kSlabBytesL2 = (size_t)62 << 20;
+
+// resident: CTAs per SM where that is fewer than MINB (0: MINB)
+template <int NT, int S, int W, int kWarps, int MINB, bool PLAN>
+cudaError_t launch_ring(const StreamArgs& a, int resident, cudaStream_t stream) {
+    const long long grid = (((long long)a.n_pieces + kWarps / W - 1) / (kWarps / W)) * a.n_tiles;
+    if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    size_t smem = kWarps * S * (NT * 32 + 512 + 8);
+    static_assert((kWarps * S * (NT * 32 + 512 + 8) + 1024) * MINB <= 228 * 1024, "shared memory of the resident CTAs");
+    if (resident && resident < MINB) smem = std::max<size_t>(smem, 228 * 1024 / (resident + 1));  // one more would not fit
+    auto kernel = spmm_bcsr_ring_kernel<NT, S, W, kWarps, MINB, PLAN>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(kernel, dim3((unsigned)grid), dim3(kWarps * 32), smem, stream, a);
+}
+
 template <bool PLAN, bool SLAB, int W>
 cudaError_t launch_nt(int nt, const StreamArgs& a, cudaStream_t stream) {
-    if constexpr (W < 8) {
+    if constexpr (SLAB && W < 8) {
+        constexpr int kWarps = W == 4 ? 4 : 2;
+        // Slices of N columns in flight per SM: 14 warps x 3 of 97 to 128 columns, 16 x 3 of 65 to 96, 20 x 2 of 33 to 64.
+        // Beyond that some 100 copies are on their way, and the kernel falls off: 18 x 3 of 96 columns take 795 us instead of
+        // 480 (power-law matrix of 262144 rows), 16 x 4 of 64 columns 575 (12 x 4) to 1000.  Slabs of more than half of L2
+        // leave it less room for A, and want fewer warps: 262144 rows, 128 columns, 653 us with 14 warps, 624 with 12; 155152
+        // rows 415 and 432.
+        if (nt == 128 && a.tile_cols > 96) return launch_ring<128, 3, W, kWarps, 14 / kWarps, PLAN>(a, (size_t)a.N * a.K * 2 > kSlabBytesL2 ? 12 / kWarps : 0, stream);
+        if (nt == 128) return launch_ring<96, 3, W, kWarps, 16 / kWarps, PLAN>(a, 0, stream);
+        if (nt == 64) return launch_ring<64, 2, W, kWarps, 20 / kWarps, PLAN>(a, 0, stream);
+    }
+    if constexpr (!SLAB && W < 8) {
         if (nt == 128) return launch_one<128, W, SLAB, PLAN>(a, stream);
     }
-    if (nt == 64) return launch_one<64, W, SLAB, PLAN>(a, stream);
+    if constexpr (!SLAB || W == 8) {
+        if (nt == 64) return launch_one<64, W, SLAB, PLAN>(a, stream);
+    }
     if (nt == 32) return launch_one<32, W, SLAB, PLAN>(a, stream);
     if constexpr (!SLAB) {
         if (nt == 16) return launch_one<16, W, SLAB, PLAN>(a, stream);

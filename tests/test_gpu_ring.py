@@ -1,0 +1,75 @@
+"""Wide products of the stream kernels from slabs, whose slices come through a ring in shared memory: block-rows shorter than the
+ring, empty ones, one, two and four warps a block-row, long block-rows in pieces, tiles of every width class and their edges, with a
+plan and without."""
+import numpy as np
+import pytest
+
+import oracle
+import smat_b200 as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(rng, Mb, Kb, most, long_row=None):
+    counts = rng.integers(0, most + 1, Mb)
+    counts[:6] = [0, 1, 2, 3, 4, min(5, Kb)]  # shorter than the ring, as long, one longer
+    if long_row is not None:
+        counts[long_row] = Kb
+    cols = [np.sort(rng.choice(Kb, c, replace=False)) for c in counts]
+    brp = np.zeros(Mb + 1, np.int32)
+    brp[1:] = np.cumsum(counts)
+    return brp, (np.concatenate(cols) * 16).astype(np.int32), (rng.standard_normal(brp[-1] * 256) * 0.25).astype(np.float16)
+
+
+@pytest.mark.parametrize("plan", [True, False])
+@pytest.mark.parametrize("Mb,Kb,most,long_row", [(2400, 300, 40, None), (1100, 260, 60, 7), (300, 700, 300, 11)])
+@pytest.mark.parametrize("N", [40, 64, 72, 96, 104, 128, 136, 200])
+def test_ring_against_oracle(plan, Mb, Kb, most, long_row, N):
+    rng = np.random.default_rng(N + Mb)
+    M, K = Mb * 16, Kb * 16
+    brp, bci, bv = _matrix(rng, Mb, Kb, most, long_row)
+    B = rng.standard_normal((N, K)).astype(np.float16)
+    A = S.SparseMatrix.from_bcsr(M, K, brp, bci, bv)
+    Bd, C = S.Matrix.from_host(B), S.Matrix(M, N, fill=float("nan"))
+    outs = []
+    S.set_variant(5)
+    try:
+        p = S.Plan(A, n_hint=N) if plan else None
+        for _ in range(2):
+            C.data.fill_(float("nan"))
+            p.spmm(Bd, C, check=True) if plan else S.spmm(A, Bd, C, check=True)
+            outs.append(C.data.cpu().numpy().copy())
+        if plan:
+            p.close()
+    finally:
+        S.set_variant(0)
+    assert np.array_equal(outs[0].view(np.uint16), outs[1].view(np.uint16))
+    ref = oracle.bcsr_spmm(bv, brp, bci, B, M, N, K, threads=8)
+    size = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B), M, N, K, threads=8)
+    # exact products, at most K additions in fp32 on either side (2^-24 of the sum of magnitudes each), one rounding to fp16 each
+    bound = 2 * K * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24
+    assert np.all(np.abs(outs[0].astype(np.float32) - ref) <= bound)
+
+
+def test_ring_skips_columns_outside_the_matrix():
+    """A block whose column lies outside the matrix is left out and reported, with the ring as with the other kernels."""
+    rng = np.random.default_rng(3)
+    Mb, Kb, N = 2400, 300, 128
+    M, K = Mb * 16, Kb * 16
+    brp, bci, bv = _matrix(rng, Mb, Kb, 40)
+    B = rng.standard_normal((N, K)).astype(np.float16)
+    row = int(np.argmax(np.diff(brp)))
+    bad, good = bci.copy(), bv.copy()
+    bad[brp[row + 1] - 1] = K
+    good[(brp[row + 1] - 1) * 256: brp[row + 1] * 256] = 0
+    C = S.Matrix(M, N, fill=float("nan"))
+    S.set_variant(5)
+    try:
+        with pytest.raises(S.SmatError):
+            S.spmm(S.SparseMatrix.from_bcsr(M, K, brp, bad, bv), S.Matrix.from_host(B), C, check=True)
+        got = C.data.cpu().numpy().copy()
+        S.spmm(S.SparseMatrix.from_bcsr(M, K, brp, bci, good), S.Matrix.from_host(B), C, check=True)
+    finally:
+        S.set_variant(0)
+    # another order of nothing but a block of zeros: the same sums
+    assert np.array_equal(got.view(np.uint16), C.data.cpu().numpy().view(np.uint16))
