@@ -22,9 +22,9 @@
 //     eight copies of a pair take 64 cycles each, 36 MMAs beside them add 107 cycles and 72 MMAs 383.
 //
 // Pipeline per step (four block-columns of a group), all hand-overs by mbarriers, every wait bounded:
-//   panel loaders (4 warps, one thread each, every 4th step): TMA box {64 k, 128 n} -> panel slot (6 slots);
+//   panel loaders (4 warps, one thread each, every 4th step): TMA box {64 k, 128 n} -> panel slot (6 slots, or 4);
 //   block loader (1 warp, one thread): per pair, one bulk copy of the packed A blocks of its steps, which follow one another in
-//     the plan, to the next free place of a ring of RING_BLOCKS blocks, and one of the pair's MMA lists.  Slots of a fixed
+//     the plan, to the next free place of a ring (Smem), and one of the pair's MMA lists.  Slots of a fixed
 //     size would have to be as large as the largest step, so steps would have to be cut short: with a ring a step holds up to
 //     kTallBlocksPerStep blocks, twice as many as with slots, and its panel is fetched and copied once (random matrix of
 //     65536 rows, 22 blocks a step: 217 000 -> 175 000 steps, 831 -> 744 us; layer 8192 x 28672, N = 4096: 737 -> 704);
@@ -48,6 +48,7 @@
 #include <stdlib.h>
 
 #include <cstdlib>
+#include <type_traits>
 
 #include "ptx_sm100.cuh"
 #include "smat_internal.h"
@@ -63,34 +64,43 @@ constexpr int NLW = 4;           // panel-loader warps
 constexpr int LW = NLW + 1;      // loader warps in all: one more loads the blocks
 constexpr int NCW = 4;           // copier warps
 constexpr int NEW = 8;           // epilogue warps
-constexpr uint32_t PS = 6;                                   // panel slots in shared memory (a slot is free once copied to tensor memory)
 constexpr uint32_t PANEL_BYTES = 128 * 64 * 2;               // 128 n x 64 k fp16
-// The blocks of a pair of steps lie one after the other in a ring (never around its end) until the pair's MMAs have completed.
-constexpr uint32_t RING_BLOCKS = 246;
+constexpr size_t kTallDenseStep = 25;                         // blocks a step, on average: Smem below
 constexpr uint32_t NLIST = 7;                                 // pairs with blocks in the ring, at most: list slots
 constexpr uint32_t META_BYTES = kTallRows / 2 * kTallListBytes;  // per pair of steps: the MMA lists of the 12 issuing warps
-constexpr uint32_t OFF_PANEL = 0;
-constexpr uint32_t OFF_BLK = OFF_PANEL + PS * PANEL_BYTES;
-constexpr uint32_t OFF_META = OFF_BLK + RING_BLOCKS * 512;
 // A thread that waits on an mbarrier by parity must see every phase of it.  Panel loader j and copier j handle the steps
-// st = j (mod 4), so the full_p ring is as long as lcm(PS, 4): barrier st % ring then always belongs to the same loader and the
-// same copier.  The per-pair rings (8 barriers) are visited by a loader or copier at every other pair, i.e. each barrier of
-// its parity class once per 8 pairs: once per phase; the block loader visits them all, in order.
-constexpr uint32_t FP = 12;                                   // full_p ring: lcm(PS, 4)
+// st = j (mod 4), so the full_p ring is a multiple of 4 and of the panel slots: barrier st % ring then always belongs to the same
+// loader and the same copier.  The per-pair rings (8 barriers) are visited by a loader or copier at every other pair, i.e. each
+// barrier of its parity class once per 8 pairs: once per phase; the block loader visits them all, in order.
+constexpr uint32_t FP = 12;                                   // full_p ring
 constexpr uint32_t NPAIR = 8;                                 // full_b / cp_done / step_done rings (pairs of steps)
-constexpr uint32_t OFF_SUBS = OFF_META + NLIST * META_BYTES;  // per step (full_p ring): its non-empty sub-columns, by the panel loader
-constexpr uint32_t OFF_AT = OFF_SUBS + FP * 4;                // per pair (NPAIR ring): place of its blocks, in blocks, by the block loader
-constexpr uint32_t OFF_END = OFF_AT + NPAIR * 4;              // ... and the count of blocks up to its end, for the block loader itself
-constexpr uint32_t OFF_BAR = OFF_END + NPAIR * 4;
 constexpr uint32_t N_BARS = FP + 3 * NPAIR + 2;
-constexpr uint32_t OFF_MISC = OFF_BAR + N_BARS * 8;
-constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;        // slack for the manual 1024-byte alignment
+// Shared memory: PS panel slots (a slot is free once copied to tensor memory), and the ring in which the blocks of a pair of steps
+// lie one after the other (never around its end) until the pair's MMAs have completed.  Six panels and 246 blocks, or, for steps
+// of kTallDenseStep blocks and more, four and 308: from there on the wait for a place in the ring is what bounds the loop (two
+// pairs of 80 blocks fill it).  Layers of 14208 rows, N = 512, cycles a step with 6 and 4 slots: 651 and 733 with 19 blocks a
+// step, 807 and 753 with 29, 1096 and 916 with 37, 1272 and 986 with 48; layer 3056 x 8176 at 35 %, N = 1000: 45.1 -> 40.9 us;
+// layer 8192 x 28672 at 20 %, N = 4096 (19 blocks): 722 and 860 us.  Eight slots and 184 blocks: 740 there, the dense ones half
+// as fast.
+template <uint32_t PS>
+struct Smem {
+    static constexpr uint32_t RING_BLOCKS = PS == 4 ? 308 : 246;
+    static constexpr uint32_t PANEL = 0;
+    static constexpr uint32_t BLK = PANEL + PS * PANEL_BYTES;
+    static constexpr uint32_t META = BLK + RING_BLOCKS * 512;
+    static constexpr uint32_t SUBS = META + NLIST * META_BYTES;  // per step (full_p ring): its non-empty sub-columns, by the panel loader
+    static constexpr uint32_t AT = SUBS + FP * 4;                // per pair (NPAIR ring): place of its blocks, in blocks, by the block loader
+    static constexpr uint32_t END = AT + NPAIR * 4;              // ... and the count of blocks up to its end, for the block loader itself
+    static constexpr uint32_t BAR = END + NPAIR * 4;
+    static constexpr uint32_t MISC = BAR + N_BARS * 8;
+    static constexpr uint32_t BYTES = MISC + 16 + 1024;          // slack for the manual 1024-byte alignment
+    static_assert(BYTES <= 227 * 1024, "shared memory budget");
+    static_assert(FP % PS == 0 && PS % 2 == 0 && BAR % 8 == 0, "the barrier phase arithmetic assumes these");
+    // a pair that does not fit behind the last one leaves less than its own size unused at the end of the ring
+    static_assert(RING_BLOCKS >= 2 * 2 * kTallBlocksPerStep, "any pair must fit an empty ring, wherever the last one ended");
+};
 constexpr uint32_t TMEM_ACC = 0;                             // accumulators: one per block-row, 16 columns each
-static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
-static_assert(NLW == 4 && NCW == 4 && FP % PS == 0 && FP % 4 == 0 && PS % 2 == 0 && NPAIR % 2 == 0 && NLIST < NPAIR && OFF_BAR % 8 == 0,
-              "the barrier phase arithmetic below assumes these");
-// a pair that does not fit behind the last one leaves less than its own size unused at the end of the ring
-static_assert(RING_BLOCKS >= 2 * 2 * kTallBlocksPerStep, "any pair must fit an empty ring, wherever the last one ended");
+static_assert(NLW == 4 && NCW == 4 && FP % 4 == 0 && NPAIR % 2 == 0 && NLIST < NPAIR, "the barrier phase arithmetic assumes these");
 static_assert(kTallRows * 16 * 128 <= kFixSlotFloats, "a partial tile must fit a scratch slot");
 
 // Shape of a work item: TRG block-rows (accumulators), two of them per MMA-issuing warp.  What tensor memory the
@@ -112,7 +122,7 @@ struct TallStep {
     uint4 a;      // {element column, packed position (256-byte units), blocks, non-empty sub-columns}
 };
 
-template <int TRG>
+template <int TRG, uint32_t PS>
 __global__ void __launch_bounds__((Shape<TRG>::kThreads), 1)
 spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* __restrict__ packed,
                       const uint4* __restrict__ steps, const uint4* __restrict__ winfo, const int* __restrict__ gsp,
@@ -121,9 +131,11 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                       int tail_parts, uint32_t panel_bytes, float* __restrict__ fix_scratch, int* status, int pf) {
     constexpr int NMW = Shape<TRG>::NMW;
     constexpr uint32_t TS_ = Shape<TRG>::TS_, TMEM_PANELS = Shape<TRG>::TMEM_PANELS;
+    using L = Smem<PS>;
+    constexpr uint32_t RING_BLOCKS = L::RING_BLOCKS;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t bar0 = base + OFF_BAR;
+    const uint32_t bar0 = base + L::BAR;
     auto full_p = [&](uint32_t s) { return bar0 + 8 * s; };
     auto full_b = [&](uint32_t p) { return bar0 + 8 * (FP + p); };  // blocks and lists of pair p (mod NPAIR) have arrived
     // The MMA warps are handed the steps two at a time (pair p = steps 2p, 2p + 1 of the CTA's sequence, whatever
@@ -132,8 +144,8 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
     auto cp_done = [&](uint32_t p) { return bar0 + 8 * (FP + NPAIR + p); };            // both panels of pair p (mod NPAIR) copied
     auto step_done = [&](uint32_t p) { return bar0 + 8 * (FP + 2 * NPAIR + p); };  // all MMAs of pair p (mod NPAIR) completed
     const uint32_t acc_full = bar0 + 8 * (FP + 3 * NPAIR), acc_empty = acc_full + 8;
-    const uint32_t tmem_slot = base + OFF_MISC;
-    const uint32_t abort_addr = base + OFF_MISC + 4;
+    const uint32_t tmem_slot = base + L::MISC;
+    const uint32_t abort_addr = base + L::MISC + 4;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -240,10 +252,10 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                     const uint32_t ps = r.st % PS, fp = r.st % FP, pi = r.st >> 1;
                     // the panel's slot is free once the copy of the step PS positions back (pair pi - PS / 2) has left it
                     if (r.st >= PS) TWAIT(cp_done((pi - PS / 2) % NPAIR), ((pi - PS / 2) / NPAIR) & 1, 1);
-                    st_shared_u32(base + OFF_SUBS + fp * 4, r.a.w);  // for the copier; ordered before its wait by the arrive below
+                    st_shared_u32(base + L::SUBS + fp * 4, r.a.w);  // for the copier; ordered before its wait by the arrive below
                     if (r.a.z) {
                         mbar_arrive_expect_tx(full_p(fp), panel_bytes);
-                        tma_load_2d(base + OFF_PANEL + ps * PANEL_BYTES, &mapB, (int)r.a.x, r.tile * 128, full_p(fp));
+                        tma_load_2d(base + L::PANEL + ps * PANEL_BYTES, &mapB, (int)r.a.x, r.tile * 128, full_p(fp));
                     } else {
                         mbar_arrive(full_p(fp));  // a step that only pads its group: no panel, the phase completes at once
                     }
@@ -282,14 +294,14 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                         used += n;
                         while (done < pi && (pi - done >= NLIST || used - freed > RING_BLOCKS)) {
                             TWAIT(step_done(done % NPAIR), (done / NPAIR) & 1, 2);
-                            freed = ld_shared_u32(base + OFF_END + (done % NPAIR) * 4);
+                            freed = ld_shared_u32(base + L::END + (done % NPAIR) * 4);
                             done++;
                         }
-                        st_shared_u32(base + OFF_AT + pl * 4, head);
-                        st_shared_u32(base + OFF_END + pl * 4, used);
+                        st_shared_u32(base + L::AT + pl * 4, head);
+                        st_shared_u32(base + L::END + pl * 4, used);
                         mbar_arrive_expect_tx(full_b(pl), n * 512u + META_BYTES);
-                        bulk_load(base + OFF_META + (pi % NLIST) * META_BYTES, winfo + (META_BYTES / 16) * (size_t)(first + i0 + a), META_BYTES, full_b(pl));
-                        if (n) bulk_load(base + OFF_BLK + head * 512u, packed + (size_t)rec[a].at * 256, n * 512u, full_b(pl));
+                        bulk_load(base + L::META + (pi % NLIST) * META_BYTES, winfo + (META_BYTES / 16) * (size_t)(first + i0 + a), META_BYTES, full_b(pl));
+                        if (n) bulk_load(base + L::BLK + head * 512u, packed + (size_t)rec[a].at * 256, n * 512u, full_b(pl));
                         head += n;
                         pi++;
                         gen(i0 + a + U, a);
@@ -318,10 +330,10 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                 // which is free once the MMAs of the step TS_ positions back (pair pi - TS_ / 2) have completed; only
                 // the copies follow that
                 if (!(j & 1u)) TWAIT(full_b(pi % NPAIR), (pi / NPAIR) & 1, 4);  // the copier of a pair's first step looks after its blocks
-                const uint64_t pdesc = smem_desc_k_sw128(base + OFF_PANEL + ps * PANEL_BYTES);
+                const uint64_t pdesc = smem_desc_k_sw128(base + L::PANEL + ps * PANEL_BYTES);
                 const uint32_t tdst = tmem_base + TMEM_PANELS + (st % TS_) * 32;
                 TWAIT(full_p(fp), (st / FP) & 1, 3);
-                const uint32_t subs = uniform(ld_shared_u32(base + OFF_SUBS + fp * 4));  // non-empty sub-columns
+                const uint32_t subs = uniform(ld_shared_u32(base + L::SUBS + fp * 4));  // non-empty sub-columns
                 if (pi >= TS_ / 2) TWAIT(step_done((pi - TS_ / 2) % NPAIR), ((pi - TS_ / 2) / NPAIR) & 1, 5);
 #ifdef SMAT_PROFILE
                 if (pi >= TS_ / 2) prof_c[13] += (unsigned int)clock() - *(volatile unsigned int*)&stamp_mma[(pi - TS_ / 2) % 8];
@@ -357,7 +369,7 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
             const uint32_t m = (uint32_t)__shfl_sync(0xffffffffu, warp - LW - NCW, 0);
             const uint32_t leader = elect_one();
             const uint32_t B_HI = (uint32_t)(smem_desc_k_sw32(0) >> 32);
-            const uint32_t b_lo0 = (uint32_t)smem_desc_k_sw32(base + OFF_BLK);
+            const uint32_t b_lo0 = (uint32_t)smem_desc_k_sw32(base + L::BLK);
             constexpr uint32_t IDESC16 = idesc_f16_f32(128, 16);
             const uint32_t acc_m = tmem_base + TMEM_ACC + 2u * m * 16u;  // this warp's two accumulators
             uint32_t st = 0, it = 0;
@@ -377,9 +389,9 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                     tc_fence_after();
                     // This warp's list for the pair (layout: kTallListBytes in smat_internal.h): which of the groups of 1, 2, 4, 8
                     // and 1 MMAs it has, and their entries.
-                    const uint32_t list = base + OFF_META + (pi % NLIST) * META_BYTES + m * kTallListBytes;
+                    const uint32_t list = base + L::META + (pi % NLIST) * META_BYTES + m * kTallListBytes;
                     const uint4 l = ld_shared_v4(list);
-                    const uint32_t b_lo = b_lo0 + uniform(ld_shared_u32(base + OFF_AT + (pi % NPAIR) * 4)) * 32u;
+                    const uint32_t b_lo = b_lo0 + uniform(ld_shared_u32(base + L::AT + (pi % NPAIR) * 4)) * 32u;
                     const uint32_t w0 = uniform(l.x), w1 = uniform(l.y), w2 = uniform(l.z), w3 = uniform(l.w);
                     const uint32_t tpanel = tmem_base + TMEM_PANELS + (st % TS_) * 32;
                     PROF_MARK(9);
@@ -542,21 +554,27 @@ int launch_spmm_tall(const PlanView& whole, const void* B, void* C, size_t N, cu
     const int n_full = (int)(n_items / (size_t)grid * (size_t)grid);
     int pf = 0;  // L2 prefetch: measured to make no difference here, and it costs copy-engine time
     if (const char* ev = std::getenv("SMAT_L2_PREFETCH")) pf = std::atoi(ev) != 0;  // tuning knob
-    auto launch = [&](auto kernel, int threads) -> int {
-        SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
-        SMAT_CUDA_TRY(launch_pdl_if(spmm_begins_early(n_items, sms), kernel, dim3(grid), dim3(threads), SMEM_BYTES, stream,
+    auto launch = [&](auto kernel, int threads, uint32_t smem_bytes) -> int {
+        SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
+        SMAT_CUDA_TRY(launch_pdl_if(spmm_begins_early(n_items, sms), kernel, dim3(grid), dim3(threads), smem_bytes, stream,
                                  mapB, reinterpret_cast<const uint8_t*>(plan.packed), reinterpret_cast<const uint4*>(plan.steps),
                                  reinterpret_cast<const uint4*>(plan.winfo), plan.gsp, plan.rowptr, reinterpret_cast<__half*>(C), ldc, (int)plan.brow_begin,
                                  (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles, (int)n_items, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, pf));
         return SMAT_OK;
     };
     // the smallest shape that holds the plan's groups: fewer accumulators leave tensor memory for more panel slots
+    auto shape = [&](auto trg) -> int {
+        constexpr int TRG = decltype(trg)::value;
+        if (plan.total_steps && plan.nnzb >= kTallDenseStep * plan.total_steps)
+            return launch(spmm_bcsr_tall_kernel<TRG, 4>, Shape<TRG>::kThreads, Smem<4>::BYTES);
+        return launch(spmm_bcsr_tall_kernel<TRG, 6>, Shape<TRG>::kThreads, Smem<6>::BYTES);
+    };
     if (plan.rg <= 16) {
-        if (int rc = launch(spmm_bcsr_tall_kernel<16>, Shape<16>::kThreads)) return rc;
+        if (int rc = shape(std::integral_constant<int, 16>{})) return rc;
     } else if (plan.rg <= 20) {
-        if (int rc = launch(spmm_bcsr_tall_kernel<20>, Shape<20>::kThreads)) return rc;
+        if (int rc = shape(std::integral_constant<int, 20>{})) return rc;
     } else {
-        if (int rc = launch(spmm_bcsr_tall_kernel<24>, Shape<24>::kThreads)) return rc;
+        if (int rc = shape(std::integral_constant<int, 24>{})) return rc;
     }
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());

@@ -58,3 +58,23 @@ def test_ring_and_lists(rows, fill):
     # magnitudes per addition, each), and both are rounded to fp16 (2^-11 of the value, 2^-25 below the normal range)
     bound = 2 * Kb * 16 * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24
     assert np.all(np.abs(C.astype(np.float32) - ref) <= bound)
+
+
+@pytest.mark.parametrize("rows,fill", [(12, 0.45), (12, 0.6), (16, 0.36), (16, 0.42), (20, 0.28), (20, 0.34), (24, 0.23), (24, 0.28)])
+def test_both_splits_of_shared_memory(rows, fill):
+    """Blocks a step just below and above the line from which panels get fewer slots and the ring more blocks, over many turns of
+    either ring."""
+    rng = np.random.default_rng(int(rows * 1000 + fill * 100))
+    Mb, Kb, N = 2 * rows, 600, 136
+    mask = rng.random((Mb, Kb)) < fill
+    mask[:, 100:140] = rng.random((Mb, 40)) < 0.05
+    brp = np.zeros(Mb + 1, np.int32)
+    brp[1:] = np.cumsum(mask.sum(axis=1))
+    bci = (np.nonzero(mask)[1] * 16).astype(np.int32)
+    bv = (rng.standard_normal(brp[-1] * 256) * 0.25).astype(np.float16)
+    B = rng.standard_normal((N, Kb * 16)).astype(np.float16)
+    C = _product(brp, bci, bv, B, Mb * 16, N, Kb * 16, rows)
+    ref = oracle.bcsr_spmm(bv, brp, bci, B, Mb * 16, N, Kb * 16, threads=8)
+    size = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B), Mb * 16, N, Kb * 16, threads=8)
+    bound = 2 * Kb * 16 * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24  # as above
+    assert np.all(np.abs(C.astype(np.float32) - ref) <= bound)
