@@ -359,10 +359,12 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
         __syncwarp();
     } else if (warp < LW + NCW + NMW) {
         // ------------------------------ MMA warp m: accumulator rows 2m, 2m + 1 ------------------------------
-        // The whole warp runs the loop converged and its MMAs are issued under a predicate of one elected lane.  Every operand of a
-        // tcgen05.mma must be a value the compiler knows to be warp-uniform (the instruction reads uniform registers): measured, the
-        // same loop run by a single lane on values loaded from shared memory is 10 % slower over the whole kernel.
-        // So the list words, read from shared memory, go through a warp reduction before anything is derived from them.
+        // The whole warp runs the loop converged and its MMAs are issued under a predicate of one elected lane: measured, the same
+        // loop run by a single lane is 10 % slower over the whole kernel.  The word that decides on branches goes through a warp
+        // reduction, so that the compiler knows them to be uniform (votes in its place: 5 % slower); the entries are left as they
+        // were read, the same in all lanes, and operands derived from them in ordinary registers (a reduction for each entry: layer
+        // 8192 x 28672 at 20 %, N = 4096, 712 -> 680 us in bursts, 797 -> 770 at the power limit; for each operand: 760).  Lists
+        // without branches, all their MMAs under predicates, are far slower (961): one that is off costs almost as much as one on.
         // In isolation (12 warps, 3 MMAs each a pair) the loop takes 500 cycles a pair; with one switch on the number of MMAs inside
         // a region of the elected lane it took 660: 120 of them the jump, 45 to 90 the region's end.
         {
@@ -390,42 +392,38 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                     // This warp's list for the pair (layout: kTallListBytes in smat_internal.h): which of the groups of 1, 2, 4, 8
                     // and 1 MMAs it has, and their entries.
                     const uint32_t list = base + L::META + (pi % NLIST) * META_BYTES + m * kTallListBytes;
-                    const uint4 l = ld_shared_v4(list);
-                    const uint32_t b_lo = b_lo0 + uniform(ld_shared_u32(base + L::AT + (pi % NPAIR) * 4)) * 32u;
-                    const uint32_t w0 = uniform(l.x), w1 = uniform(l.y), w2 = uniform(l.z), w3 = uniform(l.w);
+                    const uint4 l = ld_shared_v4(list), q = ld_shared_v4(list + 16);
+                    const uint32_t b_lo = b_lo0 + ld_shared_u32(base + L::AT + (pi % NPAIR) * 4) * 32u;
+                    const uint32_t w0 = uniform(l.x);
                     const uint32_t tpanel = tmem_base + TMEM_PANELS + (st % TS_) * 32;
                     PROF_MARK(9);
                     auto mma = [&](uint32_t e) {
                         mma_f16_ts_if(leader, acc_m + (e & 0x1fu), tpanel + ((e >> 8) & 0xffu), b_lo + ((e >> 16) & 0xfffu), B_HI, IDESC16);
                     };
-                    if (w0 & kTallList1) mma(w1);
+                    if (w0 & kTallList1) mma(l.y);
                     if (w0 & kTallList2) {
-                        mma(w2);
-                        mma(w3);
+                        mma(l.z);
+                        mma(l.w);
                     }
                     if (w0 & (kTallList4 | kTallList8 | kTallListLast)) {
                         if (w0 & kTallList4) {
-                            const uint4 q = ld_shared_v4(list + 16);
-                            const uint32_t e0 = uniform(q.x), e1 = uniform(q.y), e2 = uniform(q.z), e3 = uniform(q.w);
-                            mma(e0);
-                            mma(e1);
-                            mma(e2);
-                            mma(e3);
+                            mma(q.x);
+                            mma(q.y);
+                            mma(q.z);
+                            mma(q.w);
                         }
                         if (w0 & kTallList8) {
-                            const uint4 q = ld_shared_v4(list + 32), r = ld_shared_v4(list + 48);
-                            const uint32_t e0 = uniform(q.x), e1 = uniform(q.y), e2 = uniform(q.z), e3 = uniform(q.w);
-                            const uint32_t e4 = uniform(r.x), e5 = uniform(r.y), e6 = uniform(r.z), e7 = uniform(r.w);
-                            mma(e0);
-                            mma(e1);
-                            mma(e2);
-                            mma(e3);
-                            mma(e4);
-                            mma(e5);
-                            mma(e6);
-                            mma(e7);
+                            const uint4 r = ld_shared_v4(list + 32), t = ld_shared_v4(list + 48);
+                            mma(r.x);
+                            mma(r.y);
+                            mma(r.z);
+                            mma(r.w);
+                            mma(t.x);
+                            mma(t.y);
+                            mma(t.z);
+                            mma(t.w);
                         }
-                        if (w0 & kTallListLast) mma(w0);
+                        if (w0 & kTallListLast) mma(l.x);
                     }
                     PROF_MARK(10);
                     if (w0) tc_commit_if(leader, step_done(pi % NPAIR));
