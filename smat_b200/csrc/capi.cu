@@ -162,7 +162,10 @@ static int spmm_transient_plan(const void* vals, const int* rowptr, const int* c
         return rc;
     }
     const size_t rg = choose_rows_per_group(brow_end - brow_begin, N, ctx->sm_count, true, nnzb, K);
-    const PlanSizes sz = plan_sizes(nnzb, brow_begin, brow_end, rg);
+    PlanSizes sz = plan_sizes(nnzb, brow_begin, brow_end, rg);
+    // the kernel gathers the blocks itself, unless a variant is asked for that reads a packed copy of them
+    const bool pack = g_spmm_variant == 2 || g_spmm_variant == 3;
+    if (!pack) sz.packed_bytes = 0;
     v.n_groups = sz.n_groups;
     v.rg = rg;
     if (nnzb == 0) return launch_spmm(v, B, C, N, stream);
@@ -174,12 +177,13 @@ static int spmm_transient_plan(const void* vals, const int* rowptr, const int* c
     v.gsp = reinterpret_cast<int*>(b);
     v.steps = b + sz.gsp_bytes;
     v.blk = reinterpret_cast<int*>(b + sz.gsp_bytes + sz.steps_bytes);
-    v.packed = b + sz.gsp_bytes + sz.steps_bytes + sz.blk_bytes;
+    if (pack) v.packed = b + sz.gsp_bytes + sz.steps_bytes + sz.blk_bytes;
+    else v.vals = vals;
     int rc = plan_count_async(rowptr, colidx, K, nnzb, brow_begin, brow_end, rg, reinterpret_cast<int*>(b), stream);
     if (rc == SMAT_OK)
         rc = plan_fill_async(rowptr, colidx, K, nnzb, brow_begin, brow_end, rg, v.gsp, b + sz.gsp_bytes,
                              reinterpret_cast<int*>(b + sz.gsp_bytes + sz.steps_bytes), stream);
-    if (rc == SMAT_OK)
+    if (rc == SMAT_OK && pack)
         rc = pack_values_async(rowptr, vals, v.blk, b + sz.gsp_bytes + sz.steps_bytes + sz.blk_bytes, brow_begin, brow_end, nnzb, stream);
     if (rc == SMAT_OK) rc = launch_spmm(v, B, C, N, stream);
     const cudaError_t e = cudaFreeAsync(buf, stream);

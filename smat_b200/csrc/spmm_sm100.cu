@@ -124,10 +124,17 @@ struct StepRec {
 // NH = 1: a work item is 128 columns of C wide.  NH = 2: 256 columns -- every A block then feeds two
 //   independent MMAs (one per 128-column half, own accumulator), which doubles the MMA work per stage
 //   hand-over and halves the A traffic per MMA; the 32 accumulators fill tensor memory (one buffer).
-template <bool TS, int NH, int SCHED, int CAP>
+// GATHER: no packed copy of the blocks (a product without a plan): each block comes from where the boundary's array has it, by a
+//   tiled copy of its own whose 32-byte swizzle is what the packed copy holds ready.  `packed` is null then, `blk` the blocks'
+//   indices in walk order.  A copy takes the copy engine some 28 cycles, the MMA of a block 39 and more, so that the copies hide
+//   behind the MMAs, as often as tiles of C repeat them, and the packing (37 of 141 us for 121 MB of blocks) goes.  Products
+//   without a plan, packed and gathered: random matrix of 16384 rows, 237 000 blocks, N = 256: 141 and 107 us; 65536 rows, 3.8
+//   million blocks, N = 128: 1436 and 727, N = 1024: 5105 and 4508; dense clusters of 65536 rows, N = 128: 43 and 32, N = 1024:
+//   105 and 104; band of 32768 rows, half bandwidth 256, N = 256: 50 and 38; dense 2048 x 8192, N = 128: 68 and 59.
+template <bool TS, int NH, int SCHED, int CAP, bool GATHER = false>
 __global__ void __launch_bounds__(kThreads, 1)
-spmm_bcsr_tc_kernel(const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapC,
-                    const uint8_t* __restrict__ packed,
+spmm_bcsr_tc_kernel(const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapC, const __grid_constant__ CUtensorMap mapA,
+                    const uint8_t* __restrict__ packed, const int* __restrict__ blk,
                     const uint4* __restrict__ steps, const int* __restrict__ gsp,
                     const int* __restrict__ rowptr, __half* __restrict__ C, int brow_begin, int brow_end, int rg, int N,
                     int n_tiles, int n_items, int n_groups, int tail_parts, uint32_t panel_bytes,
@@ -324,8 +331,59 @@ spmm_bcsr_tc_kernel(const __grid_constant__ CUtensorMap mapB, const __grid_const
         const int j = warp;
         // Software pipeline over the warp's steps, unrolled U times so that every record lives in fixed
         // registers (a record whose descriptor load is still in flight is never copied): the descriptor
-        // of position i + U is requested while position i is consumed.  One thread per warp works.
-        if (lane == 0) {
+        // of position i + U is requested while position i is consumed.  One thread per warp works; gathered blocks take a lane each.
+        if constexpr (GATHER) {
+            SegGen<SCHED> sg = make_gen();
+            Seg cs;
+            bool have = sg.next(cs);
+            uint32_t h_st0 = 0, h_next = (uint32_t)j;
+            constexpr int U = 8;
+            StepRec rec[U];
+            int block[U];  // this lane's block of the step
+            const int* const from = blk + __ldg(rowptr + brow_begin);
+            auto gen = [&](StepRec& r) {
+                while (have && h_next >= h_st0 + (uint32_t)(cs.k1 - cs.k0)) {
+                    h_st0 += (uint32_t)(cs.k1 - cs.k0);
+                    have = sg.next(cs);
+                }
+                r.live = have;
+                if (have) {
+                    r.tile = cs.item % n_tiles;
+                    r.st = h_next;
+                    r.d = __ldg(steps + cs.gs + cs.k0 + (int)(h_next - h_st0));
+                    h_next += NL;
+                }
+            };
+            auto blocks = [](const StepRec& r) { return __popc(r.d.z) + __popc(r.d.w); };
+            auto find = [&](const StepRec& r, int& b) { if (r.live && lane < blocks(r)) b = __ldg(from + (r.d.y >> 1) + lane); };
+#pragma unroll
+            for (int a = 0; a < U; a++) gen(rec[a]);
+#pragma unroll
+            for (int a = 0; a < U / 2; a++) find(rec[a], block[a]);
+            bool more = true;
+            while (more) {
+#pragma unroll
+                for (int a = 0; a < U; a++) {
+                    StepRec& r = rec[a];
+                    if (!r.live) { more = false; break; }
+                    find(rec[(a + U / 2) % U], block[(a + U / 2) % U]);
+                    const uint32_t slot = r.st % S;
+                    wait_bar(empty(slot), ((r.st / S) & 1) ^ 1, abort_addr, status, 1);
+                    const uint32_t stage = base + OFF_STAGE + slot * STAGE_BYTES;
+                    const int n = blocks(r);
+                    if (lane == 0) {
+                        st_shared_u32(base + OFF_META + slot * 8, r.d.z);
+                        st_shared_u32(base + OFF_META + slot * 8 + 4, r.d.w);
+                        mbar_arrive_expect_tx(full(slot), panel_bytes + (uint32_t)n * ABLK_BYTES);
+                        tma_load_2d(stage, &mapB, (int)r.d.x, r.tile * NT, full(slot));
+                    }
+                    __syncwarp();
+                    // (an index out of range, which only arrays that were found inconsistent lead to, reads zeros)
+                    if (lane < n) tma_load_2d(stage + PANEL_BYTES + (uint32_t)lane * ABLK_BYTES, &mapA, 0, block[a] * 16, full(slot));
+                    gen(r);
+                }
+            }
+        } else if (lane == 0) {
             SegGen<SCHED> sg = make_gen();
             Seg cs;
             bool have = sg.next(cs);
@@ -709,10 +767,19 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
             kWideItemCost * rounds(plan.n_groups * ((N + 255) / 256), true) < rounds(plan.n_groups * ((N + 127) / 128), false))
             variant = 3;
     }
+    const bool gather = plan.packed == nullptr;  // a product without a plan: the blocks as the boundary has them
+    if (gather) {
+        variant = 1;
+        if (balanced || listed || plan.cap != (size_t)kPlanBlocksPerStep || !plan.vals || !plan.blk)
+            return fail(SMAT_ERR_BAD_ARG, "plan without a copy of the blocks: no kernel for it");
+    }
     const size_t NTI = variant == 3 ? 256 : 128;
     const uint32_t panel_rows = (uint32_t)(N < NTI ? N : NTI);
     CUtensorMap mapB;
     if (int rc = encode_tensor_map_2d_f16(&mapB, B, plan.K, N, plan.K * 2, 64, panel_rows, 128, 0)) return rc;
+    CUtensorMap mapA = {};
+    if (gather)
+        if (int rc = encode_tensor_map_2d_f16(&mapA, plan.vals, 16, whole.nnzb * 16, 32, 16, 16, 32, 0)) return rc;
     CUtensorMap mapC;  // C as the epilogue stores it: boxes of 16 rows x 128 columns (N columns when C is narrower)
     if (int rc = encode_tensor_map_2d_f16(&mapC, C, N, nb_rows * 16, ldc * 2, (uint32_t)(N < 128 ? N : 128), 16, 0, 0)) return rc;
     const int n_tiles = (int)((N + NTI - 1) / NTI);
@@ -739,7 +806,7 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
     auto launch = [&](auto kernel, uint32_t smem_bytes) -> int {
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
         SMAT_CUDA_TRY(launch_pdl_if(spmm_begins_early(n_items, sms), kernel, dim3(grid), dim3(kThreads), smem_bytes, stream,
-                                 mapB, mapC, reinterpret_cast<const uint8_t*>(plan.packed), reinterpret_cast<const uint4*>(plan.steps), plan.gsp,
+                                 mapB, mapC, mapA, reinterpret_cast<const uint8_t*>(plan.packed), plan.blk, reinterpret_cast<const uint4*>(plan.steps), plan.gsp,
                                  plan.rowptr, reinterpret_cast<__half*>(C), (int)plan.brow_begin, (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles,
                                  (int)n_items, (int)plan.n_groups, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, ldc,
                                  listed ? plan.sched_off : nullptr, listed ? plan.sched_list : nullptr, nm, pf));
@@ -760,7 +827,8 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
     if (plan.cap != (size_t)kPlanBlocksPerStep && plan.cap != (size_t)kPlanBlocksPerStepDense)
         return fail(SMAT_ERR_BAD_ARG, "plan with %zu blocks per step: no kernel for it", plan.cap);
     int rc;
-    if (listed) rc = launch_cap(std::integral_constant<int, 1>{});
+    if (gather) rc = launch(spmm_bcsr_tc_kernel<false, 1, 0, kPlanBlocksPerStep, true>, Cfg<1, kPlanBlocksPerStep>::SMEM_BYTES);
+    else if (listed) rc = launch_cap(std::integral_constant<int, 1>{});
     else if (balanced) rc = launch_cap(std::integral_constant<int, 2>{});
     else rc = launch_cap(std::integral_constant<int, 0>{});
     if (rc != SMAT_OK) return rc;
