@@ -515,10 +515,14 @@ PlanSizes plan_sizes(size_t nnzb, size_t brow_begin, size_t brow_end, size_t rg,
 double tc_estimate_us(const PlanView& v, size_t N, size_t sms) {
     const size_t items = v.n_groups * ((N + 127) / 128);
     const double per_group = (double)v.total_steps / (double)v.n_groups;
+    // the heaviest item is cut into as many segments as the others, or not at all
+    const double longest = v.heaviest_cycles / (items < sms ? (double)tail_parts_for(items, sms, true, (size_t)per_group) : 1.0);
     double cycles;
-    if (v.tall) cycles = tall_rounds(items, sms, per_group) * per_group * v.step_cycles + kTallExtraCycles;
-    else if (v.balanced || v.sched_list) cycles = (double)items / (double)sms * per_group * v.step_cycles;
-    else cycles = rounds_for(items, sms, true, (size_t)per_group, false) * per_group * v.step_cycles;
+    if (v.tall)
+        cycles = std::max(tall_rounds(items, sms, per_group) * per_group * std::max(v.step_cycles, kTallLeastCycles), longest) + kTallExtraCycles;
+    // (graphs, whose steps differ as much as their groups: measured 1.5 to 1.6 times the even share of the steps)
+    else if (v.balanced || v.sched_list) cycles = 1.55 * (double)items / (double)sms * per_group * v.step_cycles;
+    else cycles = std::max(rounds_for(items, sms, true, (size_t)per_group, false) * per_group * v.step_cycles, longest);
     return 8.0 + cycles / 1850.0;
 }
 
@@ -977,6 +981,8 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
     v.vertical = vertical;
     v.tall = tall;
     v.step_cycles = tall ? tall_step_cycles((double)range_blocks / (double)(steps_final > 0 ? steps_final : 1)) : step16;
+    // (a tall group of many more steps than quads holds full steps)
+    v.heaviest_cycles = total_and_max[1] * (tall && (double)total_and_max[1] > 1.2 * std::ceil((double)K / 64.0) ? tall_step_cycles(40.0) : v.step_cycles);
     // Stream plan (spmm_stream_sm100.cu): taken where its estimate is below that of the kernel chosen so far.  That one is kept
     // beside it where it is faster for wide products: each pass over the matrix with the stream kernel multiplies 128 columns
     // or as many as the hint names, so a plan made for 16 columns would take 32 passes for 4096.

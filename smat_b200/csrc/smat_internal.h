@@ -112,9 +112,11 @@ inline double tall_rounds(size_t items, size_t sms, double est_steps) {
     const size_t P = tail_parts_for(items, sms, true, (size_t)est_steps);
     return (double)(items / sms) + 1.0 / (double)P + (P > 1 ? 12.0 / est_steps : 0.0);
 }
-// Cycles of a step of the tall kernel that holds `blocks` blocks (measured on layers: 374 with 9 blocks a step, 482 with 12.5, 513
-// with 15.5, 569 with 18.6, about 800 with 31).
+// Cycles of a step of the tall kernel that holds `blocks` blocks, for the choice of heights (measured on layers of 256 steps an
+// item: 630 with 19 blocks a step, 750 with 29, 790 with 36, 1000 with 48; of many items an SM 510 with 10, 560 with 19).
 inline double tall_step_cycles(double blocks) { return 300.0 + 15.0 * blocks > 400.0 ? 300.0 + 15.0 * blocks : 400.0; }
+// ... and at least, against other kernels (steps of a few blocks take 510 to 590, estimates of the others are as low).
+constexpr double kTallLeastCycles = 440.0;
 // ... and what a launch of it costs beyond its steps: its pipeline takes longer to fill and to drain (measured, smallest plans).
 constexpr double kTallExtraCycles = 5000.0;
 // Measured cost of a 256-column item relative to a 128-column item of the same group.
@@ -176,6 +178,7 @@ struct PlanView {
     size_t total_steps = 0;  // number of steps of the range when the host knows it, else 0
     size_t cap = kPlanBlocksPerStep;  // most blocks of a step: kPlanBlocksPerStep or kPlanBlocksPerStepDense
     double step_cycles = 0.0;  // what a step is estimated to take (tc_estimate_us)
+    double heaviest_cycles = 0.0;  // ... and the heaviest group for one tile of C, in one piece
     bool vertical = false;  // most blocks have a neighbour above or below in their block-column (dense clusters)
     // Tall plan: groups of rg <= kTallRows block-rows with an even number of steps, at most kTallBlocksPerStep blocks
     // per step.  A step record is {element column of the quad, position of the first block in the packed stream in

@@ -654,14 +654,14 @@ StreamShape stream_shape(size_t N, size_t rows, size_t nnzb, size_t K, int sm_co
 }
 
 // Microseconds a product takes with this kernel (one B200), within some 20 %: a launch, the slabs, and per block and SM the
-// streaming of A (10 ns) and the fetch of the slice of B (fitted to 110 random layers, band, uniform, clustered and
-// power-law matrices with 8 to 496 columns).  Without a plan the values come in halves of eight bytes per lane and the
-// pieces less evenly: half again as much per column.
+// streaming of A (10 ns) and the fetch of the slice of B.  From slabs, fitted to 150 random, power-law, layer, band and clustered
+// matrices of 6 000 to 3.8 million blocks, with 40 to 256 columns: 0.46 ns a column, and no less than 40 ns beyond 32 columns;
+// without a plan 0.33 ns a column and 12 ns for every tile, no less than 34 ns.
 double stream_estimate_us(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count, bool plan) {
     const StreamShape s = stream_shape(N, rows, nnzb, K, sm_count, plan);
-    const double n = (double)N, slice = plan ? 0.46 : 0.75;
-    double per_block = s.slab ? std::max(N <= 32 ? 26.0 : 40.0, slice * n) : 10.0 + 0.6 * n;
-    const double warps = (double)rows * std::ceil(n / s.nt) * s.w, full = (double)sm_count * (s.nt == 128 ? 12 : s.nt == 64 ? 16 : 32);
+    const double n = (double)N, tiles = std::ceil(n / s.nt);
+    double per_block = s.slab ? std::max(N <= 32 ? 22.0 : plan ? 40.0 : 34.0, plan ? 0.46 * n : 12.0 * tiles + 0.33 * n) : 10.0 + 0.6 * n;
+    const double warps = (double)rows * tiles * s.w, full = (double)sm_count * (s.nt == 128 ? 12 : s.nt == 64 ? 16 : 32);
     if (s.slab && warps < full) per_block *= full / warps;  // block-rows too few and too short to fill the SMs' load queues
     return 4.0 + (s.slab ? 2.0 + 4e-6 * n * (double)K / 5.5 : 0.0) + (double)nnzb / sm_count * per_block * 1e-3 + (double)(rows * 16) * n * 2.0 / 6e6;
 }
@@ -673,25 +673,24 @@ double stream_passes_us(size_t N, size_t N_hint, size_t rows, size_t nnzb, size_
 }
 
 // A product without a plan takes this kernel unless building a plan inside the call and a tcgen05 kernel are estimated to be
-// faster: 24 us for the launches and small plan kernels, 0.2 ns per block for reading and writing it, and the product --
-// rounds of items at 0.26 us a step, or 20 ns per block, tile and SM, whichever is more.
+// faster: 12 us for the launches and small plan kernels, 0.02 ns per block for the walk order, and the product -- rounds of
+// items at 0.26 us a step, or 20 ns per block, tile and SM, whichever is more.
 bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count) {
     if (g_spmm_variant) return g_spmm_variant == 5;
     const size_t rg = choose_rows_per_group(rows, N, sm_count, true, nnzb, K), groups = (rows + rg - 1) / rg, tiles = (N + 127) / 128;
-    const double throughput = (double)nnzb * (double)tiles / sm_count * 20e-3, build = 24.0 + 0.2e-3 * (double)nnzb;
+    const double throughput = (double)nnzb * (double)tiles / sm_count * 20e-3, build = 12.0 + 0.02e-3 * (double)nnzb;
     const double stream = stream_estimate_us(N, rows, nnzb, K, sm_count, false);
-    if ((double)nnzb < 0.08 * (double)rows * (double)(K / 16)) {
+    if ((double)nnzb < 0.12 * (double)rows * (double)(K / 16)) {
         // Few of the possible blocks: how they lie is not known here, and no rule on these four sizes suits all.  Clustered
-        // blocks suit the other kernel: dense clusters of 65536 rows, N = 512, 71 us against 165 with this one.  Scattered
-        // ones suit this one: random matrix of 65536 rows, 123 blocks a block-row, N = 128, 251 against 474; skewed ones
-        // more (power-law graph of 65536 rows: 235 against 970), since it cuts long block-rows.  So short block-rows are
-        // taken to be clustered, and for long ones this kernel may cost twice the estimate of the other's throughput.
-        // Of 489 products (random, power-law, block-sparse layer, clusters, bands; 16 to 768 columns) the rule takes the slower
-        // kernel for random matrices where both are close (105 us against 84 at worst) and leaves them the other kernel where
-        // N > 200 (2.4 times the time at worst); what pays for it are bands of more than 24 blocks a block-row at 72 to 264
-        // columns (half bandwidth 200: 65 us against 42; 600: 190 against 101).  Counting the other kernel's rounds of
-        // steps, as below, is right for scattered blocks and takes those bands beyond 264 columns as well (120 -> 240 us).
-        return stream < (nnzb > 24 * rows ? 2.0 : 1.0) * (build + throughput);
+        // blocks and bands suit the other kernel, whose steps they fill, scattered ones this one, and skewed ones more, since
+        // it cuts long block-rows.  What sizes tell is the number of blocks of a block-row: bands and clusters have some tens,
+        // random matrices and graphs of this fill a hundred and more.  So up to 48 the other kernel is taken at the estimate of
+        // its throughput (and this one for what is close), beyond that at three times it.
+        // Both kernels timed on 216 products (40 to 400 columns), time of the chosen one to the faster one, geometric mean and
+        // worst, with this rule and before it (which drew the line at 24 and twice the throughput, with estimates from
+        // before slices came through a ring and blocks were gathered): random 1.00, 1.06 and 1.03, 1.82; power-law 1.00, 1.00
+        // and 1.45, 3.43; layers 1.01, 1.09 and 1.02, 1.18; bands 1.02, 1.21 and 1.13, 2.41; clusters 1.01, 1.14 and 1.03, 1.20.
+        return stream < (nnzb > 48 * rows ? 3.0 : 1.15) * (build + throughput);
     }
     const double quads = std::ceil((double)K / 64.0), steps = quads * (1.0 - std::exp(-(double)nnzb / (double)groups / quads));
     return stream < build + std::max(throughput, rounds_for(groups * tiles, (size_t)sm_count, true, (size_t)steps, false) * steps * 0.26);
