@@ -179,10 +179,11 @@ static int spmm_transient_plan(const void* vals, const int* rowptr, const int* c
     v.blk = reinterpret_cast<int*>(b + sz.gsp_bytes + sz.steps_bytes);
     if (pack) v.packed = b + sz.gsp_bytes + sz.steps_bytes + sz.blk_bytes;
     else v.vals = vals;
-    int rc = plan_count_async(rowptr, colidx, K, nnzb, brow_begin, brow_end, rg, reinterpret_cast<int*>(b), stream);
-    if (rc == SMAT_OK)
-        rc = plan_fill_async(rowptr, colidx, K, nnzb, brow_begin, brow_end, rg, v.gsp, b + sz.gsp_bytes,
-                             reinterpret_cast<int*>(b + sz.gsp_bytes + sz.steps_bytes), stream);
+    int* const gsp = reinterpret_cast<int*>(b);
+    int* const blk = reinterpret_cast<int*>(b + sz.gsp_bytes + sz.steps_bytes);
+    int rc = pack ? plan_count_async(rowptr, colidx, K, nnzb, brow_begin, brow_end, rg, gsp, stream)
+                  : plan_fill_loose_async(rowptr, colidx, K, nnzb, brow_begin, brow_end, rg, gsp, b + sz.gsp_bytes, blk, stream);
+    if (rc == SMAT_OK && pack) rc = plan_fill_async(rowptr, colidx, K, nnzb, brow_begin, brow_end, rg, gsp, b + sz.gsp_bytes, blk, stream);
     if (rc == SMAT_OK && pack)
         rc = pack_values_async(rowptr, vals, v.blk, b + sz.gsp_bytes + sz.steps_bytes + sz.blk_bytes, brow_begin, brow_end, nnzb, stream);
     if (rc == SMAT_OK) rc = launch_spmm(v, B, C, N, stream);

@@ -109,7 +109,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* total, int* sh) 
 template <bool FILL, int WIN>
 __global__ void __launch_bounds__(kPlanThreads)
 plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int brow_begin, int brow_end, int rg, int CAP, int Kb,
-            int n_groups, int* __restrict__ gsp, uint4* __restrict__ steps, int* __restrict__ blk, int nnzb, int* status, int* units) {
+            int n_groups, int* __restrict__ gsp, uint4* __restrict__ steps, int* __restrict__ blk, int nnzb, int* status, int* units, bool loose) {
     ptx::pdl_wait();
     extern __shared__ uint32_t sm[];
     uint32_t* masks = sm;                                 // [WIN] row mask per block-column
@@ -119,7 +119,7 @@ plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int 
     // The buffers of the plan are sized from the caller's block count: a range of row pointers that is not monotone or
     // holds more blocks than that would be written past their end.  Such a range gets an empty plan and a status code.
     if (range_is_bad(rowptr, brow_begin, brow_end, nnzb)) {
-        if (!FILL) {
+        if (!FILL || loose) {
             for (int g = blockIdx.x * blockDim.x + threadIdx.x; g <= n_groups; g += gridDim.x * blockDim.x) gsp[g] = 0;
             if (blockIdx.x == 0 && threadIdx.x == 0 && status) atomicCAS(status, 0, kStatusBadRowptr);
         }
@@ -135,7 +135,9 @@ plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int 
         const int rfirst = __ldg(rowptr + brow_begin);           // first block of the whole range
         int cur = beg;
         int steps_done = 0, blocks_done = 0;
-        const int gs = FILL ? __ldg(gsp + g) : 0;
+        // loose: nothing was counted, the group's steps (at most one a block) begin where its blocks do
+        const int gs = FILL ? (loose ? gfirst - rfirst : __ldg(gsp + g)) : 0;
+        const int room = FILL && loose ? min(max(__ldg(rowptr + min(brow_end, brow_begin + (g + 1) * rg)), r_lo), r_hi) - gfirst : INT_MAX;
         for (int w0 = 0; w0 < Kb; w0 += WIN) {
             const int cur_before = cur;
             mark_window<kPlanThreads, WIN>(colidx, cur, end, w0, Kb, masks, warp, lane, status);
@@ -161,6 +163,10 @@ plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int 
             const int pre_s = block_exclusive_scan(ns, &tot_s, scan_sh);
             if (FILL) {
                 const int pre_b = block_exclusive_scan(nb, &tot_b, scan_sh);
+                if (blocks_done + tot_b > room) {  // row pointers that go down inside the range: more blocks than the group has room for
+                    if (threadIdx.x == 0 && status) atomicCAS(status, 0, kStatusBadRowptr);
+                    break;
+                }
                 int s = steps_done + pre_s, b = blocks_done + pre_b;
                 for (int qd = 0; qd < PER / 4; qd++) {
                     unsigned long long m64 = 0;
@@ -199,6 +205,10 @@ plan_kernel(const int* __restrict__ rowptr, const int* __restrict__ colidx, int 
             __syncthreads();
         }
         if (!FILL && threadIdx.x == 0) gsp[g + 1] = steps_done;
+        if (FILL && loose) {
+            if (threadIdx.x == 0) gsp[g] = steps_done;
+            __syncthreads();  // (after a break: all have left the scans)
+        }
     }
     if (!FILL && blockIdx.x == 0 && threadIdx.x == 0) gsp[0] = 0;
 }
@@ -564,7 +574,7 @@ int plan_count_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         SMAT_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(kPlanThreads), smem, stream,
                                  rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap, (int)(K / 16),
-                                 (int)n_groups, gsp, nullptr, nullptr, (int)nnzb, ctx->d_status, units));
+                                 (int)n_groups, gsp, nullptr, nullptr, (int)nnzb, ctx->d_status, units, false));
         return SMAT_OK;
     });
     if (rc) return rc;
@@ -576,8 +586,8 @@ int plan_count_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb
     return SMAT_OK;
 }
 
-int plan_fill_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
-                    size_t rg, const int* gsp, void* steps, int* blk, cudaStream_t stream, const DeviceCtx* ctx_in, size_t cap) {
+static int plan_fill(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end, size_t rg, int* gsp,
+                     void* steps, int* blk, cudaStream_t stream, const DeviceCtx* ctx_in, size_t cap, bool loose) {
     const DeviceCtx* ctx = nullptr;
     if (int rc = plan_launch_setup(ctx_in, &ctx)) return rc;
     const size_t n_groups = (brow_end - brow_begin + rg - 1) / rg;
@@ -587,14 +597,22 @@ int plan_fill_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb,
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         SMAT_CUDA_TRY(launch_pdl(kernel, dim3(grid), dim3(kPlanThreads), smem, stream,
                                  rowptr, colidx, (int)brow_begin, (int)brow_end, (int)rg, (int)cap, (int)(K / 16),
-                                 (int)n_groups, const_cast<int*>(gsp), reinterpret_cast<uint4*>(steps), blk, (int)nnzb,
-                                 ctx->d_status, nullptr));
+                                 (int)n_groups, gsp, reinterpret_cast<uint4*>(steps), blk, (int)nnzb,
+                                 ctx->d_status, nullptr, loose));
         return SMAT_OK;
     });
     if (rc) return rc;
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;
+}
+int plan_fill_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
+                    size_t rg, const int* gsp, void* steps, int* blk, cudaStream_t stream, const DeviceCtx* ctx, size_t cap) {
+    return plan_fill(rowptr, colidx, K, nnzb, brow_begin, brow_end, rg, const_cast<int*>(gsp), steps, blk, stream, ctx, cap, false);
+}
+int plan_fill_loose_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
+                          size_t rg, int* gsp, void* steps, int* blk, cudaStream_t stream, const DeviceCtx* ctx) {
+    return plan_fill(rowptr, colidx, K, nnzb, brow_begin, brow_end, rg, gsp, steps, blk, stream, ctx, kPlanBlocksPerStep, true);
 }
 
 

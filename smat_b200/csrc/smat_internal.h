@@ -172,7 +172,7 @@ struct PlanView {
     const void* steps = nullptr;
     const int* blk = nullptr;
     const void* packed = nullptr;
-    const void* vals = nullptr;  // packed null: the boundary's array of all nnzb blocks, which the kernel reads block by block
+    const void* vals = nullptr;  // packed null: the boundary's array of all nnzb blocks, read block by block; plan_fill_loose_async
     // nnzb: blocks of block-rows [brow_begin, brow_end) when known (plans), else of the whole arrays; steers heuristics only
     size_t K = 0, nnzb = 0, brow_begin = 0, brow_end = 0, n_groups = 0, rg = kPlanRowsPerGroup;
     size_t total_steps = 0;  // number of steps of the range when the host knows it, else 0
@@ -214,6 +214,10 @@ int plan_count_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb
 int plan_fill_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
                     size_t rg, const int* gsp, void* steps, int* blk, cudaStream_t stream, const DeviceCtx* ctx = nullptr,
                     size_t cap = kPlanBlocksPerStep);
+// Both phases in one, for a product without a plan: gsp[g] becomes the number of steps of group g, which begin in `steps` where the
+// group's blocks do, counted from the range's first.
+int plan_fill_loose_async(const int* rowptr, const int* colidx, size_t K, size_t nnzb, size_t brow_begin, size_t brow_end,
+                          size_t rg, int* gsp, void* steps, int* blk, cudaStream_t stream, const DeviceCtx* ctx = nullptr);
 // Copies the value blocks of block-rows [brow_begin, brow_end) into their places in the packed stream.
 int pack_values_async(const int* rowptr, const void* vals, const int* blk, void* packed, size_t brow_begin, size_t brow_end, size_t nnzb,
                       cudaStream_t stream, const DeviceCtx* ctx = nullptr);

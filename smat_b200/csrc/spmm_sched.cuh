@@ -95,7 +95,9 @@ struct Flat {
 //    length of the items; an item that a range boundary falls into is computed in segments.
 // A cut item is assembled from fp32 partial tiles: each CTA stores its segment's result to a scratch tile (one
 // per CTA, two in the balanced schedule: the head and the tail of its range) and a small second kernel adds them.
-// SCHED: 0 = round-robin with a cut last round, 1 = listed, 2 = balanced ranges.
+// SCHED: 0 = round-robin with a cut last round, 1 = listed, 2 = balanced ranges, 3 = 0 for steps that were written without
+// having been counted first (plan_kernel, `loose`): gsp holds the number of steps of every group, and they begin where the
+// group's blocks do, counted from the range's first.
 template <int SCHED>
 struct SegGen {
     const int* gsp;
@@ -105,6 +107,18 @@ struct SegGen {
     Flat flat;
     long long p, p_begin, p_end;
     int g;
+    const int* rowptr = nullptr;  // schedule 3
+    int brow_begin = 0, brow_end = 0, rg = 0;
+    __device__ __forceinline__ void steps_of(int gg, int& gs, int& ns) const {
+        if (SCHED == 3) {
+            const int lo = __ldg(rowptr + brow_begin), hi = __ldg(rowptr + brow_end);
+            gs = min(max(__ldg(rowptr + brow_begin + gg * rg), lo), hi) - lo;
+            ns = __ldg(gsp + gg);
+        } else {
+            gs = __ldg(gsp + gg);
+            ns = __ldg(gsp + gg + 1) - gs;
+        }
+    }
     const int* list;      // listed schedule: the groups of this CTA, else null
     int li, li_end, lt;   // position in the list, its end, next tile of the current group
     __device__ __forceinline__ bool next(Seg& s) {
@@ -133,8 +147,8 @@ struct SegGen {
             return true;
         }
         if (item < n_full) {
-            const int gg = item / n_tiles;
-            const int gs = __ldg(gsp + gg), ns = __ldg(gsp + gg + 1) - gs;
+            int gs, ns;
+            steps_of(item / n_tiles, gs, ns);
             s.item = item; s.k0 = 0; s.k1 = ns; s.ns = ns; s.gs = gs; s.cut = false; s.slot = 0;
             item += n_ctas;
             return true;
@@ -143,8 +157,8 @@ struct SegGen {
         tail_done = true;
         if (cta >= (n_items - n_full) * P) return false;
         const int i = cta / P, j = cta - i * P;
-        const int gg = (n_full + i) / n_tiles;
-        const int gs = __ldg(gsp + gg), ns = __ldg(gsp + gg + 1) - gs;
+        int gs, ns;
+        steps_of((n_full + i) / n_tiles, gs, ns);
         s.item = n_full + i; s.gs = gs; s.ns = ns; s.cut = P > 1; s.slot = cta;
         const unsigned nq = (unsigned)(ns / quantum);  // P <= kMaxTailParts: the products fit 32 bits
         s.k0 = (int)(nq * (unsigned)j / (unsigned)P) * quantum;

@@ -126,8 +126,9 @@ struct StepRec {
 //   hand-over and halves the A traffic per MMA; the 32 accumulators fill tensor memory (one buffer).
 // GATHER: no packed copy of the blocks (a product without a plan): each block comes from where the boundary's array has it, by a
 //   tiled copy of its own whose 32-byte swizzle is what the packed copy holds ready.  `packed` is null then, `blk` the blocks'
-//   indices in walk order.  A copy takes the copy engine some 28 cycles, the MMA of a block 39 and more, so that the copies hide
-//   behind the MMAs, as often as tiles of C repeat them, and the packing (37 of 141 us for 121 MB of blocks) goes.  Products
+//   indices in walk order, gsp and steps as plan_kernel writes them without a count (schedule 3).  A copy takes the copy engine
+//   some 28 cycles, the MMA of a block 39 and more, so that the copies hide behind the MMAs, as often as tiles of C repeat them,
+//   and the packing (37 of 141 us for 121 MB of blocks) goes.  Products
 //   without a plan, packed and gathered: random matrix of 16384 rows, 237 000 blocks, N = 256: 141 and 107 us; 65536 rows, 3.8
 //   million blocks, N = 128: 1436 and 727, N = 1024: 5105 and 4508; dense clusters of 65536 rows, N = 128: 43 and 32, N = 1024:
 //   105 and 104; band of 32768 rows, half bandwidth 256, N = 256: 50 and 38; dense 2048 x 8192, N = 128: 68 and 59.
@@ -182,6 +183,7 @@ spmm_bcsr_tc_kernel(const __grid_constant__ CUtensorMap mapB, const __grid_const
         sg.flat = flat; sg.g = 0;
         sg.p = sg.p_begin = sg.p_end = 0;
         sg.list = sched_list; sg.li = sg.li_end = 0; sg.lt = 0;
+        if (SCHED == 3) { sg.rowptr = rowptr; sg.brow_begin = brow_begin; sg.brow_end = brow_end; sg.rg = rg; }
         if (listed) { sg.li = __ldg(sched_off + blockIdx.x); sg.li_end = __ldg(sched_off + blockIdx.x + 1); }
         if (balanced) {
             sg.p = sg.p_begin = flat.range_begin((int)gridDim.x, (int)blockIdx.x);
@@ -555,14 +557,15 @@ spmm_bcsr_tc_kernel(const __grid_constant__ CUtensorMap mapB, const __grid_const
                     pp += k1 - k0;
                 }
             }
-            for (int item = blockIdx.x; SCHED == 0 && item < n_full; item += gridDim.x) {  // the complete rounds: whole items
-                const int g = item / n_tiles;
-                run_segment(0, __ldg(gsp + g + 1) - __ldg(gsp + g));
+            constexpr bool rounds = SCHED == 0 || SCHED == 3;
+            auto steps_of = [&](int g) { return SCHED == 3 ? __ldg(gsp + g) : __ldg(gsp + g + 1) - __ldg(gsp + g); };
+            for (int item = blockIdx.x; rounds && item < n_full; item += gridDim.x) {  // the complete rounds: whole items
+                run_segment(0, steps_of(item / n_tiles));
             }
-            if (SCHED == 0 && (int)blockIdx.x < (n_items - n_full) * tail_parts) {  // the last round: one segment of an item
+            if (rounds && (int)blockIdx.x < (n_items - n_full) * tail_parts) {  // the last round: one segment of an item
                 const int i = (int)blockIdx.x / tail_parts, j = (int)blockIdx.x - i * tail_parts;
                 const int g = (n_full + i) / n_tiles;
-                const unsigned ns = (unsigned)(__ldg(gsp + g + 1) - __ldg(gsp + g));  // times j <= 4: fits 32 bits
+                const unsigned ns = (unsigned)steps_of(g);  // times j <= 4: fits 32 bits
                 const int k0 = __shfl_sync(0xffffffffu, (int)(ns * (unsigned)j / (unsigned)tail_parts), 0);
                 const int k1 = __shfl_sync(0xffffffffu, (int)(ns * (unsigned)(j + 1) / (unsigned)tail_parts), 0);
                 run_segment(k0, k1);
@@ -827,7 +830,7 @@ int launch_spmm(const PlanView& whole, const void* B, void* C, size_t N, cudaStr
     if (plan.cap != (size_t)kPlanBlocksPerStep && plan.cap != (size_t)kPlanBlocksPerStepDense)
         return fail(SMAT_ERR_BAD_ARG, "plan with %zu blocks per step: no kernel for it", plan.cap);
     int rc;
-    if (gather) rc = launch(spmm_bcsr_tc_kernel<false, 1, 0, kPlanBlocksPerStep, true>, Cfg<1, kPlanBlocksPerStep>::SMEM_BYTES);
+    if (gather) rc = launch(spmm_bcsr_tc_kernel<false, 1, 3, kPlanBlocksPerStep, true>, Cfg<1, kPlanBlocksPerStep>::SMEM_BYTES);
     else if (listed) rc = launch_cap(std::integral_constant<int, 1>{});
     else if (balanced) rc = launch_cap(std::integral_constant<int, 2>{});
     else rc = launch_cap(std::integral_constant<int, 0>{});

@@ -147,9 +147,12 @@ extern "C" int smat_spmm_bcsr_f16_static(const void* vals, const int* rowptr, co
     const bool pack = g_spmm_variant == 2 || g_spmm_variant == 3;
     if (pack) v.packed = packed;
     else v.vals = vals;
-    if (int rc = plan_count_async(rowptr, colidx, K, nnzb, 0, Mb, rg, gsp, stream, &d->ctx)) return rc;
-    if (int rc = plan_fill_async(rowptr, colidx, K, nnzb, 0, Mb, rg, gsp, steps, blk, stream, &d->ctx)) return rc;
-    if (pack)
+    if (pack) {
+        if (int rc = plan_count_async(rowptr, colidx, K, nnzb, 0, Mb, rg, gsp, stream, &d->ctx)) return rc;
+        if (int rc = plan_fill_async(rowptr, colidx, K, nnzb, 0, Mb, rg, gsp, steps, blk, stream, &d->ctx)) return rc;
         if (int rc = pack_values_async(rowptr, vals, blk, packed, 0, Mb, nnzb, stream, &d->ctx)) return rc;
+    } else if (int rc = plan_fill_loose_async(rowptr, colidx, K, nnzb, 0, Mb, rg, gsp, steps, blk, stream, &d->ctx)) {
+        return rc;
+    }
     return launch_spmm(v, B, C, N, stream, &d->ctx);
 }

@@ -52,23 +52,25 @@ def test_gather_against_oracle_and_packed(Mb, Kb, fill, N):
     assert torch.all((packed.data.float() - C.data.float()).abs() <= torch.from_numpy(2 * bound).cuda())
 
 
-@pytest.mark.parametrize("what", ["column", "order", "rowptr"])
+@pytest.mark.parametrize("what", ["column", "order", "rowptr", "dip"])
 def test_gather_reports_inconsistent_arrays(what):
-    """Columns outside the matrix, block columns that go back to an earlier window, row pointers beyond the blocks: reported, and the
-    next product is right."""
+    """Columns outside the matrix, block columns that go back to an earlier window, row pointers beyond the blocks or that go down so
+    that a block-row claims others' blocks, more than its group has room for: reported, and the next product is right."""
     rng = np.random.default_rng(9)
     Mb, Kb, N = 20, 17000, 128
     M, K = Mb * 16, Kb * 16
     brp, bci, bv = _matrix(rng, Mb, Kb, 0.002)
     B = rng.standard_normal((N, K)).astype(np.float16)
-    row = int(np.argmax(np.diff(brp)))
+    row = 5
     bad_rp, bad_ci = brp.copy(), bci.copy()
     if what == "column":
         bad_ci[brp[row + 1] - 1] = K
     elif what == "order":
         bad_ci[brp[row]] = K - 16
+    elif what == "rowptr":
+        bad_rp[-1] = brp[-1] + 5
     else:
-        bad_rp[row + 1] = brp[-1] + 5
+        bad_rp[row + 1] = brp[row - 3]
     Bd, C = S.Matrix.from_host(B), S.Matrix(M, N, fill=float("nan"))
     S.set_variant(1)
     try:
