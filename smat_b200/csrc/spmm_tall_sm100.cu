@@ -39,10 +39,10 @@
 // Groups of at most 16 or 20 block-rows use fewer accumulators and a longer tensor-memory panel ring (8 or 6 slots
 // instead of 4).  Scheduling is the round-robin-with-cut-last-round scheme of spmm_sm100.cu (SegGen<0>); the plan
 // pads every group to an even number of steps and items are cut at even positions, so a pair never spans two items.
-// What bounds the kernel on the block-sparse layer it was written for (1190 cycles per pair of steps at 24 rows): the loop copy ->
-// MMAs -> slot release, with two pairs of panels in tensor memory.  Of it 512 cycles are the copies themselves, 300 the MMAs, the
-// rest hand-overs; without panels, copies and MMAs the loop alone takes 650.  The loads (52 KB a pair) would take 740 at the rate
-// at which L2 serves a pure streaming kernel (70 bytes per cycle and SM).
+// What bounds the kernel on the block-sparse layer it was written for (1130 cycles per pair of steps at 24 rows): the loop copy ->
+// MMAs -> slot release, with two pairs of panels in tensor memory.  The tensor pipe has 860 of them (512 the copies, 350 the MMAs),
+// an issuing warp 970 (wait 170, list 160, MMAs 410, commit 230), and the loads (52 KB a pair) would take 740 at the rate at which
+// L2 serves a pure streaming kernel (70 bytes per cycle and SM).
 #include <cuda_fp16.h>
 #include <limits.h>
 #include <stdlib.h>
