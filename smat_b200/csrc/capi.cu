@@ -138,8 +138,8 @@ using namespace smat;
 
 extern "C" {
 
-// One multiplication with a plan (walk order + packed copy of the blocks) built on the fly in
-// stream-ordered scratch memory.
+// One multiplication with the stream kernel, or with the walk order built on the fly in stream-ordered scratch memory; the kernel
+// then reads the blocks where they are.
 static int spmm_transient_plan(const void* vals, const int* rowptr, const int* colidx, const void* B, void* C, size_t N,
                                size_t K, size_t nnzb, size_t brow_begin, size_t brow_end, cudaStream_t stream) {
     if (brow_end == brow_begin || N == 0) return SMAT_OK;

@@ -13,7 +13,7 @@
 // processed in windows of 16384; inside a window a shared word per block-column collects the row
 // mask (atomicOr), block-wide prefix sums number the steps and the blocks, then every block
 // scatters its own index into the (group, column, row) order.  The number of steps per group is
-// counted first (same pass without the scatter) and scanned.
+// counted first (same pass without the scatter) and scanned; a product without a plan does without the count (`loose`).
 #include <cuda_fp16.h>
 
 #include <new>

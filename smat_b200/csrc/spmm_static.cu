@@ -4,9 +4,9 @@
 // any framework allocator on top of them) is off limits -- a latency-critical serving loop whose
 // memory budget is fixed at start-up, a library callback invoked while another component holds the
 // allocator or device-synchronising locks, a process that has handed all remaining device memory
-// to a pool it does not own.  smat_spmm_bcsr_f16 builds its plan (walk order plus a copy of the
-// blocks in that order) in freshly allocated scratch on every call; this variant builds the same
-// plan in a fixed array that is part of the library image, so the call itself allocates nothing
+// to a pool it does not own.  smat_spmm_bcsr_f16 builds the blocks' walk order (and, for two of
+// the forced variants, a copy of the blocks in it) in freshly allocated scratch on every call; this variant builds the same
+// in a fixed array that is part of the library image, so the call itself allocates nothing
 // and frees nothing.
 //
 // Cost and limits: the array occupies kStaticScratchBytes (17.5 MB) on every GPU that loads
