@@ -240,7 +240,7 @@ int smat_selftest_wait_timeout(void* stream) {
     clear_error();
     DeviceCtx* ctx = nullptr;
     if (int rc = get_device_ctx(&ctx)) return rc;
-    wait_selftest_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(ctx->d_status, 400000LL);  // about 0.2 ms
+    wait_selftest_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(ctx->d_status, kSelftestWaitCycles);
     count_launch();
     SMAT_CUDA_TRY(cudaGetLastError());
     return SMAT_OK;

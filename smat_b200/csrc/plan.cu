@@ -1144,6 +1144,18 @@ int smat_plan_spmm(const smat_plan* plan, const void* B, void* C, size_t N, void
     return launch_spmm(view_for(plan, N), B, C, N, (cudaStream_t)stream);
 }
 
+int smat_selftest_plan_wait_timeout(const smat_plan* plan, const void* B, void* C, size_t N, void* stream) {
+    clear_error();
+    if (!plan || !B || !C) return fail(SMAT_ERR_BAD_ARG, "NULL argument");
+    if (N == 0 || N % 8 || N >= ((size_t)1 << 31)) return fail(SMAT_ERR_BAD_ARG, "N (%zu) must be a multiple of 8 below 2^31", N);
+    if (((uintptr_t)B | (uintptr_t)C) & 15) return fail(SMAT_ERR_BAD_ARG, "B and C must be 16-byte aligned");
+    if (int rc = check_plan_device(plan)) return rc;
+    PlanView v = view_for(plan, N);
+    if (!v.stream) return fail(SMAT_ERR_BAD_ARG, "this plan's kernel has no such self-test");
+    v.selftest = true;
+    return launch_spmm(v, B, C, N, (cudaStream_t)stream);
+}
+
 int smat_plan_spmm_host(smat_plan* plan, const void* B_host, void* C_host, size_t N, void* stream) {
     clear_error();
     if (!plan) return fail(SMAT_ERR_BAD_ARG, "plan is NULL");

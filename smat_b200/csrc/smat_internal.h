@@ -69,6 +69,8 @@ int static_status_take(int* out);
 // Device status codes (the word kernels set): 1..99 a bounded wait ran out at that wait site; 100.. the input
 // structure is inconsistent (101: row pointers disagree with the number of blocks, 102: a block column is out of range
 // or the columns of a block-row are not ascending, see kOrderWindow).
+// Limit of a wait inside a kernel, in clock cycles: about two seconds; of the waits that a self-test lets run out, about 0.2 ms.
+constexpr long long kWaitCycles = 4000000000LL, kSelftestWaitCycles = 400000LL;
 constexpr int kStatusBadRowptr = 101;
 constexpr int kStatusBadColumns = 102;
 // Most block-columns that the plan kernels look at together.  Inside such a window they sort for themselves, so the order of
@@ -179,6 +181,7 @@ struct PlanView {
     size_t cap = kPlanBlocksPerStep;  // most blocks of a step: kPlanBlocksPerStep or kPlanBlocksPerStepDense
     double step_cycles = 0.0;  // what a step is estimated to take (tc_estimate_us)
     double heaviest_cycles = 0.0;  // ... and the heaviest group for one tile of C, in one piece
+    bool selftest = false;  // the product's waits for blocks run out (smat_selftest_plan_wait_timeout)
     bool vertical = false;  // most blocks have a neighbour above or below in their block-column (dense clusters)
     // Tall plan: groups of rg <= kTallRows block-rows with an even number of steps, at most kTallBlocksPerStep blocks
     // per step.  A step record is {element column of the quad, position of the first block in the packed stream in

@@ -11,7 +11,6 @@ namespace {
 
 using namespace ptx;
 
-constexpr long long WAIT_LIMIT = 4000000000LL;  // clock cycles (about two seconds)
 constexpr int RG = kPlanRowsPerGroup;           // block-rows per work item of the 16-row kernels
 
 __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
@@ -39,7 +38,7 @@ static __device__ unsigned long long g_wait_prof[64];
 
 // Bounded mbarrier wait.  After the first time-out anywhere in the CTA every wait returns at once.
 __device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, uint32_t abort_addr, int* status, int code,
-                                         long long limit = WAIT_LIMIT) {
+                                         long long limit = kWaitCycles) {
     if (mbar_try_wait(bar, parity)) return;
     if (ld_shared_u32(abort_addr)) return;
     const long long t0 = clock64();

@@ -66,11 +66,11 @@ __device__ __forceinline__ uint2 lds8(uint32_t at) {
     return v;
 }
 constexpr int kRingWaitCode = 40;  // status word: a bounded wait of the ring kernel ran out
-__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity, long long limit) {
     if (ptx::mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     while (!ptx::mbar_try_wait_suspend(bar, parity, 2000u))
-        if (clock64() - t0 > 4000000000LL) return false;  // about two seconds
+        if (clock64() - t0 > limit) return false;
     return true;
 }
 
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_ring_kernel(const
 #pragma unroll
     for (int j = 0; j < T; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
     const int octets = min(p.tile_cols, p.N - n0) >> 3, Kb = p.K >> 4;
-    const uint32_t bytes = (uint32_t)octets * 256u;
+    const uint32_t bytes = (uint32_t)octets * 256u, awaited = bytes + 512u + p.lost_bytes;
     const uint8_t* vals = static_cast<const uint8_t*>(p.vals);
     const uint8_t* slabs = static_cast<const uint8_t*>(p.B) + (size_t)n0 * 32;
     const size_t slab = (size_t)p.N * 32;
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_ring_kernel(const
         if (at < c1 && cb >= 0) {
             ok |= 1u << s;
             if (lane == 0) {
-                ptx::mbar_arrive_expect_tx(bars + 8 * s, bytes + 512u);
+                ptx::mbar_arrive_expect_tx(bars + 8 * s, awaited);
                 ptx::bulk_load(ring + s * STAGE, slabs + (size_t)cb * slab, bytes, bars + 8 * s);
                 ptx::bulk_load_hint(ring + s * STAGE + NT * 32, vals + (size_t)at * 512, 512u, bars + 8 * s, once);
             }
@@ -396,7 +396,8 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_ring_kernel(const
 #pragma unroll
         for (int s = 0; s < S; s++) {
             if (there && (ok & (1u << s))) {
-                there = ring_wait(bars + 8 * s, (phase >> s) & 1u);
+                // (by vote: at the limit one lane may give up where the next still sees the copy arrive, and all take part in fetch())
+                there = __all_sync(0xffffffffu, ring_wait(bars + 8 * s, (phase >> s) & 1u, p.wait_cycles));
                 phase ^= 1u << s;
                 // all of the stage: what a narrower tile leaves of it goes to columns that are not stored
                 uint4 a;
@@ -813,6 +814,8 @@ int launch_stream(const PlanView& v, const void* B, void* C, size_t N, cudaStrea
             a.B = sp.slabs;
         }
         // one round of warps: see the kernel's first lines (with more, most begin long after the kernel before this one)
+        a.wait_cycles = v.selftest ? kSelftestWaitCycles : kWaitCycles;
+        a.lost_bytes = v.selftest ? 16 : 0;
         a.nnzb = (long long)a.n_pieces * a.n_tiles * s.w <= 40LL * ctx->sm_count && row_begin == 0 && row_end == rows ? (int)v.nnzb : 0;
         if (int rc = launch<true>(s, a, stream)) return rc;
     }
@@ -851,6 +854,7 @@ int stream_call(const StreamShape& s, const void* vals, const int* rowptr, const
     a.brow_end = (int)brow_end;
     a.nnzb = (int)nnzb;
     a.chunk = s.chunk;
+    a.wait_cycles = kWaitCycles;
     if (extra) {
         int* head = reinterpret_cast<int*>(b); b += 256;
         a.long_rows = head;

@@ -73,3 +73,26 @@ def test_ring_skips_columns_outside_the_matrix():
         S.set_variant(0)
     # another order of nothing but a block of zeros: the same sums
     assert np.array_equal(got.view(np.uint16), C.data.cpu().numpy().view(np.uint16))
+
+
+@pytest.mark.parametrize("Mb,Kb,most,N", [(2400, 300, 40, 128), (2400, 300, 40, 96), (1100, 260, 60, 128), (300, 700, 300, 128)])
+def test_waits_that_run_out_end_the_product_and_are_reported(Mb, Kb, most, N):
+    """One, two and four warps a block-row give up their first wait (all lanes of a warp, and all warps reach the sum of a block-row):
+    the kernel ends, the status says so once, and the plan's next product is the one before."""
+    rng = np.random.default_rng(N)
+    M, K = Mb * 16, Kb * 16
+    brp, bci, bv = _matrix(rng, Mb, Kb, most)
+    Bd, C = S.Matrix.from_host(rng.standard_normal((N, K)).astype(np.float16)), S.Matrix(M, N, fill=float("nan"))
+    S.set_variant(5)
+    try:
+        p = S.Plan(S.SparseMatrix.from_bcsr(M, K, brp, bci, bv), n_hint=N)
+    finally:
+        S.set_variant(0)
+    p.spmm(Bd, C, check=True)
+    before = C.data.cpu().numpy().copy()
+    assert S.lib().smat_selftest_plan_wait_timeout(p._h, Bd.data.data_ptr(), C.data.data_ptr(), N, None) == 0
+    assert S.lib().smat_device_status(None) == -3 and b"site code 40" in S.lib().smat_last_error_string()
+    C.data.fill_(float("nan"))
+    p.spmm(Bd, C, check=True)
+    p.close()
+    assert np.array_equal(before.view(np.uint16), C.data.cpu().numpy().view(np.uint16))
