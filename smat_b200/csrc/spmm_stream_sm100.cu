@@ -443,7 +443,9 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_ring_kernel(const
         }
         if (w != 0 || !q.live) return;
     }
-    if (there) finish_piece<T>(p, q, acc, tile, n0, octets, lane);
+    // (also after a wait that ran out: a piece of a long block-row that did not arrive would leave the row's counter, which the last
+    // one resets, part-way up for the plan's next product)
+    finish_piece<T>(p, q, acc, tile, n0, octets, lane);
 }
 
 // B ([N][K], k contiguous) -> slabs [K / 16][N][16]: the 16 x N slice of one block-column becomes contiguous.

@@ -75,13 +75,15 @@ def test_ring_skips_columns_outside_the_matrix():
     assert np.array_equal(got.view(np.uint16), C.data.cpu().numpy().view(np.uint16))
 
 
-@pytest.mark.parametrize("Mb,Kb,most,N", [(2400, 300, 40, 128), (2400, 300, 40, 96), (1100, 260, 60, 128), (300, 700, 300, 128)])
-def test_waits_that_run_out_end_the_product_and_are_reported(Mb, Kb, most, N):
+@pytest.mark.parametrize("Mb,Kb,most,long_row,N", [(2400, 300, 40, None, 128), (2400, 300, 40, None, 96), (1100, 260, 60, None, 128),
+                                                   (300, 700, 300, None, 128), (2400, 300, 40, 7, 128), (1100, 600, 60, 9, 128)])
+def test_waits_that_run_out_end_the_product_and_are_reported(Mb, Kb, most, long_row, N):
     """One, two and four warps a block-row give up their first wait (all lanes of a warp, and all warps reach the sum of a block-row):
-    the kernel ends, the status says so once, and the plan's next product is the one before."""
+    the kernel ends, the status says so once, and the plan's next products are the one before, of long block-rows too, whose pieces
+    are counted as they arrive."""
     rng = np.random.default_rng(N)
     M, K = Mb * 16, Kb * 16
-    brp, bci, bv = _matrix(rng, Mb, Kb, most)
+    brp, bci, bv = _matrix(rng, Mb, Kb, most, long_row)
     Bd, C = S.Matrix.from_host(rng.standard_normal((N, K)).astype(np.float16)), S.Matrix(M, N, fill=float("nan"))
     S.set_variant(5)
     try:
@@ -92,7 +94,8 @@ def test_waits_that_run_out_end_the_product_and_are_reported(Mb, Kb, most, N):
     before = C.data.cpu().numpy().copy()
     assert S.lib().smat_selftest_plan_wait_timeout(p._h, Bd.data.data_ptr(), C.data.data_ptr(), N, None) == 0
     assert S.lib().smat_device_status(None) == -3 and b"site code 40" in S.lib().smat_last_error_string()
-    C.data.fill_(float("nan"))
-    p.spmm(Bd, C, check=True)
+    for _ in range(3):
+        C.data.fill_(float("nan"))
+        p.spmm(Bd, C, check=True)
+        assert np.array_equal(before.view(np.uint16), C.data.cpu().numpy().view(np.uint16))
     p.close()
-    assert np.array_equal(before.view(np.uint16), C.data.cpu().numpy().view(np.uint16))
