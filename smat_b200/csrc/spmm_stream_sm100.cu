@@ -567,18 +567,19 @@ cudaError_t launch_one(const StreamArgs& a, cudaStream_t stream) {
 // slabs of more bytes than this are taken not to stay in L2 beside A (126 MB, each half of the SMs by its own half)
 constexpr size_t kSlabBytesL2 = (size_t)62 << 20;
 
-// resident: CTAs per SM where that is fewer than MINB (0: MINB)
-template <int NT, int S, int W, int kWarps, int MINB, bool PLAN>
-cudaError_t launch_ring(const StreamArgs& a, int resident, cudaStream_t stream) {
+// FEWER: CTAs per SM where `fewer` asks for them instead of MINB (0: never).  The limit that is set on the kernel is the most that
+// either launch of it wants: it belongs to the kernel, and another thread's launch may come between setting it and launching.
+template <int NT, int S, int W, int kWarps, int MINB, bool PLAN, int FEWER = 0>
+cudaError_t launch_ring(const StreamArgs& a, cudaStream_t stream, bool fewer = false) {
     const long long grid = (((long long)a.n_pieces + kWarps / W - 1) / (kWarps / W)) * a.n_tiles;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    size_t smem = kWarps * S * (NT * 32 + 512 + 8);
-    static_assert((kWarps * S * (NT * 32 + 512 + 8) + 1024) * MINB <= 228 * 1024, "shared memory of the resident CTAs");
-    if (resident && resident < MINB) smem = std::max<size_t>(smem, 228 * 1024 / (resident + 1));  // one more would not fit
+    constexpr int own = kWarps * S * (NT * 32 + 512 + 8), large = FEWER && FEWER < MINB ? 228 * 1024 / (FEWER + 1) : 0;  // large: one CTA more would not fit
+    constexpr int most = own > large ? own : large;
+    static_assert((own + 1024) * MINB <= 228 * 1024, "shared memory of the resident CTAs");
     auto kernel = spmm_bcsr_ring_kernel<NT, S, W, kWarps, MINB, PLAN>;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return e;
-    return launch_pdl(kernel, dim3((unsigned)grid), dim3(kWarps * 32), smem, stream, a);
+    return launch_pdl(kernel, dim3((unsigned)grid), dim3(kWarps * 32), fewer ? most : own, stream, a);
 }
 
 template <bool PLAN, bool SLAB, int W>
@@ -590,9 +591,9 @@ cudaError_t launch_nt(int nt, const StreamArgs& a, cudaStream_t stream) {
         // 480 (power-law matrix of 262144 rows), 16 x 4 of 64 columns 575 (12 x 4) to 1000.  Slabs of more than half of L2
         // leave it less room for A, and want fewer warps: 262144 rows, 128 columns, 653 us with 14 warps, 624 with 12; 155152
         // rows 415 and 432.
-        if (nt == 128 && a.tile_cols > 96) return launch_ring<128, 3, W, kWarps, 14 / kWarps, PLAN>(a, (size_t)a.N * a.K * 2 > kSlabBytesL2 ? 12 / kWarps : 0, stream);
-        if (nt == 128) return launch_ring<96, 3, W, kWarps, 16 / kWarps, PLAN>(a, 0, stream);
-        if (nt == 64) return launch_ring<64, 2, W, kWarps, 20 / kWarps, PLAN>(a, 0, stream);
+        if (nt == 128 && a.tile_cols > 96) return launch_ring<128, 3, W, kWarps, 14 / kWarps, PLAN, 12 / kWarps>(a, stream, (size_t)a.N * a.K * 2 > kSlabBytesL2);
+        if (nt == 128) return launch_ring<96, 3, W, kWarps, 16 / kWarps, PLAN>(a, stream);
+        if (nt == 64) return launch_ring<64, 2, W, kWarps, 20 / kWarps, PLAN>(a, stream);
     }
     if constexpr (!SLAB && W < 8) {
         if (nt == 128) return launch_one<128, W, SLAB, PLAN>(a, stream);

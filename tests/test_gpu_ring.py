@@ -1,8 +1,11 @@
 """Wide products of the stream kernels from slabs, whose slices come through a ring in shared memory: block-rows shorter than the
 ring, empty ones, one, two and four warps a block-row, long block-rows in pieces, tiles of every width class and their edges, with a
 plan and without."""
+import threading
+
 import numpy as np
 import pytest
+import torch
 
 import oracle
 import smat_b200 as S
@@ -99,3 +102,46 @@ def test_waits_that_run_out_end_the_product_and_are_reported(Mb, Kb, most, long_
         p.spmm(Bd, C, check=True)
         assert np.array_equal(before.view(np.uint16), C.data.cpu().numpy().view(np.uint16))
     p.close()
+
+
+def test_small_and_large_slabs_from_two_threads():
+    """Slabs of more than half of L2 are multiplied by the same kernel with more shared memory for each CTA: two threads that launch
+    it so and so do not refuse each other's launch, and both products are right."""
+    N, plans = 128, []
+    for Mb, Kb, most in [(2400, 16384, 120), (2400, 300, 40)]:  # 67 MB of slabs, 1.2 MB
+        rng = np.random.default_rng(Kb)
+        M, K = Mb * 16, Kb * 16
+        brp, bci, bv = _matrix(rng, Mb, Kb, most)
+        B = rng.standard_normal((N, K)).astype(np.float16)
+        A, Bd, C = S.SparseMatrix.from_bcsr(M, K, brp, bci, bv), S.Matrix.from_host(B), S.Matrix(M, N, fill=float("nan"))
+        S.set_variant(5)
+        try:
+            plan = S.Plan(A, n_hint=N)
+        finally:
+            S.set_variant(0)
+        plan.spmm(Bd, C, check=True)
+        ref = oracle.bcsr_spmm(bv, brp, bci, B, M, N, K, threads=8)
+        size = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B), M, N, K, threads=8)
+        bound = 2 * K * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24  # as above
+        assert np.all(np.abs(C.data.cpu().numpy().astype(np.float32) - ref) <= bound)
+        plans.append((plan, Bd, C, C.data.clone()))
+    errors, start = [], threading.Barrier(2)
+
+    def work(plan, Bd, C, first):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait()
+                for _ in range(300):
+                    plan.spmm(Bd, C)
+                torch.cuda.current_stream().synchronize()
+            assert torch.equal(C.data, first)
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=p) for p in plans]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    assert S.lib().smat_device_status(None) == 0
