@@ -147,10 +147,10 @@ int smat_device_status(void* stream);
  * it.  Nothing faults and the context stays usable.  No counterpart in the reference. */
 int smat_selftest_wait_timeout(void* stream);
 
-/* The same for a product with a plan whose kernel waits for slices of B and blocks in shared memory (the kernel that walks single
- * block-rows, 33 to 128 columns from slabs): every wait expects more bytes than are copied and gives up after about 0.2 ms.  C is
- * invalid, the next smat_device_status says so (SMAT_ERR_DEVICE_WAIT), and products after that are as before.  The kernel's other
- * forms wait for nothing and multiply as ever; SMAT_ERR_BAD_ARG for plans of other kernels. */
+/* The same for a product with a plan whose kernel waits for blocks in shared memory (the tall kernel; the kernel that walks single
+ * block-rows, 33 to 128 columns from slabs): the waits for blocks expect more bytes than are copied, and waits give up after about
+ * 0.2 ms.  C is invalid, the next smat_device_status says so (SMAT_ERR_DEVICE_WAIT), and products after that are as before.  The
+ * latter kernel's other forms wait for nothing and multiply as ever; SMAT_ERR_BAD_ARG for plans of other kernels. */
 int smat_selftest_plan_wait_timeout(const smat_plan* plan, const void* B, void* C, size_t N, void* stream);
 
 /* Number of this library's kernels launched so far by the calling process (all devices). */

@@ -1151,7 +1151,7 @@ int smat_selftest_plan_wait_timeout(const smat_plan* plan, const void* B, void* 
     if (((uintptr_t)B | (uintptr_t)C) & 15) return fail(SMAT_ERR_BAD_ARG, "B and C must be 16-byte aligned");
     if (int rc = check_plan_device(plan)) return rc;
     PlanView v = view_for(plan, N);
-    if (!v.stream) return fail(SMAT_ERR_BAD_ARG, "this plan's kernel has no such self-test");
+    if (!v.stream && !v.tall) return fail(SMAT_ERR_BAD_ARG, "this plan's kernel has no such self-test");
     v.selftest = true;
     return launch_spmm(v, B, C, N, (cudaStream_t)stream);
 }

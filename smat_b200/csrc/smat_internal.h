@@ -147,6 +147,7 @@ constexpr int kTallBlocksPerStep = 48;
 // word 1: the group of one; words 2, 3: of two; 4 to 7: of four; 8 to 15: of eight.
 constexpr int kTallListBytes = 64;
 constexpr uint32_t kTallList1 = 1u << 31, kTallList2 = 1u << 30, kTallList4 = 1u << 29, kTallList8 = 1u << 28, kTallListLast = 1u << 7;
+constexpr uint32_t kTallListNone = 1u << 6;  // in the kernel only: a wait was given up
 static_assert(2 * kTallBlocksPerStep * 32 <= 1 << 12, "an entry's block");
 // MMA-issuing warps of the kernel; each owns kPlanRowsPerGroup / kPlanOwners consecutive accumulators.
 #ifndef SMAT_OWNERS

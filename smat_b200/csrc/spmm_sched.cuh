@@ -36,21 +36,22 @@ __device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) {
 static __device__ unsigned long long g_wait_prof[64];
 #endif
 
-// Bounded mbarrier wait.  After the first time-out anywhere in the CTA every wait returns at once.
-__device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, uint32_t abort_addr, int* status, int code,
+// Bounded mbarrier wait; false: given up.  After the first time-out anywhere in the CTA every wait returns at once.
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, uint32_t abort_addr, int* status, int code,
                                          long long limit = kWaitCycles) {
-    if (mbar_try_wait(bar, parity)) return;
-    if (ld_shared_u32(abort_addr)) return;
+    if (mbar_try_wait(bar, parity)) return true;
+    if (ld_shared_u32(abort_addr)) return false;
     const long long t0 = clock64();
     // suspended waits: the warp sleeps in hardware until the phase completes or ~2 us pass
     while (!mbar_try_wait_suspend(bar, parity, 2000u)) {
-        if (ld_shared_u32(abort_addr)) return;
+        if (ld_shared_u32(abort_addr)) return false;
         if (clock64() - t0 > limit) {
             st_shared_u32(abort_addr, 1);
             atomicCAS(status, 0, code);
-            return;
+            return false;
         }
     }
+    return true;
 }
 
 // A segment: steps [k0, k1) of the ns steps of work item `item` (the first step of the item is steps[gs]).

@@ -128,7 +128,8 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                       const uint4* __restrict__ steps, const uint4* __restrict__ winfo, const int* __restrict__ gsp,
                       const int* __restrict__ rowptr,
                       __half* __restrict__ C, size_t ldc, int brow_begin, int brow_end, int rg, int N, int n_tiles, int n_items,
-                      int tail_parts, uint32_t panel_bytes, float* __restrict__ fix_scratch, int* status, int pf) {
+                      int tail_parts, uint32_t panel_bytes, float* __restrict__ fix_scratch, int* status, int pf,
+                      long long wait_cycles, uint32_t lost_bytes) {
     constexpr int NMW = Shape<TRG>::NMW;
     constexpr uint32_t TS_ = Shape<TRG>::TS_, TMEM_PANELS = Shape<TRG>::TMEM_PANELS;
     using L = Smem<PS>;
@@ -161,14 +162,15 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
         if (code) prof_c[code] += (unsigned int)(t_ - prof_t);   \
         prof_t = t_;                                             \
     } while (0)
-#define TWAIT(bar, par, code)                                    \
-    do {                                                         \
-        const long long t_ = clock64();                          \
-        wait_bar(bar, par, abort_addr, status, code);            \
-        prof_c[code] += (unsigned int)(clock64() - t_);          \
-    } while (0)
+    auto timed_wait = [&](uint32_t bar, uint32_t par, int code) {
+        const long long t_ = clock64();
+        const bool there = wait_bar(bar, par, abort_addr, status, code, wait_cycles);
+        prof_c[code] += (unsigned int)(clock64() - t_);
+        return there;
+    };
+#define TWAIT(bar, par, code) timed_wait(bar, par, code)
 #else
-#define TWAIT(bar, par, code) wait_bar(bar, par, abort_addr, status, code)
+#define TWAIT(bar, par, code) wait_bar(bar, par, abort_addr, status, code, wait_cycles)
 #define PROF_MARK(code)
 #endif
     const int n_full = n_items / (int)gridDim.x * (int)gridDim.x;  // items of the complete rounds
@@ -251,7 +253,7 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                     if (!r.live) { more = false; break; }
                     const uint32_t ps = r.st % PS, fp = r.st % FP, pi = r.st >> 1;
                     // the panel's slot is free once the copy of the step PS positions back (pair pi - PS / 2) has left it
-                    if (r.st >= PS) TWAIT(cp_done((pi - PS / 2) % NPAIR), ((pi - PS / 2) / NPAIR) & 1, 1);
+                    if (r.st >= PS && !TWAIT(cp_done((pi - PS / 2) % NPAIR), ((pi - PS / 2) / NPAIR) & 1, 1)) { more = false; break; }
                     st_shared_u32(base + L::SUBS + fp * 4, r.a.w);  // for the copier; ordered before its wait by the arrive below
                     if (r.a.z) {
                         mbar_arrive_expect_tx(full_p(fp), panel_bytes);
@@ -272,7 +274,8 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
             uint32_t used = 0, freed = 0;    // blocks of the ring taken (with what was left out at its end) and given back, ever
             constexpr int U = 4;             // pairs whose step records are requested ahead
             struct { uint32_t at, n; } rec[U];
-            while (sg.next(cs)) {
+            bool there = true;
+            while (there && sg.next(cs)) {
                 const int first = (cs.gs + cs.k0) >> 1, n_pairs = (cs.k1 - cs.k0) >> 1;
                 auto gen = [&](int i, int a) {
                     if (i >= n_pairs) return;
@@ -282,7 +285,7 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                 };
 #pragma unroll
                 for (int a = 0; a < U; a++) gen(a, a);
-                for (int i0 = 0; i0 < n_pairs; i0 += U) {
+                for (int i0 = 0; there && i0 < n_pairs; i0 += U) {
 #pragma unroll
                     for (int a = 0; a < U; a++) {
                         if (i0 + a >= n_pairs) break;
@@ -293,13 +296,15 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                         }
                         used += n;
                         while (done < pi && (pi - done >= NLIST || used - freed > RING_BLOCKS)) {
-                            TWAIT(step_done(done % NPAIR), (done / NPAIR) & 1, 2);
+                            there = TWAIT(step_done(done % NPAIR), (done / NPAIR) & 1, 2);
+                            if (!there) break;
                             freed = ld_shared_u32(base + L::END + (done % NPAIR) * 4);
                             done++;
                         }
+                        if (!there) break;
                         st_shared_u32(base + L::AT + pl * 4, head);
                         st_shared_u32(base + L::END + pl * 4, used);
-                        mbar_arrive_expect_tx(full_b(pl), n * 512u + META_BYTES);
+                        mbar_arrive_expect_tx(full_b(pl), n * 512u + META_BYTES + lost_bytes);
                         bulk_load(base + L::META + (pi % NLIST) * META_BYTES, winfo + (META_BYTES / 16) * (size_t)(first + i0 + a), META_BYTES, full_b(pl));
                         if (n) bulk_load(base + L::BLK + head * 512u, packed + (size_t)rec[a].at * 256, n * 512u, full_b(pl));
                         head += n;
@@ -333,7 +338,8 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                 const uint64_t pdesc = smem_desc_k_sw128(base + L::PANEL + ps * PANEL_BYTES);
                 const uint32_t tdst = tmem_base + TMEM_PANELS + (st % TS_) * 32;
                 TWAIT(full_p(fp), (st / FP) & 1, 3);
-                const uint32_t subs = uniform(ld_shared_u32(base + L::SUBS + fp * 4));  // non-empty sub-columns
+                const uint32_t subs = uniform(ld_shared_u32(base + L::SUBS + fp * 4) | ld_shared_u32(abort_addr) << 4);  // non-empty sub-columns
+                if (subs & 16u) break;
                 if (pi >= TS_ / 2) TWAIT(step_done((pi - TS_ / 2) % NPAIR), ((pi - TS_ / 2) / NPAIR) & 1, 5);
 #ifdef SMAT_PROFILE
                 if (pi >= TS_ / 2) prof_c[13] += (unsigned int)clock() - *(volatile unsigned int*)&stamp_mma[(pi - TS_ / 2) % 8];
@@ -375,9 +381,10 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
             constexpr uint32_t IDESC16 = idesc_f16_f32(128, 16);
             const uint32_t acc_m = tmem_base + TMEM_ACC + 2u * m * 16u;  // this warp's two accumulators
             uint32_t st = 0, it = 0;
+            bool there = true;
             SegGen<0> sg = make_gen();
             Seg cs;
-            while (sg.next(cs)) {
+            while (there && sg.next(cs)) {
                 TWAIT(acc_empty, (it & 1) ^ 1, 6);
                 tc_fence_after();
                 // segments hold an even number of steps and start at an even position: a pair never spans two of them
@@ -394,11 +401,15 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                     const uint32_t list = base + L::META + (pi % NLIST) * META_BYTES + m * kTallListBytes;
                     const uint4 l = ld_shared_v4(list), q = ld_shared_v4(list + 16);
                     const uint32_t b_lo = b_lo0 + ld_shared_u32(base + L::AT + (pi % NPAIR) * 4) * 32u;
-                    const uint32_t w0 = uniform(l.x);
+                    // Once a wait was given up, lists and places may never have arrived, and their MMAs could reach anywhere: none from
+                    // here on.  (Who gave up says so before it arrives at anything, and the loaders stop, so what is read above was there
+                    // if the word is still zero.)
+                    const uint32_t w0 = uniform(ld_shared_u32(abort_addr) ? kTallListNone : l.x);
+                    if (w0 & kTallListNone) { there = false; break; }
                     const uint32_t tpanel = tmem_base + TMEM_PANELS + (st % TS_) * 32;
                     PROF_MARK(9);
                     auto mma = [&](uint32_t e) {
-                        mma_f16_ts_if(leader, acc_m + (e & 0x1fu), tpanel + ((e >> 8) & 0xffu), b_lo + ((e >> 16) & 0xfffu), B_HI, IDESC16);
+                        mma_f16_ts_if(leader, acc_m + (e & 0x10u), tpanel + ((e >> 8) & 0x38u), b_lo + ((e >> 16) & 0xfe0u), B_HI, IDESC16);
                     };
                     if (w0 & kTallList1) mma(l.y);
                     if (w0 & kTallList2) {
@@ -557,7 +568,8 @@ int launch_spmm_tall(const PlanView& whole, const void* B, void* C, size_t N, cu
         SMAT_CUDA_TRY(launch_pdl_if(spmm_begins_early(n_items, sms), kernel, dim3(grid), dim3(threads), smem_bytes, stream,
                                  mapB, reinterpret_cast<const uint8_t*>(plan.packed), reinterpret_cast<const uint4*>(plan.steps),
                                  reinterpret_cast<const uint4*>(plan.winfo), plan.gsp, plan.rowptr, reinterpret_cast<__half*>(C), ldc, (int)plan.brow_begin,
-                                 (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles, (int)n_items, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, pf));
+                                 (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles, (int)n_items, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, pf,
+                                 whole.selftest ? kSelftestWaitCycles : kWaitCycles, whole.selftest ? 16u : 0u));
         return SMAT_OK;
     };
     // the smallest shape that holds the plan's groups: fewer accumulators leave tensor memory for more panel slots

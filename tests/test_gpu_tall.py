@@ -78,3 +78,32 @@ def test_both_splits_of_shared_memory(rows, fill):
     size = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B), Mb * 16, N, Kb * 16, threads=8)
     bound = 2 * Kb * 16 * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24  # as above
     assert np.all(np.abs(C.astype(np.float32) - ref) <= bound)
+
+
+@pytest.mark.parametrize("rows,fill", [(16, 0.1), (24, 0.35), (24, 0.9)])
+def test_waits_that_run_out_end_the_product_and_are_reported(rows, fill):
+    """The waits for blocks run out before the first list has arrived: no MMA takes its operands from shared memory that nothing was
+    written to, the kernel ends, the status says so once, and the plan's next products are the one before."""
+    rng = np.random.default_rng(rows)
+    Mb, Kb, N = 4 * rows, 120, 264
+    mask = rng.random((Mb, Kb)) < fill
+    brp = np.zeros(Mb + 1, np.int32)
+    brp[1:] = np.cumsum(mask.sum(axis=1))
+    bci = (np.nonzero(mask)[1] * 16).astype(np.int32)
+    bv = (rng.standard_normal(brp[-1] * 256) * 0.25).astype(np.float16)
+    S.set_variant(4)
+    try:
+        plan = S.Plan(S.SparseMatrix.from_bcsr(Mb * 16, Kb * 16, brp, bci, bv), n_hint=N)
+    finally:
+        S.set_variant(0)
+    assert plan.info()["tall"]
+    Bd, C = S.Matrix.from_host(rng.standard_normal((N, Kb * 16)).astype(np.float16)), S.Matrix(Mb * 16, N, fill=float("nan"))
+    plan.spmm(Bd, C, check=True)
+    before = C.data.cpu().numpy().copy()
+    assert S.lib().smat_selftest_plan_wait_timeout(plan._h, Bd.data.data_ptr(), C.data.data_ptr(), N, None) == 0
+    assert S.lib().smat_device_status(None) == -3
+    for _ in range(3):
+        C.data.fill_(float("nan"))
+        plan.spmm(Bd, C, check=True)
+        assert np.array_equal(before.view(np.uint16), C.data.cpu().numpy().view(np.uint16))
+    plan.close()
