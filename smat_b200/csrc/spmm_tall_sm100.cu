@@ -437,6 +437,9 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                         if (w0 & kTallListLast) mma(l.x);
                     }
                     PROF_MARK(10);
+#ifdef SMAT_PROFILE
+                    if (leader) atomicMax(&stamp_mma[pi % 8], (unsigned int)clock());
+#endif
                     if (w0) tc_commit_if(leader, step_done(pi % NPAIR));
                     else if (leader) mbar_arrive(step_done(pi % NPAIR));
                     PROF_MARK(11);
