@@ -908,12 +908,12 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
         }
     }
     // Tall plan: groups of up to 24 block-rows for the kernel that reads the B panels from tensor memory.  Its steps
-    // cost a little more than those of the 16-row kernels (tall_step_cycles() against ~480 cycles, the latter growing with
+    // cost as much as those of the 16-row kernels or more (tall_step_cycles(), at least 500, against ~480 cycles, the latter growing with
     // the MMAs of the step: ~58 cycles each with the hand-overs, the shared-memory operand port; vertical neighbours
     // share one, which is what keeps dense clusters with this kernel), so it pays where taller groups mean
     // fewer steps: matrices whose quads mostly hold a block (a block-sparse layer, a reordered random matrix: three
-    // quarters of the steps), not scattered ones (as many steps as before) and not dense clusters (steps of 32 blocks
-    // already).  Both plans are counted and the estimates compared; smat_spmm_set_variant(4) forces a tall plan,
+    // quarters of the steps), not those of a block or less a quad (as many steps as before) and not dense clusters (steps of 32
+    // blocks already).  Both plans are counted and the estimates compared; smat_spmm_set_variant(4) forces a tall plan,
     // 1..3 exclude it.
     const double mma_per_step = total_steps > 0 ? (double)mmas16 / (double)total_steps : 0.0;
     // cycles of a 16-row step: an MMA per block or pair of vertical neighbours, or, where whole columns of blocks are there
@@ -974,7 +974,7 @@ int smat_plan_create(smat_plan** out, const void* bcsrValuesA, const int* bcsrRo
             const double steps_per_tall = (double)tall_total_and_max[0] / (double)sz_tall.n_groups;
             const double est_tall =
                 tall_rounds(sz_tall.n_groups * tiles, (size_t)ctx->sm_count, steps_per_tall) * steps_per_tall *
-                    tall_step_cycles((double)range_blocks / (double)(tall_total_and_max[0] > 0 ? tall_total_and_max[0] : 1)) +
+                    std::max(tall_step_cycles((double)range_blocks / (double)(tall_total_and_max[0] > 0 ? tall_total_and_max[0] : 1)), kTallLeastCycles16) +
                 kTallExtraCycles;
             tall = tall_forced || est_tall < est16;
             if (std::getenv("SMAT_PLAN_DEBUG"))

@@ -117,8 +117,10 @@ inline double tall_rounds(size_t items, size_t sms, double est_steps) {
 // Cycles of a step of the tall kernel that holds `blocks` blocks, for the choice of heights (measured on layers of 256 steps an
 // item: 630 with 19 blocks a step, 750 with 29, 790 with 36, 1000 with 48; of many items an SM 510 with 10, 560 with 19).
 inline double tall_step_cycles(double blocks) { return 300.0 + 15.0 * blocks > 400.0 ? 300.0 + 15.0 * blocks : 400.0; }
-// ... and at least, against other kernels (steps of a few blocks take 510 to 590, estimates of the others are as low).
-constexpr double kTallLeastCycles = 440.0;
+// ... and at least: against the stream kernel, and against the 16-row kernels, whose steps are counted at 480 at least.  (Steps of a
+// few blocks take 410 to 440 where a CTA has many items, 500 where it has one: random matrix of 16384 rows with a tenth of its
+// blocks, N = 256, 6.4 blocks a step: 68 us with items of 16 rows, 63.5 with the 16-row kernel.)
+constexpr double kTallLeastCycles = 440.0, kTallLeastCycles16 = 500.0;
 // ... and what a launch of it costs beyond its steps: its pipeline takes longer to fill and to drain (measured, smallest plans).
 constexpr double kTallExtraCycles = 5000.0;
 // Measured cost of a 256-column item relative to a 128-column item of the same group.

@@ -159,3 +159,17 @@ def test_order_inside_a_window_does_not_matter(route):
     C = S.Matrix(640, 16, fill=float("nan"))
     assert _status_of(route, A, S.Matrix.from_host(B_nk), C) == (0, False)
     assert _error(C.data.cpu().numpy(), brp, bci, bv, B_nk, (0, 40)) <= TOL
+
+
+@pytest.mark.parametrize("N,tall", [(256, False), (1024, True)])
+def test_plan_of_few_blocks_a_step_is_tall_only_where_that_is_faster(N, tall):
+    """Some 105 000 scattered blocks, six of them a step: one round of items either way at 256 columns, which the 16-row kernel takes 63 us
+    for and the tall kernel 68; several at 1024 (228 and 173)."""
+    rng = np.random.default_rng(1)
+    mask = rng.random((1024, 1024)) < 0.1
+    brp = np.zeros(1025, np.int32)
+    brp[1:] = np.cumsum(mask.sum(axis=1))
+    A = S.SparseMatrix.from_bcsr(16384, 16384, brp, (np.nonzero(mask)[1] * 16).astype(np.int32), np.zeros(brp[-1] * 256, np.float16))
+    plan = S.Plan(A, n_hint=N)
+    assert plan.info()["tall"] == tall
+    plan.close()
