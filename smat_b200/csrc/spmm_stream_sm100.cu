@@ -185,14 +185,11 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
     const int tile = (int)(blockIdx.x % (unsigned)p.n_tiles);
     const int piece = (int)(blockIdx.x / (unsigned)p.n_tiles) * (kWarps / W) + warp / W;
     const int n0 = tile * p.tile_cols;
-    if (PLAN && p.nnzb && lane == 0 && tile == 0 && piece < p.n_pieces) {
+    if (PLAN && p.ahead > 0.0f && lane == 0 && tile == 0 && piece < p.n_pieces) {
         // about where this warp's blocks begin, were they dealt out evenly: on their way to L2 before the kernel before this one
-        // has ended (nothing is read here, so it matters neither whether that one writes them nor whether the place is right).
-        // Layer 8192 x 28672 at 20 %, N = 16: 24.4 -> 23.4 us (32 blocks instead of eight: 24.3); 8192 x 8192 at 10 %, N = 32:
-        // 10.7 -> 9.6; 4096 x 14336 at 20 %: 12.3 -> 12.3; a pass after which the device is waited for takes as long as before.
-        const long long at = (long long)p.nnzb * (piece * W + warp % W) / ((long long)p.n_pieces * W);
-        const int n = min(p.nnzb - (int)at, 8);
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const uint8_t*>(p.vals) + at * 512), "r"(n * 512) : "memory");
+        // has ended (nothing is read here, so it matters neither whether that one writes them nor whether the place is right)
+        const int at = min((int)(p.ahead * (float)(piece * W + warp % W)), p.nnzb - 1), n = min(p.nnzb - at, 8);
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const uint8_t*>(p.vals) + (size_t)at * 512), "r"(n * 512) : "memory");
     }
     ptx::pdl_wait();
     Piece q = piece_of<PLAN>(p, piece, lane);
@@ -632,6 +629,9 @@ int make_slabs(const void* B, void* slabs, size_t N, size_t K, cudaStream_t stre
     return SMAT_OK;
 }
 
+// Plans of fewer bytes of blocks than this do without the prefetch at the kernel's start: they are in L2 anyway.
+constexpr size_t kAheadBytes = (size_t)64 << 20;
+
 // Columns of a tile: N spread evenly over the tiles, in octets.
 int tile_cols(size_t N, int tiles) { return (int)((N / 8 + (size_t)tiles - 1) / (size_t)tiles) * 8; }
 
@@ -816,10 +816,13 @@ int launch_stream(const PlanView& v, const void* B, void* C, size_t N, cudaStrea
             if (int rc = make_slabs(a.B, sp.slabs, n, v.K, stream)) return rc;
             a.B = sp.slabs;
         }
-        // one round of warps: see the kernel's first lines (with more, most begin long after the kernel before this one)
         a.wait_cycles = v.selftest ? kSelftestWaitCycles : kWaitCycles;
         a.lost_bytes = v.selftest ? 16 : 0;
-        a.nnzb = (long long)a.n_pieces * a.n_tiles * s.w <= 40LL * ctx->sm_count && row_begin == 0 && row_end == rows ? (int)v.nnzb : 0;
+        // The kernel's first lines, where they can pay: one round of warps (with more, most begin long after the kernel before this
+        // one), and more blocks than stay in L2 from one product to the next.
+        const long long warps = (long long)a.n_pieces * a.n_tiles * s.w;
+        a.nnzb = (int)v.nnzb;
+        a.ahead = warps <= 40LL * ctx->sm_count && row_begin == 0 && row_end == rows && v.nnzb * 512 > kAheadBytes ? (float)((double)v.nnzb / ((double)a.n_pieces * s.w)) : 0.0f;
         if (int rc = launch<true>(s, a, stream)) return rc;
     }
     return SMAT_OK;
