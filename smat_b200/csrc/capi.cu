@@ -139,7 +139,7 @@ using namespace smat;
 extern "C" {
 
 // One multiplication with the stream kernel, or with the walk order built on the fly in stream-ordered scratch memory; the kernel
-// then reads the blocks where they are.
+// then reads the blocks where they are, or a copy of them in walk order (pack_for_call).
 static int spmm_transient_plan(const void* vals, const int* rowptr, const int* colidx, const void* B, void* C, size_t N,
                                size_t K, size_t nnzb, size_t brow_begin, size_t brow_end, cudaStream_t stream) {
     if (brow_end == brow_begin || N == 0) return SMAT_OK;
@@ -162,16 +162,24 @@ static int spmm_transient_plan(const void* vals, const int* rowptr, const int* c
         return rc;
     }
     const size_t rg = choose_rows_per_group(brow_end - brow_begin, N, ctx->sm_count, true, nnzb, K);
-    PlanSizes sz = plan_sizes(nnzb, brow_begin, brow_end, rg);
-    // the kernel gathers the blocks itself, unless a variant is asked for that reads a packed copy of them
-    const bool pack = g_spmm_variant == 2 || g_spmm_variant == 3;
-    if (!pack) sz.packed_bytes = 0;
+    const PlanSizes sz = plan_sizes(nnzb, brow_begin, brow_end, rg);
+    bool pack = pack_for_call(N, brow_end - brow_begin, nnzb);
     v.n_groups = sz.n_groups;
     v.rg = rg;
     if (nnzb == 0) return launch_spmm(v, B, C, N, stream);
     void* buf = nullptr;
-    const size_t plan_bytes = (sz.gsp_bytes + sz.steps_bytes + sz.blk_bytes + sz.packed_bytes + 255) / 256 * 256;
-    SMAT_CUDA_TRY(cudaMallocFromPoolAsync(&buf, plan_bytes + fix_scratch_bytes(ctx->sm_count), ctx->pool, stream));
+    size_t plan_bytes = 0;
+    auto allocate = [&]() {
+        plan_bytes = (sz.gsp_bytes + sz.steps_bytes + sz.blk_bytes + (pack ? sz.packed_bytes : 0) + 255) / 256 * 256;
+        return cudaMallocFromPoolAsync(&buf, plan_bytes + fix_scratch_bytes(ctx->sm_count), ctx->pool, stream);
+    };
+    cudaError_t got = allocate();
+    if (got == cudaErrorMemoryAllocation && pack && g_spmm_variant != 2 && g_spmm_variant != 3) {  // no room for a second copy of the blocks
+        cudaGetLastError();
+        pack = false;
+        got = allocate();
+    }
+    SMAT_CUDA_TRY(got);
     char* b = static_cast<char*>(buf);
     v.fix_scratch = reinterpret_cast<float*>(b + plan_bytes);
     v.gsp = reinterpret_cast<int*>(b);

@@ -534,6 +534,16 @@ PlanSizes plan_sizes(size_t nnzb, size_t brow_begin, size_t brow_end, size_t rg,
     return s;
 }
 
+// Packing costs its launches and a pass over the blocks (15 us for 65 000 of them), gathering a copy for every block of every tile of
+// C: 28 cycles each, which hide behind the MMA of a block (39 and more) but not behind one MMA for several blocks above one another,
+// as dense clusters and bands have them.  Sizes tell those by their short block-rows.  us, packed and gathered: clusters of 65536
+// rows, N = 1024: 104 and 98, 2048: 172 and 182, 4096: 322 and 340; band of 32768 rows, half bandwidth 256, 97.5 and 90, 165 and
+// 175, 300 and 324.  Not so scattered blocks of longer block-rows: layer 4096 x 8192 at 20 %, N = 4096, 180 and 170.
+bool pack_for_call(size_t N, size_t rows, size_t nnzb) {
+    if (g_spmm_variant == 2 || g_spmm_variant == 3) return true;  // these read a packed copy
+    return (N + 127) / 128 > 12 && nnzb <= 48 * rows;
+}
+
 double tc_estimate_us(const PlanView& v, size_t N, size_t sms) {
     const size_t items = v.n_groups * ((N + 127) / 128);
     const double per_group = (double)v.total_steps / (double)v.n_groups;

@@ -123,6 +123,8 @@ inline double tall_step_cycles(double blocks) { return 300.0 + 15.0 * blocks > 4
 constexpr double kTallLeastCycles = 440.0, kTallLeastCycles16 = 500.0;
 // ... and what a launch of it costs beyond its steps: its pipeline takes longer to fill and to drain (measured, smallest plans).
 constexpr double kTallExtraCycles = 5000.0;
+// Whether a product without a plan copies its blocks into walk order first instead of having the kernel gather them.
+bool pack_for_call(size_t N, size_t rows, size_t nnzb);
 // Measured cost of a 256-column item relative to a 128-column item of the same group.
 constexpr double kWideItemCost = 1.95;
 // Group height for a range of `block_rows` block-rows when C is N columns wide (0 = unknown): the height in

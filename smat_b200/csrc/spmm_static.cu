@@ -4,10 +4,10 @@
 // any framework allocator on top of them) is off limits -- a latency-critical serving loop whose
 // memory budget is fixed at start-up, a library callback invoked while another component holds the
 // allocator or device-synchronising locks, a process that has handed all remaining device memory
-// to a pool it does not own.  smat_spmm_bcsr_f16 builds the blocks' walk order (and, for two of
-// the forced variants, a copy of the blocks in it) in freshly allocated scratch on every call; this variant builds the same
-// in a fixed array that is part of the library image, so the call itself allocates nothing
-// and frees nothing.
+// to a pool it does not own.  smat_spmm_bcsr_f16 builds the blocks' walk order (and, for some
+// products, see pack_for_call, a copy of the blocks in it) in freshly allocated scratch on every
+// call; this variant builds the same in a fixed array that is part of the library image, so the call
+// itself allocates nothing and frees nothing.
 //
 // Cost and limits: the array occupies kStaticScratchBytes (17.5 MB) on every GPU that loads
 // the library, until the process exits, and therefore bounds the problem: at most
@@ -143,8 +143,7 @@ extern "C" int smat_spmm_bcsr_f16_static(const void* vals, const int* rowptr, co
     v.gsp = gsp;
     v.steps = steps;
     v.blk = blk;
-    // the kernel gathers the blocks itself, unless a variant is asked for that reads a packed copy of them
-    const bool pack = g_spmm_variant == 2 || g_spmm_variant == 3;
+    const bool pack = pack_for_call(N, Mb, nnzb);
     if (pack) v.packed = packed;
     else v.vals = vals;
     if (pack) {

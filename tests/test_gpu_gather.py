@@ -52,6 +52,35 @@ def test_gather_against_oracle_and_packed(Mb, Kb, fill, N):
     assert torch.all((packed.data.float() - C.data.float()).abs() <= torch.from_numpy(2 * bound).cuda())
 
 
+@pytest.mark.parametrize("call", ["spmm", "static"])
+@pytest.mark.parametrize("Kb,fill,N,packed", [(70, 0.3, 1536, False), (70, 0.3, 1544, True), (131, 0.6, 1544, False)])
+def test_wide_products_of_short_block_rows_read_a_packed_copy(call, Kb, fill, N, packed):
+    """Beyond twelve tiles of C block-rows of up to 48 blocks are copied into walk order first (three launches more), others are
+    gathered; either way the product is the oracle's."""
+    rng = np.random.default_rng(Kb + N)
+    Mb = 40
+    M, K = Mb * 16, Kb * 16
+    brp, bci, bv = _matrix(rng, Mb, Kb, fill)
+    B = rng.standard_normal((N, K)).astype(np.float16)
+    A, Bd, C = S.SparseMatrix.from_bcsr(M, K, brp, bci, bv), S.Matrix.from_host(B), S.Matrix(M, N, fill=float("nan"))
+    S.set_variant(1)
+    before = S.launch_count()
+    try:
+        if call == "spmm":
+            S.spmm(A, Bd, C)
+        else:
+            assert S.lib().smat_spmm_bcsr_f16_static(A.getBcsrValues(), A.getBcsrRowPtr(), A.getBcsrColIdx(), Bd.data.data_ptr(),
+                                                     C.data.data_ptr(), M, N, K, A.nnzb, None) == 0
+    finally:
+        S.set_variant(0)
+    assert S.lib().smat_device_status(None) == 0
+    assert (S.launch_count() - before >= 5) == packed
+    ref = oracle.bcsr_spmm(bv, brp, bci, B, M, N, K, threads=8)
+    size = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B), M, N, K, threads=8)
+    bound = 2 * K * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24  # as above
+    assert np.all(np.abs(C.data.cpu().numpy().astype(np.float32) - ref) <= bound)
+
+
 @pytest.mark.parametrize("what", ["column", "order", "rowptr", "dip"])
 def test_gather_reports_inconsistent_arrays(what):
     """Columns outside the matrix, block columns that go back to an earlier window, row pointers beyond the blocks or that go down so
