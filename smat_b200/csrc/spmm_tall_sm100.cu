@@ -66,7 +66,6 @@ constexpr int NCW = 4;           // copier warps
 constexpr int NEW = 8;           // epilogue warps
 constexpr uint32_t PANEL_BYTES = 128 * 64 * 2;               // 128 n x 64 k fp16
 constexpr size_t kTallDenseStep = 25;                         // blocks a step, on average: Smem below
-constexpr size_t kTallHalvesStep = 12;                        // blocks a step, on average, from which panels are copied in halves
 constexpr uint32_t NLIST = 7;                                 // pairs with blocks in the ring, at most: list slots
 constexpr uint32_t META_BYTES = kTallRows / 2 * kTallListBytes;  // per pair of steps: the MMA lists of the 12 issuing warps
 // A thread that waits on an mbarrier by parity must see every phase of it.  Panel loader j and copier j handle the steps
@@ -130,7 +129,7 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                       const int* __restrict__ rowptr,
                       __half* __restrict__ C, size_t ldc, int brow_begin, int brow_end, int rg, int N, int n_tiles, int n_items,
                       int tail_parts, uint32_t panel_bytes, float* __restrict__ fix_scratch, int* status, int pf,
-                      long long wait_cycles, uint32_t lost_bytes, int halves) {
+                      long long wait_cycles, uint32_t lost_bytes) {
     constexpr int NMW = Shape<TRG>::NMW;
     constexpr uint32_t TS_ = Shape<TRG>::TS_, TMEM_PANELS = Shape<TRG>::TMEM_PANELS;
     using L = Smem<PS>;
@@ -348,17 +347,10 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
 #endif
                 tc_fence_after();
                 if (leader) {
-                    if (halves) {
-                        if (subs & 1u) tc_cp_2x128x128b(tdst, pdesc);
-                        if (subs & 2u) tc_cp_2x128x128b(tdst + 8, pdesc + 2);
-                        if (subs & 4u) tc_cp_2x128x128b(tdst + 16, pdesc + 4);
-                        if (subs & 8u) tc_cp_2x128x128b(tdst + 24, pdesc + 6);
-                    } else {
-                        if (subs & 1u) tc_cp_128x256b(tdst, pdesc);
-                        if (subs & 2u) tc_cp_128x256b(tdst + 8, pdesc + 2);
-                        if (subs & 4u) tc_cp_128x256b(tdst + 16, pdesc + 4);
-                        if (subs & 8u) tc_cp_128x256b(tdst + 24, pdesc + 6);
-                    }
+                    if (subs & 1u) tc_cp_128x256b(tdst, pdesc);
+                    if (subs & 2u) tc_cp_128x256b(tdst + 8, pdesc + 2);
+                    if (subs & 4u) tc_cp_128x256b(tdst + 16, pdesc + 4);
+                    if (subs & 8u) tc_cp_128x256b(tdst + 24, pdesc + 6);
                     tc_commit(cp_done(pi % NPAIR));
                     // A plain arrive beside the commit's: it is ordered after this thread's wait for the blocks and
                     // lists of the step, so whoever passes cp_done may read them (the MMA warps wait for nothing else).
@@ -574,14 +566,13 @@ int launch_spmm_tall(const PlanView& whole, const void* B, void* C, size_t N, cu
     const int n_full = (int)(n_items / (size_t)grid * (size_t)grid);
     int pf = 0;  // L2 prefetch: measured to make no difference here, and it costs copy-engine time
     if (const char* ev = std::getenv("SMAT_L2_PREFETCH")) pf = std::atoi(ev) != 0;  // tuning knob
-    const int halves = plan.total_steps && plan.nnzb >= kTallHalvesStep * plan.total_steps;
     auto launch = [&](auto kernel, int threads, uint32_t smem_bytes) -> int {
         SMAT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
         SMAT_CUDA_TRY(launch_pdl_if(spmm_begins_early(n_items, sms), kernel, dim3(grid), dim3(threads), smem_bytes, stream,
                                  mapB, reinterpret_cast<const uint8_t*>(plan.packed), reinterpret_cast<const uint4*>(plan.steps),
                                  reinterpret_cast<const uint4*>(plan.winfo), plan.gsp, plan.rowptr, reinterpret_cast<__half*>(C), ldc, (int)plan.brow_begin,
                                  (int)plan.brow_end, (int)plan.rg, (int)N, n_tiles, (int)n_items, parts, panel_rows * 128u, plan.fix_scratch, ctx->d_status, pf,
-                                 whole.selftest ? kSelftestWaitCycles : kWaitCycles, whole.selftest ? 16u : 0u, halves));
+                                 whole.selftest ? kSelftestWaitCycles : kWaitCycles, whole.selftest ? 16u : 0u));
         return SMAT_OK;
     };
     // the smallest shape that holds the plan's groups: fewer accumulators leave tensor memory for more panel slots
