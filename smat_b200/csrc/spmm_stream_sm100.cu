@@ -629,8 +629,10 @@ int make_slabs(const void* B, void* slabs, size_t N, size_t K, cudaStream_t stre
     return SMAT_OK;
 }
 
-// Plans of fewer bytes of blocks than this do without the prefetch at the kernel's start: they are in L2 anyway.
-constexpr size_t kAheadBytes = (size_t)64 << 20;
+// Plans of fewer bytes of blocks than this do without the prefetch at the kernel's start.  Without and with it, one plan and four in
+// turn, us: 0.8 MB of blocks, N = 16: 3.7 and 3.7, 3.7 and 3.6; 8.4 MB, N = 32: 6.02 and 6.02, 6.25 and 6.07; 13 MB, N = 32: 9.0 and
+// 8.9, 10.2 and 9.2; 27 MB: 12.8 and 11.7, 15.6 and 14.4; 94 MB, N = 16: 22.6 and 22.3, 24.4 and 23.7.
+constexpr size_t kAheadBytes = (size_t)4 << 20;
 
 // Columns of a tile: N spread evenly over the tiles, in octets.
 int tile_cols(size_t N, int tiles) { return (int)((N / 8 + (size_t)tiles - 1) / (size_t)tiles) * 8; }
@@ -819,7 +821,7 @@ int launch_stream(const PlanView& v, const void* B, void* C, size_t N, cudaStrea
         a.wait_cycles = v.selftest ? kSelftestWaitCycles : kWaitCycles;
         a.lost_bytes = v.selftest ? 16 : 0;
         // The kernel's first lines, where they can pay: one round of warps (with more, most begin long after the kernel before this
-        // one), and more blocks than stay in L2 from one product to the next.
+        // one), and not the smallest products, which are all launch.
         const long long warps = (long long)a.n_pieces * a.n_tiles * s.w;
         a.nnzb = (int)v.nnzb;
         a.ahead = warps <= 40LL * ctx->sm_count && row_begin == 0 && row_end == rows && v.nnzb * 512 > kAheadBytes ? (float)((double)v.nnzb / ((double)a.n_pieces * s.w)) : 0.0f;
