@@ -534,14 +534,19 @@ PlanSizes plan_sizes(size_t nnzb, size_t brow_begin, size_t brow_end, size_t rg,
     return s;
 }
 
-// Packing costs its launches and a pass over the blocks (15 us for 65 000 of them), gathering a copy for every block of every tile of
-// C: 28 cycles each, which hide behind the MMA of a block (39 and more) but not behind one MMA for several blocks above one another,
-// as dense clusters and bands have them.  Sizes tell those by their short block-rows.  us, packed and gathered: clusters of 65536
-// rows, N = 1024: 104 and 98, 2048: 172 and 182, 4096: 322 and 340; band of 32768 rows, half bandwidth 256, 97.5 and 90, 165 and
-// 175, 300 and 324.  Not so scattered blocks of longer block-rows: layer 4096 x 8192 at 20 %, N = 4096, 180 and 170.
+// Packing costs its launches and a pass over the blocks, gathering a copy for every block of every tile of C: 28 cycles each, which
+// hide behind the MMA of a block (39 and more), not behind one MMA for several blocks above one another, and not all of the time
+// where many CTAs gather at once.  us, packed and gathered, by columns:
+//   4096 block-rows, clusters, 65 536 blocks: 1024: 104 and 98, 1536: 135 and 135, 2048: 165 and 175, 8192: 546 and 603
+//   2048, band of 67 000: 1024: 98 and 90, 1536: 139 and 146, 2048: 160 and 170, 8192: 531 and 609; of 164 000: 1024: 192 and 177,
+//     2048: 330 and 350, 4096: 609 and 648; of 10 000: 2048: 82 and 76, 4096: 130 and 126, 8192: 229 and 225
+//   1024, clusters, 16 384: 1536: 56 and 51, 2560: 72 and 72, 8192: 155 and 170; random, 237 000: 2048: 647 and 624, 4096: 1278 and 1277
+//   512, layer, 183 000: 2048: 560 and 534, 3072: 827 and 844, 4096: 1020 and 1055; dense, 262 000: 2048: 523 and 506, 4096: 898 and 951
+//   256, layer, 26 000: 4096: 180 and 170, 8192: 303 and 305;  128, dense, 65 536: 4096: 308 and 280, 8192: 603 and 578
 bool pack_for_call(size_t N, size_t rows, size_t nnzb) {
     if (g_spmm_variant == 2 || g_spmm_variant == 3) return true;  // these read a packed copy
-    return (N + 127) / 128 > 12 && nnzb <= 48 * rows;
+    const size_t tiles = (N + 127) / 128;
+    return rows >= 512 && tiles > (rows >= 2048 ? 12u : 24u) && tiles * nnzb > 350000;
 }
 
 double tc_estimate_us(const PlanView& v, size_t N, size_t sms) {

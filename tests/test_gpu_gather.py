@@ -53,12 +53,12 @@ def test_gather_against_oracle_and_packed(Mb, Kb, fill, N):
 
 
 @pytest.mark.parametrize("call", ["spmm", "static"])
-@pytest.mark.parametrize("Kb,fill,N,packed", [(70, 0.3, 1536, False), (70, 0.3, 1544, True), (131, 0.6, 1544, False)])
-def test_wide_products_of_short_block_rows_read_a_packed_copy(call, Kb, fill, N, packed):
-    """Beyond twelve tiles of C block-rows of up to 48 blocks are copied into walk order first (three launches more), others are
+@pytest.mark.parametrize("Mb,Kb,fill,N,packed", [(2048, 70, 0.2, 1536, False), (2048, 70, 0.2, 1544, True), (2048, 20, 0.2, 1544, False),
+                                                 (512, 70, 0.4, 3072, False), (512, 70, 0.4, 3080, True), (511, 70, 0.4, 3080, False)])
+def test_wide_products_read_a_packed_copy(call, Mb, Kb, fill, N, packed):
+    """Many tiles of C, block-rows and blocks: the blocks are copied into walk order first (three launches more), else they are
     gathered; either way the product is the oracle's."""
     rng = np.random.default_rng(Kb + N)
-    Mb = 40
     M, K = Mb * 16, Kb * 16
     brp, bci, bv = _matrix(rng, Mb, Kb, fill)
     B = rng.standard_normal((N, K)).astype(np.float16)
@@ -75,10 +75,13 @@ def test_wide_products_of_short_block_rows_read_a_packed_copy(call, Kb, fill, N,
         S.set_variant(0)
     assert S.lib().smat_device_status(None) == 0
     assert (S.launch_count() - before >= 5) == packed
-    ref = oracle.bcsr_spmm(bv, brp, bci, B, M, N, K, threads=8)
-    size = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B), M, N, K, threads=8)
-    bound = 2 * K * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24  # as above
-    assert np.all(np.abs(C.data.cpu().numpy().astype(np.float32) - ref) <= bound)
+    got = C.data.cpu().numpy().astype(np.float32)
+    assert np.all(np.isfinite(got))
+    for b0 in (0, Mb // 2 - 4, Mb - 8):
+        ref = oracle.bcsr_spmm(bv, brp, bci, B, M, N, K, b0, b0 + 8, threads=8)
+        size = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B), M, N, K, b0, b0 + 8, threads=8)
+        bound = 2 * K * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24  # as above
+        assert np.all(np.abs(got[b0 * 16: b0 * 16 + 128] - ref) <= bound)
 
 
 @pytest.mark.parametrize("what", ["column", "order", "rowptr", "dip"])
