@@ -273,7 +273,8 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
             uint32_t head = 0;               // where its blocks go if they fit before the end of the ring
             uint32_t used = 0, freed = 0;    // blocks of the ring taken (with what was left out at its end) and given back, ever
             constexpr int U = 4;             // pairs whose step records are requested ahead
-            struct { uint32_t at, n; } rec[U];
+            // (kept as loaded: the sum of the two counts, taken here, would wait for each record as it is requested)
+            struct { uint32_t at, n0, n1; } rec[U];
             bool there = true;
             while (there && sg.next(cs)) {
                 const int first = (cs.gs + cs.k0) >> 1, n_pairs = (cs.k1 - cs.k0) >> 1;
@@ -281,7 +282,8 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                     if (i >= n_pairs) return;
                     const uint4 s0 = __ldg(steps + 2 * (first + i)), s1 = __ldg(steps + 2 * (first + i) + 1);
                     rec[a].at = s0.y;
-                    rec[a].n = s0.z + s1.z;  // the blocks of a group's steps follow one another
+                    rec[a].n0 = s0.z;
+                    rec[a].n1 = s1.z;
                 };
 #pragma unroll
                 for (int a = 0; a < U; a++) gen(a, a);
@@ -289,7 +291,7 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
 #pragma unroll
                     for (int a = 0; a < U; a++) {
                         if (i0 + a >= n_pairs) break;
-                        const uint32_t n = rec[a].n, pl = pi % NPAIR;
+                        const uint32_t n = rec[a].n0 + rec[a].n1, pl = pi % NPAIR;  // the blocks of a group's steps follow one another
                         if (head + n > RING_BLOCKS) {
                             used += RING_BLOCKS - head;
                             head = 0;
