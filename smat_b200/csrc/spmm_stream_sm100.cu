@@ -66,12 +66,15 @@ __device__ __forceinline__ uint2 lds8(uint32_t at) {
     return v;
 }
 constexpr int kRingWaitCode = 40;  // status word: a bounded wait of the ring kernel ran out
-__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity, long long limit) {
-    if (ptx::mbar_try_wait(bar, parity)) return true;
+// late: a wait of this lane ran out, here or before; no wait is waited for after that.
+__device__ __forceinline__ void ring_wait(uint32_t bar, uint32_t parity, long long limit, bool& late) {
+    if (ptx::mbar_try_wait(bar, parity) || late) return;
     const long long t0 = clock64();
     while (!ptx::mbar_try_wait_suspend(bar, parity, 2000u))
-        if (clock64() - t0 > limit) return false;
-    return true;
+        if (clock64() - t0 > limit) {
+            late = true;
+            return;
+        }
 }
 
 // The blocks [b0, b1) of block-row `row` that a warp (or several) multiplies; count > 1: one of `count` pieces of a long block-row.
@@ -369,6 +372,10 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_ring_kernel(const
     };
     int cols_at = c0, cols = load_cols(c0), cols_next = load_cols(c0 + 32);
     uint32_t ok = 0, phase = 0;  // bit s: stage s holds a block; parity of its next wait
+    // At the limit of a wait one lane may give up where the next still sees the copy arrive.  Giving up changes no branch that all
+    // lanes take part in: the lane goes on with what the stage holds, and lane 0 starts no more copies, so that the others' next
+    // waits run out too.  (A vote after every wait instead: 2 to 3 % at 64 columns.)
+    bool late = false;
     auto fetch = [&](int s, int at) {
         if (at - cols_at >= 32) {
             cols_at += 32;
@@ -379,7 +386,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_ring_kernel(const
         ok &= ~(1u << s);
         if (at < c1 && cb >= 0) {
             ok |= 1u << s;
-            if (lane == 0) {
+            if (lane == 0 && !late) {
                 ptx::mbar_arrive_expect_tx(bars + 8 * s, awaited);
                 ptx::bulk_load(ring + s * STAGE, slabs + (size_t)cb * slab, bytes, bars + 8 * s);
                 ptx::bulk_load_hint(ring + s * STAGE + NT * 32, vals + (size_t)at * 512, 512u, bars + 8 * s, once);
@@ -388,13 +395,12 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_ring_kernel(const
     };
 #pragma unroll
     for (int s = 0; s < S; s++) fetch(s, c0 + s);
-    bool there = true;
-    for (int at = c0; at < c1 && there; at += S) {
+    for (int at = c0; at < c1; at += S) {
 #pragma unroll
         for (int s = 0; s < S; s++) {
-            if (there && (ok & (1u << s))) {
-                // (by vote: at the limit one lane may give up where the next still sees the copy arrive, and all take part in fetch())
-                there = __all_sync(0xffffffffu, ring_wait(bars + 8 * s, (phase >> s) & 1u, p.wait_cycles));
+            if (ok & (1u << s)) {
+                ring_wait(bars + 8 * s, (phase >> s) & 1u, p.wait_cycles, late);
+                __syncwarp();  // for the MMAs
                 phase ^= 1u << s;
                 // all of the stage: what a narrower tile leaves of it goes to columns that are not stored
                 uint4 a;
@@ -411,13 +417,14 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_ring_kernel(const
                 for (int j = 0; j < T; j++) mma_16816(acc[j], a, b[j]);
             }
             __syncwarp();  // all lanes have read the stage before it is filled again
-            if (there) fetch(s, at + S + s);
+            fetch(s, at + S + s);
         }
     }
-    if (!there) {  // a copy did not arrive in time: the host sees a status, copies in flight get time to land
-        if (lane == 0) atomicCAS(p.status, 0, kRingWaitCode);
+    if (late) {  // a copy did not arrive in time: the host sees a status, copies in flight get time to land
+        atomicCAS(p.status, 0, kRingWaitCode);
         for (int i = 0; i < 64; i++) __nanosleep(1000);
     }
+    __syncwarp();
     if constexpr (W > 1) {  // sum over the W warps of the piece (fixed order), in the rings
         const int w = warp % W;
 #pragma unroll
