@@ -24,7 +24,7 @@ struct StreamArgs {
     int* counters;         // arrivals per long block-row (first slot) and tile, zero between launches
     int* status;
     size_t ldc;
-    int n_pieces, n_tiles, tile_cols, N, K, brow_begin, brow_end, nnzb, chunk;
+    int n_pieces, n_tiles, tile_cols, N, K, brow_begin, brow_end, nnzb, chunk, sm_count;
     float ahead;            // plan: blocks of a warp, on average, where its first ones are prefetched early; else 0
     long long wait_cycles;  // limit of a wait
     unsigned lost_bytes;    // bytes that a wait expects beyond those that are copied: 0, but for a self-test

@@ -586,16 +586,28 @@ cudaError_t launch_ring(const StreamArgs& a, cudaStream_t stream, bool fewer = f
     return launch_pdl(kernel, dim3((unsigned)grid), dim3(kWarps * 32), fewer ? most : own, stream, a);
 }
 
+// Whether 97 to 128 columns take 12 warps an SM instead of 14 (launch_nt): where slabs of more than half of L2 leave it less room for
+// A, and, with a plan, where 14 warps would have more than some 170 KB of slices an SM on their way, from 113 columns on.  There they
+// fall off, but for products that are one round of 14 warps and for short block-rows.  us, 14 and 12 warps, 128 columns: random
+// matrices of 65536 rows with 120 blocks a block-row 224 and 172, 20 blocks 41 and 44, of 131072 rows with 60 blocks 183 and 176, of
+// 16384 rows (one round) 29 and 35; power-law in given order, 98304 rows 285 and 274, 160000 rows 383 and 412; sorted by degree, 65536
+// rows 206 and 158, 160000 rows 432 and 356.  112 columns: 150 and 171, 264 and 271, 377 and 408, 333 and 346.  Without a plan 14 are
+// the better more often: 184 and 194, 430 and 469, 199 and 186.
+bool ring_fewer_warps(const StreamArgs& a, int w, bool plan) {
+    if ((size_t)a.N * a.K * 2 > kSlabBytesL2) return true;
+    const long long warps = (long long)a.n_pieces * a.n_tiles * w;
+    if (!plan || a.tile_cols <= 112 || (warps > 12LL * a.sm_count && warps <= 14LL * a.sm_count)) return false;
+    return a.nnzb >= 40LL * a.n_pieces;
+}
+
 template <bool PLAN, bool SLAB, int W>
 cudaError_t launch_nt(int nt, const StreamArgs& a, cudaStream_t stream) {
     if constexpr (SLAB && W < 8) {
         constexpr int kWarps = W == 4 ? 4 : 2;
-        // Slices of N columns in flight per SM: 14 warps x 3 of 97 to 128 columns, 16 x 3 of 65 to 96, 20 x 2 of 33 to 64.
-        // Beyond that some 100 copies are on their way, and the kernel falls off: 18 x 3 of 96 columns take 795 us instead of
-        // 480 (power-law matrix of 262144 rows), 16 x 4 of 64 columns 575 (12 x 4) to 1000.  Slabs of more than half of L2
-        // leave it less room for A, and want fewer warps: 262144 rows, 128 columns, 653 us with 14 warps, 624 with 12; 155152
-        // rows 415 and 432.
-        if (nt == 128 && a.tile_cols > 96) return launch_ring<128, 3, W, kWarps, 14 / kWarps, PLAN, 12 / kWarps>(a, stream, (size_t)a.N * a.K * 2 > kSlabBytesL2);
+        // Slices of N columns in flight per SM: 14 warps x 3 (or 12 x 3) of 97 to 128 columns, 16 x 3 of 65 to 96, 20 x 2 of 33 to
+        // 64.  Beyond that the kernel falls off: 18 x 3 of 96 columns take 795 us instead of 480 (power-law matrix of 262144 rows), 16
+        // x 4 of 64 columns 575 (12 x 4) to 1000.
+        if (nt == 128 && a.tile_cols > 96) return launch_ring<128, 3, W, kWarps, 14 / kWarps, PLAN, 12 / kWarps>(a, stream, ring_fewer_warps(a, W, PLAN));
         if (nt == 128) return launch_ring<96, 3, W, kWarps, 16 / kWarps, PLAN>(a, stream);
         if (nt == 64) return launch_ring<64, 2, W, kWarps, 20 / kWarps, PLAN>(a, stream);
     }
@@ -831,6 +843,7 @@ int launch_stream(const PlanView& v, const void* B, void* C, size_t N, cudaStrea
         // one), and not the smallest products, which are all launch.
         const long long warps = (long long)a.n_pieces * a.n_tiles * s.w;
         a.nnzb = (int)v.nnzb;
+        a.sm_count = ctx->sm_count;
         a.ahead = warps <= 40LL * ctx->sm_count && row_begin == 0 && row_end == rows && v.nnzb * 512 > kAheadBytes ? (float)((double)v.nnzb / ((double)a.n_pieces * s.w)) : 0.0f;
         if (int rc = launch<true>(s, a, stream)) return rc;
     }
@@ -869,6 +882,7 @@ int stream_call(const StreamShape& s, const void* vals, const int* rowptr, const
     a.brow_end = (int)brow_end;
     a.nnzb = (int)nnzb;
     a.chunk = s.chunk;
+    a.sm_count = ctx->sm_count;
     a.wait_cycles = kWaitCycles;
     if (extra) {
         int* head = reinterpret_cast<int*>(b); b += 256;

@@ -104,6 +104,31 @@ def test_waits_that_run_out_end_the_product_and_are_reported(Mb, Kb, most, long_
     p.close()
 
 
+@pytest.mark.parametrize("N", [112, 120, 128])
+def test_block_rows_that_take_fewer_warps(N):
+    """Some 60 blocks a block-row and more than one round of warps: 12 warps an SM from 113 columns on."""
+    rng = np.random.default_rng(N)
+    Mb, Kb = 2400, 300
+    M, K = Mb * 16, Kb * 16
+    brp, bci, bv = _matrix(rng, Mb, Kb, 120)
+    B = rng.standard_normal((N, K)).astype(np.float16)
+    A, Bd, C = S.SparseMatrix.from_bcsr(M, K, brp, bci, bv), S.Matrix.from_host(B), S.Matrix(M, N, fill=float("nan"))
+    S.set_variant(5)
+    try:
+        p = S.Plan(A, n_hint=N)
+    finally:
+        S.set_variant(0)
+    p.spmm(Bd, C, check=True)
+    p.close()
+    got = C.data.cpu().numpy().astype(np.float32)
+    assert np.all(np.isfinite(got))
+    for b0 in (0, 1000, Mb - 200):
+        ref = oracle.bcsr_spmm(bv, brp, bci, B, M, N, K, b0, b0 + 200, threads=8)
+        size = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B), M, N, K, b0, b0 + 200, threads=8)
+        bound = 2 * K * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24  # as above
+        assert np.all(np.abs(got[b0 * 16: (b0 + 200) * 16] - ref) <= bound)
+
+
 def test_small_and_large_slabs_from_two_threads():
     """Slabs of more than half of L2 are multiplied by the same kernel with more shared memory for each CTA: two threads that launch
     it so and so do not refuse each other's launch, and both products are right."""
