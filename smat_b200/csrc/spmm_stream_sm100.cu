@@ -586,6 +586,16 @@ cudaError_t launch_ring(const StreamArgs& a, cudaStream_t stream, bool fewer = f
     return launch_pdl(kernel, dim3((unsigned)grid), dim3(kWarps * 32), fewer ? most : own, stream, a);
 }
 
+// Whether 33 to 64 columns from slabs stay with the loads in registers: slabs of a few megabytes come fast enough, and a block's two
+// copies cost more than its bytes.  us, registers and ring, 64 columns, without a plan: random matrices of 16384 rows 26 and 28, 38
+// and 41, of 32768 rows 40 and 42, 103 and 109; power-law 32768 rows 83 and 82; block-rows of very different length 48 and 56, 120 and
+// 118; of 65536 rows random 125 and 132, power-law 153 and 144, 131 and 129; 131072 rows 131 and 116, 270 and 229.  With a plan the
+// ring is the better from 65 000 blocks on (32768 rows: 68 and 65, 126 and 103) and below 32 000 (11.7 and 11.6), not between (19.8
+// and 21.4, 16.2 and 17.8, unequal block-rows 36 and 43).
+bool ring_not_for_64(const StreamArgs& a, bool plan) {
+    return (size_t)a.N * a.K * 2 <= (size_t)9 << 19 && (!plan || (a.nnzb >= 32768 && a.nnzb < 65536));
+}
+
 // Whether 97 to 128 columns take 12 warps an SM instead of 14 (launch_nt): where slabs of more than half of L2 leave it less room for
 // A, and, with a plan, where 14 warps would have more than some 170 KB of slices an SM on their way, from 113 columns on.  There they
 // fall off, but for products that are one round of 14 warps and for short block-rows.  us, 14 and 12 warps, 128 columns: random
@@ -609,6 +619,7 @@ cudaError_t launch_nt(int nt, const StreamArgs& a, cudaStream_t stream) {
         // x 4 of 64 columns 575 (12 x 4) to 1000.
         if (nt == 128 && a.tile_cols > 96) return launch_ring<128, 3, W, kWarps, 14 / kWarps, PLAN, 12 / kWarps>(a, stream, ring_fewer_warps(a, W, PLAN));
         if (nt == 128) return launch_ring<96, 3, W, kWarps, 16 / kWarps, PLAN>(a, stream);
+        if (nt == 64 && ring_not_for_64(a, PLAN)) return launch_one<64, W, SLAB, PLAN>(a, stream);
         if (nt == 64) return launch_ring<64, 2, W, kWarps, 20 / kWarps, PLAN>(a, stream);
     }
     if constexpr (!SLAB && W < 8) {

@@ -54,6 +54,34 @@ def test_ring_against_oracle(plan, Mb, Kb, most, long_row, N):
     assert np.all(np.abs(outs[0].astype(np.float32) - ref) <= bound)
 
 
+@pytest.mark.parametrize("plan", [True, False])
+@pytest.mark.parametrize("Mb,Kb,most,blocks", [(2400, 300, 30, (32768, 65536)), (2400, 300, 60, (65536, 1 << 30)), (300, 2400, 260, (32768, 65536))])
+@pytest.mark.parametrize("N", [40, 64])
+def test_both_kernels_of_33_to_64_columns(plan, Mb, Kb, most, blocks, N):
+    """From slabs, with the loads in registers (without a plan; with one between 32768 and 65536 blocks) and through the ring, one and
+    four warps a block-row; beyond 4.5 MB of slabs (Kb = 2400, 64 columns) all through the ring."""
+    rng = np.random.default_rng(Mb + most + N)
+    M, K = Mb * 16, Kb * 16
+    brp, bci, bv = _matrix(rng, Mb, Kb, most)
+    assert blocks[0] <= brp[-1] < blocks[1]
+    B = rng.standard_normal((N, K)).astype(np.float16)
+    A, Bd, C = S.SparseMatrix.from_bcsr(M, K, brp, bci, bv), S.Matrix.from_host(B), S.Matrix(M, N, fill=float("nan"))
+    S.set_variant(5)
+    try:
+        if plan:
+            p = S.Plan(A, n_hint=N)
+            p.spmm(Bd, C, check=True)
+            p.close()
+        else:
+            S.spmm(A, Bd, C, check=True)
+    finally:
+        S.set_variant(0)
+    ref = oracle.bcsr_spmm(bv, brp, bci, B, M, N, K, threads=8)
+    size = oracle.bcsr_spmm(np.abs(bv), brp, bci, np.abs(B), M, N, K, threads=8)
+    bound = 2 * K * 2.0 ** -24 * size + 2 * 2.0 ** -11 * np.abs(ref) + 2.0 ** -24  # as above
+    assert np.all(np.abs(C.data.cpu().numpy().astype(np.float32) - ref) <= bound)
+
+
 def test_ring_skips_columns_outside_the_matrix():
     """A block whose column lies outside the matrix is left out and reported, with the ring as with the other kernels."""
     rng = np.random.default_rng(3)
