@@ -555,7 +555,8 @@ class Plan:
         _check(lib().smat_plan_set_values(self._h, self.A.getBcsrValues(), _stream()))
 
     def info(self):
-        """{'tall': bool, 'rows_per_item': int, 'steps': int, 'kernel': name of the CUDA kernel that multiplies}."""
+        """{'tall': bool, 'rows_per_item': int, 'steps': int, 'kernel': name of the CUDA kernel that multiplies; of a plan for
+        spmm_bcsr_stream_kernel, products with tiles of 33 to 128 columns from slabs take spmm_bcsr_ring_kernel}."""
         t, r, n = C.c_int(0), C.c_int(0), C.c_size_t(0)
         _check(lib().smat_plan_info(self._h, C.addressof(t), C.addressof(r), C.addressof(n)))
         return {"tall": bool(t.value), "rows_per_item": r.value, "steps": n.value,

@@ -15,12 +15,11 @@
 // cycle (60 cycles; 33 out of L1).  So where the blocks outnumber the block-columns enough, B is first rewritten as slabs
 // [K / 16][N][16], one pass over B.  mma.sync runs at 2.1-2.6 cycles per 16x8x16 MMA and SM (34 cycles per block of 128
 // columns) and is not what bounds it; a tcgen05.mma on one block would need its slice in shared memory (39 cycles for the
-// operand port alone) and a barrier round trip per hand-over.  At 128 columns from slabs no unit is full (ncu, power-law matrix of
-// 464 000 blocks: L2 at 45 % of its peak, tensor pipe 34 %, HBM 17 %): 166 registers leave 12 warps per SM, each with the
-// loads of one block in flight, 49 bytes per cycle and SM at an L2 latency of about a thousand cycles.
+// operand port alone) and a barrier round trip per hand-over.  Most tiles of more than 32 columns from slabs have a kernel of
+// their own below, with the loads in flight in shared memory instead of registers.
 //
-// Measured against the tcgen05 kernels (before -> now, inputs that change from pass to pass): 8192 x 28672 layer, 183 000
-// blocks, N = 16: 67.7 -> 24.7 us (3.9 TB/s); power-law matrix of 2.05 million blocks, N = 128: 1706 -> 795 us, N = 8 (1.78
+// Measured against the tcgen05 kernels (theirs -> these, inputs that change from pass to pass): 8192 x 28672 layer, 183 000
+// blocks, N = 16: 67.7 -> 24.4 us (3.9 TB/s); power-law matrix of 2.05 million blocks, N = 128: 1706 -> 694 us, N = 8 (1.78
 // million): 2076 -> 208 us; band matrix of 2284 blocks, N = 64: 10 -> 4.1 us.  Where blocks share their slices of B (a layer
 // or a random matrix at N >= 128: the tall kernel takes 8-10 ns per block, 128 columns and SM, this one 55-60) the tcgen05
 // kernels stay.
@@ -319,8 +318,8 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) spmm_bcsr_stream_kernel(con
 }
 
 // The same product for wide tiles whose B is slabs: a warp's next S slices and blocks are on their way to a ring in shared memory
-// (a bulk copy each) while it multiplies, so that the loads in flight are not bounded by registers: 12 warps of the kernel above
-// (166 registers) have one block of 4.6 KB each on its way.  Power-law matrix of 262144 rows, 128 columns: 826 -> 630 us (58 of
+// (a bulk copy each) while it multiplies, so that the loads in flight are not bounded by registers: at 128 columns 12 warps of the
+// kernel above (166 registers) would have one block of 4.6 KB each on its way.  Power-law matrix of 262144 rows, 128 columns: 826 -> 630 us (58 of
 // the 67-72 bytes per cycle and SM that L2 serves to a pure streaming kernel), 96 columns 731 -> 480, 64 columns 515 -> 403;
 // 65536 rows without a plan, 128 columns: 266 -> 212.  32 columns stay with the kernel above (179 us against 234): a
 // block then costs its two copies, 28 cycles each, more than its bytes.  The blocks of A come as copies too, although a lane
@@ -730,7 +729,9 @@ bool stream_for_call(size_t N, size_t rows, size_t nnzb, size_t K, int sm_count)
         // blocks and bands suit the other kernel, whose steps they fill, scattered ones this one, and skewed ones more, since
         // it cuts long block-rows.  What sizes tell is the number of blocks of a block-row: bands and clusters have some tens,
         // random matrices and graphs of this fill a hundred and more.  So up to 48 the other kernel is taken at the estimate of
-        // its throughput (and this one for what is close), beyond that at three times it.
+        // its throughput (and this one for what is close), beyond that at three times it.  What that gets wrong are bands of more
+        // than 48 blocks a block-row (half bandwidth beyond some 380; none among the products below): this kernel is taken for
+        // them and takes up to twice the other's time.
         // Both kernels timed on 216 products (40 to 400 columns), time of the chosen one to the faster one, geometric mean and
         // worst, with this rule and before it (which drew the line at 24 and twice the throughput, with estimates from
         // before slices came through a ring and blocks were gathered): random 1.00, 1.06 and 1.03, 1.82; power-law 1.00, 1.00
