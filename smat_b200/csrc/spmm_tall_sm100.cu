@@ -336,12 +336,13 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                 // what is usually there already first: blocks and panel wait in shared memory for a tensor-memory slot,
                 // which is free once the MMAs of the step TS_ positions back (pair pi - TS_ / 2) have completed; only
                 // the copies follow that
-                if (!(j & 1u)) TWAIT(full_b(pi % NPAIR), (pi / NPAIR) & 1, 4);  // the copier of a pair's first step looks after its blocks
+                bool there = true;
+                if (!(j & 1u)) there = TWAIT(full_b(pi % NPAIR), (pi / NPAIR) & 1, 4);  // the copier of a pair's first step looks after its blocks
                 const uint64_t pdesc = smem_desc_k_sw128(base + L::PANEL + ps * PANEL_BYTES);
                 const uint32_t tdst = tmem_base + TMEM_PANELS + (st % TS_) * 32;
-                TWAIT(full_p(fp), (st / FP) & 1, 3);
-                const uint32_t subs = uniform(ld_shared_u32(base + L::SUBS + fp * 4) | ld_shared_u32(abort_addr) << 4);  // non-empty sub-columns
-                if (subs & 16u) break;
+                there &= TWAIT(full_p(fp), (st / FP) & 1, 3);
+                const uint32_t subs = uniform(ld_shared_u32(base + L::SUBS + fp * 4) | (there ? 0u : 16u));  // non-empty sub-columns
+                if (subs & 16u) break;  // a wait was given up: the pair's cp_done stays open
                 if (pi >= TS_ / 2) TWAIT(step_done((pi - TS_ / 2) % NPAIR), ((pi - TS_ / 2) / NPAIR) & 1, 5);
 #ifdef SMAT_PROFILE
                 if (pi >= TS_ / 2) prof_c[13] += (unsigned int)clock() - *(volatile unsigned int*)&stamp_mma[(pi - TS_ / 2) % 8];
@@ -393,7 +394,7 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                 for (int k = cs.k0; k < cs.k1; k += 2, st += 2) {
                     const uint32_t pi = st >> 1;
                     PROF_MARK(0);
-                    TWAIT(cp_done(pi % NPAIR), (pi / NPAIR) & 1, 7);
+                    there = TWAIT(cp_done(pi % NPAIR), (pi / NPAIR) & 1, 7);
 #ifdef SMAT_PROFILE
                     prof_c[12] += (unsigned int)clock() - *(volatile unsigned int*)&stamp_cp[pi % 8];
 #endif
@@ -404,9 +405,8 @@ spmm_bcsr_tall_kernel(const __grid_constant__ CUtensorMap mapB, const uint8_t* _
                     const uint4 l = ld_shared_v4(list), q = ld_shared_v4(list + 16);
                     const uint32_t b_lo = b_lo0 + ld_shared_u32(base + L::AT + (pi % NPAIR) * 4) * 32u;
                     // Once a wait was given up, lists and places may never have arrived, and their MMAs could reach anywhere: none from
-                    // here on.  (Who gave up says so before it arrives at anything, and the loaders stop, so what is read above was there
-                    // if the word is still zero.)
-                    const uint32_t w0 = uniform(ld_shared_u32(abort_addr) ? kTallListNone : l.x);
+                    // here on.  (A copier that gave up does not arrive at cp_done, and the loaders stop: what is read above was there.)
+                    const uint32_t w0 = uniform(there ? l.x : kTallListNone);
                     if (w0 & kTallListNone) { there = false; break; }
                     const uint32_t tpanel = tmem_base + TMEM_PANELS + (st % TS_) * 32;
                     PROF_MARK(9);
